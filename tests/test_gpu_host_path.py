@@ -1,0 +1,100 @@
+"""The host path of a call: where images come from, how results leave, and launches that are recorded as graphs. Needs a GPU.
+
+The same frames must give the same bits whichever way their images take (inside the staging block, through the upload helpers,
+straight from pinned memory, already on the device) and whether the chunk's kernels are launched one by one (a shape's first
+call) or as a graph (the calls that follow)."""
+import numpy as np
+import pytest
+
+import golden_io as G
+from visualmesh_b200 import workloads as W
+from visualmesh_b200.engine import Engine, FrameInput, Mesh, pinned_empty, pinned_free
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(a, b):
+    for name in ("pixel_coordinates", "global_indices", "neighbourhood", "classifications"):
+        assert np.array_equal(G.bits(getattr(a, name)) if getattr(a, name).dtype == np.float32 else getattr(a, name),
+                              G.bits(getattr(b, name)) if getattr(b, name).dtype == np.float32 else getattr(b, name)), name
+
+
+# bytes of an RGBA frame: inside the staging block (up to 128 KB in all), one slice, around the 256 KB slices, many slices
+@pytest.mark.parametrize("width,height", [(96, 64), (181, 181), (256, 256), (257, 256), (1280, 1024)])
+def test_images_from_every_kind_of_memory_give_the_same_results(width, height):
+    import torch
+    case = G.Case("ring6_equisolid_rgba")
+    mesh = Mesh.from_arrays(case.rays, case.nbrs, case.bsp)
+    lens = W.Lens((width, height), W.EQUISOLID, 0.35 * width, (0.0, 0.0), (0.0, 0.0), np.pi)
+    engine = Engine(case.network)
+    code = W.fourcc("RGBA")
+    image = W.random_bytes(7, width * height * 4)
+    pinned = pinned_empty(image.size)
+    pinned[:] = image
+    device = torch.from_numpy(image).cuda()
+    torch.cuda.synchronize()
+    frames = {"pageable": FrameInput(mesh, case.frames[0]["Hoc"], lens, image, code, None),
+              "pinned": FrameInput(mesh, case.frames[0]["Hoc"], lens, pinned, code, None),
+              "device": FrameInput(mesh, case.frames[0]["Hoc"], lens, device.data_ptr(), code, None, True)}
+    want = engine.run_batch([frames["device"]]).frame(0)
+    assert len(want.global_indices) > 100
+    for kind, frame in frames.items():
+        for _ in range(3):
+            _same(engine.run_batch([frame]).frame(0), want)
+    # unaligned, and one batch of all three kinds
+    shifted = np.empty(image.size + 1, np.uint8)[1:]
+    shifted[:] = image
+    order = ["pinned", "pageable", "device"]
+    for _ in range(3):
+        batch = engine.run_batch([frames[k] for k in order] + [FrameInput(mesh, case.frames[0]["Hoc"], lens, shifted, code, None)])
+        for f in range(4):
+            _same(batch.frame(f), want)
+    engine.close()
+    pinned_free(pinned)
+
+
+def test_host_ranges_of_changing_poses_leave_nothing_behind():
+    """With host ranges the node table is not cleared between calls: entries of an earlier pose must not be taken for points."""
+    case = G.Case("ring6_equisolid_rgba")
+    mesh = Mesh.from_arrays(case.rays, case.nbrs, case.bsp)
+    engine = Engine(case.network)
+    for f in (0, 1, 0, 2, 1, 0):
+        fr = case.frames[f]
+        out = engine.run_batch([FrameInput(mesh, fr["Hoc"], case.lens, fr["image"], case.format, fr["ranges"])]).frame(0)
+        assert np.array_equal(out.global_indices, fr["global_indices"])
+        assert np.array_equal(out.neighbourhood, fr["neighbourhood"])
+    engine.close()
+
+
+@pytest.mark.parametrize("n_frames", [1, 2, 37])
+def test_batches_left_on_the_device_and_copied_to_the_host_agree(n_frames):
+    """Results written to the host by the device (one small chunk), copied by the copy engines (several chunks) and left behind."""
+    import ctypes
+    import torch
+    wl = W.config(1, n_frames=n_frames)
+    mesh = Mesh.from_spec(wl.frames[0].mesh)
+    engine = Engine(wl.network)
+    images = torch.randint(0, 256, (n_frames, wl.frames[0].image_bytes), dtype=torch.uint8)
+    frames = [FrameInput(mesh, fr.Hoc, fr.lens, images[i].numpy(), fr.format, None) for i, fr in enumerate(wl.frames)]
+    on_device = images.cuda()
+    torch.cuda.synchronize()
+    device_frames = [FrameInput(mesh, fr.Hoc, fr.lens, on_device[i].data_ptr(), fr.format, None, True) for i, fr in enumerate(wl.frames)]
+    for _ in range(3):
+        left = engine.run_batch(device_frames, results_on_device=True)
+        n_cls, total = left.n_classes, left.total_points
+
+        class Array:
+            def __init__(self, pointer, shape, kind):
+                self.__cuda_array_interface__ = {"data": (ctypes.cast(pointer, ctypes.c_void_p).value, False), "shape": shape, "typestr": kind, "version": 3}
+        cls = torch.as_tensor(Array(left.raw.classifications, (total + n_frames, n_cls), "<f4"), device="cuda").cpu().numpy()
+        gi = torch.as_tensor(Array(left.raw.global_indices, (total,), "<i4"), device="cuda").cpu().numpy()
+        nb = torch.as_tensor(Array(left.raw.neighbourhood, (total + n_frames, 6), "<i4"), device="cuda").cpu().numpy()
+        for some in (frames, device_frames):
+            batch = engine.run_batch(some)
+            for f in range(n_frames):
+                out = batch.frame(f, copy=False)
+                p0, p1 = left.offsets[f], left.offsets[f + 1]
+                assert np.array_equal(out.global_indices, gi[p0:p1])
+                assert np.array_equal(out.neighbourhood, nb[p0 + f:p1 + f + 1])
+                assert np.array_equal(G.bits(out.classifications), G.bits(cls[p0 + f:p1 + f + 1]))
+    engine.close()

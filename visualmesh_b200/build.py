@@ -20,7 +20,7 @@ LIB = os.path.join(HERE, "libvmcuda.so")
 ABI_HEADER = os.path.join("..", "..", "include", "vmcuda.h")
 # translation unit -> headers it includes (directly or not)
 UNITS = {
-    "engine.cu": ["kernels.cuh", "tile_plan.cuh", "device_math.cuh", "host_math.hpp", "libm_tables.hpp", "conv_dispatch.hpp", "conv_args.hpp",
+    "engine.cu": ["kernels.cuh", "tile_plan.cuh", "device_math.cuh", "host_math.hpp", "libm_tables.hpp", "upload.hpp", "conv_dispatch.hpp", "conv_args.hpp",
                   ABI_HEADER],
     "conv_ffma.cu": ["conv_ffma.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
     "conv_tc.cu": ["conv_tc.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],

@@ -28,9 +28,18 @@ struct ConvArgs {
     int32_t out_stride;     // rows per planar chunk of `out`
     int32_t out_planar;     // write `out` chunk-planar (needs COUT % 4 == 0 and !out_global)
     int32_t out_split;      // write `out` as fp16 hi/lo planes for a tensor-core consumer (needs COUT % 8 == 0)
-    int32_t* range_flag;    // raised (to 3) when a value is too large for the fp16 split
+    int32_t* range_flag;    // the engine's abort flags: ABORT_RANGE is raised when a value is too large for the fp16 split
 };
 
 constexpr int CONV_THREADS = 128;
+
+// Why a call had to be given up: one flag per reason, in pinned host memory. A kernel raises one with a plain store, so a healthy
+// call neither clears nor copies anything.
+enum AbortReason { ABORT_BSP_DEPTH = 1, ABORT_TC_TIMEOUT = 2, ABORT_TC_RANGE = 3, ABORT_FLAGS = 4 };
+#ifdef __CUDACC__
+__device__ __forceinline__ void raise_flag(int32_t* flags, int reason) {
+    *static_cast<volatile int32_t*>(flags + reason) = 1;
+}
+#endif
 
 }  // namespace vm

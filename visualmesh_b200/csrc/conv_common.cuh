@@ -52,8 +52,6 @@ __device__ __forceinline__ void activate(float* v, int act) {
 // x), in the shape the tensor-core kernel copies straight into shared memory: 16-byte chunks of 8 channels, chunk
 // plane p of row r at byte ((p * stride + r) * 16), the C/8 hi planes first, then the C/8 lo planes. Same footprint as
 // fp32. Values beyond the fp16 range raise the range flag; the host then recomputes without the tensor-core path.
-constexpr int ABORT_RANGE = 3;
-
 template <int COUT>
 __device__ __forceinline__ void store_split(float* out, int stride, size_t row, const float* v, int32_t* range_flag) {
     static_assert(COUT % 8 == 0, "split layout needs whole 8-channel chunks");
@@ -77,7 +75,7 @@ __device__ __forceinline__ void store_split(float* out, int stride, size_t row, 
         *reinterpret_cast<uint4*>(base + (static_cast<size_t>(p) * stride + row) * 16)     = make_uint4(h[0], h[1], h[2], h[3]);
         *reinterpret_cast<uint4*>(base + (static_cast<size_t>(P + p) * stride + row) * 16) = make_uint4(l[0], l[1], l[2], l[3]);
     }
-    if (bad) atomicCAS(range_flag, 0, ABORT_RANGE);
+    if (bad) raise_flag(range_flag, ABORT_TC_RANGE);
 }
 
 }  // namespace vm

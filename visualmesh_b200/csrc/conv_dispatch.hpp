@@ -63,14 +63,12 @@ bool has_fast_ffma_kernel(int cin, int cout);
 void launch_conv_ffma(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, cudaStream_t s);
 
 // ---- conv_tc.cu: layers on the tensor cores, gather by global loads ----------------------------------------------
-constexpr int TC_MAX_FRAMES    = 64;  // frames per launch of a tensor-core layer (shared table of tile counts)
-constexpr int ABORT_TC_TIMEOUT = 2;   // abort flag: a bounded wait of a tensor-core kernel ran out
-constexpr int ABORT_TC_RANGE   = 3;   // abort flag: a feature value too large for the fp16 split
+constexpr int TC_MAX_FRAMES    = 256;  // frames per launch of a tensor-core layer (shared table of tile counts)
 constexpr uint32_t TC_DEFAULT_WAIT_LIMIT = 4000000;
 bool has_tc_gather_kernel(const DenseLayer& L);  // gathers fp32 rows and splits them itself
 bool has_tc_split_kernel(const DenseLayer& L);   // fed from the split feature layout
-bool launch_conv_tc_gather(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, int32_t* abort_flag, uint32_t wait_limit, cudaStream_t s);
-bool launch_conv_tc_split(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, int32_t* abort_flag, uint32_t wait_limit, cudaStream_t s);
+bool launch_conv_tc_gather(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, int32_t* abort_flags, uint32_t wait_limit, cudaStream_t s);
+bool launch_conv_tc_split(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, int32_t* abort_flags, uint32_t wait_limit, cudaStream_t s);
 
 // ---- conv_staged.cu: layers on the tensor cores, gather from shared-memory windows --------------------------------
 // What the tile plan of a chunk holds (device pointers), see conv_staged.cuh.
@@ -83,7 +81,7 @@ constexpr int STAGED_NBL_STRIDE = 8;    // 16-bit neighbour positions per row
 constexpr int STAGED_ST         = 256;  // rows of a super-tile
 constexpr int STAGED_HALO       = 192;  // halo slots of a super-tile
 bool has_staged_kernel(const DenseLayer& L);
-bool launch_conv_staged(const DenseLayer& L, const ConvArgs& a, const StagedPlan& plan, int n_frames, int max_rows, int32_t* abort_flag,
+bool launch_conv_staged(const DenseLayer& L, const ConvArgs& a, const StagedPlan& plan, int n_frames, int max_rows, int32_t* abort_flags,
                         uint32_t wait_limit, cudaStream_t s);
 // the plan for a neighbourhood that is already in memory (the hot path makes it inside the neighbour-remap kernel)
 void launch_tile_plan_kernel(int n_neighbours, const int32_t* offsets, const int32_t* nb, uint16_t* nbl, int32_t* halo_rows, int32_t* halo_count,

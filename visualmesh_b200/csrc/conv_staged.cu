@@ -11,7 +11,7 @@ static_assert(STAGED_NBL_STRIDE == st::NBL_STRIDE && STAGED_ST == st::ST && STAG
               "the engine sizes the plan with the kernels' own constants");
 
 template <int CIN, int COUT, int NSLOTS>
-static void launch_conv_staged_t(const DenseLayer& L, const ConvArgs& a, const st::Plan& plan, int n_frames, int max_rows, int32_t* abort_flag,
+static void launch_conv_staged_t(const DenseLayer& L, const ConvArgs& a, const st::Plan& plan, int n_frames, int max_rows, int32_t* abort_flags,
                                  uint32_t wait_limit, cudaStream_t s) {
     constexpr int THREADS = (CIN == 16 ? 8 : 16) * 32 + 32;  // compute warps + the loader warp
     constexpr auto kernel = st::k_graph_conv_mma<CIN, COUT, NSLOTS, THREADS>;
@@ -31,7 +31,7 @@ static void launch_conv_staged_t(const DenseLayer& L, const ConvArgs& a, const s
     st::Args t{};
     t.n_frames   = n_frames;
     t.cout       = L.cout;
-    t.abort_flag = abort_flag;
+    t.abort_flags = abort_flags;
     t.wait_limit = wait_limit;
     const int tiles_upper = n_frames * ((max_rows + st::ST - 1) / st::ST);
     const int grid        = std::max(1, std::min(tiles_upper, lp.n_sms * lp.ctas_per_sm));
@@ -46,12 +46,12 @@ bool has_staged_kernel(const DenseLayer& L) {
            && (L.n_slots == 5 || L.n_slots == 7 || L.n_slots == 9) && L.activation != VM_SOFTMAX;
 }
 
-bool launch_conv_staged(const DenseLayer& L, const ConvArgs& a, const StagedPlan& plan, int n_frames, int max_rows, int32_t* abort_flag,
+bool launch_conv_staged(const DenseLayer& L, const ConvArgs& a, const StagedPlan& plan, int n_frames, int max_rows, int32_t* abort_flags,
                         uint32_t wait_limit, cudaStream_t s) {
     const st::Plan p{plan.nbl, plan.halo_rows, plan.halo_count};
 #define VM_STG(CI, CO, NS)                                                                             \
     if (L.cin == CI && L.cout == CO && L.n_slots == NS) {                                                \
-        launch_conv_staged_t<CI, CO, NS>(L, a, p, n_frames, max_rows, abort_flag, wait_limit, s);        \
+        launch_conv_staged_t<CI, CO, NS>(L, a, p, n_frames, max_rows, abort_flags, wait_limit, s);        \
         return true;                                                                                     \
     }
     VM_STG(16, 8, 5) VM_STG(16, 8, 7) VM_STG(16, 8, 9) VM_STG(16, 16, 5) VM_STG(16, 16, 7) VM_STG(16, 16, 9)

@@ -108,7 +108,7 @@ namespace st {
     struct Args {
         int32_t n_frames;
         int32_t cout;
-        int32_t* abort_flag;
+        int32_t* abort_flags;
         uint32_t wait_limit;  // polls of one wait for a window before the kernel gives up (0: the first wait fails at once)
     };
 
@@ -180,15 +180,7 @@ namespace st {
         }
         for (int f = tid; f <= t.n_frames; f += THREADS) frame_start[f] = a.offsets[a.f0 + f];
         __syncthreads();
-        if (tid == 0) {
-            int run = 0;
-            for (int f = 0; f < t.n_frames; ++f) {
-                tile_prefix[f] = run;
-                const int rows = frame_start[f + 1] - frame_start[f] + 1;
-                run += (rows + ST - 1) / ST;
-            }
-            tile_prefix[t.n_frames] = run;
-        }
+        tc::tiles_before<ST>(tile_prefix, frame_start, t.n_frames);
 
         // ---- B fragments: weights [k][n] split into fp16 hi and lo, in the register layout of mma.m16n8k16 ----
         // fragment of (slot s, K step ks, column block nb), lane (g, tq): b0 = {W[k0 + 2 tq][n], W[k0 + 2 tq + 1][n]} and b1 =
@@ -473,7 +465,7 @@ namespace st {
                         }
                     }
                 }
-                if (bad) atomicCAS(a.range_flag, 0, ABORT_RANGE);
+                if (bad) raise_flag(a.range_flag, ABORT_TC_RANGE);
             }
             // this warp is done with the window: the loader may refill it once every compute warp has said so
             __syncwarp();
@@ -481,7 +473,7 @@ namespace st {
         }
         }
         __syncthreads();
-        if (tid == 0 && failed_s) atomicExch(t.abort_flag, tc::ABORT_TC_TIMEOUT);
+        if (tid == 0 && failed_s) raise_flag(t.abort_flags, ABORT_TC_TIMEOUT);
     }
 
 }  // namespace st

@@ -6,12 +6,11 @@
 
 namespace vm {
 
-static_assert(TC_MAX_FRAMES == tc::MAX_FRAMES && ABORT_TC_TIMEOUT == tc::ABORT_TC_TIMEOUT && ABORT_TC_RANGE == tc::ABORT_TC_RANGE
-                && TC_DEFAULT_WAIT_LIMIT == tc::WAIT_LIMIT,
+static_assert(TC_MAX_FRAMES == tc::MAX_FRAMES && TC_DEFAULT_WAIT_LIMIT == tc::WAIT_LIMIT,
               "the constants the engine sees are the kernels' own");
 
 template <int CIN, int NP, int NSLOTS, bool HALF>
-static void launch_conv_tc_t(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, int32_t* abort_flag, uint32_t wait_limit, cudaStream_t s) {
+static void launch_conv_tc_t(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, int32_t* abort_flags, uint32_t wait_limit, cudaStream_t s) {
     constexpr int STAGES = CIN >= 32 ? 2 : 3;  // 32-channel stages are 16 KB: two of them leave room for a third CTA per SM
     const size_t smem    = tc::smem_bytes<CIN, NP, STAGES, HALF>(NSLOTS);
     static LaunchPlans plans;
@@ -34,7 +33,7 @@ static void launch_conv_tc_t(const DenseLayer& L, const ConvArgs& a, int n_frame
     t.bias       = L.d_tc_bias;
     t.n_frames   = n_frames;
     t.cout       = L.cout;
-    t.abort_flag = abort_flag;
+    t.abort_flags = abort_flags;
     t.wait_limit = wait_limit;
     const int tiles_upper = n_frames * ((max_rows + tc::TILE_ROWS - 1) / tc::TILE_ROWS);
     const int grid        = std::max(1, std::min(tiles_upper, plan.n_sms * plan.ctas_per_sm));
@@ -42,7 +41,7 @@ static void launch_conv_tc_t(const DenseLayer& L, const ConvArgs& a, int n_frame
 }
 
 template <int CIN, int NP, int NSLOTS>
-static void launch_conv_tc_tmem_t(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, int32_t* abort_flag, uint32_t wait_limit, cudaStream_t s) {
+static void launch_conv_tc_tmem_t(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, int32_t* abort_flags, uint32_t wait_limit, cudaStream_t s) {
     const size_t smem = tc::smem_bytes_tmem<CIN, NP>(NSLOTS);
     static LaunchPlans plans;
     const LaunchPlan& plan = plans.get([smem](int dev) {
@@ -67,7 +66,7 @@ static void launch_conv_tc_tmem_t(const DenseLayer& L, const ConvArgs& a, int n_
     t.bias       = L.d_tc_bias;
     t.n_frames   = n_frames;
     t.cout       = L.cout;
-    t.abort_flag = abort_flag;
+    t.abort_flags = abort_flags;
     t.wait_limit = wait_limit;
     const int tiles_upper = n_frames * ((max_rows + tc::TILE_ROWS - 1) / tc::TILE_ROWS);
     const int grid        = std::max(1, std::min(tiles_upper, plan.n_sms * plan.ctas_per_sm));
@@ -79,10 +78,10 @@ bool has_tc_split_kernel(const DenseLayer& L) {
     return L.tc_np != 0 && L.tc_half && (L.cin == 16 || L.cin == 32) && (L.n_slots == 5 || L.n_slots == 7 || L.n_slots == 9);
 }
 
-bool launch_conv_tc_split(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, int32_t* abort_flag, uint32_t wait_limit, cudaStream_t s) {
+bool launch_conv_tc_split(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, int32_t* abort_flags, uint32_t wait_limit, cudaStream_t s) {
 #define VM_TCS(CI, NPAD, NS)                                                              \
     if (L.cin == CI && L.tc_np == NPAD && L.n_slots == NS) {                               \
-        launch_conv_tc_tmem_t<CI, NPAD, NS>(L, a, n_frames, max_rows, abort_flag, wait_limit, s);       \
+        launch_conv_tc_tmem_t<CI, NPAD, NS>(L, a, n_frames, max_rows, abort_flags, wait_limit, s);       \
         return true;                                                                       \
     }
     VM_TCS(16, 16, 5) VM_TCS(16, 16, 7) VM_TCS(16, 16, 9) VM_TCS(16, 32, 5) VM_TCS(16, 32, 7) VM_TCS(16, 32, 9)
@@ -91,11 +90,11 @@ bool launch_conv_tc_split(const DenseLayer& L, const ConvArgs& a, int n_frames, 
     return false;
 }
 
-bool launch_conv_tc_gather(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, int32_t* abort_flag, uint32_t wait_limit, cudaStream_t s) {
+bool launch_conv_tc_gather(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, int32_t* abort_flags, uint32_t wait_limit, cudaStream_t s) {
     if (L.tc_np == 0 || n_frames > tc::MAX_FRAMES) return false;
 #define VM_TC(CI, NPAD, NS, HF)                                                      \
     if (L.cin == CI && L.tc_np == NPAD && L.n_slots == NS && L.tc_half == HF) {        \
-        launch_conv_tc_t<CI, NPAD, NS, HF>(L, a, n_frames, max_rows, abort_flag, wait_limit, s);   \
+        launch_conv_tc_t<CI, NPAD, NS, HF>(L, a, n_frames, max_rows, abort_flags, wait_limit, s);   \
         return true;                                                                  \
     }
     VM_TC(8, 16, 5, false) VM_TC(8, 16, 7, false) VM_TC(8, 16, 9, false)

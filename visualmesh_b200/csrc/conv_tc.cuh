@@ -27,9 +27,8 @@ namespace vm {
 namespace tc {
 
     constexpr int TILE_ROWS     = 128;
-    constexpr int MAX_FRAMES    = 64;       // frames per launch whose tile counts fit the shared prefix table
+    constexpr int MAX_FRAMES    = 256;      // frames per launch whose tile counts fit the shared prefix table
     constexpr uint32_t WAIT_LIMIT = 4000000;  // default polls of mbarrier.try_wait before giving up (Args::wait_limit)
-    constexpr int ABORT_TC_TIMEOUT = 2;
 
     __device__ __forceinline__ uint32_t smem_u32(const void* p) {
         return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -58,6 +57,29 @@ namespace tc {
         return false;
     }
 
+    // prefix[f] = tiles of the frames before frame f of the launch, prefix[n_frames] = all of them; by the first warp of the block,
+    // 32 frames at a time. The caller synchronises.
+    template <int ROWS>
+    __device__ __forceinline__ void tiles_before(int32_t* prefix, const int32_t* frame_start, int n_frames) {
+        if (threadIdx.x >= 32) return;
+        const int lane = threadIdx.x;
+        int run        = 0;
+        for (int f0 = 0; f0 < n_frames; f0 += 32) {
+            const int f     = f0 + lane;
+            const int tiles = f < n_frames ? (frame_start[f + 1] - frame_start[f] + 1 + ROWS - 1) / ROWS : 0;
+            int incl        = tiles;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += v;
+            }
+            if (f < n_frames) prefix[f] = run + incl - tiles;
+            run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) prefix[n_frames] = run;
+        __syncwarp();
+    }
+
     // K-major, no swizzle: 8-row x 16-byte core matrices; LBO = distance between the two 16-byte K chunks of one MMA,
     // SBO = distance between 8-row groups. Version 1 = Blackwell descriptor.
     __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
@@ -84,11 +106,9 @@ namespace tc {
         const float* bias;  // [NP]
         int32_t n_frames;
         int32_t cout;
-        int32_t* abort_flag;
+        int32_t* abort_flags;
         uint32_t wait_limit;  // polls of one mbarrier wait before the kernel gives up (0: every wait fails at once)
     };
-
-    constexpr int ABORT_TC_RANGE = ABORT_RANGE;  // a feature value too large for the fp16 split: the host falls back to FFMA
 
     // Element formats of the split. HALF: x = h + l with h, l fp16 (kind::f16, 8 channels per 16-byte chunk, K = 16
     // per MMA) - half the shared-memory traffic of the fp32 container formats, needs |x| < 65504. Otherwise TF32:
@@ -170,6 +190,7 @@ namespace tc {
         __shared__ uint64_t bars[2 * STAGES + 5];
         __shared__ uint32_t tmem_base_slot;
         __shared__ int32_t tile_prefix[MAX_FRAMES + 1];
+        __shared__ int32_t frame_start[MAX_FRAMES + 1];
         __shared__ int32_t failed_s;
         volatile int32_t* failed = &failed_s;
 
@@ -197,14 +218,10 @@ namespace tc {
             }
             mbar_init(bar_drain, 1);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            int run = 0;
-            for (int f = 0; f < t.n_frames; ++f) {
-                tile_prefix[f] = run;
-                const int rows = a.offsets[a.f0 + f + 1] - a.offsets[a.f0 + f] + 1;
-                run += (rows + TILE_ROWS - 1) / TILE_ROWS;
-            }
-            tile_prefix[t.n_frames] = run;
         }
+        for (int f = tid; f <= t.n_frames; f += CTA_THREADS) frame_start[f] = a.offsets[a.f0 + f];
+        __syncthreads();
+        tiles_before<TILE_ROWS>(tile_prefix, frame_start, t.n_frames);
         if (warp == 0) {
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(TMEM_COLS)
                          : "memory");
@@ -450,9 +467,9 @@ namespace tc {
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         const int any_range = __syncthreads_or(out_of_range ? 1 : 0);
         if (tid == 0) {
-            if (failed_s) { atomicExch(t.abort_flag, ABORT_TC_TIMEOUT); }
+            if (failed_s) { raise_flag(t.abort_flags, ABORT_TC_TIMEOUT); }
             else if (any_range) {
-                atomicCAS(t.abort_flag, 0, ABORT_TC_RANGE);
+                raise_flag(t.abort_flags, ABORT_TC_RANGE);
             }
         }
         if (warp == 0) {
@@ -557,15 +574,7 @@ namespace tc {
         }
         for (int f = tid; f <= t.n_frames; f += CTA_THREADS) frame_start[f] = a.offsets[a.f0 + f];
         __syncthreads();
-        if (tid == 0) {
-            int run = 0;
-            for (int f = 0; f < t.n_frames; ++f) {
-                tile_prefix[f] = run;
-                const int rows = frame_start[f + 1] - frame_start[f] + 1;
-                run += (rows + TILE_ROWS - 1) / TILE_ROWS;
-            }
-            tile_prefix[t.n_frames] = run;
-        }
+        tiles_before<TILE_ROWS>(tile_prefix, frame_start, t.n_frames);
         if (warp == 0) {
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(TMEM_COLS)
                          : "memory");
@@ -803,7 +812,7 @@ namespace tc {
 
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
-        if (tid == 0 && failed_s) atomicExch(t.abort_flag, ABORT_TC_TIMEOUT);
+        if (tid == 0 && failed_s) raise_flag(t.abort_flags, ABORT_TC_TIMEOUT);
         if (warp == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");

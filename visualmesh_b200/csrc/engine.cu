@@ -2,8 +2,10 @@
 //
 // One engine instance owns its streams, its grow-only device scratch and its pinned result buffers; like the
 // reference engines it is not thread-safe - use one instance per host thread. A batch is cut into chunks of frames;
-// chunks rotate over a few lanes (stream + scratch) so that the host-to-device copy of one chunk's images, the
-// kernels of another and the device-to-host copy of a third overlap.
+// chunks rotate over a few lanes (streams + scratch) so that the host-to-device copy of one chunk's images, the
+// kernels of another and the device-to-host copy of a third overlap. Nothing waits for the device before the batch's end:
+// offsets, results and abort flags are written into pinned host memory by the kernels themselves, and a chunk of a shape that
+// returns is one launch of a recorded graph.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
@@ -22,6 +24,7 @@
 #include "host_math.hpp"
 #include "kernels.cuh"
 #include "conv_dispatch.hpp"
+#include "upload.hpp"
 #include "libm_tables.hpp"
 
 namespace vm {
@@ -43,14 +46,15 @@ template <typename T>
 struct DeviceArray {
     T* p       = nullptr;
     size_t cap = 0;
-    void ensure(size_t n) {
-        if (n <= cap) return;
+    bool ensure(size_t n) {  // true when the array was reallocated
+        if (n <= cap) return false;
         if (p != nullptr) VM_CUDA(cudaFree(p));
         p   = nullptr;
         cap = 0;
         const size_t want = n + n / 8 + 64;
         VM_CUDA(cudaMalloc(reinterpret_cast<void**>(&p), want * sizeof(T)));
         cap = want;
+        return true;
     }
     void release() {
         if (p != nullptr) cudaFree(p);
@@ -63,14 +67,15 @@ template <typename T>
 struct PinnedArray {
     T* p       = nullptr;
     size_t cap = 0;
-    void ensure(size_t n) {
-        if (n <= cap) return;
+    bool ensure(size_t n) {  // true when the array was reallocated
+        if (n <= cap) return false;
         if (p != nullptr) VM_CUDA(cudaFreeHost(p));
         p   = nullptr;
         cap = 0;
         const size_t want = n + n / 8 + 64;
         VM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p), want * sizeof(T), cudaHostAllocDefault));
         cap = want;
+        return true;
     }
     void release() {
         if (p != nullptr) cudaFreeHost(p);
@@ -106,20 +111,20 @@ static const uint32_t* libm_table(int device, int fn, bool build_if_missing) {
     return g_libm_device[device][fn];
 }
 
-constexpr int MAX_LANES = 3;
+constexpr int MAX_LANES = 4;
 
 struct Lane {
-    cudaStream_t stream   = nullptr;
-    cudaEvent_t ev_staged = nullptr;   // host staging of this lane has been consumed
-    cudaEvent_t ev_scan   = nullptr;   // this chunk's offsets are on the device
-    cudaEvent_t ev_offsets = nullptr;  // ... and on the host
-    cudaEvent_t ev_done   = nullptr;   // everything of this chunk, copies included, has finished
-    bool busy             = false;
-    int f0 = 0, f1 = 0;
-    PinnedArray<FrameParams> h_frames;
-    DeviceArray<FrameParams> d_frames;
-    PinnedArray<int32_t> h_ranges;  // int2 ranges then range starts
-    DeviceArray<int32_t> d_ranges;
+    cudaStream_t stream = nullptr;
+    cudaStream_t side   = nullptr;     // runs beside `stream` within a chunk: sampling next to the neighbour remap, result copies
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_offsets = nullptr;  // this chunk's offsets are on the device
+    cudaEvent_t ev_images  = nullptr;  // its images are
+    cudaEvent_t ev_done    = nullptr;  // everything of this chunk, result copies included, has finished
+    bool busy = false;
+    // staging block of a chunk, copied to the device in one piece: header, frame constants, range pairs and starts, group counts
+    // (zeros), small images
+    PinnedArray<uint8_t> h_staging;
+    DeviceArray<uint8_t> d_staging;
     DeviceArray<uint8_t> d_state;
     DeviceArray<float2> d_cand_px;
     DeviceArray<int32_t> d_cand_node;
@@ -127,17 +132,33 @@ struct Lane {
     DeviceArray<int32_t> d_node_rank;
     DeviceArray<float> d_feat[2];
     DeviceArray<uint8_t> d_images;
+    PinnedArray<uint8_t> h_images;  // staging of images that come from pageable memory
     // tile plan of the chunk for the staged tensor-core layers (conv_staged.cuh)
     DeviceArray<uint16_t> d_nbl;
     DeviceArray<int32_t> d_halo_rows;
     DeviceArray<int32_t> d_halo_count;
-    bool plan_valid = false;
 };
 
 struct StageTimer {
     const char* name;
     cudaEvent_t start, stop;
 };
+
+// What the recorded graph of a chunk's kernels depends on besides the contents of its buffers. Compared byte for byte.
+struct GraphKey {
+    int32_t part, lane, n_frames, f0, n_neighbours, blocks_per_frame, bsp_blocks, options;
+    uint32_t wait_limit;
+    int32_t feature_stride;
+    uint64_t staging_bytes;
+};
+struct GraphEntry {
+    GraphKey key;
+    cudaGraphExec_t exec = nullptr;
+    int64_t kernels      = 0;
+    uint64_t last_use    = 0;
+    bool refused         = false;  // could not be recorded: its kernels are launched one by one
+};
+constexpr size_t MAX_GRAPHS = 48;  // per engine; the least recently used one goes first
 
 }  // namespace vm
 
@@ -158,23 +179,33 @@ struct vm_engine {
     int n_classes = 0;
     vm::Lane lanes[vm::MAX_LANES];
     int n_lanes = vm::MAX_LANES;
+    cudaStream_t copy_stream = nullptr;  // images on their way to the device, chunk after chunk
     int64_t chunk_candidates = 2 << 20;
     int chunk_frames         = 16;
     bool chunk_override      = false;  // set by the environment: use the limits above for every batch
     // batch-wide results
     vm::DeviceArray<int32_t> d_offsets;
-    vm::PinnedArray<int32_t> h_offsets;
     vm::DeviceArray<float2> d_px;
     vm::DeviceArray<int32_t> d_gi;
     vm::DeviceArray<int32_t> d_nb;
     vm::DeviceArray<float> d_cls;
+    vm::PinnedArray<int32_t> h_offsets;
     vm::PinnedArray<float2> h_px;
     vm::PinnedArray<int32_t> h_gi;
     vm::PinnedArray<int32_t> h_nb;
     vm::PinnedArray<float> h_cls;
-    int32_t* d_abort = nullptr;
-    int32_t* h_abort = nullptr;
+    int32_t* flags = nullptr;  // abort flags, pinned host memory that the kernels raise them in
     std::vector<vm_mesh*> meshes;
+    // recorded graphs
+    bool use_graphs       = true;
+    uint64_t graph_uses   = 0;
+    bool buffers_moved    = false;  // a device buffer was reallocated: the recorded graphs name addresses that are gone
+    std::vector<vm::GraphEntry> graphs;
+    // constants of the last lens seen
+    vm_lens lens{};
+    bool lens_known = false;
+    vm::host::EdgeRays lens_rays{};
+    float lens_cos_fov = 0, lens_sin_fov = 0;
     // stage timing
     std::vector<vm::StageTimer> timers;
     std::vector<cudaEvent_t> event_pool;
@@ -190,13 +221,18 @@ struct vm_engine {
     bool may_stage       = false;   // some layer could run as a staged tensor-core layer under the engine's policy
     uint32_t tc_wait_limit = vm::TC_DEFAULT_WAIT_LIMIT;  // polls of one mbarrier wait in the tensor-core kernels (vm_set_wait_limit)
     cudaEvent_t ev_timer_start = nullptr, ev_timer_stop = nullptr;
-    cudaEvent_t ev_batch_start = nullptr;  // the start-of-batch clears (offsets[0], abort flag) are done
-    cudaEvent_t ev_batch_done  = nullptr;  // everything of the batch, the abort flag's copy included, has finished
     bool blocking_sync         = false;    // host waits sleep instead of spinning
     bool nvtx                  = false;    // NVTX ranges around every kernel launch and batch (VMCUDA_NVTX=1)
+    std::shared_ptr<vm::UploadHelpers> helpers;  // taken at the first upload from pageable memory
 };
 
 namespace vm {
+
+// Device buffers and staging blocks of the batch path: a reallocation makes the recorded graphs stale.
+template <typename Array>
+static void need(vm_engine* e, Array& a, size_t n) {
+    if (a.ensure(n)) e->buffers_moved = true;
+}
 
 // A stage is one kernel launch. With VMCUDA_NVTX=1 every launch sits in an NVTX range of the stage's name (the header-only
 // NVTX does nothing unless a profiler is attached); with stage timing on, between two CUDA events.
@@ -215,6 +251,7 @@ static void begin_stage(vm_engine* e, cudaStream_t s, const char* name) {
     e->timers.push_back(t);
 }
 static void end_stage(vm_engine* e, cudaStream_t s) {
+    VM_CUDA(cudaGetLastError());
     if (e->nvtx) nvtxRangePop();
     if (!e->timing) return;
     VM_CUDA(cudaEventRecord(e->timers.back().stop, s));
@@ -232,10 +269,12 @@ static bool producer_writes_split(const DenseLayer& L, ConvKind kind) {
 }
 
 // Scratch of a chunk's tile plan (tile_plan.cuh): neighbour positions per row, halo lists per super-tile.
-static st::PlanOut ensure_tile_plan(Lane& lane, size_t rows_cap, size_t supertiles_cap) {
-    lane.d_nbl.ensure(rows_cap * STAGED_NBL_STRIDE + 64);
-    lane.d_halo_rows.ensure(supertiles_cap * STAGED_HALO + 64);
-    lane.d_halo_count.ensure(supertiles_cap + 64);
+static void ensure_tile_plan(vm_engine* e, Lane& lane, size_t rows_cap, size_t supertiles_cap) {
+    need(e, lane.d_nbl, rows_cap * STAGED_NBL_STRIDE + 64);
+    need(e, lane.d_halo_rows, supertiles_cap * STAGED_HALO + 64);
+    need(e, lane.d_halo_count, supertiles_cap + 64);
+}
+static st::PlanOut tile_plan(Lane& lane) {
     return st::PlanOut{lane.d_nbl.p, lane.d_halo_rows.p, lane.d_halo_count.p};
 }
 
@@ -245,19 +284,19 @@ static void launch_conv(vm_engine* e, const DenseLayer& L, ConvArgs a, int n_fra
     a.n_slots     = L.n_slots;
     a.activation  = L.activation;
     begin_stage(e, s, L.stage.c_str());
-    if (kind == CONV_TC_STAGED && launch_conv_staged(L, a, plan, n_frames, max_rows, e->d_abort, e->tc_wait_limit, s)) {}
-    else if ((kind == CONV_TC_SPLIT || kind == CONV_TC_STAGED) && launch_conv_tc_split(L, a, n_frames, max_rows, e->d_abort, e->tc_wait_limit, s)) {}
-    else if (kind == CONV_TC_GATHER && launch_conv_tc_gather(L, a, n_frames, max_rows, e->d_abort, e->tc_wait_limit, s)) {}
+    if (kind == CONV_TC_STAGED && launch_conv_staged(L, a, plan, n_frames, max_rows, e->flags, e->tc_wait_limit, s)) {}
+    else if ((kind == CONV_TC_SPLIT || kind == CONV_TC_STAGED) && launch_conv_tc_split(L, a, n_frames, max_rows, e->flags, e->tc_wait_limit, s)) {}
+    else if (kind == CONV_TC_GATHER && launch_conv_tc_gather(L, a, n_frames, max_rows, e->flags, e->tc_wait_limit, s)) {}
     else {
         launch_conv_ffma(L, a, n_frames, max_rows, s);
     }
-    VM_CUDA(cudaGetLastError());
     end_stage(e, s);
 }
 
 // Runs all layers over a chunk whose input features are in feat[0]; the last layer writes out_final.
 static void run_network(vm_engine* e,
                         Lane& lane,
+                        bool plan_valid,
                         const int32_t* d_offsets,
                         const int32_t* d_nb,
                         int n_neighbours,
@@ -279,7 +318,7 @@ static void run_network(vm_engine* e,
         if (!e->use_tc || L.tc_np == 0 || L.n_slots == 1 || n_frames > TC_MAX_FRAMES) continue;
         const bool producer_can_split = l > 0 && producer_writes_split(e->layers[l - 1], kind[l - 1]) && !e->tc_no_split;
         // the staged kernel wherever it exists (it writes features, not results: never the last layer)
-        if (e->staged && lane.plan_valid && producer_can_split && has_staged_kernel(L) && l + 1 < n_layers) {
+        if (e->staged && plan_valid && producer_can_split && has_staged_kernel(L) && l + 1 < n_layers) {
             kind[l] = CONV_TC_STAGED;
             continue;
         }
@@ -305,7 +344,7 @@ static void run_network(vm_engine* e,
         a.out_stride   = feature_stride;
         a.out_planar   = (!last && e->layers[l].cout % 4 == 0) ? 1 : 0;
         a.out_split    = (!last && (kind[l + 1] == CONV_TC_SPLIT || kind[l + 1] == CONV_TC_STAGED)) ? 1 : 0;
-        a.range_flag   = e->d_abort;
+        a.range_flag   = e->flags;
         launch_conv(e, e->layers[l], a, n_frames, max_rows, lane.stream, kind[l], plan);
         cur ^= 1;
     }
@@ -313,7 +352,7 @@ static void run_network(vm_engine* e,
 
 // ---- per-frame constants -----------------------------------------------------------------------------------------
 
-static bool fill_frame_params(const vm_frame& fr, FrameParams& p, int device, bool may_allocate = true) {
+static bool fill_frame_params(vm_engine* e, const vm_frame& fr, FrameParams& p, bool may_allocate = true) {
     const float* H = fr.Hoc;
     // Rco = block<3,3>(transpose(Hoc)), cpp/visualmesh/engine/cpu/engine.hpp:95
     for (int i = 0; i < 3; ++i)
@@ -328,12 +367,21 @@ static bool fill_frame_params(const vm_frame& fr, FrameParams& p, int device, bo
     p.dims[1]    = fr.lens.dimensions[1];
     p.projection = fr.lens.projection;
     p.format     = fr.format;
-    // cpp/visualmesh/mesh.hpp:503-504
-    p.cos_fov = std::cos(fr.lens.fov * 0.5f);
-    p.sin_fov = std::sin(fr.lens.fov * 0.5f);
+    // what depends on the lens alone and takes a dozen libm calls is worked out when the lens changes
+    if (!e->lens_known || std::memcmp(&e->lens, &fr.lens, sizeof(vm_lens)) != 0) {
+        e->lens_known = false;
+        if (!host::edge_rays(fr.lens, e->lens_rays)) return false;
+        // cpp/visualmesh/mesh.hpp:503-504
+        e->lens_cos_fov = std::cos(fr.lens.fov * 0.5f);
+        e->lens_sin_fov = std::sin(fr.lens.fov * 0.5f);
+        e->lens         = fr.lens;
+        e->lens_known   = true;
+    }
+    p.cos_fov = e->lens_cos_fov;
+    p.sin_fov = e->lens_sin_fov;
     if (fr.ranges == nullptr) {
         std::array<host::Cone, 4> edges;
-        if (!host::screen_edges(H, fr.lens, edges)) return false;
+        host::screen_edges(H, fr.lens, e->lens_rays, edges);
         for (int i = 0; i < 4; ++i) {
             p.edges[i][0] = edges[i].axis[0];
             p.edges[i][1] = edges[i].axis[1];
@@ -342,9 +390,9 @@ static bool fill_frame_params(const vm_frame& fr, FrameParams& p, int device, bo
             p.edges[i][4] = edges[i].sin_t;
         }
     }
-    p.libm_acos = libm_table(device, libm::ACOS, may_allocate);
-    p.libm_sin  = fr.lens.projection == VM_EQUISOLID ? libm_table(device, libm::SIN, may_allocate) : nullptr;
-    p.libm_tan  = fr.lens.projection == VM_RECTILINEAR ? libm_table(device, libm::TAN, may_allocate) : nullptr;
+    p.libm_acos = libm_table(e->device, libm::ACOS, may_allocate);
+    p.libm_sin  = fr.lens.projection == VM_EQUISOLID ? libm_table(e->device, libm::SIN, may_allocate) : nullptr;
+    p.libm_tan  = fr.lens.projection == VM_RECTILINEAR ? libm_table(e->device, libm::TAN, may_allocate) : nullptr;
     const vm_mesh* m = fr.mesh;
     p.rays           = m->d_rays;
     p.neighbours     = m->d_neighbours;
@@ -368,228 +416,465 @@ static int64_t frame_candidates(const vm_frame& fr) {
     return n;
 }
 
-// ---- one chunk: enqueue everything up to the last kernel -----------------------------------------------------
-
-static void enqueue_chunk(vm_engine* e, Lane& lane, Lane* prev, const vm_frame* frames, int f0, int f1, bool classify) {
-    const int nf = f1 - f0;
-    cudaStream_t s = lane.stream;
-    lane.f0 = f0;
-    lane.f1 = f1;
-
-    // host staging: frame constants and the concatenated ranges
-    lane.h_frames.ensure(nf);
-    lane.d_frames.ensure(nf);
-    size_t n_ranges_total = 0;
-    for (int f = f0; f < f1; ++f) n_ranges_total += frames[f].ranges != nullptr ? frames[f].n_ranges : 0;
-    lane.h_ranges.ensure(3 * n_ranges_total + 4);
-    lane.d_ranges.ensure(3 * n_ranges_total + 4);
-
-    int64_t cand_total = 0, node_total = 0, bsp_total = 0, image_total = 0;
-    const int plan_st     = STAGED_ST;
-    size_t supertiles_cap = 0;
-    lane.plan_valid       = false;
-    int32_t max_cand = 0;
-    bool any_device_lookup = false, any_host_ranges = false;
-    size_t range_cursor = 0;
-    for (int f = f0; f < f1; ++f) {
-        const vm_frame& fr = frames[f];
-        FrameParams& p     = lane.h_frames.p[f - f0];
-        std::memset(&p, 0, sizeof(p));
-        if (!fill_frame_params(fr, p, e->device)) throw UnsupportedLens{};
-        const int64_t nc = frame_candidates(fr);
-        p.n_candidates   = static_cast<int32_t>(nc);
-        p.cand_off       = static_cast<int32_t>(cand_total);
-        p.node_off       = static_cast<int32_t>(node_total);
-        p.bsp_off        = static_cast<int32_t>(bsp_total);
-        if (fr.ranges != nullptr) {
-            any_host_ranges = true;
-            // device layout: [int2 ranges of all frames][starts of all frames]; pointers are patched below
-            p.n_ranges = fr.n_ranges;
-        }
-        else {
-            any_device_lookup = true;
-            bsp_total += fr.mesh->n_bsp;
-        }
-        cand_total += nc;
-        supertiles_cap += static_cast<size_t>((nc + 1 + plan_st - 1) / plan_st);
-        node_total += fr.mesh->n_nodes;
-        max_cand = std::max<int32_t>(max_cand, static_cast<int32_t>(nc));
-        if (classify && !fr.image_on_device) image_total += (image_bytes(fr) + 255) & ~size_t(255);
-    }
-    // ranges and their exclusive prefix sums
-    {
-        int32_t* pairs  = lane.h_ranges.p;
-        int32_t* starts = lane.h_ranges.p + 2 * n_ranges_total;
-        for (int f = f0; f < f1; ++f) {
-            const vm_frame& fr = frames[f];
-            if (fr.ranges == nullptr) continue;
-            FrameParams& p = lane.h_frames.p[f - f0];
-            p.ranges       = reinterpret_cast<const int2*>(lane.d_ranges.p + 2 * range_cursor);
-            p.range_starts = lane.d_ranges.p + 2 * n_ranges_total + range_cursor;
-            int32_t run    = 0;
-            for (int r = 0; r < fr.n_ranges; ++r) {
-                pairs[2 * (range_cursor + r) + 0] = fr.ranges[2 * r];
-                pairs[2 * (range_cursor + r) + 1] = fr.ranges[2 * r + 1];
-                starts[range_cursor + r]          = run;
-                run += std::max(0, fr.ranges[2 * r + 1] - fr.ranges[2 * r]);
-            }
-            if (fr.n_ranges == 0) {
-                // keep the "host ranges" marker non-null for an empty frame
-                p.ranges       = reinterpret_cast<const int2*>(lane.d_ranges.p);
-                p.range_starts = lane.d_ranges.p;
-            }
-            range_cursor += fr.n_ranges;
-        }
-    }
-
-    lane.d_cand_px.ensure(cand_total + 1);
-    lane.d_cand_node.ensure(cand_total + 1);
-    lane.d_node_rank.ensure(node_total + 1);
-    if (any_device_lookup) lane.d_state.ensure(bsp_total + 1);
-    const int blocks_per_frame = std::max(1, (max_cand + SELECT_THREADS - 1) / SELECT_THREADS);
-    const int n_blocks         = blocks_per_frame * nf;
-    lane.d_block_counts.ensure(n_blocks + 1);
-    const int64_t rows_cap = cand_total + nf;
-    if (classify) {
-        lane.d_feat[0].ensure(static_cast<size_t>(rows_cap) * e->max_width);
-        lane.d_feat[1].ensure(static_cast<size_t>(rows_cap) * e->max_width);
-        lane.d_images.ensure(image_total + 256);
-    }
-
-    // images: host frames go through the lane's device buffer, device frames are read in place. Frames that follow
-    // one another in host memory (a caller's ring of camera buffers, the rows of one big array) travel as ONE copy:
-    // sixteen 5 MB copies per chunk cost measurably more host time and bus turn-around than one 84 MB copy.
-    if (classify) {
-        size_t cursor = 0;
-        const uint8_t* run_src = nullptr;
-        size_t run_dst = 0, run_bytes = 0;
-        auto flush = [&] {
-            if (run_bytes > 0) VM_CUDA(cudaMemcpyAsync(lane.d_images.p + run_dst, run_src, run_bytes, cudaMemcpyHostToDevice, s));
-            run_bytes = 0;
-        };
-        for (int f = f0; f < f1; ++f) {
-            const vm_frame& fr = frames[f];
-            FrameParams& p     = lane.h_frames.p[f - f0];
-            if (fr.image_on_device) {
-                p.image = static_cast<const uint8_t*>(fr.image);
-                continue;
-            }
-            const size_t bytes = image_bytes(fr);
-            const uint8_t* src = static_cast<const uint8_t*>(fr.image);
-            if (run_bytes > 0 && src == run_src + run_bytes && cursor == run_dst + run_bytes) { run_bytes += bytes; }
-            else {
-                flush();
-                run_src   = src;
-                run_dst   = cursor;
-                run_bytes = bytes;
-            }
-            p.image = lane.d_images.p + cursor;
-            cursor += (bytes + 255) & ~size_t(255);
-        }
-        flush();
-    }
-    VM_CUDA(cudaMemcpyAsync(lane.d_frames.p, lane.h_frames.p, sizeof(FrameParams) * nf, cudaMemcpyHostToDevice, s));
-    if (n_ranges_total > 0) {
-        VM_CUDA(cudaMemcpyAsync(lane.d_ranges.p, lane.h_ranges.p, sizeof(int32_t) * 3 * n_ranges_total, cudaMemcpyHostToDevice, s));
-    }
-    VM_CUDA(cudaEventRecord(lane.ev_staged, s));
-
-    if (any_host_ranges) VM_CUDA(cudaMemsetAsync(lane.d_node_rank.p, 0xFF, sizeof(int32_t) * node_total, s));
-
-    if (any_device_lookup) {
-        int32_t max_bsp = 0;
-        for (int f = f0; f < f1; ++f)
-            if (frames[f].ranges == nullptr) max_bsp = std::max(max_bsp, frames[f].mesh->n_bsp);
-        dim3 g((max_bsp + SELECT_THREADS - 1) / SELECT_THREADS, nf);
-        begin_stage(e, s, "bsp_state");
-        k_bsp_state<<<g, SELECT_THREADS, 0, s>>>(lane.d_frames.p, lane.d_state.p);
-        VM_CUDA(cudaGetLastError());
-        end_stage(e, s);
-    }
-    {
-        dim3 g(blocks_per_frame, nf);
-        begin_stage(e, s, "select_project");
-        k_select<<<g, SELECT_THREADS, 0, s>>>(lane.d_frames.p, lane.d_state.p, lane.d_cand_px.p, lane.d_cand_node.p,
-                                              lane.d_block_counts.p, e->d_abort);
-        VM_CUDA(cudaGetLastError());
-        end_stage(e, s);
-    }
-    // the scan continues the batch-wide offsets from the previous chunk's scan
-    if (prev != nullptr && prev != &lane) VM_CUDA(cudaStreamWaitEvent(s, prev->ev_scan, 0));
-    begin_stage(e, s, "scan");
-    k_scan<<<1, 1024, 0, s>>>(lane.d_block_counts.p, n_blocks, blocks_per_frame, nf, e->d_offsets.p, f0);
-    VM_CUDA(cudaGetLastError());
-    end_stage(e, s);
-    VM_CUDA(cudaEventRecord(lane.ev_scan, s));
-    VM_CUDA(cudaMemcpyAsync(e->h_offsets.p + f0 + 1, e->d_offsets.p + f0 + 1, sizeof(int32_t) * nf, cudaMemcpyDeviceToHost, s));
-    VM_CUDA(cudaEventRecord(lane.ev_offsets, s));
-    {
-        dim3 g((blocks_per_frame + SCATTER_UNITS - 1) / SCATTER_UNITS, nf);
-        begin_stage(e, s, "scatter_compact");
-        k_scatter<SCATTER_UNITS><<<g, SELECT_THREADS, 0, s>>>(lane.d_frames.p, lane.d_cand_px.p, lane.d_cand_node.p, lane.d_block_counts.p,
-                                                              blocks_per_frame, e->d_offsets.p, f0, e->d_px.p, e->d_gi.p, lane.d_node_rank.p);
-        VM_CUDA(cudaGetLastError());
-        end_stage(e, s);
-    }
-    const int max_rows = max_cand + 1;
-    {
-        dim3 g((max_rows + ROW_THREADS - 1) / ROW_THREADS, nf);
-        const int N = frames[f0].mesh->n_neighbours;
-        begin_stage(e, s, "remap_neighbours");
-        // the staged layer kernels want a tile plan of the chunk: the remap makes it while it has the indices in hand
-        const bool with_plan = classify && e->staged && e->use_tc && e->may_stage && nf <= TC_MAX_FRAMES;
-        const st::PlanOut plan = with_plan ? ensure_tile_plan(lane, static_cast<size_t>(rows_cap), supertiles_cap) : st::PlanOut{nullptr, nullptr, nullptr};
-#define VM_REMAP(NN)                                                                                                                    \
-    if (N == NN) {                                                                                                                      \
-        if (with_plan) k_remap<NN, true><<<g, ROW_THREADS, 0, s>>>(lane.d_frames.p, e->d_offsets.p, f0, e->d_gi.p, lane.d_node_rank.p, e->d_nb.p, plan); \
-        else k_remap<NN, false><<<g, ROW_THREADS, 0, s>>>(lane.d_frames.p, e->d_offsets.p, f0, e->d_gi.p, lane.d_node_rank.p, e->d_nb.p, plan); \
-    }
-        VM_REMAP(4) VM_REMAP(6) VM_REMAP(8)
-#undef VM_REMAP
-        lane.plan_valid = with_plan;
-        VM_CUDA(cudaGetLastError());
-        end_stage(e, s);
-        if (classify) {
-            begin_stage(e, s, "sample_image");
-            bool packed4 = true;
-            for (int f = f0; f < f1; ++f) {
-                const int cls = format_class(frames[f].format);
-                packed4 &= cls == FMT_RGBA || cls == FMT_BGRA;
-            }
-            const dim3 gs((max_rows + ROW_THREADS * SAMPLE_ROWS - 1) / (ROW_THREADS * SAMPLE_ROWS), nf);
-            if (packed4) {
-                k_sample<true><<<gs, ROW_THREADS, 0, s>>>(lane.d_frames.p, e->d_offsets.p, f0, e->d_px.p,
-                                                         reinterpret_cast<float4*>(lane.d_feat[0].p));
-            }
-            else {
-                k_sample<false><<<gs, ROW_THREADS, 0, s>>>(lane.d_frames.p, e->d_offsets.p, f0, e->d_px.p,
-                                                          reinterpret_cast<float4*>(lane.d_feat[0].p));
-            }
-            VM_CUDA(cudaGetLastError());
-            end_stage(e, s);
-            run_network(e, lane, e->d_offsets.p, e->d_nb.p, N, f0, nf, max_rows, e->d_cls.p, true, static_cast<int>(rows_cap));
-        }
-    }
-    lane.busy = true;
+static size_t aligned(size_t n) {
+    return (n + 255) & ~size_t(255);
 }
 
-// Copies a finished chunk's results to the host. Needs the chunk's offsets on the host first.
-static void enqueue_chunk_readback(vm_engine* e, Lane& lane, int N, bool classify, bool to_host) {
+// Sizes that shape the launches are rounded up (by an eighth at most), so that calls whose poses differ a little share a graph.
+static int64_t rounded(int64_t n) {
+    int64_t step = 1024;
+    while (step * 16 <= n) step *= 2;
+    return (n + step - 1) / step * step;
+}
+
+// ---- one chunk -----------------------------------------------------------------------------------------------------
+
+// Images up to this size travel inside the chunk's staging block: for them a copy of their own costs more than the bytes.
+constexpr size_t SMALL_IMAGES = 128 << 10;
+
+// Results of a single chunk up to this size are written to the host by the device; more are copied by the copy engines, which leave
+// the SMs alone (a persistent layer kernel that finds some of its SM occupied runs in two waves), at the price of a wait for the
+// number of points in the middle of the call.
+constexpr int64_t MAX_EXPORT = 16 << 20;
+
+// Host images of one chunk of a batch.
+constexpr size_t CHUNK_IMAGE_BYTES = 21 << 20;
+
+struct Chunk {
+    int f0 = 0, f1 = 0, n_neighbours = 0;
+    bool classify = false, device_lookup = false, packed4 = false, with_plan = false;
+    bool images_apart = false;  // host images that travel on the copy stream
+    bool exported     = false;  // results are written to the host by k_export
+    bool copied       = false;  // ... or copied there once the host knows how many there are
+    int blocks_per_frame = 0, n_groups = 0, bsp_blocks = 0, max_rows = 0, stride = 0;
+    size_t staging_bytes = 0, counts_at = 0;
+};
+
+// Where a chunk's host images go in the lane's buffers: pageable ones first (their slices are sent as runs of the staging
+// buffer), then the pinned ones.
+struct ImagePlan {
+    std::vector<size_t> at;  // per frame of the chunk
+    size_t total = 0, pageable = 0;
+    bool small = false;
+};
+
+static bool is_pageable(const void* p) {
+    cudaPointerAttributes attributes{};
+    if (cudaPointerGetAttributes(&attributes, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return attributes.type == cudaMemoryTypeUnregistered;
+}
+
+static ImagePlan plan_images(const vm_frame* frames, int f0, int f1) {
+    ImagePlan plan;
+    plan.at.assign(f1 - f0, 0);
+    for (int f = f0; f < f1; ++f)
+        if (!frames[f].image_on_device) plan.total += aligned(image_bytes(frames[f]));
+    plan.small = plan.total <= SMALL_IMAGES;
+    std::vector<char> pageable(f1 - f0, 0);
+    for (int f = f0; f < f1 && !plan.small; ++f) pageable[f - f0] = !frames[f].image_on_device && is_pageable(frames[f].image);
+    size_t cursor = 0;
+    for (const char wanted : {1, 0}) {
+        for (int f = f0; f < f1; ++f) {
+            if (frames[f].image_on_device || pageable[f - f0] != wanted) continue;
+            plan.at[f - f0] = cursor;
+            cursor += aligned(image_bytes(frames[f]));
+        }
+        if (wanted) plan.pageable = cursor;
+    }
+    return plan;
+}
+
+// Starts the images of a chunk on their way. Pinned frames that follow one another in host memory (a caller's ring of camera
+// buffers, the rows of one big array) travel as ONE copy: sixteen 5 MB copies per chunk cost measurably more host time and bus
+// turn-around than one 84 MB copy. Pageable frames go through the upload helpers.
+static std::unique_ptr<Upload> start_images(vm_engine* e, Lane& lane, const vm_frame* frames, int f0, int f1, const ImagePlan& plan) {
+    need(e, lane.d_images, plan.total + 256);
+    std::unique_ptr<Upload> upload;
+    if (plan.pageable > 0) {
+        if (!e->helpers) e->helpers = UploadHelpers::get();
+        lane.h_images.ensure(plan.pageable);
+        upload.reset(new Upload(e->helpers.get(), lane.d_images.p, e->copy_stream));
+        for (int f = f0; f < f1; ++f)
+            if (!frames[f].image_on_device && plan.at[f - f0] < plan.pageable)
+                upload->job.add(static_cast<const uint8_t*>(frames[f].image), plan.at[f - f0], image_bytes(frames[f]));
+        upload->start(lane.h_images.p);
+    }
+    const uint8_t* run_src = nullptr;
+    size_t run_dst = 0, run_bytes = 0;
+    auto flush = [&] {
+        if (run_bytes > 0) VM_CUDA(cudaMemcpyAsync(lane.d_images.p + run_dst, run_src, run_bytes, cudaMemcpyHostToDevice, e->copy_stream));
+        run_bytes = 0;
+    };
+    for (int f = f0; f < f1; ++f) {
+        if (frames[f].image_on_device || plan.at[f - f0] < plan.pageable) continue;
+        const size_t bytes = image_bytes(frames[f]);
+        const uint8_t* src = static_cast<const uint8_t*>(frames[f].image);
+        if (run_bytes > 0 && src == run_src + run_bytes && plan.at[f - f0] == run_dst + run_bytes) { run_bytes += bytes; }
+        else {
+            flush();
+            run_src   = src;
+            run_dst   = plan.at[f - f0];
+            run_bytes = bytes;
+        }
+    }
+    flush();
+    return upload;
+}
+
+// Fills the chunk's staging block and works out its launches.
+static Chunk stage_chunk(vm_engine* e, Lane& lane, const vm_frame* frames, int f0, int f1, bool classify, bool to_host, bool only_chunk, const ImagePlan& images) {
+    const int nf = f1 - f0;
+    Chunk c;
+    c.f0           = f0;
+    c.f1           = f1;
+    c.classify     = classify;
+    c.n_neighbours = frames[f0].mesh->n_neighbours;
+    size_t n_ranges = 0, supertiles_cap = 0;
+    int64_t cand_total = 0, node_total = 0, bsp_total = 0, max_cand = 0, max_bsp = 0;
+    bool on_device = true;
+    c.packed4      = true;
+    for (int f = f0; f < f1; ++f) {
+        const vm_frame& fr = frames[f];
+        const int64_t nc   = frame_candidates(fr);
+        if (fr.ranges != nullptr) { n_ranges += fr.n_ranges; }
+        else {
+            c.device_lookup = true;
+            bsp_total += fr.mesh->n_bsp;
+            max_bsp = std::max<int64_t>(max_bsp, fr.mesh->n_bsp);
+        }
+        cand_total += nc;
+        node_total += fr.mesh->n_nodes;
+        max_cand = std::max(max_cand, nc);
+        supertiles_cap += static_cast<size_t>((nc + 1 + STAGED_ST - 1) / STAGED_ST);
+        const int cls = format_class(fr.format);
+        c.packed4     = c.packed4 && (cls == FMT_RGBA || cls == FMT_BGRA);
+        on_device     = on_device && fr.image_on_device;
+    }
+    c.images_apart     = classify && !on_device && !images.small;
+    c.exported         = to_host && only_chunk && cand_total * (12 + 4 * c.n_neighbours + 4 * (classify ? e->n_classes : 0)) <= MAX_EXPORT;
+    c.copied           = to_host && !c.exported;
+    c.blocks_per_frame = static_cast<int>(std::max<int64_t>(1, (rounded(max_cand) + SELECT_THREADS - 1) / SELECT_THREADS));
+    c.n_groups         = (c.blocks_per_frame + GROUP_BLOCKS - 1) / GROUP_BLOCKS;
+    c.bsp_blocks       = static_cast<int>((max_bsp + SELECT_THREADS - 1) / SELECT_THREADS);
+    c.max_rows         = c.blocks_per_frame * SELECT_THREADS + 1;
+    c.stride           = static_cast<int>(rounded(cand_total + nf));
+    // the staged layer kernels want a tile plan of the chunk: the remap makes it while it has the indices in hand
+    c.with_plan = classify && e->staged && e->use_tc && e->may_stage && nf <= TC_MAX_FRAMES;
+
+    // layout of the staging block
+    const size_t frames_at = aligned(sizeof(ChunkHeader));
+    const size_t ranges_at = aligned(frames_at + sizeof(FrameParams) * nf);
+    const size_t n_slots   = n_ranges == 0 ? 0 : std::max<size_t>(64, rounded(n_ranges));  // rounded like every size a graph depends on
+    c.counts_at            = aligned(ranges_at + 3 * sizeof(int32_t) * n_slots);
+    const size_t images_at = aligned(c.counts_at + sizeof(int32_t) * nf * c.n_groups);
+    c.staging_bytes        = images_at + (classify && images.small ? images.total : 0);
+    need(e, lane.h_staging, c.staging_bytes);
+    need(e, lane.d_staging, c.staging_bytes);
+    need(e, lane.d_cand_px, cand_total + 1);
+    need(e, lane.d_cand_node, cand_total + 1);
+    need(e, lane.d_node_rank, node_total + 1);
+    need(e, lane.d_block_counts, static_cast<size_t>(c.blocks_per_frame) * nf);
+    if (c.device_lookup) need(e, lane.d_state, bsp_total + 1);
+    if (classify) {
+        need(e, lane.d_feat[0], static_cast<size_t>(c.stride) * e->max_width);
+        need(e, lane.d_feat[1], static_cast<size_t>(c.stride) * e->max_width);
+    }
+    if (c.with_plan) ensure_tile_plan(e, lane, static_cast<size_t>(c.stride), supertiles_cap);
+
+    uint8_t* h = lane.h_staging.p;
+    uint8_t* d = lane.d_staging.p;
+    *reinterpret_cast<ChunkHeader*>(h) = ChunkHeader{e->h_px.p, e->h_gi.p, e->h_nb.p, e->h_cls.p, e->h_offsets.p};
+    int32_t* pairs  = reinterpret_cast<int32_t*>(h + ranges_at);
+    int32_t* starts = pairs + 2 * n_slots;
+    auto on_gpu     = [&](const void* p) { return d + (static_cast<const uint8_t*>(p) - h); };
+    size_t cursor   = 0;
+    int64_t cand_off = 0, node_off = 0, bsp_off = 0;
+    for (int f = f0; f < f1; ++f) {
+        const vm_frame& fr = frames[f];
+        FrameParams& p     = reinterpret_cast<FrameParams*>(h + frames_at)[f - f0];
+        std::memset(&p, 0, sizeof(p));
+        if (!fill_frame_params(e, fr, p)) throw UnsupportedLens{};
+        p.cand_off = static_cast<int32_t>(cand_off);
+        p.node_off = static_cast<int32_t>(node_off);
+        p.bsp_off  = static_cast<int32_t>(bsp_off);
+        if (fr.ranges == nullptr) {
+            p.n_candidates = fr.mesh->n_nodes;
+            bsp_off += fr.mesh->n_bsp;
+        }
+        else {
+            // ranges and their exclusive prefix sums; an empty frame keeps non-null pointers, which mark host ranges
+            p.n_ranges     = fr.n_ranges;
+            p.ranges       = reinterpret_cast<const int2*>(on_gpu(pairs + 2 * cursor));
+            p.range_starts = reinterpret_cast<const int32_t*>(on_gpu(starts + cursor));
+            int32_t run    = 0;
+            for (int r = 0; r < fr.n_ranges; ++r, ++cursor) {
+                pairs[2 * cursor + 0] = fr.ranges[2 * r];
+                pairs[2 * cursor + 1] = fr.ranges[2 * r + 1];
+                starts[cursor]        = run;
+                run += std::max(0, fr.ranges[2 * r + 1] - fr.ranges[2 * r]);
+            }
+            p.n_candidates = run;
+        }
+        cand_off += p.n_candidates;
+        node_off += fr.mesh->n_nodes;
+        if (!classify) continue;
+        if (fr.image_on_device) { p.image = static_cast<const uint8_t*>(fr.image); }
+        else if (images.small) {
+            p.image = d + images_at + images.at[f - f0];
+            std::memcpy(h + images_at + images.at[f - f0], fr.image, image_bytes(fr));
+        }
+        else {
+            p.image = lane.d_images.p + images.at[f - f0];
+        }
+    }
+    std::memset(h + c.counts_at, 0, sizeof(int32_t) * nf * c.n_groups);
+    return c;
+}
+
+static const FrameParams* device_frames(const Lane& lane) {
+    return reinterpret_cast<const FrameParams*>(lane.d_staging.p + aligned(sizeof(ChunkHeader)));
+}
+static const ChunkHeader* device_header(const Lane& lane) {
+    return reinterpret_cast<const ChunkHeader*>(lane.d_staging.p);
+}
+
+// Exported arrays are copied by a few blocks that leave the SMs to the layers: 32 blocks of 512 threads keep the bus busy.
+constexpr int EXPORT_BLOCKS = 32;
+
+static void issue_export_points(vm_engine* e, Lane& lane, const Chunk& c, cudaStream_t s) {
+    begin_stage(e, s, "export_points");
+    k_export<0><<<EXPORT_BLOCKS, EXPORT_THREADS, 0, s>>>(device_header(lane), e->d_offsets.p, c.f0, c.f1, c.n_neighbours, e->d_px.p, e->d_gi.p, e->d_nb.p);
+    end_stage(e, s);
+}
+
+static void issue_sample(vm_engine* e, Lane& lane, const Chunk& c, cudaStream_t s) {
+    const dim3 g((c.max_rows + ROW_THREADS * SAMPLE_ROWS - 1) / (ROW_THREADS * SAMPLE_ROWS), c.f1 - c.f0);
+    float4* features = reinterpret_cast<float4*>(lane.d_feat[0].p);
+    begin_stage(e, s, "sample_image");
+    if (c.packed4) { k_sample<true><<<g, ROW_THREADS, 0, s>>>(device_frames(lane), e->d_offsets.p, c.f0, e->d_px.p, features); }
+    else {
+        k_sample<false><<<g, ROW_THREADS, 0, s>>>(device_frames(lane), e->d_offsets.p, c.f0, e->d_px.p, features);
+    }
+    end_stage(e, s);
+}
+
+// Staging copy, lookup, projection, compaction, neighbour remap; images that are on the device already are sampled beside the
+// remap (neither needs the other: 178 -> 140 us on 4.4 M rows).
+static void issue_projection(vm_engine* e, Lane& lane, const Chunk& c, bool sample) {
+    cudaStream_t s            = lane.stream;
+    const int nf              = c.f1 - c.f0;
+    const FrameParams* frames = device_frames(lane);
+    int32_t* groups           = reinterpret_cast<int32_t*>(lane.d_staging.p + c.counts_at);
+    VM_CUDA(cudaMemcpyAsync(lane.d_staging.p, lane.h_staging.p, c.staging_bytes, cudaMemcpyHostToDevice, s));
+    if (c.device_lookup) {
+        begin_stage(e, s, "bsp_state");
+        k_bsp_state<<<dim3(c.bsp_blocks, nf), SELECT_THREADS, 0, s>>>(frames, lane.d_state.p);
+        end_stage(e, s);
+    }
+    begin_stage(e, s, "select_project");
+    k_select<<<dim3(c.blocks_per_frame, nf), SELECT_THREADS, 0, s>>>(frames, lane.d_state.p, lane.d_cand_px.p, lane.d_cand_node.p, lane.d_block_counts.p,
+                                                                     groups, c.n_groups, e->flags);
+    end_stage(e, s);
+    begin_stage(e, s, "scatter_compact");
+    k_scatter<SCATTER_UNITS><<<dim3((c.blocks_per_frame + SCATTER_UNITS - 1) / SCATTER_UNITS, nf), SELECT_THREADS, 0, s>>>(
+      frames, device_header(lane), lane.d_cand_px.p, lane.d_cand_node.p, lane.d_block_counts.p, groups, c.blocks_per_frame, c.n_groups, e->d_offsets.p,
+      c.f0, e->d_px.p, e->d_gi.p, lane.d_node_rank.p);
+    end_stage(e, s);
+    const bool fork = sample && !e->timing;
+    if (fork) {
+        VM_CUDA(cudaEventRecord(lane.ev_fork, s));
+        VM_CUDA(cudaStreamWaitEvent(lane.side, lane.ev_fork, 0));
+    }
+    if (sample) issue_sample(e, lane, c, fork ? lane.side : s);
+    if (fork) VM_CUDA(cudaEventRecord(lane.ev_join, lane.side));
+    const dim3 g((c.max_rows + ROW_THREADS - 1) / ROW_THREADS, nf);
+    const st::PlanOut plan = c.with_plan ? tile_plan(lane) : st::PlanOut{nullptr, nullptr, nullptr};
+    begin_stage(e, s, "remap_neighbours");
+#define VM_REMAP(NN)                                                                                                                      \
+    if (c.n_neighbours == NN) {                                                                                                           \
+        if (c.with_plan) k_remap<NN, true><<<g, ROW_THREADS, 0, s>>>(frames, e->d_offsets.p, c.f0, e->d_gi.p, lane.d_node_rank.p, e->d_nb.p, plan); \
+        else k_remap<NN, false><<<g, ROW_THREADS, 0, s>>>(frames, e->d_offsets.p, c.f0, e->d_gi.p, lane.d_node_rank.p, e->d_nb.p, plan);  \
+    }
+    VM_REMAP(4) VM_REMAP(6) VM_REMAP(8)
+#undef VM_REMAP
+    end_stage(e, s);
+    if (fork) VM_CUDA(cudaStreamWaitEvent(s, lane.ev_join, 0));
+}
+
+// All layers, and the classifications to the host when they are wanted there.
+static void issue_layers(vm_engine* e, Lane& lane, const Chunk& c, bool sample) {
+    if (sample) issue_sample(e, lane, c, lane.stream);
+    run_network(e, lane, c.with_plan, e->d_offsets.p, e->d_nb.p, c.n_neighbours, c.f0, c.f1 - c.f0, c.max_rows, e->d_cls.p, true, c.stride);
+    if (!c.exported) return;
+    begin_stage(e, lane.stream, "export_classes");
+    k_export<1><<<EXPORT_BLOCKS, EXPORT_THREADS, 0, lane.stream>>>(device_header(lane), e->d_offsets.p, c.f0, c.f1, e->n_classes, nullptr, nullptr, e->d_cls.p);
+    end_stage(e, lane.stream);
+}
+
+// ---- recorded graphs -------------------------------------------------------------------------------------------------
+
+enum GraphPart { PART_ALL = 0, PART_PROJECTION = 1, PART_LAYERS = 2 };
+
+static void forget_graphs(vm_engine* e) {
+    for (auto& g : e->graphs)
+        if (g.exec != nullptr) cudaGraphExecDestroy(g.exec);
+    e->graphs.clear();
+}
+
+static GraphKey graph_key(const vm_engine* e, const Lane& lane, const Chunk& c, int part) {
+    GraphKey k;
+    std::memset(&k, 0, sizeof(k));
+    k.part             = part;
+    k.lane             = static_cast<int32_t>(&lane - e->lanes);
+    k.n_frames         = c.f1 - c.f0;
+    k.f0               = c.f0;
+    k.n_neighbours     = c.n_neighbours;
+    k.blocks_per_frame = c.blocks_per_frame;
+    k.bsp_blocks       = c.bsp_blocks;
+    k.options          = c.classify | c.exported << 1 | c.device_lookup << 2 | c.packed4 << 3 | c.with_plan << 4 | c.images_apart << 5 | int(e->use_tc) << 6;
+    k.wait_limit       = e->tc_wait_limit;
+    k.feature_stride   = c.stride;
+    k.staging_bytes    = c.staging_bytes;
+    return k;
+}
+
+// Enqueues what `issue` enqueues on the lane's stream. A chunk of this shape that comes back is recorded as a CUDA graph and from
+// then on costs one launch: on the B200 box a launch takes 2.7 to 3.8 us of host time, so that 8 small kernels and a wait take
+// 32 us one by one and 11 us as a graph, 16 kernels 49 and 15 us. The first time nothing is recorded: recording and instantiating
+// costs more than it saves on a shape that may never return.
+template <typename Issue>
+static void run_part(vm_engine* e, Lane& lane, const Chunk& c, int part, Issue issue) {
+    if (!e->use_graphs || e->timing || e->nvtx) {
+        issue();
+        return;
+    }
+    const GraphKey key = graph_key(e, lane, c, part);
+    GraphEntry* entry  = nullptr;
+    for (auto& g : e->graphs)
+        if (std::memcmp(&g.key, &key, sizeof(key)) == 0) entry = &g;
+    if (entry == nullptr || entry->refused) {
+        if (entry == nullptr) {
+            if (e->graphs.size() >= MAX_GRAPHS) {
+                auto oldest = std::min_element(e->graphs.begin(), e->graphs.end(), [](const GraphEntry& a, const GraphEntry& b) { return a.last_use < b.last_use; });
+                if (oldest->exec != nullptr) {
+                    // it may still be running on its lane
+                    VM_CUDA(cudaStreamSynchronize(e->lanes[oldest->key.lane].stream));
+                    cudaGraphExecDestroy(oldest->exec);
+                }
+                e->graphs.erase(oldest);
+            }
+            GraphEntry fresh;
+            fresh.key      = key;
+            fresh.last_use = ++e->graph_uses;
+            e->graphs.push_back(fresh);
+        }
+        issue();
+        return;
+    }
+    entry->last_use = ++e->graph_uses;
+    if (entry->exec == nullptr) {
+        const int64_t before = e->launches;
+        cudaGraph_t graph    = nullptr;
+        VM_CUDA(cudaStreamBeginCapture(lane.stream, cudaStreamCaptureModeThreadLocal));
+        bool recorded = true;
+        try {
+            issue();
+        }
+        catch (const CudaFailure&) {
+            recorded = false;
+        }
+        recorded         = cudaStreamEndCapture(lane.stream, &graph) == cudaSuccess && recorded;
+        entry->kernels   = e->launches - before;
+        e->launches      = before;
+        recorded         = recorded && cudaGraphInstantiate(&entry->exec, graph, 0) == cudaSuccess;
+        if (graph != nullptr) cudaGraphDestroy(graph);
+        if (!recorded) {
+            cudaGetLastError();
+            entry->exec    = nullptr;
+            entry->refused = true;
+            issue();
+            return;
+        }
+    }
+    VM_CUDA(cudaGraphLaunch(entry->exec, lane.stream));
+    e->launches += entry->kernels;
+}
+
+// ---- one batch -------------------------------------------------------------------------------------------------------
+
+// Enqueues a whole chunk except for results that are copied once their number is known; nothing here waits for the device.
+static Chunk enqueue_chunk(vm_engine* e, Lane& lane, Lane* prev, bool after_prev, const vm_frame* frames, int f0, int f1, bool classify, bool to_host,
+                           bool only_chunk, const ImagePlan& images, Upload* upload) {
+    const Chunk c = stage_chunk(e, lane, frames, f0, f1, classify, to_host, only_chunk, images);
+    if (upload != nullptr) upload->pump();
+    if (e->buffers_moved) {
+        // graphs of other lanes may be running: they stay valid until they have finished
+        for (auto& l : e->lanes)
+            if (l.busy) VM_CUDA(cudaStreamSynchronize(l.stream));
+        forget_graphs(e);
+        e->buffers_moved = false;
+    }
+    // this chunk's offsets continue those of the one before
+    if (prev != nullptr && prev != &lane) VM_CUDA(cudaStreamWaitEvent(lane.stream, after_prev ? prev->ev_done : prev->ev_offsets, 0));
+    lane.busy = true;
+    if (only_chunk && !c.images_apart && !c.copied) {
+        // everything as one graph, the results of the projection on their way to the host beside the layers
+        run_part(e, lane, c, PART_ALL, [&] {
+            issue_projection(e, lane, c, classify);
+            const bool fork = c.exported && classify && !e->timing;
+            if (fork) {
+                VM_CUDA(cudaEventRecord(lane.ev_fork, lane.stream));
+                VM_CUDA(cudaStreamWaitEvent(lane.side, lane.ev_fork, 0));
+            }
+            if (c.exported) issue_export_points(e, lane, c, fork ? lane.side : lane.stream);
+            if (fork) VM_CUDA(cudaEventRecord(lane.ev_join, lane.side));
+            if (classify) issue_layers(e, lane, c, false);
+            if (fork) VM_CUDA(cudaStreamWaitEvent(lane.stream, lane.ev_join, 0));
+        });
+    }
+    else {
+        run_part(e, lane, c, PART_PROJECTION, [&] { issue_projection(e, lane, c, classify && !c.images_apart); });
+        VM_CUDA(cudaEventRecord(lane.ev_offsets, lane.stream));
+        if (c.exported) {
+            cudaStream_t beside = e->timing ? lane.stream : lane.side;
+            VM_CUDA(cudaStreamWaitEvent(beside, lane.ev_offsets, 0));
+            issue_export_points(e, lane, c, beside);
+            VM_CUDA(cudaEventRecord(lane.ev_join, beside));
+        }
+        if (upload != nullptr) upload->finish();
+        if (c.images_apart) {
+            VM_CUDA(cudaEventRecord(lane.ev_images, e->copy_stream));
+            VM_CUDA(cudaStreamWaitEvent(lane.stream, lane.ev_images, 0));
+        }
+        if (classify) run_part(e, lane, c, PART_LAYERS, [&] { issue_layers(e, lane, c, c.images_apart); });
+        if (c.exported) VM_CUDA(cudaStreamWaitEvent(lane.stream, lane.ev_join, 0));
+    }
+    VM_CUDA(cudaEventRecord(lane.ev_done, lane.stream));
+    return c;
+}
+
+// Copies a chunk's results to the host; waits for its offsets first. The projection's results leave while its layers run.
+static void copy_results(vm_engine* e, Lane& lane, const Chunk& c) {
+    if (!c.copied) return;
     VM_CUDA(cudaEventSynchronize(lane.ev_offsets));
-    if (to_host) {
-        const int32_t* off = e->h_offsets.p;
-        const size_t p0 = off[lane.f0], p1 = off[lane.f1];
-        const size_t r0 = p0 + lane.f0, r1 = p1 + lane.f1;
-        cudaStream_t s = lane.stream;
-        if (p1 > p0) {
-            VM_CUDA(cudaMemcpyAsync(e->h_px.p + p0, e->d_px.p + p0, sizeof(float2) * (p1 - p0), cudaMemcpyDeviceToHost, s));
-            VM_CUDA(cudaMemcpyAsync(e->h_gi.p + p0, e->d_gi.p + p0, sizeof(int32_t) * (p1 - p0), cudaMemcpyDeviceToHost, s));
-        }
-        VM_CUDA(cudaMemcpyAsync(e->h_nb.p + r0 * N, e->d_nb.p + r0 * N, sizeof(int32_t) * (r1 - r0) * N, cudaMemcpyDeviceToHost, s));
-        if (classify) {
-            const size_t C = e->n_classes;
-            VM_CUDA(cudaMemcpyAsync(e->h_cls.p + r0 * C, e->d_cls.p + r0 * C, sizeof(float) * (r1 - r0) * C, cudaMemcpyDeviceToHost, s));
-        }
+    const int32_t* off = e->h_offsets.p;
+    const size_t p0 = off[c.f0], p1 = off[c.f1];
+    const size_t r0 = p0 + c.f0, r1 = p1 + c.f1;
+    const size_t N = c.n_neighbours, C = e->n_classes;
+    cudaStream_t beside = e->timing ? lane.stream : lane.side;
+    VM_CUDA(cudaStreamWaitEvent(beside, lane.ev_offsets, 0));
+    if (p1 > p0) {
+        VM_CUDA(cudaMemcpyAsync(e->h_px.p + p0, e->d_px.p + p0, sizeof(float2) * (p1 - p0), cudaMemcpyDeviceToHost, beside));
+        VM_CUDA(cudaMemcpyAsync(e->h_gi.p + p0, e->d_gi.p + p0, sizeof(int32_t) * (p1 - p0), cudaMemcpyDeviceToHost, beside));
+    }
+    VM_CUDA(cudaMemcpyAsync(e->h_nb.p + r0 * N, e->d_nb.p + r0 * N, sizeof(int32_t) * (r1 - r0) * N, cudaMemcpyDeviceToHost, beside));
+    if (c.classify) VM_CUDA(cudaMemcpyAsync(e->h_cls.p + r0 * C, e->d_cls.p + r0 * C, sizeof(float) * (r1 - r0) * C, cudaMemcpyDeviceToHost, lane.stream));
+    if (beside != lane.stream) {
+        VM_CUDA(cudaEventRecord(lane.ev_join, beside));
+        VM_CUDA(cudaStreamWaitEvent(lane.stream, lane.ev_join, 0));
     }
     VM_CUDA(cudaEventRecord(lane.ev_done, lane.stream));
 }
@@ -642,6 +927,14 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
     if (classify && e->layers.front().n_slots != N + 1) return fail(VM_ERR_NETWORK_SHAPE, "network was built for a different n_neighbours");
     if (cand_all + n_frames > (int64_t(1) << 31) - 1024) return fail(VM_ERR_INVALID_ARGUMENT, "batch too large: split it");
 
+    auto drain = [&] {
+        for (auto& lane : e->lanes) {
+            cudaStreamSynchronize(lane.stream);
+            cudaStreamSynchronize(lane.side);
+            lane.busy = false;
+        }
+        cudaStreamSynchronize(e->copy_stream);
+    };
     try {
         VM_CUDA(cudaSetDevice(e->device));
         e->timing = (flags & VM_TIME_STAGES) != 0;
@@ -649,44 +942,46 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
         e->events_used = 0;
         e->stage_ms.clear();
         const bool to_host = (flags & VM_RESULTS_ON_DEVICE) == 0;
-        const int n_lanes  = e->timing ? 1 : e->n_lanes;
+        const int n_lanes  = e->timing ? 1 : e->n_lanes;  // with the stages timed, one chunk after another
 
         const size_t rows_all = static_cast<size_t>(cand_all) + n_frames;
-        e->d_offsets.ensure(n_frames + 1);
+        need(e, e->d_offsets, n_frames + 1);
+        need(e, e->d_px, cand_all + 1);
+        need(e, e->d_gi, cand_all + 1);
+        need(e, e->d_nb, rows_all * N);
+        if (classify) need(e, e->d_cls, rows_all * e->n_classes);
         e->h_offsets.ensure(n_frames + 1);
-        e->d_px.ensure(cand_all + 1);
-        e->d_gi.ensure(cand_all + 1);
-        e->d_nb.ensure(rows_all * N);
-        if (classify) e->d_cls.ensure(rows_all * e->n_classes);
         if (to_host) {
             e->h_px.ensure(cand_all + 1);
             e->h_gi.ensure(cand_all + 1);
             e->h_nb.ensure(rows_all * N);
             if (classify) e->h_cls.ensure(rows_all * e->n_classes);
         }
-        e->h_offsets.p[0] = 0;
-        *e->h_abort       = 0;
-        VM_CUDA(cudaMemsetAsync(e->d_offsets.p, 0, sizeof(int32_t), e->lanes[0].stream));
-        VM_CUDA(cudaMemsetAsync(e->d_abort, 0, sizeof(int32_t), e->lanes[0].stream));
-        // kernels of the other lanes raise the same abort flag: their first chunk must not start before the clear
-        VM_CUDA(cudaEventRecord(e->ev_batch_start, e->lanes[0].stream));
-        for (int l = 1; l < n_lanes; ++l) VM_CUDA(cudaStreamWaitEvent(e->lanes[l].stream, e->ev_batch_start, 0));
+        for (int i = 0; i < ABORT_FLAGS; ++i) e->flags[i] = 0;
 
-        // chunks: runs of frames bounded by a candidate budget and a frame count. Small chunks let the copies of one
-        // chunk overlap the kernels of another; when there is nothing to copy in (frames already on the device, or
-        // projection only) larger chunks mean fewer, fuller launches.
+        // Chunks: runs of frames bounded by a candidate budget, a frame count and the bytes of their host images. Small ones let the
+        // copies of one chunk overlap the kernels of another: 20 MB are 0.4 ms of the bus (32 frames of 5 MB to results on the
+        // host: 4.28 ms in chunks of 16 frames, 3.98 in chunks of 4, 4.11 in chunks of 2; both directions' bytes alone take 3.45). When no images are to be copied in, a batch is one chunk as far as the scratch allows, and
+        // chunks follow one another: fewer and fuller launches (64 frames of 1280 x 1024 pixels in one chunk: 1.61 ms, in two that
+        // overlap 1.99, in eight 2.06 - persistent layer kernels of two chunks get in one another's way).
         bool host_images = false;
         for (int f = 0; f < n_frames; ++f) host_images = host_images || (classify && !frames[f].image_on_device);
-        const int64_t max_chunk_candidates = (e->chunk_override || host_images) ? e->chunk_candidates : 4 * e->chunk_candidates;
-        const int max_chunk_frames         = (e->chunk_override || host_images) ? e->chunk_frames : std::min(4 * e->chunk_frames, static_cast<int>(TC_MAX_FRAMES));
+        const bool small_chunks = e->chunk_override || host_images;
+        const int64_t max_chunk_candidates = small_chunks ? e->chunk_candidates : 8 * e->chunk_candidates;
+        const int max_chunk_frames         = small_chunks ? e->chunk_frames : TC_MAX_FRAMES;
         int f0 = 0, chunk = 0;
         Lane* prev = nullptr;
-        std::vector<Lane*> order;
+        Chunk last;
         while (f0 < n_frames) {
             int f1 = f0;
-            int64_t c = 0;
-            while (f1 < n_frames && (f1 == f0 || (c + frame_candidates(frames[f1]) <= max_chunk_candidates && f1 - f0 < max_chunk_frames))) {
-                c += frame_candidates(frames[f1]);
+            int64_t c    = 0;
+            size_t bytes = 0;
+            while (f1 < n_frames) {
+                const int64_t more      = frame_candidates(frames[f1]);
+                const size_t more_bytes = classify && !frames[f1].image_on_device ? image_bytes(frames[f1]) : 0;
+                if (f1 > f0 && (c + more > max_chunk_candidates || f1 - f0 >= max_chunk_frames || (bytes + more_bytes > CHUNK_IMAGE_BYTES && !e->chunk_override))) break;
+                c += more;
+                bytes += more_bytes;
                 ++f1;
             }
             Lane& lane = e->lanes[chunk % n_lanes];
@@ -695,40 +990,37 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
                 VM_CUDA(cudaEventSynchronize(lane.ev_done));
                 lane.busy = false;
             }
-            enqueue_chunk(e, lane, prev, frames, f0, f1, classify);
-            // while this chunk runs, read back the one before it
-            if (prev != nullptr) enqueue_chunk_readback(e, *prev, N, classify, to_host);
-            if (n_lanes == 1) {
-                enqueue_chunk_readback(e, lane, N, classify, to_host);
-                prev = nullptr;
-                // a single lane still has to chain its scans: same stream, already ordered
+            ImagePlan images;
+            std::unique_ptr<Upload> upload;
+            if (classify) {
+                images = plan_images(frames, f0, f1);
+                if (images.total > 0 && !images.small) upload = start_images(e, lane, frames, f0, f1, images);
             }
-            else {
-                prev = &lane;
+            const Chunk current = enqueue_chunk(e, lane, prev, !host_images, frames, f0, f1, classify, to_host, f0 == 0 && f1 == n_frames, images, upload.get());
+            // while this chunk runs, fetch the results of the one before it
+            if (n_lanes == 1) { copy_results(e, lane, current); }
+            else if (prev != nullptr) {
+                copy_results(e, *prev, last);
             }
-            f0 = f1;
+            prev = &lane;
+            last = current;
+            f0   = f1;
             ++chunk;
         }
-        if (prev != nullptr) enqueue_chunk_readback(e, *prev, N, classify, to_host);
-        // the abort flag is read once, after the last kernel of EVERY lane: the chunks before the last one run on
-        // other streams and may still be in their network layers when the last chunk's stream gets here
-        cudaStream_t last_stream = e->lanes[(chunk - 1) % n_lanes].stream;
-        for (int l = 0; l < n_lanes; ++l) {
-            if (e->lanes[l].busy && e->lanes[l].stream != last_stream) VM_CUDA(cudaStreamWaitEvent(last_stream, e->lanes[l].ev_done, 0));
+        if (n_lanes > 1) copy_results(e, *prev, last);
+        for (auto& lane : e->lanes) {
+            if (lane.busy) VM_CUDA(cudaEventSynchronize(lane.ev_done));
+            lane.busy = false;
         }
-        VM_CUDA(cudaMemcpyAsync(e->h_abort, e->d_abort, sizeof(int32_t), cudaMemcpyDeviceToHost, last_stream));
-        // the last stream has waited for every other lane: one event behind the flag's copy marks the end of the batch
-        VM_CUDA(cudaEventRecord(e->ev_batch_done, last_stream));
-        VM_CUDA(cudaEventSynchronize(e->ev_batch_done));
-        for (int l = 0; l < n_lanes; ++l) e->lanes[l].busy = false;
-        if (*e->h_abort == ABORT_TC_RANGE && e->use_tc) {
+        // read once, after the last kernel of EVERY lane
+        if (e->flags[ABORT_TC_TIMEOUT]) return fail(VM_ERR_DEVICE_ABORT, "a tensor-core kernel gave up waiting on an mbarrier");
+        if (e->flags[ABORT_BSP_DEPTH]) return fail(VM_ERR_DEVICE_ABORT, "a kernel gave up on a bounded loop (BSP deeper than 128 levels)");
+        if (e->flags[ABORT_TC_RANGE] && e->use_tc) {
             // a feature value beyond the range of the fp16 split: this engine goes back to the FFMA kernels for good and
             // the batch is computed again
             e->use_tc = false;
             return run_batch(e, frames, n_frames, flags, out);
         }
-        if (*e->h_abort == ABORT_TC_TIMEOUT) return fail(VM_ERR_DEVICE_ABORT, "a tensor-core kernel gave up waiting on an mbarrier");
-        if (*e->h_abort != 0) return fail(VM_ERR_DEVICE_ABORT, "a kernel gave up on a bounded loop (BSP deeper than 128 levels)");
 
         if (e->timing) {
             for (const auto& t : e->timers) {
@@ -759,15 +1051,13 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
     }
     catch (const CudaFailure& f) {
         cudaGetLastError();
+        drain();
+        cudaGetLastError();
         const vm_status s = f.code == cudaErrorMemoryAllocation ? VM_ERR_OUT_OF_MEMORY : VM_ERR_CUDA;
         return fail(s, std::string(cudaGetErrorName(f.code)) + ": " + cudaGetErrorString(f.code) + " in " + f.what);
     }
     catch (const UnsupportedLens&) {
-        // work already enqueued for earlier chunks finishes on its own; the lanes are drained before the next batch
-        for (int l = 0; l < MAX_LANES; ++l) {
-            cudaStreamSynchronize(e->lanes[l].stream);
-            e->lanes[l].busy = false;
-        }
+        drain();
         return fail(VM_ERR_UNSUPPORTED_LENS, "Cannot project: Unknown lens type");
     }
 }
@@ -844,24 +1134,24 @@ vm_status vm_engine_create(int device, const vm_layer* layers, const int32_t* la
         if (const char* v = std::getenv("VMCUDA_STAGED")) e->staged = std::atoi(v) != 0;
         if (const char* v = std::getenv("VMCUDA_BLOCKING_SYNC")) e->blocking_sync = std::atoi(v) != 0;
         if (const char* v = std::getenv("VMCUDA_NVTX")) e->nvtx = std::atoi(v) != 0;
+        if (const char* v = std::getenv("VMCUDA_GRAPHS")) e->use_graphs = std::atoi(v) != 0;
         if (const char* v = std::getenv("VMCUDA_LANES")) e->n_lanes = std::min(MAX_LANES, std::max(1, std::atoi(v)));
         for (int l = 0; l < MAX_LANES; ++l) {
             Lane& lane = e->lanes[l];
             VM_CUDA(cudaStreamCreateWithFlags(&lane.stream, cudaStreamNonBlocking));
-            VM_CUDA(cudaEventCreateWithFlags(&lane.ev_staged, cudaEventDisableTiming));
-            VM_CUDA(cudaEventCreateWithFlags(&lane.ev_scan, cudaEventDisableTiming));
-            // the two events the host waits on: spinning (lowest latency) or, with VMCUDA_BLOCKING_SYNC=1, sleeping - for
-            // boxes where several engines' host threads share few cores
-            const unsigned wait_flags = cudaEventDisableTiming | (e->blocking_sync ? cudaEventBlockingSync : 0);
-            VM_CUDA(cudaEventCreateWithFlags(&lane.ev_offsets, wait_flags));
-            VM_CUDA(cudaEventCreateWithFlags(&lane.ev_done, wait_flags));
+            VM_CUDA(cudaStreamCreateWithFlags(&lane.side, cudaStreamNonBlocking));
+            for (cudaEvent_t* ev : {&lane.ev_fork, &lane.ev_join, &lane.ev_images}) VM_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
+            // the events the host waits on: spinning (lowest latency) or, with VMCUDA_BLOCKING_SYNC=1, sleeping - for boxes where
+            // several engines' host threads share few cores
+            for (cudaEvent_t* ev : {&lane.ev_offsets, &lane.ev_done}) {
+                VM_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming | (e->blocking_sync ? cudaEventBlockingSync : 0)));
+            }
         }
+        VM_CUDA(cudaStreamCreateWithFlags(&e->copy_stream, cudaStreamNonBlocking));
         VM_CUDA(cudaEventCreate(&e->ev_timer_start));
         VM_CUDA(cudaEventCreate(&e->ev_timer_stop));
-        VM_CUDA(cudaEventCreateWithFlags(&e->ev_batch_start, cudaEventDisableTiming));
-        VM_CUDA(cudaEventCreateWithFlags(&e->ev_batch_done, cudaEventDisableTiming | (e->blocking_sync ? cudaEventBlockingSync : 0)));
-        VM_CUDA(cudaMalloc(reinterpret_cast<void**>(&e->d_abort), sizeof(int32_t)));
-        VM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&e->h_abort), sizeof(int32_t), cudaHostAllocDefault));
+        VM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&e->flags), sizeof(int32_t) * ABORT_FLAGS, cudaHostAllocDefault));
+        for (int i = 0; i < ABORT_FLAGS; ++i) e->flags[i] = 0;
         int l = 0;
         int width = 4;
         for (int g = 0; g < n_groups; ++g) {
@@ -963,11 +1253,10 @@ void vm_engine_destroy(vm_engine* e) {
         cudaFree(L.d_tc_cat);
         cudaFree(L.d_tc_bias);
     }
+    forget_graphs(e);
     for (auto& lane : e->lanes) {
-        lane.h_frames.release();
-        lane.d_frames.release();
-        lane.h_ranges.release();
-        lane.d_ranges.release();
+        lane.h_staging.release();
+        lane.d_staging.release();
         lane.d_state.release();
         lane.d_cand_px.release();
         lane.d_cand_node.release();
@@ -976,15 +1265,16 @@ void vm_engine_destroy(vm_engine* e) {
         lane.d_feat[0].release();
         lane.d_feat[1].release();
         lane.d_images.release();
+        lane.h_images.release();
         lane.d_nbl.release();
         lane.d_halo_rows.release();
         lane.d_halo_count.release();
         if (lane.stream) cudaStreamDestroy(lane.stream);
-        if (lane.ev_staged) cudaEventDestroy(lane.ev_staged);
-        if (lane.ev_scan) cudaEventDestroy(lane.ev_scan);
-        if (lane.ev_offsets) cudaEventDestroy(lane.ev_offsets);
-        if (lane.ev_done) cudaEventDestroy(lane.ev_done);
+        if (lane.side) cudaStreamDestroy(lane.side);
+        for (cudaEvent_t ev : {lane.ev_fork, lane.ev_join, lane.ev_offsets, lane.ev_images, lane.ev_done})
+            if (ev) cudaEventDestroy(ev);
     }
+    if (e->copy_stream) cudaStreamDestroy(e->copy_stream);
     e->d_offsets.release();
     e->h_offsets.release();
     e->d_px.release();
@@ -998,10 +1288,7 @@ void vm_engine_destroy(vm_engine* e) {
     for (auto ev : e->event_pool) cudaEventDestroy(ev);
     if (e->ev_timer_start) cudaEventDestroy(e->ev_timer_start);
     if (e->ev_timer_stop) cudaEventDestroy(e->ev_timer_stop);
-    if (e->ev_batch_start) cudaEventDestroy(e->ev_batch_start);
-    if (e->ev_batch_done) cudaEventDestroy(e->ev_batch_done);
-    cudaFree(e->d_abort);
-    cudaFreeHost(e->h_abort);
+    cudaFreeHost(e->flags);
     delete e;
 }
 
@@ -1132,9 +1419,9 @@ vm_status vm_sample(vm_engine* e, const float* px, int32_t n, const void* image,
         VM_CUDA(cudaSetDevice(e->device));
         Lane& lane        = e->lanes[0];
         const size_t bytes = static_cast<size_t>(width) * height * format_bytes_per_pixel(cls);
-        lane.d_images.ensure(bytes);
-        lane.d_cand_px.ensure(n);
-        lane.d_feat[0].ensure(static_cast<size_t>(n) * 4);
+        need(e, lane.d_images, bytes);
+        need(e, lane.d_cand_px, n);
+        need(e, lane.d_feat[0], static_cast<size_t>(n) * 4);
         VM_CUDA(cudaMemcpyAsync(lane.d_images.p, image, bytes, cudaMemcpyHostToDevice, lane.stream));
         VM_CUDA(cudaMemcpyAsync(lane.d_cand_px.p, px, sizeof(float2) * n, cudaMemcpyHostToDevice, lane.stream));
         ++e->launches;
@@ -1164,11 +1451,11 @@ vm_status vm_network(vm_engine* e, const float* input, const int32_t* neighbourh
         VM_CUDA(cudaSetDevice(e->device));
         Lane& lane = e->lanes[0];
         const size_t rows = n_rows;
-        e->d_offsets.ensure(2);
-        e->d_nb.ensure(rows * n_neighbours);
-        e->d_cls.ensure(rows * e->n_classes);
-        lane.d_feat[0].ensure(rows * e->max_width);
-        lane.d_feat[1].ensure(rows * e->max_width);
+        need(e, e->d_offsets, 2);
+        need(e, e->d_nb, rows * n_neighbours);
+        need(e, e->d_cls, rows * e->n_classes);
+        need(e, lane.d_feat[0], rows * e->max_width);
+        need(e, lane.d_feat[1], rows * e->max_width);
         const int32_t offsets[2] = {0, n_rows - 1};
         VM_CUDA(cudaMemcpyAsync(e->d_offsets.p, offsets, sizeof(offsets), cudaMemcpyHostToDevice, lane.stream));
         VM_CUDA(cudaMemcpyAsync(e->d_nb.p, neighbourhood, sizeof(int32_t) * rows * n_neighbours, cudaMemcpyHostToDevice, lane.stream));
@@ -1176,24 +1463,23 @@ vm_status vm_network(vm_engine* e, const float* input, const int32_t* neighbourh
         for (int attempt = 0; attempt < 2; ++attempt) {
             // the layers ping-pong over the feature buffers, so a second attempt needs the input again
             VM_CUDA(cudaMemcpyAsync(lane.d_feat[0].p, input, sizeof(float) * rows * 4, cudaMemcpyHostToDevice, lane.stream));
-            VM_CUDA(cudaMemsetAsync(e->d_abort, 0, sizeof(int32_t), lane.stream));
-            lane.plan_valid = false;
-            if (e->staged && e->use_tc && e->may_stage) {
-                const st::PlanOut plan = ensure_tile_plan(lane, rows, (rows + STAGED_ST - 1) / STAGED_ST + 1);
+            for (int i = 0; i < ABORT_FLAGS; ++i) e->flags[i] = 0;
+            const bool with_plan = e->staged && e->use_tc && e->may_stage;
+            if (with_plan) {
+                ensure_tile_plan(e, lane, rows, (rows + STAGED_ST - 1) / STAGED_ST + 1);
+                const st::PlanOut plan = tile_plan(lane);
                 ++e->launches;
                 launch_tile_plan_kernel(n_neighbours, e->d_offsets.p, e->d_nb.p, plan.nbl, plan.halo_rows, plan.halo_count, 0, 1, n_rows, lane.stream);
                 VM_CUDA(cudaGetLastError());
-                lane.plan_valid = true;
             }
-            run_network(e, lane, e->d_offsets.p, e->d_nb.p, n_neighbours, 0, 1, n_rows, e->d_cls.p, true, n_rows);
+            run_network(e, lane, with_plan, e->d_offsets.p, e->d_nb.p, n_neighbours, 0, 1, n_rows, e->d_cls.p, true, n_rows);
             VM_CUDA(cudaMemcpyAsync(out, e->d_cls.p, sizeof(float) * rows * e->n_classes, cudaMemcpyDeviceToHost, lane.stream));
-            VM_CUDA(cudaMemcpyAsync(e->h_abort, e->d_abort, sizeof(int32_t), cudaMemcpyDeviceToHost, lane.stream));
             VM_CUDA(cudaStreamSynchronize(lane.stream));
-            if (*e->h_abort == ABORT_TC_RANGE && e->use_tc) {
+            if (e->flags[ABORT_TC_TIMEOUT]) return fail(VM_ERR_DEVICE_ABORT, "a kernel gave up on a bounded wait");
+            if (e->flags[ABORT_TC_RANGE] && e->use_tc) {
                 e->use_tc = false;  // a value beyond the fp16 split's range: recompute with the FFMA kernels
                 continue;
             }
-            if (*e->h_abort != 0) return fail(VM_ERR_DEVICE_ABORT, "a kernel gave up on a bounded wait");
             break;
         }
     }
@@ -1212,9 +1498,12 @@ constexpr size_t align256(size_t v) {
     return (v + 255) & ~size_t(255);
 }
 constexpr size_t ST_FRAME   = 0;
-constexpr size_t ST_CELLS   = ST_FRAME + align256(sizeof(vm::FrameParams));  // offsets[2], abort flag
-constexpr size_t ST_BLOCKS  = ST_CELLS + 256;
+constexpr size_t ST_CELLS   = ST_FRAME + align256(sizeof(vm::FrameParams));  // offsets[2], the offsets' second copy, abort flags, group counts
+constexpr size_t ST_HEADER  = ST_CELLS + 256;
+constexpr size_t ST_BLOCKS  = ST_HEADER + align256(sizeof(vm::ChunkHeader));
 constexpr size_t ST_STATE   = ST_BLOCKS + align256(sizeof(int32_t) * (VM_STATIC_MAX_NODES / vm::SELECT_THREADS + 2));
+constexpr int ST_GROUPS     = VM_STATIC_MAX_NODES / (vm::SELECT_THREADS * vm::GROUP_BLOCKS) + 1;
+static_assert(8 + ST_GROUPS <= 64, "the cells hold offsets, flags and group counts");
 constexpr size_t ST_CAND_PX = ST_STATE + align256(VM_STATIC_MAX_BSP);
 constexpr size_t ST_CAND_ID = ST_CAND_PX + align256(sizeof(float2) * VM_STATIC_MAX_NODES);
 constexpr size_t ST_RANK    = ST_CAND_ID + align256(sizeof(int32_t) * VM_STATIC_MAX_NODES);
@@ -1267,7 +1556,8 @@ vm_status vm_project_static(vm_engine* e,
         unsigned char* base = g_static_address[e->device];
         if (base == nullptr) return fail(VM_ERR_CUDA, "the address of the static scratch array could not be looked up on this device");
         auto* d_frame         = reinterpret_cast<FrameParams*>(base + ST_FRAME);
-        auto* d_cells         = reinterpret_cast<int32_t*>(base + ST_CELLS);  // [0], [1] offsets, [2] abort
+        auto* d_cells         = reinterpret_cast<int32_t*>(base + ST_CELLS);  // [0..1] offsets, [2..3] copy, [4..7] abort flags, [8..] group counts
+        auto* d_header        = reinterpret_cast<ChunkHeader*>(base + ST_HEADER);
         auto* d_blocks        = reinterpret_cast<int32_t*>(base + ST_BLOCKS);
         auto* d_state         = reinterpret_cast<uint8_t*>(base + ST_STATE);
         auto* d_cand_px       = reinterpret_cast<float2*>(base + ST_CAND_PX);
@@ -1281,18 +1571,20 @@ vm_status vm_project_static(vm_engine* e,
         FrameParams p;
         std::memset(&p, 0, sizeof(p));
         // never builds the libm last-bit tables here (that allocates): they are used only if an earlier call built them
-        if (!fill_frame_params(fr, p, e->device, false)) return fail(VM_ERR_UNSUPPORTED_LENS, "Cannot project: Unknown lens type");
+        if (!fill_frame_params(e, fr, p, false)) return fail(VM_ERR_UNSUPPORTED_LENS, "Cannot project: Unknown lens type");
         p.n_candidates = mesh->n_nodes;
 
         cudaStream_t s = e->lanes[0].stream;
         VM_CUDA(cudaMemcpyAsync(d_frame, &p, sizeof(p), cudaMemcpyHostToDevice, s));
         // the array keeps the last call's contents: the running offset and the abort flag must start at zero
-        VM_CUDA(cudaMemsetAsync(d_cells, 0, 4 * sizeof(int32_t), s));
+        VM_CUDA(cudaMemsetAsync(d_cells, 0, 64 * sizeof(int32_t), s));
+        const ChunkHeader header{nullptr, nullptr, nullptr, nullptr, d_cells + 2};
+        VM_CUDA(cudaMemcpyAsync(d_header, &header, sizeof(header), cudaMemcpyHostToDevice, s));
         const int blocks = (mesh->n_nodes + SELECT_THREADS - 1) / SELECT_THREADS;
         k_bsp_state<<<dim3((mesh->n_bsp + SELECT_THREADS - 1) / SELECT_THREADS, 1), SELECT_THREADS, 0, s>>>(d_frame, d_state);
-        k_select<<<dim3(blocks, 1), SELECT_THREADS, 0, s>>>(d_frame, d_state, d_cand_px, d_cand_node, d_blocks, d_cells + 2);
-        k_scan<<<1, 1024, 0, s>>>(d_blocks, blocks, blocks, 1, d_cells, 0);
-        k_scatter<1><<<dim3(blocks, 1), SELECT_THREADS, 0, s>>>(d_frame, d_cand_px, d_cand_node, d_blocks, blocks, d_cells, 0,
+        const int groups = (blocks + GROUP_BLOCKS - 1) / GROUP_BLOCKS;
+        k_select<<<dim3(blocks, 1), SELECT_THREADS, 0, s>>>(d_frame, d_state, d_cand_px, d_cand_node, d_blocks, d_cells + 8, groups, d_cells + 4);
+        k_scatter<1><<<dim3(blocks, 1), SELECT_THREADS, 0, s>>>(d_frame, d_header, d_cand_px, d_cand_node, d_blocks, d_cells + 8, blocks, groups, d_cells, 0,
                                                              reinterpret_cast<float2*>(d_px), d_gi, d_rank);
         dim3 g((mesh->n_nodes + 1 + ROW_THREADS - 1) / ROW_THREADS, 1);
         const st::PlanOut no_plan{nullptr, nullptr, nullptr};
@@ -1300,12 +1592,12 @@ vm_status vm_project_static(vm_engine* e,
         else if (mesh->n_neighbours == 6) k_remap<6, false><<<g, ROW_THREADS, 0, s>>>(d_frame, d_cells, 0, d_gi, d_rank, d_nb, no_plan);
         else k_remap<8, false><<<g, ROW_THREADS, 0, s>>>(d_frame, d_cells, 0, d_gi, d_rank, d_nb, no_plan);
         VM_CUDA(cudaGetLastError());
-        e->launches += 5;
+        e->launches += 4;
         if (d_n_points != nullptr) VM_CUDA(cudaMemcpyAsync(d_n_points, d_cells + 1, sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
-        int32_t cells[3] = {0, 0, 0};
+        int32_t cells[8] = {};
         VM_CUDA(cudaMemcpyAsync(cells, d_cells, sizeof(cells), cudaMemcpyDeviceToHost, s));
         VM_CUDA(cudaStreamSynchronize(s));
-        if (cells[2] != 0) return fail(VM_ERR_DEVICE_ABORT, "a kernel gave up on a bounded loop (BSP deeper than 128 levels)");
+        if (cells[4 + ABORT_BSP_DEPTH] != 0) return fail(VM_ERR_DEVICE_ABORT, "a kernel gave up on a bounded loop (BSP deeper than 128 levels)");
         if (n_points != nullptr) *n_points = cells[1];
     }
     catch (const CudaFailure& f) {
@@ -1345,8 +1637,8 @@ vm_status vm_timer_stop(vm_engine* e, float* milliseconds) {
         VM_CUDA(cudaSetDevice(e->device));
         // lane 0 waits for the other lanes, then stamps the end
         for (int l = 1; l < MAX_LANES; ++l) {
-            VM_CUDA(cudaEventRecord(e->lanes[l].ev_staged, e->lanes[l].stream));
-            VM_CUDA(cudaStreamWaitEvent(e->lanes[0].stream, e->lanes[l].ev_staged, 0));
+            VM_CUDA(cudaEventRecord(e->lanes[l].ev_fork, e->lanes[l].stream));
+            VM_CUDA(cudaStreamWaitEvent(e->lanes[0].stream, e->lanes[l].ev_fork, 0));
         }
         VM_CUDA(cudaEventRecord(e->ev_timer_stop, e->lanes[0].stream));
         VM_CUDA(cudaEventSynchronize(e->ev_timer_stop));

@@ -141,36 +141,47 @@ namespace host {
         return true;
     }
 
-    // cpp/visualmesh/mesh.hpp:265-349: the four screen-edge cones (planes for a rectilinear lens) in world space
-    inline bool screen_edges(const float* Hoc, const vm_lens& lens, std::array<Cone, 4>& edges) {
-        const m3 Roc{{v3{{Hoc[0], Hoc[1], Hoc[2]}}, v3{{Hoc[4], Hoc[5], Hoc[6]}}, v3{{Hoc[8], Hoc[9], Hoc[10]}}}};
+    // cpp/visualmesh/mesh.hpp:265-349: the four screen-edge cones (planes for a rectilinear lens) in world space. The rays through
+    // the image corners and edge centres depend on the lens alone: frames of one camera share them.
+    struct EdgeRays {
+        std::array<v3, 4> corners;
+        std::array<v3, 4> mids;
+    };
+    inline bool edge_rays(const vm_lens& lens, EdgeRays& rays) {
         const v2 dims{{float(lens.dimensions[0]) - 1.0f, float(lens.dimensions[1]) - 1.0f}};
         const std::array<v2, 4> corners{{v2{{1.0f, 1.0f}}, v2{{dims[0], 1.0f}}, v2{{dims[0], dims[1]}}, v2{{1.0f, dims[1]}}}};
+        for (int i = 0; i < 4; ++i)
+            if (!unproject(corners[i], lens, rays.corners[i])) return false;
+        if (lens.projection == VM_RECTILINEAR) return true;
+        const v2 centre{{dims[0] * 0.5f + lens.centre[0], dims[1] * 0.5f + lens.centre[1]}};
+        const std::array<v2, 4> mids{{v2{{centre[0], 1.0f}}, v2{{dims[0], centre[1]}}, v2{{centre[0], dims[1]}}, v2{{1.0f, centre[1]}}}};
+        for (int i = 0; i < 4; ++i)
+            if (!unproject(mids[i], lens, rays.mids[i])) return false;
+        return true;
+    }
+    inline void screen_edges(const float* Hoc, const vm_lens& lens, const EdgeRays& rays, std::array<Cone, 4>& edges) {
+        const m3 Roc{{v3{{Hoc[0], Hoc[1], Hoc[2]}}, v3{{Hoc[4], Hoc[5], Hoc[6]}}, v3{{Hoc[8], Hoc[9], Hoc[10]}}}};
         std::array<v3, 4> rNCo;
-        for (int i = 0; i < 4; ++i) {
-            v3 cam;
-            if (!unproject(corners[i], lens, cam)) return false;
-            rNCo[i] = mul(Roc, cam);
-        }
+        for (int i = 0; i < 4; ++i) rNCo[i] = mul(Roc, rays.corners[i]);
         if (lens.projection == VM_RECTILINEAR) {
             for (int i = 0; i < 4; ++i) {
                 edges[i].axis  = normalise(cross(rNCo[(i + 1) & 3], rNCo[i]));
                 edges[i].cos_t = 0.0f;
                 edges[i].sin_t = 1.0f;
             }
-            return true;
+            return;
         }
-        const v2 centre{{dims[0] * 0.5f + lens.centre[0], dims[1] * 0.5f + lens.centre[1]}};
-        const std::array<v2, 4> mids{{v2{{centre[0], 1.0f}}, v2{{dims[0], centre[1]}}, v2{{centre[0], dims[1]}}, v2{{1.0f, centre[1]}}}};
         for (int i = 0; i < 4; ++i) {
-            v3 cam;
-            if (!unproject(mids[i], lens, cam)) return false;
-            const v3 rECo  = mul(Roc, cam);
-            const auto c   = cone_from_points(rNCo[(i + 1) & 3], rECo, rNCo[i]);
+            const auto c   = cone_from_points(rNCo[(i + 1) & 3], mul(Roc, rays.mids[i]), rNCo[i]);
             edges[i].axis  = c.first;
             edges[i].cos_t = c.second;
             edges[i].sin_t = std::sqrt(1.0f - c.second * c.second);
         }
+    }
+    inline bool screen_edges(const float* Hoc, const vm_lens& lens, std::array<Cone, 4>& edges) {
+        EdgeRays rays;
+        if (!edge_rays(lens, rays)) return false;
+        screen_edges(Hoc, lens, rays, edges);
         return true;
     }
 

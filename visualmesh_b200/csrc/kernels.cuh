@@ -3,7 +3,7 @@
 // A chunk is a run of frames of one batch processed by one set of launches. Grids are two-dimensional:
 // blockIdx.y is the frame within the chunk, blockIdx.x walks that frame's candidates (or rows). Blocks past the end of
 // their frame exit at once, so no launch needs a count that only the device knows and the host never waits in the
-// middle of a chunk. No kernel waits on another block: compaction is count -> scan -> scatter in three launches.
+// middle of a chunk. No kernel waits on another block: compaction is count -> scatter in two launches.
 //
 // Row spaces: points of frame f start at offsets[f] in the batch-wide result arrays; rows (points + one off-screen
 // row per frame) start at offsets[f] + f. Feature buffers are chunk-local: rows start at
@@ -13,6 +13,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "conv_args.hpp"
 #include "device_math.cuh"
 #include "tile_plan.cuh"
 
@@ -21,6 +22,18 @@ namespace vm {
 constexpr int SELECT_THREADS = 256;
 constexpr int ROW_THREADS    = 256;
 constexpr int SCATTER_UNITS  = 4;    // runs of SELECT_THREADS candidates per block of k_scatter
+constexpr int GROUP_BLOCKS   = 64;   // blocks of k_select whose counts are also summed as a group (a multiple of SCATTER_UNITS)
+constexpr int EXPORT_THREADS = 512;
+
+// Where a chunk's results go when they are wanted on the host: pinned memory that the device writes directly. It heads the
+// chunk's staging block, so that a recorded graph of the chunk's kernels serves results buffers that change from call to call.
+struct alignas(16) ChunkHeader {
+    float2* px;
+    int32_t* gi;
+    int32_t* nb;
+    float* cls;
+    int32_t* offsets;  // every chunk: the batch's offsets array in pinned memory
+};
 constexpr int SAMPLE_ROWS    = 2;    // points per thread of k_sample
 
 enum : uint8_t { BSP_DESCEND = 0, BSP_INSIDE = 1, BSP_OUTSIDE = 2 };
@@ -71,14 +84,16 @@ __global__ void __launch_bounds__(SELECT_THREADS) k_bsp_state(const FrameParams*
 // node of the concatenated ranges. With device lookup every node is a candidate and the thread first walks the BSP
 // from the root: an INSIDE ancestor selects the node, an OUTSIDE one drops it, a leaf tests the node itself
 // (cpp/visualmesh/mesh.hpp:559-583: inside the field of view and loosely on screen). Selected nodes then take the
-// engine's strict on-screen test. Writes the pixel and node id (-1 = dropped) per candidate and the number kept per
-// block.
+// engine's strict on-screen test. Writes the pixel and node id (-1 = dropped) per candidate, the number kept per block and,
+// added up in group_counts (which starts at zero), per group of GROUP_BLOCKS blocks.
 __global__ void __launch_bounds__(SELECT_THREADS) k_select(const FrameParams* __restrict__ frames,
                                                            const uint8_t* __restrict__ state,
                                                            float2* __restrict__ cand_px,
                                                            int32_t* __restrict__ cand_node,
                                                            int32_t* __restrict__ block_counts,
-                                                           int32_t* __restrict__ abort_flag) {
+                                                           int32_t* __restrict__ group_counts,
+                                                           int32_t n_groups,
+                                                           int32_t* __restrict__ abort_flags) {
     const FrameParams& p = frames[blockIdx.y];
     const int c          = blockIdx.x * SELECT_THREADS + threadIdx.x;
     bool keep            = false;
@@ -119,7 +134,7 @@ __global__ void __launch_bounds__(SELECT_THREADS) k_select(const FrameParams* __
             }
             if (steps == 128) {
                 // a tree deeper than any the builder makes: give up on this node and report it
-                atomicExch(abort_flag, 1);
+                raise_flag(abort_flags, ABORT_BSP_DEPTH);
                 selected = false;
             }
         }
@@ -135,67 +150,9 @@ __global__ void __launch_bounds__(SELECT_THREADS) k_select(const FrameParams* __
         cand_node[p.cand_off + c] = keep ? g : -1;
     }
     const int n = __syncthreads_count(keep);
-    if (threadIdx.x == 0) block_counts[blockIdx.y * gridDim.x + blockIdx.x] = n;
-}
-
-// ---- scan of the per-block counts --------------------------------------------------------------------------------
-// One block. Turns block_counts into exclusive block offsets relative to the chunk's first point and extends the
-// batch-wide offsets array: offsets[f0 + y + 1] for every frame y of the chunk, continuing from offsets[f0].
-// Each warp owns a contiguous run of the counts and walks it 32 at a time, so every load and store is one coalesced
-// line; the first pass sums the runs, the second redoes each run as a shuffle scan carried from line to line.
-__global__ void __launch_bounds__(1024) k_scan(int32_t* __restrict__ block_counts,
-                                               int32_t n_blocks,
-                                               int32_t blocks_per_frame,
-                                               int32_t n_frames,
-                                               int32_t* __restrict__ offsets,
-                                               int32_t f0) {
-    __shared__ int32_t warp_base[33];
-    const int t     = threadIdx.x;
-    const int lane  = t & 31;
-    const int warp  = t >> 5;
-    const int lines = (n_blocks + 1023) / 1024;  // 32-count lines per warp
-    const int begin = min(warp * lines * 32, n_blocks);
-    const int end   = min(begin + lines * 32, n_blocks);
-    int sum         = 0;
-#pragma unroll 4
-    for (int i = begin + lane; i < end; i += 32) sum += block_counts[i];
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
-    if (lane == 0) warp_base[warp + 1] = sum;
-    __syncthreads();
-    if (warp == 0) {
-        // exclusive scan of the 32 run totals; warp_base[32] keeps the grand total
-        int v = warp_base[lane + 1];
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, v, d);
-            if (lane >= d) v += u;
-        }
-        warp_base[lane + 1] = v;
-        if (lane == 0) warp_base[0] = 0;
-    }
-    __syncthreads();
-    const int total = warp_base[32];
-    int run         = warp_base[warp];
-    for (int i0 = begin; i0 < end; i0 += 32) {
-        const int i = i0 + lane;
-        const int c = (i < end) ? block_counts[i] : 0;
-        int v       = c;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, v, d);
-            if (lane >= d) v += u;
-        }
-        if (i < end) block_counts[i] = run + v - c;
-        run += __shfl_sync(0xffffffffu, v, 31);
-    }
-    __syncthreads();
-    // frame y starts at block y * blocks_per_frame
-    const int base = offsets[f0];
-    for (int y = t; y < n_frames; y += 1024) {
-        const int first = (y + 1) * blocks_per_frame;
-        const int upto  = (first < n_blocks) ? block_counts[first] : total;
-        offsets[f0 + y + 1] = base + upto;
+    if (threadIdx.x == 0) {
+        block_counts[blockIdx.y * gridDim.x + blockIdx.x] = n;
+        if (n > 0) atomicAdd(group_counts + blockIdx.y * n_groups + blockIdx.x / GROUP_BLOCKS, n);
     }
 }
 
@@ -203,56 +160,109 @@ __global__ void __launch_bounds__(1024) k_scan(int32_t* __restrict__ block_count
 // Kept candidates, in candidate order, become the frame's points: global_indices ascending
 // (cpp/visualmesh/engine/cpu/engine.hpp:110-120). Also fills the node -> local index table that k_remap reads in
 // place of the reference's r_lookup (engine.hpp:128-131); with device lookup every entry is written, with host
-// ranges the table was cleared to -1 beforehand.
+// ranges only the candidates' (k_remap then checks what it reads).
+// A block adds up what comes before it itself: the groups of the frames before, the groups of its own frame, the blocks
+// of its own group. That is a few hundred counts that sit in L2 (64 frames x 8 groups for a mesh of 121 k nodes, 8 x 106
+// for 1.7 M), read side by side, where a scan kernel of one block cost a launch and 6 to 9 us of every call.
+// The batch-wide offsets array continues from offsets[f0], which the chunk before has written (0 for the first chunk).
 template <int UNITS>
 __global__ void __launch_bounds__(SELECT_THREADS) k_scatter(const FrameParams* __restrict__ frames,
+                                                            const ChunkHeader* __restrict__ header,
                                                             const float2* __restrict__ cand_px,
                                                             const int32_t* __restrict__ cand_node,
-                                                            const int32_t* __restrict__ block_offsets,
+                                                            const int32_t* __restrict__ block_counts,
+                                                            const int32_t* __restrict__ group_counts,
                                                             int32_t blocks_per_frame,
-                                                            const int32_t* __restrict__ offsets,
+                                                            int32_t n_groups,
+                                                            int32_t* offsets,
                                                             int32_t f0,
                                                             float2* __restrict__ out_px,
                                                             int32_t* __restrict__ out_gi,
                                                             int32_t* __restrict__ node_rank) {
-    // a block compacts UNITS runs of SELECT_THREADS candidates (the unit k_select counted and k_scan scanned); their
-    // loads are issued together
-    __shared__ int32_t warp_counts[UNITS][SELECT_THREADS / 32];
+    static_assert(GROUP_BLOCKS % UNITS == 0, "a block's runs lie in one group");
+    constexpr int WARPS = SELECT_THREADS / 32;
+    // a block compacts UNITS runs of SELECT_THREADS candidates (the unit k_select counted); their loads are issued together
+    __shared__ int32_t warp_counts[UNITS][WARPS];
+    __shared__ int32_t sums[3][WARPS];
     const FrameParams& p = frames[blockIdx.y];
     const int lane       = threadIdx.x & 31;
     const int warp       = threadIdx.x >> 5;
     const int frame      = f0 + blockIdx.y;
+    const int unit0      = blockIdx.x * UNITS;
     int c[UNITS], g[UNITS];
     unsigned mask[UNITS];
 #pragma unroll
     for (int u = 0; u < UNITS; ++u) {
-        c[u] = (blockIdx.x * UNITS + u) * SELECT_THREADS + threadIdx.x;
+        c[u] = (unit0 + u) * SELECT_THREADS + threadIdx.x;
         g[u] = (c[u] < p.n_candidates) ? cand_node[p.cand_off + c[u]] : -1;
+    }
+    // points of the frames before, points of this frame before this block, and (first block only) points of this frame
+    int before_frame = 0, before_block = 0, of_frame = 0;
+    const int own_first = blockIdx.y * n_groups;
+    for (int i = threadIdx.x; i < own_first; i += SELECT_THREADS) before_frame += group_counts[i];
+    const int group = unit0 / GROUP_BLOCKS;
+    for (int i = threadIdx.x; i < group; i += SELECT_THREADS) before_block += group_counts[own_first + i];
+    if (static_cast<int>(threadIdx.x) < unit0 - group * GROUP_BLOCKS) {
+        before_block += block_counts[blockIdx.y * blocks_per_frame + group * GROUP_BLOCKS + threadIdx.x];
+    }
+    if (blockIdx.x == 0) {
+        for (int i = threadIdx.x; i < n_groups; i += SELECT_THREADS) of_frame += group_counts[own_first + i];
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        before_frame += __shfl_xor_sync(0xffffffffu, before_frame, d);
+        before_block += __shfl_xor_sync(0xffffffffu, before_block, d);
+        of_frame += __shfl_xor_sync(0xffffffffu, of_frame, d);
+    }
+    if (lane == 0) {
+        sums[0][warp] = before_frame;
+        sums[1][warp] = before_block;
+        sums[2][warp] = of_frame;
     }
 #pragma unroll
     for (int u = 0; u < UNITS; ++u) {
         mask[u] = __ballot_sync(0xffffffffu, g[u] >= 0);
         if (lane == 0) warp_counts[u][warp] = __popc(mask[u]);
     }
+    const int chunk_base = (f0 == 0) ? 0 : *static_cast<volatile int32_t*>(offsets + f0);
     __syncthreads();
-    const int chunk_base = offsets[f0];
-    const int frame_base = offsets[frame];
+    int frame_base = chunk_base, in_frame = 0;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+        frame_base += sums[0][w];
+        in_frame += sums[1][w];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        int total = frame_base;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) total += sums[2][w];
+        offsets[frame + 1]         = total;
+        header->offsets[frame + 1] = total;
+        if (frame == 0) {
+            offsets[0]         = 0;
+            header->offsets[0] = 0;
+        }
+    }
 #pragma unroll
     for (int u = 0; u < UNITS; ++u) {
-        const int unit = blockIdx.x * UNITS + u;
-        if (unit >= blocks_per_frame) break;
-        int before = 0;
-        for (int w = 0; w < warp; ++w) before += warp_counts[u][w];
-        const int in_chunk = block_offsets[blockIdx.y * blocks_per_frame + unit] + before + __popc(mask[u] & ((1u << lane) - 1u));
+        if (unit0 + u >= blocks_per_frame) break;
+        int before = in_frame, of_unit = 0;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+            if (w < warp) before += warp_counts[u][w];
+            of_unit += warp_counts[u][w];
+        }
         if (g[u] >= 0) {
-            const int o  = chunk_base + in_chunk;
+            const int k  = before + __popc(mask[u] & ((1u << lane) - 1u));
+            const int o  = frame_base + k;
             out_px[o]    = cand_px[p.cand_off + c[u]];
             out_gi[o]    = g[u];
-            node_rank[p.node_off + g[u]] = o - frame_base;
+            node_rank[p.node_off + g[u]] = k;
         }
         else if (c[u] < p.n_candidates && p.ranges == nullptr) {
             node_rank[p.node_off + c[u]] = -1;
         }
+        in_frame += of_unit;
     }
 }
 
@@ -291,7 +301,11 @@ __global__ void __launch_bounds__(ROW_THREADS) k_remap(const FrameParams* __rest
                 const int t = __ldg(nbrs + j);
                 if (t >= 0 && t < p.n_nodes) {
                     const int k = node_rank[p.node_off + t];
-                    v[j]        = (k < 0) ? n : k;
+                    bool known  = k >= 0;
+                    // with host ranges the table holds what earlier frames left for the nodes that were no candidates now: an
+                    // entry counts only if its point is this node
+                    if (p.ranges != nullptr) known = known && k < n && out_gi[start + k] == t;
+                    v[j] = known ? k : n;
                 }
             }
         }
@@ -339,6 +353,50 @@ __global__ void __launch_bounds__(ROW_THREADS) k_sample(const FrameParams* __res
         }
         features[row0 + i] = v;
     }
+}
+
+// ---- results to the host -----------------------------------------------------------------------------------------
+// Writes a chunk's results into pinned host memory. The device knows how many there are, so the copy needs no count on the host
+// and no wait for one in the middle of a call; the bus takes 64 KB in 3 us more than a copy engine would and 5 MB in 10 us more
+// (112 us against 102). WHICH: 0 = pixel coordinates, node indices and neighbourhood; 1 = classifications.
+__device__ __forceinline__ void export_words(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, size_t begin, size_t end) {
+    // 16-byte pieces between the first and the last whole one (both arrays start on 256-byte boundaries), words at the ends
+    const size_t first = (begin + 3) / 4, last = end / 4;
+    const size_t t = static_cast<size_t>(blockIdx.x) * EXPORT_THREADS + threadIdx.x, step = static_cast<size_t>(gridDim.x) * EXPORT_THREADS;
+    if (first >= last) {
+        if (t < end - begin) dst[begin + t] = src[begin + t];
+        return;
+    }
+    if (t < first * 4 - begin) dst[begin + t] = src[begin + t];
+    if (t < end - last * 4) dst[last * 4 + t] = src[last * 4 + t];
+    const uint4* s4 = reinterpret_cast<const uint4*>(src);
+    uint4* d4       = reinterpret_cast<uint4*>(dst);
+    size_t i        = first + t;
+    for (; i + 3 * step < last; i += 4 * step) {
+        const uint4 a = s4[i], b = s4[i + step], c = s4[i + 2 * step], d = s4[i + 3 * step];
+        d4[i]            = a;
+        d4[i + step]     = b;
+        d4[i + 2 * step] = c;
+        d4[i + 3 * step] = d;
+    }
+    for (; i < last; i += step) d4[i] = s4[i];
+}
+template <int WHICH>
+__global__ void __launch_bounds__(EXPORT_THREADS) k_export(const ChunkHeader* __restrict__ header,
+                                                           const int32_t* __restrict__ offsets,
+                                                           int32_t f0,
+                                                           int32_t f1,
+                                                           int32_t width,  // neighbours or classes
+                                                           const float2* __restrict__ px,
+                                                           const int32_t* __restrict__ gi,
+                                                           const void* __restrict__ rows) {
+    const size_t p0 = offsets[f0], p1 = offsets[f1];
+    if (WHICH == 0) {
+        export_words(reinterpret_cast<uint32_t*>(header->px), reinterpret_cast<const uint32_t*>(px), 2 * p0, 2 * p1);
+        export_words(reinterpret_cast<uint32_t*>(header->gi), reinterpret_cast<const uint32_t*>(gi), p0, p1);
+    }
+    uint32_t* dst = WHICH == 0 ? reinterpret_cast<uint32_t*>(header->nb) : reinterpret_cast<uint32_t*>(header->cls);
+    export_words(dst, static_cast<const uint32_t*>(rows), (p0 + f0) * width, (p1 + f1) * width);
 }
 
 // The same sampler on a flat list of pixel coordinates (stand-alone stage for unit parity tests).

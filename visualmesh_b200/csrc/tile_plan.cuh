@@ -51,7 +51,7 @@ namespace st {
         if (tid == 0) tiles_before = 0;
         for (int i = tid; i < HASH_SIZE; i += ST) keys[i] = -1;
         __syncthreads();
-        // super-tiles of the frames before this one (at most 64 frames per launch)
+        // super-tiles of the frames before this one (at most ST frames per launch)
         if (tid < f) {
             const int r = offsets[f0 + tid + 1] - offsets[f0 + tid] + 1;
             atomicAdd(&tiles_before, (r + ST - 1) / ST);
