@@ -166,6 +166,29 @@ VM_API vm_status vm_classify(vm_engine* engine,
                       uint32_t format,
                       vm_batch_result* out);
 
+/* The reference's calls with their lookup (cpp/visualmesh/engine/opencl/engine.hpp:581): Mesh::lookup runs on the host inside the
+ * call, while the image is on its way to the device. lookup: the host tables that `mesh` was uploaded from (vm_hostmesh, below);
+ * image NULL: projection only. Otherwise vm_classify and vm_project. */
+struct vm_hostmesh;
+VM_API vm_status vm_call(vm_engine* engine,
+                         const vm_mesh* mesh,
+                         const struct vm_hostmesh* lookup,
+                         const float Hoc[16],
+                         const vm_lens* lens,
+                         const void* image,
+                         uint32_t format,
+                         vm_batch_result* out);
+
+/* No counterpart in the reference: the reference's results are the caller's own, the arrays of a vm_batch_result belong to the
+ * engine and are overwritten by its next call. vm_results_keep hands the host arrays of the engine's last call over to the caller
+ * instead of having them copied: they stay valid until vm_results_release, whatever becomes of the engine, and then serve it again.
+ * At most VM_MAX_KEPT_RESULTS are kept per engine; one more fails with VM_ERR_OUT_OF_MEMORY and leaves the results where they
+ * are. vm_results_release may be called from any thread. */
+#define VM_MAX_KEPT_RESULTS 4
+typedef struct vm_results vm_results;
+VM_API vm_status vm_results_keep(vm_engine* engine, vm_results** kept);
+VM_API void vm_results_release(vm_results* kept);
+
 /* No counterpart in the reference.
  * Projection of one frame (operator()(mesh, Hoc, lens) with the lookup on the device) for callers that must not
  * allocate device memory while they run: a camera thread inside a fixed-period control loop, where the driver lock and

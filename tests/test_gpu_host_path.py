@@ -98,3 +98,23 @@ def test_batches_left_on_the_device_and_copied_to_the_host_agree(n_frames):
                 assert np.array_equal(out.neighbourhood, nb[p0 + f:p1 + f + 1])
                 assert np.array_equal(G.bits(out.classifications), G.bits(cls[p0 + f:p1 + f + 1]))
     engine.close()
+
+
+def test_results_of_a_call_are_the_callers_own():
+    """Results kept over later calls (more of them than the engine hands over without a copy), over the engine's end, and given
+    back in another order."""
+    case = G.Case("ring6_equisolid_rgba")
+    mesh = Mesh.from_arrays(case.rays, case.nbrs, case.bsp)
+    engine = Engine(case.network)
+    frames = [case.frames[i] for i in (0, 1, 0, 1, 1, 0, 2)]
+    kept = [engine(mesh, fr["Hoc"], case.lens, fr["image"], case.format, fr["ranges"]) for fr in frames]
+    del kept[2]
+    kept.insert(2, engine(mesh, frames[2]["Hoc"], case.lens, frames[2]["image"], case.format, "device"))
+    columns = kept[1].pixel_coordinates[:, 0]
+    engine.close()
+    for out, fr in zip(kept, frames):
+        assert np.array_equal(out.global_indices, fr["global_indices"]) and np.array_equal(out.neighbourhood, fr["neighbourhood"])
+        assert out.pixel_coordinates.shape == fr["pixel_coordinates"].shape and np.abs(out.classifications - fr["classifications"]).max(initial=0.0) < 1e-4
+    want = frames[1]["pixel_coordinates"][:, 0].copy()
+    kept.clear()
+    assert np.array_equal(columns, want)

@@ -79,6 +79,10 @@ SYMBOLS = {
                              C.POINTER(vm_batch_result)]),
     "vm_classify": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p, C.POINTER(vm_lens), C.c_void_p,
                               C.c_uint32, C.POINTER(vm_batch_result)]),
+    "vm_call": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(vm_lens), C.c_void_p, C.c_uint32,
+                          C.POINTER(vm_batch_result)]),
+    "vm_results_keep": (C.c_int, [C.c_void_p, C.POINTER(C.c_void_p)]),
+    "vm_results_release": (None, [C.c_void_p]),
     "vm_project_static": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(vm_lens), C.c_void_p, C.c_void_p,
                                     C.c_void_p, C.c_void_p, C.POINTER(C.c_int32)]),
     "vm_sample": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p, C.c_int32, C.c_int32, C.c_uint32, C.c_void_p]),
@@ -121,6 +125,22 @@ def load():
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+_native = None
+
+
+def native():
+    """The extension module that marshals frames and results (csrc/native.cpp), linked against the same library."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise RuntimeError("visualmesh_b200._native cannot be imported: build it with `python -m visualmesh_b200.build`") from e
+        _native = module
+    return _native
 
 
 class VisualMeshError(RuntimeError):

@@ -1,4 +1,5 @@
-"""Builds libvmcuda.so (the CUDA engine and its C ABI) in-tree for sm_100a with nvcc.
+"""Builds libvmcuda.so (the CUDA engine and its C ABI) in-tree for sm_100a with nvcc, and the extension module _native (marshalling
+for engine.py) against it with g++.
 
     python -m visualmesh_b200.build            # rebuild what is older than its sources
     python -m visualmesh_b200.build --force [-v]
@@ -11,22 +12,25 @@ the way the reference CPU engine does. The graph-convolution kernels call fmaf()
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "_build")
 LIB = os.path.join(HERE, "libvmcuda.so")
+NATIVE = os.path.join(HERE, "_native" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 ABI_HEADER = os.path.join("..", "..", "include", "vmcuda.h")
 # translation unit -> headers it includes (directly or not)
 UNITS = {
-    "engine.cu": ["kernels.cuh", "tile_plan.cuh", "device_math.cuh", "host_math.hpp", "libm_tables.hpp", "upload.hpp", "conv_dispatch.hpp", "conv_args.hpp",
+    "engine.cu": ["kernels.cuh", "tile_plan.cuh", "device_math.cuh", "host_math.hpp", "libm_tables.hpp", "upload.hpp", "hostmesh.hpp", "conv_dispatch.hpp", "conv_args.hpp",
                   ABI_HEADER],
     "conv_ffma.cu": ["conv_ffma.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
     "conv_tc.cu": ["conv_tc.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
     "conv_staged.cu": ["conv_staged.cuh", "tile_plan.cuh", "conv_tc.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
-    "hostmesh.cpp": ["host_math.hpp", ABI_HEADER],
+    "hostmesh.cpp": ["host_math.hpp", "hostmesh.hpp", ABI_HEADER],
 }
+NATIVE_SOURCES = ["native.cpp", ABI_HEADER]
 
 
 def _nvcc():
@@ -51,6 +55,10 @@ def _stale(unit):
 
 def needs_build():
     """The library is missing or older than one of its sources (object files may be absent: they do not travel)."""
+    return _library_stale() or _native_stale()
+
+
+def _library_stale():
     if not os.path.exists(LIB):
         return True
     t = os.path.getmtime(LIB)
@@ -58,9 +66,25 @@ def needs_build():
     return any(os.path.getmtime(os.path.join(CSRC, f)) > t for f in files if os.path.exists(os.path.join(CSRC, f)))
 
 
+def _native_stale():
+    if not os.path.exists(NATIVE):
+        return True
+    t = os.path.getmtime(NATIVE)
+    return any(os.path.getmtime(os.path.join(CSRC, f)) > t for f in NATIVE_SOURCES if os.path.exists(os.path.join(CSRC, f)))
+
+
 def build(force=False, verbose=False):
-    if not force and not needs_build():
-        return LIB
+    if force or _library_stale():
+        _build_library(force, verbose)
+    if force or _native_stale():
+        import numpy
+        subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-I", sysconfig.get_paths()["include"],
+                        "-I", numpy.get_include(), os.path.join(CSRC, "native.cpp"), "-o", NATIVE, LIB, "-Wl,-rpath,$ORIGIN"],
+                       check=True, cwd=CSRC)
+    return LIB
+
+
+def _build_library(force, verbose):
     os.makedirs(OBJ, exist_ok=True)
     flags = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17", "-fmad=false",
              "-Xcompiler", "-fPIC,-ffp-contract=off,-fvisibility=hidden"]
@@ -79,9 +103,8 @@ def build(force=False, verbose=False):
                 sys.stderr.write(f"---- {unit}\n{out.stdout}{out.stderr}")
             if out.returncode != 0:
                 raise subprocess.CalledProcessError(out.returncode, f"nvcc -c {unit}")
-    subprocess.run([_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", LIB] + [_obj(u) for u in UNITS],
+    subprocess.run([_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xlinker", "-soname=libvmcuda.so", "-o", LIB] + [_obj(u) for u in UNITS],
                    check=True, cwd=CSRC)
-    return LIB
 
 
 if __name__ == "__main__":

@@ -22,6 +22,7 @@
 
 #include "../../include/vmcuda.h"
 #include "host_math.hpp"
+#include "hostmesh.hpp"
 #include "kernels.cuh"
 #include "conv_dispatch.hpp"
 #include "upload.hpp"
@@ -139,6 +140,37 @@ struct Lane {
     DeviceArray<int32_t> d_halo_count;
 };
 
+// One set of result arrays in pinned host memory. An engine writes its results into the set it holds; a caller may keep the set
+// of the last call (vm_results_keep), and the engine takes another one for the next.
+struct Results {
+    PinnedArray<int32_t> offsets;
+    PinnedArray<float2> px;
+    PinnedArray<int32_t> gi;
+    PinnedArray<int32_t> nb;
+    PinnedArray<float> cls;
+    ~Results() {
+        offsets.release();
+        px.release();
+        gi.release();
+        nb.release();
+        cls.release();
+    }
+};
+// The sets of an engine that are not in its hands: kept by callers, or given back and free. Outlives the engine while some are kept,
+// and is given back to from any thread.
+constexpr int MAX_KEPT_RESULTS = 4;
+static_assert(MAX_KEPT_RESULTS == VM_MAX_KEPT_RESULTS, "as the header says");
+struct ResultPool {
+    std::mutex mutex;
+    std::vector<std::unique_ptr<Results>> free;
+    int kept    = 0;
+    bool closed = false;  // the engine is gone: sets that come back are freed
+};
+struct KeptResults {
+    std::shared_ptr<ResultPool> pool;
+    std::unique_ptr<Results> results;
+};
+
 struct StageTimer {
     const char* name;
     cudaEvent_t start, stop;
@@ -189,11 +221,9 @@ struct vm_engine {
     vm::DeviceArray<int32_t> d_gi;
     vm::DeviceArray<int32_t> d_nb;
     vm::DeviceArray<float> d_cls;
-    vm::PinnedArray<int32_t> h_offsets;
-    vm::PinnedArray<float2> h_px;
-    vm::PinnedArray<int32_t> h_gi;
-    vm::PinnedArray<int32_t> h_nb;
-    vm::PinnedArray<float> h_cls;
+    std::unique_ptr<vm::Results> host;  // ... and where they arrive on the host
+    std::shared_ptr<vm::ResultPool> pool = std::make_shared<vm::ResultPool>();
+    std::vector<std::pair<int, int>> looked_up;  // ranges of the frame whose lookup runs inside the call
     int32_t* flags = nullptr;  // abort flags, pinned host memory that the kernels raise them in
     std::vector<vm_mesh*> meshes;
     // recorded graphs
@@ -416,6 +446,8 @@ static int64_t frame_candidates(const vm_frame& fr) {
     return n;
 }
 
+static_assert(sizeof(std::pair<int, int>) == 2 * sizeof(int32_t), "range pairs as the frames hold them");
+
 static size_t aligned(size_t n) {
     return (n + 255) & ~size_t(255);
 }
@@ -586,7 +618,7 @@ static Chunk stage_chunk(vm_engine* e, Lane& lane, const vm_frame* frames, int f
 
     uint8_t* h = lane.h_staging.p;
     uint8_t* d = lane.d_staging.p;
-    *reinterpret_cast<ChunkHeader*>(h) = ChunkHeader{e->h_px.p, e->h_gi.p, e->h_nb.p, e->h_cls.p, e->h_offsets.p};
+    *reinterpret_cast<ChunkHeader*>(h) = ChunkHeader{e->host->px.p, e->host->gi.p, e->host->nb.p, e->host->cls.p, e->host->offsets.p};
     int32_t* pairs  = reinterpret_cast<int32_t*>(h + ranges_at);
     int32_t* starts = pairs + 2 * n_slots;
     auto on_gpu     = [&](const void* p) { return d + (static_cast<const uint8_t*>(p) - h); };
@@ -860,18 +892,19 @@ static Chunk enqueue_chunk(vm_engine* e, Lane& lane, Lane* prev, bool after_prev
 static void copy_results(vm_engine* e, Lane& lane, const Chunk& c) {
     if (!c.copied) return;
     VM_CUDA(cudaEventSynchronize(lane.ev_offsets));
-    const int32_t* off = e->h_offsets.p;
+    Results& to = *e->host;
+    const int32_t* off = to.offsets.p;
     const size_t p0 = off[c.f0], p1 = off[c.f1];
     const size_t r0 = p0 + c.f0, r1 = p1 + c.f1;
     const size_t N = c.n_neighbours, C = e->n_classes;
     cudaStream_t beside = e->timing ? lane.stream : lane.side;
     VM_CUDA(cudaStreamWaitEvent(beside, lane.ev_offsets, 0));
     if (p1 > p0) {
-        VM_CUDA(cudaMemcpyAsync(e->h_px.p + p0, e->d_px.p + p0, sizeof(float2) * (p1 - p0), cudaMemcpyDeviceToHost, beside));
-        VM_CUDA(cudaMemcpyAsync(e->h_gi.p + p0, e->d_gi.p + p0, sizeof(int32_t) * (p1 - p0), cudaMemcpyDeviceToHost, beside));
+        VM_CUDA(cudaMemcpyAsync(to.px.p + p0, e->d_px.p + p0, sizeof(float2) * (p1 - p0), cudaMemcpyDeviceToHost, beside));
+        VM_CUDA(cudaMemcpyAsync(to.gi.p + p0, e->d_gi.p + p0, sizeof(int32_t) * (p1 - p0), cudaMemcpyDeviceToHost, beside));
     }
-    VM_CUDA(cudaMemcpyAsync(e->h_nb.p + r0 * N, e->d_nb.p + r0 * N, sizeof(int32_t) * (r1 - r0) * N, cudaMemcpyDeviceToHost, beside));
-    if (c.classify) VM_CUDA(cudaMemcpyAsync(e->h_cls.p + r0 * C, e->d_cls.p + r0 * C, sizeof(float) * (r1 - r0) * C, cudaMemcpyDeviceToHost, lane.stream));
+    VM_CUDA(cudaMemcpyAsync(to.nb.p + r0 * N, e->d_nb.p + r0 * N, sizeof(int32_t) * (r1 - r0) * N, cudaMemcpyDeviceToHost, beside));
+    if (c.classify) VM_CUDA(cudaMemcpyAsync(to.cls.p + r0 * C, e->d_cls.p + r0 * C, sizeof(float) * (r1 - r0) * C, cudaMemcpyDeviceToHost, lane.stream));
     if (beside != lane.stream) {
         VM_CUDA(cudaEventRecord(lane.ev_join, beside));
         VM_CUDA(cudaStreamWaitEvent(lane.stream, lane.ev_join, 0));
@@ -879,7 +912,8 @@ static void copy_results(vm_engine* e, Lane& lane, const Chunk& c) {
     VM_CUDA(cudaEventRecord(lane.ev_done, lane.stream));
 }
 
-static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frames, uint32_t flags, vm_batch_result* out) {
+// lookup: host mesh tables of the one frame of the batch, whose ranges are looked up inside the call, beside its image's upload.
+static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frames, uint32_t flags, vm_batch_result* out, const vm_hostmesh* lookup = nullptr) {
     if (e == nullptr || out == nullptr || n_frames < 0 || (n_frames > 0 && frames == nullptr)) {
         return fail(VM_ERR_INVALID_ARGUMENT, "null engine, frames or result");
     }
@@ -909,7 +943,7 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
         }
         if (fr.lens.dimensions[0] <= 0 || fr.lens.dimensions[1] <= 0) return fail(VM_ERR_INVALID_ARGUMENT, "lens dimensions must be positive");
         if (fr.ranges == nullptr && fr.n_ranges != 0) return fail(VM_ERR_INVALID_ARGUMENT, "n_ranges without ranges");
-        if (fr.ranges == nullptr && fr.mesh->n_bsp == 0) return fail(VM_ERR_NO_BSP, "device lookup needs vm_mesh_set_bsp");
+        if (fr.ranges == nullptr && fr.mesh->n_bsp == 0 && lookup == nullptr) return fail(VM_ERR_NO_BSP, "device lookup needs vm_mesh_set_bsp");
         if (fr.n_ranges < 0) return fail(VM_ERR_INVALID_ARGUMENT, "negative n_ranges");
         for (int r = 0; r < fr.n_ranges; ++r) {
             if (fr.ranges[2 * r] < 0 || fr.ranges[2 * r + 1] > fr.mesh->n_nodes || fr.ranges[2 * r] > fr.ranges[2 * r + 1]) {
@@ -921,7 +955,7 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
             char code[5] = {char(fr.format & 0xFF), char(fr.format >> 8 & 0xFF), char(fr.format >> 16 & 0xFF), char(fr.format >> 24 & 0xFF), 0};
             return fail(VM_ERR_UNSUPPORTED_FORMAT, std::string("Unsupported image format ") + code);
         }
-        cand_all += frame_candidates(fr);
+        if (lookup == nullptr) cand_all += frame_candidates(fr);
     }
     if (classify && e->layers.front().cin != 4) return fail(VM_ERR_NETWORK_SHAPE, "first layer must take 4 channels");
     if (classify && e->layers.front().n_slots != N + 1) return fail(VM_ERR_NETWORK_SHAPE, "network was built for a different n_neighbours");
@@ -944,18 +978,45 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
         const bool to_host = (flags & VM_RESULTS_ON_DEVICE) == 0;
         const int n_lanes  = e->timing ? 1 : e->n_lanes;  // with the stages timed, one chunk after another
 
+        ImagePlan images;
+        std::unique_ptr<Upload> upload;
+        vm_frame looked_up;
+        if (lookup != nullptr) {
+            if (classify) {
+                images = plan_images(frames, 0, 1);
+                if (images.total > 0 && !images.small) upload = start_images(e, e->lanes[0], frames, 0, 1, images);
+            }
+            e->looked_up.clear();
+            if (!vm_hostmesh_ranges_(lookup, frames[0].Hoc, &frames[0].lens, e->looked_up)) throw UnsupportedLens{};
+            if (upload) upload->pump();
+            static const int32_t none[2] = {0, 0};
+            looked_up          = frames[0];
+            looked_up.ranges   = e->looked_up.empty() ? none : &e->looked_up.front().first;
+            looked_up.n_ranges = static_cast<int32_t>(e->looked_up.size());
+            frames             = &looked_up;
+            cand_all           = frame_candidates(looked_up);
+        }
+
         const size_t rows_all = static_cast<size_t>(cand_all) + n_frames;
         need(e, e->d_offsets, n_frames + 1);
         need(e, e->d_px, cand_all + 1);
         need(e, e->d_gi, cand_all + 1);
         need(e, e->d_nb, rows_all * N);
         if (classify) need(e, e->d_cls, rows_all * e->n_classes);
-        e->h_offsets.ensure(n_frames + 1);
+        if (!e->host) {
+            std::lock_guard<std::mutex> lock(e->pool->mutex);
+            if (!e->pool->free.empty()) {
+                e->host = std::move(e->pool->free.back());
+                e->pool->free.pop_back();
+            }
+        }
+        if (!e->host) e->host.reset(new Results());
+        e->host->offsets.ensure(n_frames + 1);
         if (to_host) {
-            e->h_px.ensure(cand_all + 1);
-            e->h_gi.ensure(cand_all + 1);
-            e->h_nb.ensure(rows_all * N);
-            if (classify) e->h_cls.ensure(rows_all * e->n_classes);
+            e->host->px.ensure(cand_all + 1);
+            e->host->gi.ensure(cand_all + 1);
+            e->host->nb.ensure(rows_all * N);
+            if (classify) e->host->cls.ensure(rows_all * e->n_classes);
         }
         for (int i = 0; i < ABORT_FLAGS; ++i) e->flags[i] = 0;
 
@@ -990,10 +1051,9 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
                 VM_CUDA(cudaEventSynchronize(lane.ev_done));
                 lane.busy = false;
             }
-            ImagePlan images;
-            std::unique_ptr<Upload> upload;
-            if (classify) {
+            if (classify && lookup == nullptr) {
                 images = plan_images(frames, f0, f1);
+                upload.reset();
                 if (images.total > 0 && !images.small) upload = start_images(e, lane, frames, f0, f1, images);
             }
             const Chunk current = enqueue_chunk(e, lane, prev, !host_images, frames, f0, f1, classify, to_host, f0 == 0 && f1 == n_frames, images, upload.get());
@@ -1019,7 +1079,7 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
             // a feature value beyond the range of the fp16 split: this engine goes back to the FFMA kernels for good and
             // the batch is computed again
             e->use_tc = false;
-            return run_batch(e, frames, n_frames, flags, out);
+            return run_batch(e, frames, n_frames, flags, out);  // the frames have their ranges by now
         }
 
         if (e->timing) {
@@ -1034,12 +1094,12 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
         out->n_neighbours = N;
         out->n_classes    = classify ? e->n_classes : 0;
         out->on_device    = to_host ? 0 : 1;
-        out->offsets      = e->h_offsets.p;
+        out->offsets      = e->host->offsets.p;
         if (to_host) {
-            out->pixel_coordinates = reinterpret_cast<const float*>(e->h_px.p);
-            out->global_indices    = e->h_gi.p;
-            out->neighbourhood     = e->h_nb.p;
-            out->classifications   = classify ? e->h_cls.p : nullptr;
+            out->pixel_coordinates = reinterpret_cast<const float*>(e->host->px.p);
+            out->global_indices    = e->host->gi.p;
+            out->neighbourhood     = e->host->nb.p;
+            out->classifications   = classify ? e->host->cls.p : nullptr;
         }
         else {
             out->pixel_coordinates = reinterpret_cast<const float*>(e->d_px.p);
@@ -1276,15 +1336,15 @@ void vm_engine_destroy(vm_engine* e) {
     }
     if (e->copy_stream) cudaStreamDestroy(e->copy_stream);
     e->d_offsets.release();
-    e->h_offsets.release();
     e->d_px.release();
     e->d_gi.release();
     e->d_nb.release();
     e->d_cls.release();
-    e->h_px.release();
-    e->h_gi.release();
-    e->h_nb.release();
-    e->h_cls.release();
+    {
+        std::lock_guard<std::mutex> lock(e->pool->mutex);
+        e->pool->closed = true;
+        e->pool->free.clear();
+    }
     for (auto ev : e->event_pool) cudaEventDestroy(ev);
     if (e->ev_timer_start) cudaEventDestroy(e->ev_timer_start);
     if (e->ev_timer_stop) cudaEventDestroy(e->ev_timer_stop);
@@ -1397,6 +1457,40 @@ vm_status vm_classify(vm_engine* e, const vm_mesh* mesh, const int32_t* ranges, 
     fr.image  = image;
     fr.format = format;
     return run_batch(e, &fr, 1, 0, out);
+}
+
+vm_status vm_call(vm_engine* e, const vm_mesh* mesh, const vm_hostmesh* lookup, const float Hoc[16], const vm_lens* lens, const void* image, uint32_t format, vm_batch_result* out) {
+    if (lookup == nullptr || mesh == nullptr || Hoc == nullptr || lens == nullptr) return fail(VM_ERR_INVALID_ARGUMENT, "null mesh, Hoc or lens");
+    if (image != nullptr && e != nullptr && e->layers.empty()) return fail(VM_ERR_NETWORK_SHAPE, "this engine was created without a network");
+    if (vm_hostmesh_n_nodes(lookup) != mesh->n_nodes) return fail(VM_ERR_INVALID_ARGUMENT, "the host mesh is not the one that was uploaded");
+    vm_frame fr{};
+    fr.mesh = mesh;
+    std::memcpy(fr.Hoc, Hoc, sizeof(fr.Hoc));
+    fr.lens   = *lens;
+    fr.image  = image;
+    fr.format = format;
+    return run_batch(e, &fr, 1, 0, out, lookup);
+}
+
+vm_status vm_results_keep(vm_engine* e, vm_results** kept) {
+    if (e == nullptr || kept == nullptr) return fail(VM_ERR_INVALID_ARGUMENT, "null argument");
+    *kept = nullptr;
+    if (!e->host) return fail(VM_ERR_INVALID_ARGUMENT, "the engine has no results");
+    {
+        std::lock_guard<std::mutex> lock(e->pool->mutex);
+        if (e->pool->kept >= MAX_KEPT_RESULTS) return fail(VM_ERR_OUT_OF_MEMORY, "VM_MAX_KEPT_RESULTS results of this engine are kept already");
+        ++e->pool->kept;
+    }
+    *kept = reinterpret_cast<vm_results*>(new KeptResults{e->pool, std::move(e->host)});
+    return VM_OK;
+}
+
+void vm_results_release(vm_results* kept) {
+    std::unique_ptr<KeptResults> k(reinterpret_cast<KeptResults*>(kept));
+    if (!k) return;
+    std::lock_guard<std::mutex> lock(k->pool->mutex);
+    --k->pool->kept;
+    if (!k->pool->closed) k->pool->free.push_back(std::move(k->results));
 }
 
 vm_status vm_sample(vm_engine* e, const float* px, int32_t n, const void* image, int32_t width, int32_t height, uint32_t format, float* out) {

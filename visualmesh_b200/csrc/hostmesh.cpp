@@ -24,6 +24,7 @@
 
 #include "../../include/vmcuda.h"
 #include "host_math.hpp"
+#include "hostmesh.hpp"
 
 namespace vm {
 namespace host {
@@ -477,8 +478,8 @@ struct vm_hostmesh {
     std::unique_ptr<vm::host::HostMesh> mesh;
 };
 
-namespace {
-thread_local std::string g_hostmesh_error;
+bool vm_hostmesh_ranges_(const vm_hostmesh* mesh, const float Hoc[16], const vm_lens* lens, std::vector<std::pair<int, int>>& ranges) {
+    return mesh->mesh->lookup(Hoc, *lens, ranges);
 }
 
 extern "C" {

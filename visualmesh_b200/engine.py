@@ -185,15 +185,8 @@ class BatchResult:
         self.n_neighbours = raw.n_neighbours
         self.n_classes = raw.n_classes
         self.on_device = bool(raw.on_device)
-        self.offsets = np.ctypeslib.as_array(raw.offsets, shape=(raw.n_frames + 1,)).copy()
+        self.offsets, self._px, self._gi, self._nb, self._cls = abi.native().views(C.addressof(raw))
         self.total_points = int(self.offsets[-1])
-        if not self.on_device:
-            total, rows = self.total_points, self.total_points + self.n_frames
-            N, Cn = self.n_neighbours, self.n_classes
-            self._px = np.ctypeslib.as_array(raw.pixel_coordinates, shape=(max(total, 1), 2))[:total]
-            self._gi = np.ctypeslib.as_array(raw.global_indices, shape=(max(total, 1),))[:total]
-            self._nb = np.ctypeslib.as_array(raw.neighbourhood, shape=(rows, N))
-            self._cls = np.ctypeslib.as_array(raw.classifications, shape=(rows, Cn)) if Cn > 0 else None
 
     def frame(self, f: int, copy: bool = True):
         if self.on_device:
@@ -212,6 +205,10 @@ class BatchResult:
         if self._cls is None:
             return ProjectedMesh(cp(self._px[p0:p1]), cp(self._nb[r0:r1]), cp(self._gi[p0:p1]))
         return ClassifiedMesh(cp(self._px[p0:p1]), cp(self._nb[r0:r1]), cp(self._gi[p0:p1]), cp(self._cls[r0:r1]))
+
+
+def _mesh_at(mesh, Hoc) -> Mesh:
+    return mesh.height(Hoc[2][3]) if isinstance(mesh, VisualMesh) else mesh
 
 
 class Engine:
@@ -286,29 +283,8 @@ class Engine:
         n = len(frames)
         arr = (abi.vm_frame * max(n, 1))()
         keep = []
-        for i, fr in enumerate(frames):
-            mesh = fr.mesh.height(fr.Hoc[2][3]) if isinstance(fr.mesh, VisualMesh) else fr.mesh
-            arr[i].mesh = self._device_mesh(mesh)
-            if fr.ranges is not None:
-                r = np.ascontiguousarray(fr.ranges, dtype=np.int32).reshape(-1, 2)
-                keep.append(r)
-                # a non-null pointer even for zero ranges: NULL means "look up on the device"
-                arr[i].ranges = r.ctypes.data if r.shape[0] > 0 else C.addressof(arr)
-                arr[i].n_ranges = r.shape[0]
-            H = np.ascontiguousarray(fr.Hoc, dtype=np.float32).reshape(16)
-            for j in range(16):
-                arr[i].Hoc[j] = float(H[j])
-            arr[i].lens = _c_lens(fr.lens)
-            if fr.image is not None:
-                if fr.image_on_device:
-                    arr[i].image = int(fr.image)
-                    arr[i].image_on_device = 1
-                else:
-                    img = fr.image if isinstance(fr.image, np.ndarray) and fr.image.flags["C_CONTIGUOUS"] \
-                        and fr.image.dtype == np.uint8 else np.ascontiguousarray(fr.image, dtype=np.uint8)
-                    keep.append(img)
-                    arr[i].image = img.ctypes.data
-                arr[i].format = int(fr.format)
+        plain = _mesh_at if any(isinstance(fr.mesh, VisualMesh) for fr in frames) else None
+        abi.native().marshal(frames, arr, self._device_mesh, plain, keep)
         return (arr, n, keep)
 
     def run_prepared(self, prepared, results_on_device=False, time_stages=False, raw=False):
@@ -324,16 +300,21 @@ class Engine:
     def __call__(self, mesh, Hoc, lens, image=None, format=None, ranges="host"):
         """The two reference calls. ranges="host" runs Mesh::lookup on the host as the reference engines do
         (cpp/visualmesh/engine/opencl/engine.hpp:581), ranges="device" walks the BSP on the GPU, or pass the ranges."""
-        Hoc = np.asarray(Hoc, dtype=np.float32).reshape(4, 4)
-        m = mesh.height(Hoc[2][3]) if isinstance(mesh, VisualMesh) else mesh
+        m = mesh.height(np.asarray(Hoc, dtype=np.float32).reshape(4, 4)[2][3]) if isinstance(mesh, VisualMesh) else mesh
+        host = None
         if isinstance(ranges, str):
-            r = m.lookup(Hoc, lens) if ranges == "host" else None
-        else:
-            r = ranges
+            if ranges == "host":
+                if m._ptr is None:
+                    raise VisualMeshError(abi.VM_ERR_NO_BSP, "this mesh was made from arrays: it has no host lookup")
+                host = m._ptr.value
+            ranges = None
         if image is not None and self.n_classes == 0:
             raise VisualMeshError(abi.VM_ERR_NETWORK_SHAPE, "this engine was created without a network")
-        fr = FrameInput(m, Hoc, lens, image, int(format or 0), r)
-        return self.run_batch([fr]).frame(0)
+        out = abi.native().call(self._ptr.value, self._device_mesh(m).value, host or 0, ranges, Hoc, lens, image, format or 0)
+        if isinstance(out, int):
+            abi.check(out)
+        px, nb, gi, cls = out
+        return ProjectedMesh(px, nb, gi) if cls is None else ClassifiedMesh(px, nb, gi, cls)
 
     def stage_times(self):
         """(name, milliseconds) of every kernel of the last run_batch(time_stages=True), in launch order."""
