@@ -1,0 +1,48 @@
+"""Graph-convolution layers of every width against the CPU oracle, at the sizes where a kernel's tiles begin and end."""
+import numpy as np
+import pytest
+
+import oracle as O
+import parity as P
+from visualmesh_b200 import workloads as W
+from visualmesh_b200.engine import Engine
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(n, n_neighbours, seed):
+    x = W.uniform(seed, n * 4, -1.0, 1.0).reshape(n, 4).astype(np.float32)
+    nb = (W.splitmix64(seed + 1, n * n_neighbours) % np.uint64(n)).astype(np.int32).reshape(n, n_neighbours)
+    nb[-1] = n - 1
+    return x, nb
+
+
+def _check(net, n, n_neighbours):
+    x, nb = _rows(n, n_neighbours, 31 + n)
+    engine = Engine(net)
+    got = engine.network(x, nb)
+    engine.close()
+    assert np.abs(got.astype(np.float64) - O.network(x, nb, net).astype(np.float64)).max() <= P.TOL_CLS / 4
+
+
+# one row per thread up to 147 blocks of 512 rows, two from there on (75776 is the last size of the one, 75777 the first of the other)
+@pytest.mark.parametrize("n", [1, 127, 129, 75_776, 75_777])
+@pytest.mark.parametrize("n_neighbours,widths", [(4, [24, 20, 12, 5]), (6, [7, 13, 3]), (8, [28, 32, 31, 2])])
+def test_widths_without_a_kernel_of_their_own(n, n_neighbours, widths):
+    _check(W.make_network(41, n_neighbours, widths), n, n_neighbours)
+
+
+@pytest.mark.parametrize("activation", [W.SELU, W.RELU, W.TANH, W.SOFTMAX])
+def test_odd_widths_inside_a_group(activation):
+    """Dense layers behind a gather, their widths padded with channels of zeros: a softmax in the middle must not count them."""
+    rng = np.random.default_rng(3)
+    net, width = [], 4
+    for group in ([6, 5], [9, 3]):
+        net.append([])
+        for i, out in enumerate(group):
+            fan_in = width * (7 if i == 0 else 1)
+            w = rng.uniform(-1, 1, (fan_in, out)).astype(np.float32) * np.float32(np.sqrt(6.0 / (fan_in + out)))
+            net[-1].append(W.Layer(w, rng.uniform(-0.1, 0.1, out).astype(np.float32), activation))
+            width = out
+    net[-1][-1].activation = W.SOFTMAX
+    _check(net, 1000, 6)

@@ -35,7 +35,14 @@ static void launch_conv_t(const ConvArgs& a, dim3 grid_rows, int max_rows, cudaS
     k_graph_conv<CIN, COUT, R, T, MINB><<<grid, T, smem, s>>>(a);
 }
 
-constexpr int CW_MAX = 2320;  // floats: a 16 -> 16 layer with 8 neighbours and its biases
+constexpr int CW_MAX  = 2320;  // floats: a 16 -> 16 layer with 8 neighbours and its biases
+constexpr int CW_MOST = 8120;  // what the parameter space holds beside the other arguments: 28 -> 32 with 8 neighbours
+
+// Two rows per thread and 256 threads per block would leave SMs without a block (148 of them): such launches run one row per thread
+// in blocks of 128 threads.
+static bool few_rows(int max_rows, int n_frames) {
+    return static_cast<int64_t>((max_rows + 511) / 512) * n_frames < 148;
+}
 
 template <int CIN, int COUT, int R, int WMAX, int T = CONV_THREADS>
 static bool launch_conv_cw(const DenseLayer& L, const ConvArgs& a, dim3 grid_rows, int max_rows, cudaStream_t s) {
@@ -72,11 +79,10 @@ static bool launch_conv_fast(const DenseLayer& L, const ConvArgs& a, dim3 grid, 
         const char* v = std::getenv("VMCUDA_CONST_WEIGHTS");
         return v == nullptr || v[0] != '0';
     }();
-    // the 16 -> 16 layer measured best with two rows per thread and 256 threads
-    if (const_weights && L.cin == 16 && L.cout == 16 && launch_conv_cw<16, 16, 2, CW_MAX, 256>(L, a, grid, max_rows, s)) return true;
 #define VM_CONV(CI, CO, RR)                                                                       \
     if (L.cin == CI && L.cout == CO) {                                                            \
         /* parameter-space weights: two rows per thread and 256 threads measured best for every shape tried */ \
+        if (const_weights && few_rows(max_rows, grid.y) && launch_conv_cw<CI, CO, 1, CW_MAX, 128>(L, a, grid, max_rows, s)) return true; \
         if (const_weights && launch_conv_cw<CI, CO, 2, CW_MAX, 256>(L, a, grid, max_rows, s)) return true; \
         launch_conv_t<CI, CO, RR>(a, grid, max_rows, s);                                          \
         return true;                                                                              \
@@ -86,10 +92,39 @@ static bool launch_conv_fast(const DenseLayer& L, const ConvArgs& a, dim3 grid, 
     return false;
 }
 
+// Shapes without a kernel of their own, in multiples of 4 up to 32. One row per thread and small blocks until two rows per thread
+// still give every SM a block (the rule of launch_conv_fast, for the same reason).
+template <int COUTP, int WMAX>
+static void launch_conv_any_t(const DenseLayer& L, const ConvArgs& a, dim3 grid_rows, int max_rows, cudaStream_t s) {
+    ConvWeights<WMAX> wp;
+    std::memcpy(wp.w, L.host_packed.data(), L.host_packed.size() * sizeof(float));
+    constexpr int threads = 128;
+    if (few_rows(max_rows, grid_rows.y)) {
+        dim3 grid((max_rows + threads - 1) / threads, grid_rows.y);
+        k_graph_conv_any<COUTP, 1, threads, WMAX><<<grid, threads, 0, s>>>(a, L.cin / 4, L.cout, wp);
+    }
+    else {
+        dim3 grid((max_rows + 2 * threads - 1) / (2 * threads), grid_rows.y);
+        k_graph_conv_any<COUTP, 2, threads, WMAX><<<grid, threads, 0, s>>>(a, L.cin / 4, L.cout, wp);
+    }
+}
+static bool launch_conv_any(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s) {
+    if (L.cin % 4 != 0 || L.host_packed.size() > static_cast<size_t>(CW_MOST) || a.out_split) return false;
+    const bool small = L.host_packed.size() <= static_cast<size_t>(CW_MAX);
+#define VM_ANY(CP)                                                             \
+    if (L.coutp == CP) {                                                       \
+        if (small) launch_conv_any_t<CP, CW_MAX>(L, a, grid, max_rows, s);     \
+        else launch_conv_any_t<CP, CW_MOST>(L, a, grid, max_rows, s);          \
+        return true;                                                           \
+    }
+    VM_ANY(4) VM_ANY(8) VM_ANY(12) VM_ANY(16) VM_ANY(20) VM_ANY(24) VM_ANY(28) VM_ANY(32)
+#undef VM_ANY
+    return false;
+}
 
 void launch_conv_ffma(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, cudaStream_t s) {
     dim3 grid(1, n_frames);
-    if (!launch_conv_fast(L, a, grid, max_rows, s)) {
+    if (!launch_conv_fast(L, a, grid, max_rows, s) && !launch_conv_any(L, a, grid, max_rows, s)) {
         dim3 g((max_rows + CONV_THREADS - 1) / CONV_THREADS, n_frames);
         k_graph_conv_generic<<<g, CONV_THREADS, 0, s>>>(a, L.cin, L.cout, L.coutp);
     }

@@ -241,6 +241,127 @@ __global__ void __launch_bounds__(T, (CIN == 8 && COUT <= 8 && T == 256) ? 6 : 0
     }
 }
 
+// Layers whose widths are multiples of 4 up to 32 but have no kernel of their own: the padded output width is a template parameter,
+// the input width is not. Input chunks come in batches of four, the next batch (and the next slot's neighbour index) on its way
+// while one is multiplied: with one row per thread an SM holds few warps, and what bounds the layer is the chain of its gathers.
+// Weights in the parameter space as above. Measured on 29 k rows with four neighbours, against the
+// kernel that reads its weights through the cache: 24 -> 20 85 -> 21 us, 20 -> 12 47 -> 15 us, 4 -> 24 30 -> 13 us.
+template <int COUTP, int R, int T, int WMAX>
+__global__ void __launch_bounds__(T) k_graph_conv_any(const ConvArgs a, int32_t cin4, int32_t cout, const __grid_constant__ ConvWeights<WMAX> wp) {
+    constexpr int BATCH      = 4;  // chunks of 4 channels
+    const int frame_in_chunk = blockIdx.y;
+    const int frame          = a.f0 + frame_in_chunk;
+    const int start          = a.offsets[frame];
+    const int rows           = a.offsets[frame + 1] - start + 1;
+    const int first          = blockIdx.x * (T * R);
+    if (first >= rows) return;
+    const int local_base = start - a.offsets[a.f0] + frame_in_chunk;
+    const size_t nb_base = static_cast<size_t>(start + frame);
+    const float4* in4    = reinterpret_cast<const float4*>(a.in);
+
+    int row[R], src[R], next_src[R];
+    unsigned long long acc[R][COUTP / 2];
+    float4 x[R][BATCH], next[R][BATCH];
+    auto fetch_index = [&](int s) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) next_src[q] = local_base + __ldg(a.nb + (nb_base + row[q]) * a.n_neighbours + (s - 1));
+    };
+    auto fetch = [&](int c) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+#pragma unroll
+            for (int k = 0; k < BATCH; ++k) {
+                if (c + k < cin4) next[q][k] = __ldg(in4 + static_cast<size_t>(c + k) * a.in_stride + src[q]);
+            }
+        }
+    };
+    const int biases = a.n_slots * cin4 * 4 * COUTP;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        row[q] = min(first + q * T + static_cast<int>(threadIdx.x), rows - 1);
+        src[q] = local_base + row[q];
+#pragma unroll
+        for (int j = 0; j < COUTP / 2; ++j) acc[q][j] = pack2(wp.w[biases + 2 * j], wp.w[biases + 2 * j + 1]);
+    }
+    if (a.n_slots > 1) fetch_index(1);
+    fetch(0);
+    int at = 0;  // weights of the channel
+    for (int s = 0; s < a.n_slots; ++s) {
+        for (int c = 0; c < cin4; c += BATCH) {
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+#pragma unroll
+                for (int k = 0; k < BATCH; ++k) x[q][k] = next[q][k];
+            }
+            if (c + BATCH < cin4) { fetch(c + BATCH); }
+            else if (s + 1 < a.n_slots) {
+#pragma unroll
+                for (int q = 0; q < R; ++q) src[q] = next_src[q];
+                fetch(0);
+                if (s + 2 < a.n_slots) fetch_index(s + 2);
+            }
+#pragma unroll
+            for (int k = 0; k < BATCH; ++k) {
+                if (c + k >= cin4) break;
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {
+                    unsigned long long xx[R];
+#pragma unroll
+                    for (int q = 0; q < R; ++q) {
+                        const float xv = kk == 0 ? x[q][k].x : kk == 1 ? x[q][k].y : kk == 2 ? x[q][k].z : x[q][k].w;
+                        xx[q]          = pack2(xv, xv);
+                    }
+#pragma unroll
+                    for (int j = 0; j < COUTP / 2; ++j) {
+                        const unsigned long long w = pack2(wp.w[at + 2 * j], wp.w[at + 2 * j + 1]);
+#pragma unroll
+                        for (int q = 0; q < R; ++q) ffma2(acc[q][j], xx[q], w);
+                    }
+                    at += COUTP;
+                }
+            }
+        }
+    }
+    const size_t out_base = a.out_global ? nb_base : static_cast<size_t>(local_base);
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        const int i = first + q * T + static_cast<int>(threadIdx.x);
+        if (i >= rows) continue;
+        float v[COUTP];
+#pragma unroll
+        for (int j = 0; j < COUTP / 2; ++j) unpack2(acc[q][j], v[2 * j], v[2 * j + 1]);
+        if (a.activation == VM_SOFTMAX) {
+            float total = 0.0f;
+#pragma unroll
+            for (int j = 0; j < COUTP; ++j) {
+                if (j < cout) {
+                    v[j]  = expf(v[j]);
+                    total = __fadd_rn(total, v[j]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < COUTP; ++j) v[j] = __fdiv_rn(v[j], total);
+        }
+        else {
+            activate<COUTP>(v, a.activation);
+        }
+        if (a.out_planar) {
+            float4* out4 = reinterpret_cast<float4*>(a.out);
+#pragma unroll
+            for (int j4 = 0; j4 < COUTP / 4; ++j4) {
+                out4[static_cast<size_t>(j4) * a.out_stride + out_base + i] = make_float4(v[j4 * 4], v[j4 * 4 + 1], v[j4 * 4 + 2], v[j4 * 4 + 3]);
+            }
+        }
+        else {
+            float* dst = a.out + (out_base + i) * cout;
+#pragma unroll
+            for (int j = 0; j < COUTP; ++j) {
+                if (j < cout) dst[j] = v[j];
+            }
+        }
+    }
+}
+
 // Any layer shape: one row per thread, outputs in tiles of 8, weights read through the read-only cache.
 __global__ void __launch_bounds__(CONV_THREADS) k_graph_conv_generic(const ConvArgs a, int32_t cin, int32_t cout, int32_t coutp) {
     const int frame_in_chunk = blockIdx.y;

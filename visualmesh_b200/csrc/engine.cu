@@ -1213,17 +1213,35 @@ vm_status vm_engine_create(int device, const vm_layer* layers, const int32_t* la
         VM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&e->flags), sizeof(int32_t) * ABORT_FLAGS, cudaHostAllocDefault));
         for (int i = 0; i < ABORT_FLAGS; ++i) e->flags[i] = 0;
         int l = 0;
-        int width = 4;
+        int logical = 4, width = 4;  // channels of the layer before, as the network has them and as they are stored
         for (int g = 0; g < n_groups; ++g) {
             for (int i = 0; i < layers_per_group[g]; ++i, ++l) {
-                const vm_layer& L = layers[l];
+                const vm_layer& given = layers[l];
                 DenseLayer d;
-                d.n_slots    = i == 0 ? L.n_in / width : 1;
+                d.n_slots    = i == 0 ? given.n_in / logical : 1;
                 d.cin        = width;
-                d.cout       = L.n_out;
-                d.coutp      = (L.n_out + 3) & ~3;
-                d.activation = L.activation;
-                d.stage      = std::string(i == 0 ? "graph_conv_" : "dense_") + std::to_string(width) + "x" + std::to_string(L.n_out);
+                d.activation = given.activation;
+                d.stage      = std::string(i == 0 ? "graph_conv_" : "dense_") + std::to_string(logical) + "x" + std::to_string(given.n_out);
+                // Features of a width that is no multiple of 4 are stored with channels of zeros up to the next one: the kernels with
+                // 16-byte loads then serve every width. (Every activation but softmax maps 0 to 0; weights of the zeros are zeros.)
+                const bool last = g + 1 == n_groups && i + 1 == layers_per_group[g];
+                d.cout  = last || given.activation == VM_SOFTMAX ? given.n_out : (given.n_out + 3) & ~3;
+                d.coutp = (d.cout + 3) & ~3;
+                vm_layer L = given;
+                std::vector<float> padded_weights, padded_biases;
+                if (width != logical || d.cout != given.n_out) {
+                    L.n_in  = d.n_slots * width;
+                    L.n_out = d.cout;
+                    padded_weights.assign(static_cast<size_t>(L.n_in) * L.n_out, 0.0f);
+                    padded_biases.assign(L.n_out, 0.0f);
+                    for (int r = 0; r < given.n_in; ++r) {
+                        std::memcpy(&padded_weights[(static_cast<size_t>(r / logical) * width + r % logical) * L.n_out],
+                                    given.weights + static_cast<size_t>(r) * given.n_out, sizeof(float) * given.n_out);
+                    }
+                    std::memcpy(padded_biases.data(), given.biases, sizeof(float) * given.n_out);
+                    L.weights = padded_weights.data();
+                    L.biases  = padded_biases.data();
+                }
                 // [n_in][n_out] as handed over (cpp/visualmesh/network_structure.hpp:25-27), padded to coutp columns
                 std::vector<float> packed((static_cast<size_t>(L.n_in) + 1) * d.coutp, 0.0f);
                 for (int r = 0; r < L.n_in; ++r)
@@ -1278,6 +1296,7 @@ vm_status vm_engine_create(int device, const vm_layer* layers, const int32_t* la
                 }
                 e->layers.push_back(d);
                 width        = L.n_out;
+                logical      = given.n_out;
                 e->max_width = std::max(e->max_width, width);
             }
         }
