@@ -46,3 +46,23 @@ def test_odd_widths_inside_a_group(activation):
             width = out
     net[-1][-1].activation = W.SOFTMAX
     _check(net, 1000, 6)
+
+
+# 256-row super-tiles of two 128-row tiles; 9472 rows are 37 super-tiles, 75776 and more are several per SM
+@pytest.mark.parametrize("n", [1, 128, 129, 256, 257, 9_472, 90_001])
+@pytest.mark.parametrize("n_neighbours,widths", [(4, [32, 32, 32, 3]), (6, [16, 32, 32, 16, 16, 2]), (8, [32, 32, 20, 32, 32])])
+def test_layers_of_32_channels(n, n_neighbours, widths):
+    _check(W.make_network(43, n_neighbours, widths), n, n_neighbours)
+
+
+def test_layers_of_32_channels_with_neighbours_close_by():
+    """Neighbours inside the window (random ones all over the rows mostly are not)."""
+    net = W.make_network(47, 8, [32, 32, 32, 4])
+    n = 50_000
+    x, _ = _rows(n, 8, 5)
+    near = (W.splitmix64(6, n * 8) % np.uint64(61)).astype(np.int64).reshape(n, 8) - 30
+    nb = np.clip(np.arange(n)[:, None] + near, 0, n - 1).astype(np.int32)
+    engine = Engine(net)
+    got = engine.network(x, nb)
+    engine.close()
+    assert np.abs(got.astype(np.float64) - O.network(x, nb, net).astype(np.float64)).max() <= P.TOL_CLS / 4

@@ -28,6 +28,7 @@ UNITS = {
     "conv_ffma.cu": ["conv_ffma.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
     "conv_tc.cu": ["conv_tc.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
     "conv_staged.cu": ["conv_staged.cuh", "tile_plan.cuh", "conv_tc.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
+    "conv_window.cu": ["conv_window.cuh", "tile_plan.cuh", "conv_tc.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
     "hostmesh.cpp": ["host_math.hpp", "hostmesh.hpp", ABI_HEADER],
 }
 NATIVE_SOURCES = ["native.cpp", ABI_HEADER]

@@ -47,6 +47,18 @@ __device__ __forceinline__ void activate(float* v, int act) {
     }
 }
 
+__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// x = h + l with h = fp16(x), l = fp16(x - h), for two values at once
+__device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& h, uint32_t& l) {
+    h               = pack_half2(x0, x1);
+    const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&h));
+    l               = pack_half2(x0 - hf.x, x1 - hf.y);
+}
+
 // The "split" feature layout, produced for a layer that runs on the tensor cores. Every fp32 value x is stored as two
 // fp16 values, hi = fp16(x) and lo = fp16(x - hi) (x = hi + lo to ~2^-22 relative, absolute error <= 3e-8 for small
 // x), in the shape the tensor-core kernel copies straight into shared memory: 16-byte chunks of 8 channels, chunk
@@ -76,6 +88,39 @@ __device__ __forceinline__ void store_split(float* out, int stride, size_t row, 
         *reinterpret_cast<uint4*>(base + (static_cast<size_t>(P + p) * stride + row) * 16) = make_uint4(l[0], l[1], l[2], l[3]);
     }
     if (bad) raise_flag(range_flag, ABORT_TC_RANGE);
+}
+
+// The same values row after row (32 hi parts, then 32 lo parts) for the window kernel. Stores the rows of a warp, one per thread and one
+// after another; all threads call (valid: the row exists; those that do come first). stage: shared memory of the warp, 4 KB. A thread
+// that stored its own row would write 16-byte pieces 128 bytes apart, half a sector and one line per thread and store; from shared
+// memory a store writes 512 consecutive bytes. Pieces are swizzled by their row, so that neither side meets bank conflicts.
+constexpr int SPLIT_ROW_STAGE = 32 * 128;  // bytes of shared memory per warp
+__device__ __forceinline__ void store_split_rows(float* out, size_t row, bool valid, const float* v, uint4* stage, int32_t* range_flag) {
+    constexpr int P = 4, Q = 8;  // 16-byte pieces of the hi (or lo) part, of a row
+    const int lane  = threadIdx.x & 31;
+    bool bad        = false;
+    __syncwarp();
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        uint32_t h[4], l[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float x0 = v[8 * p + 2 * q], x1 = v[8 * p + 2 * q + 1];
+            bad |= fabsf(x0) > 60000.0f || fabsf(x1) > 60000.0f;
+            split_pair(x0, x1, h[q], l[q]);
+        }
+        stage[lane * Q + (p ^ (lane & (Q - 1)))]       = make_uint4(h[0], h[1], h[2], h[3]);
+        stage[lane * Q + ((P + p) ^ (lane & (Q - 1)))] = make_uint4(l[0], l[1], l[2], l[3]);
+    }
+    if (bad && valid) raise_flag(range_flag, ABORT_TC_RANGE);
+    __syncwarp();
+    const int pieces = __popc(__ballot_sync(0xffffffffu, valid)) * Q;
+    uint4* dst       = reinterpret_cast<uint4*>(out) + (row - lane) * Q;
+#pragma unroll
+    for (int k = 0; k < Q; ++k) {
+        const int i = k * 32 + lane, r = i / Q, p = i % Q;
+        if (i < pieces) dst[i] = stage[r * Q + (p ^ (r & (Q - 1)))];
+    }
 }
 
 }  // namespace vm

@@ -32,6 +32,7 @@ struct DenseLayer {
     std::vector<float> host_packed;  // [K][coutp] weights then biases, as on the device (for parameter-space kernels)
     // tensor-core path (conv_tc.cuh): weights split into TF32 hi/lo parts in the UMMA K-major layout, padded bias
     void* d_tc_cat   = nullptr;  // [K / KCH chunks][2 * NP rows][16 B]: hi rows then lo rows
+    void* d_tc_win   = nullptr;  // conv_window.cuh: columns and channels permuted (32-channel inputs)
     float* d_tc_bias = nullptr;
     int tc_np        = 0;      // padded output width of the tensor-core tile, 0 = no tensor-core path for this shape
     bool tc_half     = false;  // fp16 hi/lo split (16- and 32-channel inputs) or TF32 split (8-channel inputs)
@@ -82,6 +83,12 @@ constexpr int STAGED_ST         = 256;  // rows of a super-tile
 constexpr int STAGED_HALO       = 192;  // halo slots of a super-tile
 bool has_staged_kernel(const DenseLayer& L);
 bool launch_conv_staged(const DenseLayer& L, const ConvArgs& a, const StagedPlan& plan, int n_frames, int max_rows, int32_t* abort_flags,
+                        uint32_t wait_limit, cudaStream_t s);
+// ---- conv_window.cu: 32-channel layers on the tensor cores (tcgen05), gather from shared-memory windows ------------
+bool has_window_kernel(const DenseLayer& L);
+// the layer's weights as the kernel wants them in shared memory; weights is [n_slots * 32][cout]
+std::vector<unsigned char> pack_window_weights(const float* weights, int n_slots, int cout);
+bool launch_conv_window(const DenseLayer& L, const ConvArgs& a, const StagedPlan& plan, int n_frames, int max_rows, int32_t* abort_flags,
                         uint32_t wait_limit, cudaStream_t s);
 // the plan for a neighbourhood that is already in memory (the hot path makes it inside the neighbour-remap kernel)
 void launch_tile_plan_kernel(int n_neighbours, const int32_t* offsets, const int32_t* nb, uint16_t* nbl, int32_t* halo_rows, int32_t* halo_count,

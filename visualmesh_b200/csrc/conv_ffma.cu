@@ -22,13 +22,18 @@ bool has_fast_ffma_kernel(int cin, int cout) {
     return false;
 }
 
+// shared memory in which the warps of a block arrange split rows before they store them
+static size_t split_stage_bytes(const ConvArgs& a, int threads) {
+    return a.out_split == SPLIT_ROWS ? static_cast<size_t>(threads / 32) * SPLIT_ROW_STAGE : 0;
+}
+
 template <int CIN, int COUT, int R, int T = CONV_THREADS, int MINB = 1>
 static void launch_conv_t(const ConvArgs& a, dim3 grid_rows, int max_rows, cudaStream_t s) {
     constexpr int COUTP = (COUT + 3) & ~3;
-    const size_t smem   = (static_cast<size_t>(a.n_slots) * CIN * COUTP + COUTP) * sizeof(float);
+    const size_t smem   = (static_cast<size_t>(a.n_slots) * CIN * COUTP + COUTP) * sizeof(float) + split_stage_bytes(a, T);
     static LaunchPlans plans;
     plans.get([](int) {
-        VM_CUDA(cudaFuncSetAttribute(k_graph_conv<CIN, COUT, R, T, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        VM_CUDA(cudaFuncSetAttribute(k_graph_conv<CIN, COUT, R, T, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 120 * 1024));
         return LaunchPlan{};
     });
     dim3 grid((max_rows + T * R - 1) / (T * R), grid_rows.y);
@@ -55,16 +60,17 @@ static bool launch_conv_cw(const DenseLayer& L, const ConvArgs& a, dim3 grid_row
     // next slots are then issued ahead of the current slot's arithmetic. Measured on 4.4 M rows: 4 -> 16 183 -> 114 us
     // (with the weights in the parameter space instead of shared memory), 8 -> 8 133 -> 112 us, 32 -> 4 448 -> 413 us;
     // the 16- and 32-channel layers in between, bound by the FP32 pipe, measured 3-6 % slower unrolled and stay rolled.
+    const size_t smem            = split_stage_bytes(a, T);
     constexpr bool LATENCY_BOUND = (CIN == 8 && COUT == 8) || CIN == 4 || COUT <= 4;
-    if (LATENCY_BOUND && a.n_slots == 5) { k_graph_conv_cw<CIN, COUT, R, WMAX, T, LATENCY_BOUND ? 5 : 0><<<grid, T, 0, s>>>(a, wp); }
+    if (LATENCY_BOUND && a.n_slots == 5) { k_graph_conv_cw<CIN, COUT, R, WMAX, T, LATENCY_BOUND ? 5 : 0><<<grid, T, smem, s>>>(a, wp); }
     else if (LATENCY_BOUND && a.n_slots == 7) {
-        k_graph_conv_cw<CIN, COUT, R, WMAX, T, LATENCY_BOUND ? 7 : 0><<<grid, T, 0, s>>>(a, wp);
+        k_graph_conv_cw<CIN, COUT, R, WMAX, T, LATENCY_BOUND ? 7 : 0><<<grid, T, smem, s>>>(a, wp);
     }
     else if (LATENCY_BOUND && a.n_slots == 9) {
-        k_graph_conv_cw<CIN, COUT, R, WMAX, T, LATENCY_BOUND ? 9 : 0><<<grid, T, 0, s>>>(a, wp);
+        k_graph_conv_cw<CIN, COUT, R, WMAX, T, LATENCY_BOUND ? 9 : 0><<<grid, T, smem, s>>>(a, wp);
     }
     else {
-        k_graph_conv_cw<CIN, COUT, R, WMAX, T><<<grid, T, 0, s>>>(a, wp);
+        k_graph_conv_cw<CIN, COUT, R, WMAX, T><<<grid, T, smem, s>>>(a, wp);
     }
     return true;
 }

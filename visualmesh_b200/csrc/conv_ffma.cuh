@@ -102,8 +102,15 @@ __global__ void __launch_bounds__(T, MINB) k_graph_conv(const ConvArgs a) {
 #pragma unroll
     for (int q = 0; q < R; ++q) {
         const int i = first + q * T + static_cast<int>(threadIdx.x);
-        if (i >= rows) continue;
         activate<COUT>(acc[q], a.activation);
+        if constexpr (COUT == 32) {
+            if (a.out_split == SPLIT_ROWS) {
+                uint4* stage = reinterpret_cast<uint4*>(smem4 + (K * COUTP + COUTP) / 4) + (threadIdx.x >> 5) * (SPLIT_ROW_STAGE / 16);
+                store_split_rows(a.out, out_base + i, i < rows, acc[q], stage, a.range_flag);
+                continue;
+            }
+        }
+        if (i >= rows) continue;
         float* dst = a.out + (out_base + i) * COUT;
         if (COUT % 8 == 0 && a.out_split) { store_split<(COUT % 8 == 0 ? COUT : 8)>(a.out, a.out_stride, out_base + i, acc[q], a.range_flag); }
         else if (COUT % 4 == 0 && a.out_planar) {
@@ -158,6 +165,7 @@ template <int CIN, int COUT, int R, int WMAX, int T = CONV_THREADS, int NS = 0>
 __global__ void __launch_bounds__(T, (CIN == 8 && COUT <= 8 && T == 256) ? 6 : 0) k_graph_conv_cw(const ConvArgs a, const __grid_constant__ ConvWeights<WMAX> wp) {
     static_assert(CIN % 4 == 0, "vector loads of the input rows");
     constexpr int COUTP = (COUT + 3) & ~3;
+    extern __shared__ uint4 split_stage[];  // SPLIT_ROW_STAGE bytes per warp when the output is split in rows
     const int frame_in_chunk = blockIdx.y;
     const int frame          = a.f0 + frame_in_chunk;
     const int start          = a.offsets[frame];
@@ -214,11 +222,17 @@ __global__ void __launch_bounds__(T, (CIN == 8 && COUT <= 8 && T == 256) ? 6 : 0
 #pragma unroll
     for (int q = 0; q < R; ++q) {
         const int i = first + q * T + static_cast<int>(threadIdx.x);
-        if (i >= rows) continue;
         float v[COUTP];
 #pragma unroll
         for (int j = 0; j < COUTP / 2; ++j) unpack2(acc[q][j], v[2 * j], v[2 * j + 1]);
         activate<COUT>(v, a.activation);
+        if constexpr (COUT == 32) {
+            if (a.out_split == SPLIT_ROWS) {
+                store_split_rows(a.out, out_base + i, i < rows, v, split_stage + (threadIdx.x >> 5) * (SPLIT_ROW_STAGE / 16), a.range_flag);
+                continue;
+            }
+        }
+        if (i >= rows) continue;
         float* dst = a.out + (out_base + i) * COUT;
         if (COUT % 8 == 0 && a.out_split) { store_split<(COUT % 8 == 0 ? COUT : 8)>(a.out, a.out_stride, out_base + i, v, a.range_flag); }
         else if (COUT % 4 == 0 && a.out_planar) {

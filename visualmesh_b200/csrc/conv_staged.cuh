@@ -93,18 +93,6 @@ namespace st {
                      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
     }
-    __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
-        uint32_t r;
-        asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-        return r;
-    }
-    // x = h + l with h = fp16(x), l = fp16(x - h), for two values at once
-    __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& h, uint32_t& l) {
-        h               = pack_half2(x0, x1);
-        const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&h));
-        l               = pack_half2(x0 - hf.x, x1 - hf.y);
-    }
-
     struct Args {
         int32_t n_frames;
         int32_t cout;
@@ -244,7 +232,7 @@ namespace st {
             int n_halo = 0;
             int32_t halo_row[PER_LANE];
             auto fetch_halo_list = [&](int st) {
-                n_halo                = __ldg(plan.halo_count + st);
+                n_halo                = min(__ldg(plan.halo_count + st), HALO);
                 const int32_t* h_rows = plan.halo_rows + static_cast<size_t>(st) * HALO;
 #pragma unroll
                 for (int k = 0; k < PER_LANE; ++k) halo_row[k] = __ldg(h_rows + min(lane + 32 * k, HALO - 1));  // entries past n_halo are never used
@@ -451,6 +439,11 @@ namespace st {
                                 uint32_t h, l;
                                 split_pair(v[nb][0], v[nb][1], h, l);
                                 bad |= fabsf(v[nb][0]) > 60000.0f || fabsf(v[nb][1]) > 60000.0f;
+                                if (COUT == 32 && a.out_split == SPLIT_ROWS) {
+                                    *reinterpret_cast<uint32_t*>(out_b + out_row * 128 + nb * 16 + tq * 4)      = h;
+                                    *reinterpret_cast<uint32_t*>(out_b + out_row * 128 + 64 + nb * 16 + tq * 4) = l;
+                                    continue;
+                                }
                                 *reinterpret_cast<uint32_t*>(out_b + (static_cast<size_t>(nb) * a.out_stride + out_row) * 16 + tq * 4)        = h;
                                 *reinterpret_cast<uint32_t*>(out_b + (static_cast<size_t>(NBLK + nb) * a.out_stride + out_row) * 16 + tq * 4) = l;
                             }

@@ -287,15 +287,19 @@ static void end_stage(vm_engine* e, cudaStream_t s) {
     VM_CUDA(cudaEventRecord(e->timers.back().stop, s));
 }
 
-enum ConvKind { CONV_FFMA = 0, CONV_TC_GATHER = 1, CONV_TC_SPLIT = 2, CONV_TC_STAGED = 3 };
+enum ConvKind { CONV_FFMA = 0, CONV_TC_GATHER = 1, CONV_TC_SPLIT = 2, CONV_TC_STAGED = 3, CONV_TC_WINDOW = 4 };
 
 // Whether the kernel that runs layer L as `kind` honours ConvArgs::out_split. The tensor-core kernels write the split
 // layout when their tile is exactly as wide as the layer; the specialised FFMA kernels when the width is a multiple
 // of 8; the generic kernel never does.
 static bool producer_writes_split(const DenseLayer& L, ConvKind kind) {
-    if (kind == CONV_TC_STAGED) return L.cout % 8 == 0;
+    if (kind == CONV_TC_STAGED || kind == CONV_TC_WINDOW) return L.cout % 8 == 0;
     if (kind != CONV_FFMA) return L.cout == L.tc_np;
     return has_fast_ffma_kernel(L.cin, L.cout) && L.cout % 8 == 0;
+}
+// the same for SPLIT_ROWS, the layout of the window kernel's 32 input channels
+static bool producer_writes_rows(const DenseLayer& L, ConvKind kind) {
+    return L.cout == 32 && kind != CONV_TC_GATHER && kind != CONV_TC_SPLIT && producer_writes_split(L, kind);
 }
 
 // Scratch of a chunk's tile plan (tile_plan.cuh): neighbour positions per row, halo lists per super-tile.
@@ -314,7 +318,8 @@ static void launch_conv(vm_engine* e, const DenseLayer& L, ConvArgs a, int n_fra
     a.n_slots     = L.n_slots;
     a.activation  = L.activation;
     begin_stage(e, s, L.stage.c_str());
-    if (kind == CONV_TC_STAGED && launch_conv_staged(L, a, plan, n_frames, max_rows, e->flags, e->tc_wait_limit, s)) {}
+    if (kind == CONV_TC_WINDOW && launch_conv_window(L, a, plan, n_frames, max_rows, e->flags, e->tc_wait_limit, s)) {}
+    else if (kind == CONV_TC_STAGED && launch_conv_staged(L, a, plan, n_frames, max_rows, e->flags, e->tc_wait_limit, s)) {}
     else if ((kind == CONV_TC_SPLIT || kind == CONV_TC_STAGED) && launch_conv_tc_split(L, a, n_frames, max_rows, e->flags, e->tc_wait_limit, s)) {}
     else if (kind == CONV_TC_GATHER && launch_conv_tc_gather(L, a, n_frames, max_rows, e->flags, e->tc_wait_limit, s)) {}
     else {
@@ -337,8 +342,8 @@ static void run_network(vm_engine* e,
                         bool final_global,
                         int feature_stride) {
     // Which kernel runs each layer (VMCUDA_TC: 0 = CUDA cores only; 1, the default, and 2 = tensor cores too).
-    // A 16- or 32-channel layer whose producer can write the split layout runs as a staged layer (conv_staged.cuh,
-    // VMCUDA_STAGED=0 turns it off). Otherwise the tcgen05 kernels take a layer when its contraction is dense enough to
+    // A 16-channel layer whose producer can write the split layout runs as a staged layer (conv_staged.cuh), a dense one with 32
+    // channels in on the window kernel (conv_window.cuh; VMCUDA_STAGED=0 turns both off). Otherwise the tcgen05 kernels take a layer when its contraction is dense enough to
     // pay (mode 1: C_in x C_out >= 512) or whenever one exists (mode 2): fed by plain copies from the split layout
     // (CONV_TC_SPLIT) or gathering and splitting fp32 themselves (CONV_TC_GATHER).
     const size_t n_layers = e->layers.size();
@@ -353,8 +358,10 @@ static void run_network(vm_engine* e,
             continue;
         }
         // the tcgen05 kernels where the contraction is dense enough for them to pay (mode 1) or wherever they exist (mode 2)
+        const bool producer_can_rows = l > 0 && producer_writes_rows(e->layers[l - 1], kind[l - 1]) && !e->tc_no_split;
         if (e->tc_mode == 1 && L.cin * L.cout < e->tc_min_product) continue;
-        if (has_tc_split_kernel(L) && producer_can_split) kind[l] = CONV_TC_SPLIT;
+        if (e->staged && plan_valid && producer_can_rows && has_window_kernel(L) && (l + 1 == n_layers || L.cout % 4 == 0)) kind[l] = CONV_TC_WINDOW;
+        else if (has_tc_split_kernel(L) && producer_can_split) kind[l] = CONV_TC_SPLIT;
         else if (has_tc_gather_kernel(L)) kind[l] = CONV_TC_GATHER;
         // anything else (dense-only layers, shapes without a tensor-core instantiation) stays on the FFMA kernels
     }
@@ -373,7 +380,7 @@ static void run_network(vm_engine* e,
         a.in_stride    = feature_stride;
         a.out_stride   = feature_stride;
         a.out_planar   = (!last && e->layers[l].cout % 4 == 0) ? 1 : 0;
-        a.out_split    = (!last && (kind[l + 1] == CONV_TC_SPLIT || kind[l + 1] == CONV_TC_STAGED)) ? 1 : 0;
+        a.out_split    = last ? SPLIT_NONE : kind[l + 1] == CONV_TC_WINDOW ? SPLIT_ROWS : kind[l + 1] >= CONV_TC_SPLIT ? SPLIT_PLANES : SPLIT_NONE;
         a.range_flag   = e->flags;
         launch_conv(e, e->layers[l], a, n_frames, max_rows, lane.stream, kind[l], plan);
         cur ^= 1;
@@ -1290,6 +1297,11 @@ vm_status vm_engine_create(int device, const vm_layer* layers, const int32_t* la
                         VM_CUDA(cudaMalloc(reinterpret_cast<void**>(&d.d_tc_bias), bias.size() * sizeof(float)));
                         VM_CUDA(cudaMemcpy(d.d_tc_cat, cat.data(), cat.size(), cudaMemcpyHostToDevice));
                         VM_CUDA(cudaMemcpy(d.d_tc_bias, bias.data(), bias.size() * sizeof(float), cudaMemcpyHostToDevice));
+                        if (half && width == 32) {
+                            const std::vector<unsigned char> win = pack_window_weights(L.weights, d.n_slots, L.n_out);
+                            VM_CUDA(cudaMalloc(&d.d_tc_win, win.size()));
+                            VM_CUDA(cudaMemcpy(d.d_tc_win, win.data(), win.size(), cudaMemcpyHostToDevice));
+                        }
                         d.tc_np   = np;
                         d.tc_half = half;
                     }
@@ -1301,7 +1313,11 @@ vm_status vm_engine_create(int device, const vm_layer* layers, const int32_t* la
             }
         }
         e->n_classes = e->layers.empty() ? 0 : e->layers.back().cout;
-        for (size_t l = 1; l + 1 < e->layers.size(); ++l) e->may_stage = e->may_stage || has_staged_kernel(e->layers[l]);
+        for (size_t l = 1; l < e->layers.size(); ++l) {
+            const DenseLayer& L = e->layers[l];
+            e->may_stage        = e->may_stage || (l + 1 < e->layers.size() && has_staged_kernel(L));
+            e->may_stage        = e->may_stage || (has_window_kernel(L) && (e->tc_mode != 1 || L.cin * L.cout >= e->tc_min_product));
+        }
     }
     catch (const CudaFailure& f) {
         cudaGetLastError();
@@ -1330,6 +1346,7 @@ void vm_engine_destroy(vm_engine* e) {
     for (auto& L : e->layers) {
         cudaFree(L.d_weights);
         cudaFree(L.d_tc_cat);
+        cudaFree(L.d_tc_win);
         cudaFree(L.d_tc_bias);
     }
     forget_graphs(e);

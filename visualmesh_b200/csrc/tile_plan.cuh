@@ -24,7 +24,7 @@ namespace st {
     struct Plan {
         const uint16_t* nbl;        // [chunk rows][NBL_STRIDE]: neighbour j of a row as a position in its super-tile's window
         const int32_t* halo_rows;   // [super-tiles][HALO]: chunk-local feature row of every halo slot
-        const int32_t* halo_count;  // [super-tiles]
+        const int32_t* halo_count;  // [super-tiles]: outside rows; more than HALO: some neighbours are marked NBL_GLOBAL
     };
     struct PlanOut {
         uint16_t* nbl;
@@ -101,7 +101,7 @@ namespace st {
                 ++slot;
             }
         }
-        if (tid == 0) out.halo_count[st_id] = total < HALO ? total : HALO;
+        if (tid == 0) out.halo_count[st_id] = total;
         __syncthreads();
         // ---- 3: every neighbour as a position in the window ----
         if (valid) {
