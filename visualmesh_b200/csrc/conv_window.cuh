@@ -14,11 +14,15 @@
 //   - the columns of D are permuted so that the epilogue's thread holds neighbouring output channels of a row, four threads a row:
 //     features are written in whole 32-byte sectors without a detour through shared memory.
 //
-// Roles: gather groups of four warps (128 rows, one MMA tile) that store units of up to three slots of A into a ring in tensor memory,
-// one warp that issues the MMAs, a group of four warps for the epilogue, one loader warp. They meet at mbarriers only.
-// What bounds a 128-row tile with eight neighbours, in cycles of its SM: the shared-memory path with 1152 for the gather, 180 to fill
-// the window and 576 for the B operand; the MMAs take 1190 (16.5 each). Measured on the 32 -> 32 layer over 7.4 M rows: 978 us, against
-// 1394 us for the kernel that gathers with global loads (conv_tc.cuh).
+// Roles: two gather groups of four warps (128 rows, one MMA tile) that store units of up to three slots of A into a ring in tensor
+// memory, one warp that issues the MMAs (the weights' hi and lo parts side by side as N, so half as many to issue), a group of four
+// warps for the epilogue, one loader warp. They meet at mbarriers only. 14 warps leave 128 registers a thread, and two steps of the
+// gather in flight; three groups with 96 registers and one step measured 6 % slower, with two steps (spills) 28 %, a second group for
+// the epilogue 10 % slower, units of one slot 10 % slower (the barriers).
+// What bounds a 128-row tile with eight neighbours: the load/store path of its SM, about 2300 cycles for the gather's loads (1152 and
+// their conflicts), the stores to tensor memory, the window and the output, while the MMAs take 1190; the tile takes about 4000,
+// the rest being the chain load -> store -> settle -> MMA of a unit with only two groups to overlap it. Measured on the 32 -> 32 layer
+// over 7.4 M rows: 834 us, against 1394 us for the kernel that gathers with global loads (conv_tc.cuh).
 //
 // Every wait is bounded: a wait that runs out raises the abort flag, the CTA stops issuing work, waits (bounded) for its own copies
 // and MMAs, frees its tensor memory and returns. No multicast; all copies read this GPU's own memory.
@@ -36,13 +40,13 @@ namespace win {
     constexpr int HALO          = st::HALO;
     constexpr int CIN           = 32;
     constexpr int ROW           = 4 * CIN;  // bytes of a feature row: hi part, lo part
-    constexpr int GATHER_GROUPS = 3;        // groups of four warps: the 128 rows of one MMA tile
+    constexpr int GATHER_GROUPS = 2;        // groups of four warps: the 128 rows of one MMA tile
     constexpr int GATHER_WARPS  = 4 * GATHER_GROUPS;
     constexpr int OUT_WARPS     = 4;
     constexpr int LOADER        = GATHER_WARPS + OUT_WARPS;
     constexpr int ISSUER        = LOADER + 1;
     constexpr int THREADS       = 32 * (ISSUER + 1);
-    constexpr int ACCS          = 4;  // accumulators: tiles between their first MMA and their epilogue's load
+    constexpr int ACCS          = 2;  // accumulators: tiles between their first MMA and their epilogue's load
     constexpr int BUFFERS       = 3;  // windows that are being read or on their way
     constexpr int WINDOW        = (ST + HALO) * ROW;
     constexpr int NBL_BYTES     = ST * st::NBL_STRIDE * 2;
@@ -70,7 +74,7 @@ namespace win {
         static constexpr int COUNT  = (NSLOTS + 2) / 3;
         static constexpr int SLOTS  = (NSLOTS + COUNT - 1) / COUNT;
         static constexpr int COLS   = SLOTS * CIN;  // a column holds two fp16 values
-        static constexpr int FIT    = (512 - ACCS * NP) / COLS;
+        static constexpr int FIT    = (512 - ACCS * 2 * NP) / COLS;
         static constexpr int STAGES = FIT < 8 ? FIT : 8;
         static_assert(COUNT <= 3 && STAGES >= GATHER_GROUPS, "every gather group has a unit to store into");
     };
@@ -153,7 +157,8 @@ namespace win {
         constexpr int STAGES   = Unit::STAGES;
         constexpr int WCHUNK   = 2 * NP * 16;
         constexpr int OWN      = NP / 4;     // output channels of a thread
-        constexpr int A_COLUMN = ACCS * NP;  // first tensor-memory column of the units of A, behind the accumulators
+        constexpr int ACC_COLS = 2 * NP;     // products with the weights' hi parts, then with their lo parts
+        constexpr int A_COLUMN = ACCS * ACC_COLS;  // first tensor-memory column of the units of A, behind the accumulators
 
         extern __shared__ __align__(1024) unsigned char smem_raw[];
         // window: full, free; unit of A: stored, read; accumulator: full, free; drain
@@ -328,7 +333,7 @@ namespace win {
         }
         else if (warp == ISSUER) {
             // ================= MMAs, issued by one lane =================
-            constexpr uint32_t IDESC = (1u << 4) | (static_cast<uint32_t>(tc::TILE_ROWS >> 4) << 24) | (static_cast<uint32_t>(NP >> 3) << 17);
+            constexpr uint32_t IDESC = (1u << 4) | (static_cast<uint32_t>(tc::TILE_ROWS >> 4) << 24) | (static_cast<uint32_t>(ACC_COLS >> 3) << 17);
             const uint64_t b0        = tc::smem_desc(w_addr, WCHUNK, 128);
             uint32_t stage = 0, stage_phase = 0, acc = 0, acc_phase = 0;
             bool ok = true;
@@ -336,7 +341,7 @@ namespace win {
                 const Item r = locate(item);
                 for (int tile = r.first; ok && tile < r.end; ++tile) {
                     ok = wait(bar_acc_free + 8 * acc, acc_phase ^ 1u);  // passes at once the first time round
-                    const uint32_t d = tmem_base + acc * NP;
+                    const uint32_t d = tmem_base + acc * ACC_COLS;
 #pragma unroll 1
                     for (int u = 0; ok && u < Unit::COUNT; ++u) {
                         ok = wait(bar_stored + 8 * stage, stage_phase);
@@ -352,9 +357,7 @@ namespace win {
 #pragma unroll
                                     for (int ks = 0; ks < CIN / 8; ++ks) {
                                         // K step ks & 1 of the slot's weights: NP rows of hi parts, behind them NP rows of lo parts
-                                        const uint64_t b = bu + (i * 4 + (ks & 1) * 2) * (WCHUNK / 16);
-                                        mma_ts(d, a0 + i * CIN + 8 * ks, b, IDESC, u != 0 || i != 0 || ks != 0);
-                                        mma_ts(d, a0 + i * CIN + 8 * ks, b + NP, IDESC, true);
+                                        mma_ts(d, a0 + i * CIN + 8 * ks, bu + (i * 4 + (ks & 1) * 2) * (WCHUNK / 16), IDESC, u != 0 || i != 0 || ks != 0);
                                     }
                                 }
                             }
@@ -383,7 +386,7 @@ namespace win {
         }
         else if (warp < GATHER_WARPS) {
             // ================= gather: window -> units of A =================
-            constexpr int DEPTH       = 1;             // steps of 16 rows of a slot whose loads are in flight
+            constexpr int DEPTH       = 2;             // steps of 16 rows of a slot whose loads are in flight
             const int group           = warp >> 2;
             const int quad            = lane >> 2;     // this thread's rows of the warp's 32: quad, quad + 8, + 16, + 24
             const int piece           = lane & 3;
@@ -525,13 +528,22 @@ namespace win {
                     ok = wait(bar_acc_full + 8 * acc, acc_phase);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    uint32_t d[2][NP / 2];  // all columns of 16 rows over 32 threads, twice
+                    float v[4][OWN];  // rows first_row, + 8, + 16, + 24
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
+                        uint32_t d[ACC_COLS / 2];  // all columns of 16 rows over 32 threads
 #pragma unroll
-                        for (int c = 0; c < NP; c += 16) load_d(tmem_base + acc * NP + lanes + (static_cast<uint32_t>(16 * h) << 16) + c, d[h] + c / 2);
+                        for (int c = 0; c < ACC_COLS; c += 16) load_d(tmem_base + acc * ACC_COLS + lanes + (static_cast<uint32_t>(16 * h) << 16) + c, d + c / 2);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+#pragma unroll
+                            for (int i = 0; i < OWN; ++i) {
+                                const int at    = 4 * (i / 2) + 2 * j + i % 2;
+                                v[2 * h + j][i] = (__uint_as_float(d[at]) + __uint_as_float(d[NP / 2 + at])) + bias[i];
+                            }
+                        }
                     }
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
                     if (lane == 0) tc::mbar_arrive(bar_acc_free + 8 * acc);
@@ -540,12 +552,6 @@ namespace win {
                         acc_phase ^= 1u;
                     }
                     const int first_row = r.t0 + tile * tc::TILE_ROWS + (warp & 3) * 32 + quad;  // within the frame
-                    float v[4][OWN];  // rows first_row, + 8, + 16, + 24
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-#pragma unroll
-                        for (int i = 0; i < OWN; ++i) v[j][i] = __uint_as_float(d[j >> 1][4 * (i / 2) + 2 * (j & 1) + i % 2]) + bias[i];
-                    }
                     if (a.activation == VM_SOFTMAX) {
                         // exp of each, summed in channel order from thread to thread of the row
 #pragma unroll
