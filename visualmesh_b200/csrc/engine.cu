@@ -1505,6 +1505,10 @@ vm_status vm_call(vm_engine* e, const vm_mesh* mesh, const vm_hostmesh* lookup, 
     fr.lens   = *lens;
     fr.image  = image;
     fr.format = format;
+    // With the mesh's BSP on the device the lookup runs there, with the host's arithmetic and the host's result: one more small kernel
+    // against 10 to 140 us on the calling thread, which is then free to copy the image (thumbnail on a mesh of 7 k nodes: 62 -> 48 us a
+    // call, 21 MB frame on one of 1.7 M: 2.49 -> 2.27 ms, ten calls of both grid models and all sizes: -3 % to +29 %).
+    if (mesh->n_bsp > 0) lookup = nullptr;
     return run_batch(e, &fr, 1, 0, out, lookup);
 }
 

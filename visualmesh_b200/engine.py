@@ -298,8 +298,9 @@ class Engine:
         return self.run_prepared(self.prepare_batch(frames), results_on_device, time_stages)
 
     def __call__(self, mesh, Hoc, lens, image=None, format=None, ranges="host"):
-        """The two reference calls. ranges="host" runs Mesh::lookup on the host as the reference engines do
-        (cpp/visualmesh/engine/opencl/engine.hpp:581), ranges="device" walks the BSP on the GPU, or pass the ranges."""
+        """The two reference calls. ranges="host" looks up the nodes of a mesh with host tables as the reference engines do
+        (cpp/visualmesh/engine/opencl/engine.hpp:581; the work itself is done wherever it is faster, with the same result),
+        ranges="device" walks the BSP on the GPU, or pass the ranges."""
         m = mesh.height(np.asarray(Hoc, dtype=np.float32).reshape(4, 4)[2][3]) if isinstance(mesh, VisualMesh) else mesh
         host = None
         if isinstance(ranges, str):
