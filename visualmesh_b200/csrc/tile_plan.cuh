@@ -58,18 +58,34 @@ namespace st {
         }
         const int local_base = offsets[f0 + f] - offsets[f0] + f;
         // ---- 1: the set of outside rows ----
-        if (valid) {
+        // Of the 256 N neighbours of a super-tile one in eight lies outside, so a warp meets the insertion for every j. The first tries
+        // of all j are in flight together; an entry is kept, so that nothing is searched again in step 3. (One after the other, and a
+        // second search: PLAN_MEASURED.)
+        int entry[N];
+        int prev[N];
 #pragma unroll
-            for (int j = 0; j < N; ++j) {
-                const int i = idx[j];
-                if (i >= t0 && i < t0 + ST) continue;
-                uint32_t h = hash_row(i);
-                for (int probe = 0; probe < HASH_SIZE; ++probe) {
-                    const int prev = atomicCAS(&keys[h], -1, i);
-                    if (prev == -1 || prev == i) break;
-                    h = (h + 1) & (HASH_SIZE - 1);
+        for (int j = 0; j < N; ++j) {
+            const int i = idx[j];
+            entry[j]    = -1;
+            prev[j]     = i;
+            if (valid && (i < t0 || i >= t0 + ST)) {
+                entry[j] = static_cast<int>(hash_row(i));
+                prev[j]  = atomicCAS(&keys[entry[j]], -1, i);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            if (prev[j] == -1 || prev[j] == idx[j]) continue;
+            // taken by another row: on to the next entries; a full table leaves the row out (NBL_GLOBAL)
+            int e = entry[j];
+            entry[j] = HASH_SIZE;
+            for (int probe = 1; probe < HASH_SIZE; ++probe) {
+                e           = (e + 1) & (HASH_SIZE - 1);
+                const int p = atomicCAS(&keys[e], -1, idx[j]);
+                if (p == -1 || p == idx[j]) {
+                    entry[j] = e;
+                    break;
                 }
-                // a full table leaves the row out: it is then fetched from global memory by the layer kernels
             }
         }
         __syncthreads();
@@ -110,24 +126,11 @@ namespace st {
             for (int j = 0; j < NBL_STRIDE; ++j) v[j] = 0;
 #pragma unroll
             for (int j = 0; j < N; ++j) {
-                const int i = idx[j];
-                if (i >= t0 && i < t0 + ST) {
-                    v[j] = static_cast<uint32_t>(i - t0);
-                    continue;
+                if (entry[j] < 0) { v[j] = static_cast<uint32_t>(idx[j] - t0); }
+                else {
+                    const uint32_t s = entry[j] < HASH_SIZE ? slot_of[entry[j]] : NBL_GLOBAL;
+                    v[j]             = s == NBL_GLOBAL ? NBL_GLOBAL : static_cast<uint32_t>(ST) + s;
                 }
-                uint32_t h   = hash_row(i);
-                uint32_t pos = NBL_GLOBAL;
-                for (int probe = 0; probe < HASH_SIZE; ++probe) {
-                    const int k = keys[h];
-                    if (k == i) {
-                        const uint32_t s = slot_of[h];
-                        pos              = s == NBL_GLOBAL ? NBL_GLOBAL : static_cast<uint32_t>(ST) + s;
-                        break;
-                    }
-                    if (k == -1) break;
-                    h = (h + 1) & (HASH_SIZE - 1);
-                }
-                v[j] = pos;
             }
             uint4 packed;
             packed.x = v[0] | (v[1] << 16);
