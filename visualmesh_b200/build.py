@@ -21,11 +21,14 @@ OBJ = os.path.join(CSRC, "_build")
 LIB = os.path.join(HERE, "libvmcuda.so")
 NATIVE = os.path.join(HERE, "_native" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 ABI_HEADER = os.path.join("..", "..", "include", "vmcuda.h")
+FFMA_HEADERS = ["conv_ffma_launch.cuh", "conv_ffma.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER]
 # translation unit -> headers it includes (directly or not)
 UNITS = {
     "engine.cu": ["kernels.cuh", "tile_plan.cuh", "device_math.cuh", "host_math.hpp", "libm_tables.hpp", "upload.hpp", "hostmesh.hpp", "conv_dispatch.hpp", "conv_args.hpp",
                   ABI_HEADER],
-    "conv_ffma.cu": ["conv_ffma.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
+    "conv_ffma.cu": FFMA_HEADERS,
+    "conv_ffma_mid.cu": FFMA_HEADERS,
+    "conv_ffma_wide.cu": FFMA_HEADERS,
     "conv_tc.cu": ["conv_tc.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
     "conv_staged.cu": ["conv_staged.cuh", "tile_plan.cuh", "conv_tc.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
     "conv_window.cu": ["conv_window.cuh", "tile_plan.cuh", "conv_tc.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],

@@ -28,6 +28,7 @@ struct ConvArgs {
     int32_t out_stride;     // rows per planar chunk of `out`
     int32_t out_planar;     // write `out` chunk-planar (needs COUT % 4 == 0 and !out_global)
     int32_t out_split;      // write `out` as fp16 hi/lo parts for a tensor-core consumer: SPLIT_PLANES (COUT % 8 == 0) or SPLIT_ROWS
+    float* const* out_host; // where the batch-wide classifications go instead of `out`: the device address of a pointer to pinned memory
     int32_t* range_flag;    // the engine's abort flags: ABORT_RANGE is raised when a value is too large for the fp16 split
 };
 

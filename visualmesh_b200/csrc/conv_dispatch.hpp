@@ -61,6 +61,7 @@ struct LaunchPlans {
 // ---- conv_ffma.cu: layers on the CUDA cores ----------------------------------------------------------------------
 // a specialised kernel exists for this shape (anything else runs the generic kernel, which ignores ConvArgs::out_split)
 bool has_fast_ffma_kernel(int cin, int cout);
+bool ffma_stores_to_host(const DenseLayer& L);  // the layer's kernel honours ConvArgs::out_host
 void launch_conv_ffma(const DenseLayer& L, const ConvArgs& a, int n_frames, int max_rows, cudaStream_t s);
 
 // ---- conv_tc.cu: layers on the tensor cores, gather by global loads ----------------------------------------------

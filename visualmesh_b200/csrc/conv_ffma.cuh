@@ -135,6 +135,23 @@ __global__ void __launch_bounds__(T, MINB) k_graph_conv(const ConvArgs a) {
     }
 }
 
+// The last layer's results straight into pinned host memory. The rows of a block lie one after another there; threads that stored
+// their own would send the bus pieces of a few bytes, so the block arranges them in shared memory first and writes whole lines.
+// All threads call; stage holds T * R rows. rows_left: rows of the frame from the block's first on.
+template <int R, int T, int COUTP>
+__device__ __forceinline__ void store_rows_to_host(float* dst, int rows_left, int cout, const float (&v)[R][COUTP], float* stage) {
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+#pragma unroll
+        for (int j = 0; j < COUTP; ++j) {
+            if (j < cout) stage[(q * T + static_cast<int>(threadIdx.x)) * cout + j] = v[q][j];
+        }
+    }
+    __syncthreads();
+    const int words = min(rows_left, T * R) * cout;
+    for (int k = threadIdx.x; k < words; k += T) dst[k] = stage[k];
+}
+
 // The same layer with the weights in the kernel's parameter space (constant bank) instead of shared memory: every
 // weight read is a constant-cache load that all lanes share and does not touch the L1/shared data path that the
 // gather loads. Layers whose weights fit the parameter space (WMAX floats).
@@ -165,7 +182,7 @@ template <int CIN, int COUT, int R, int WMAX, int T = CONV_THREADS, int NS = 0>
 __global__ void __launch_bounds__(T, (CIN == 8 && COUT <= 8 && T == 256) ? 6 : 0) k_graph_conv_cw(const ConvArgs a, const __grid_constant__ ConvWeights<WMAX> wp) {
     static_assert(CIN % 4 == 0, "vector loads of the input rows");
     constexpr int COUTP = (COUT + 3) & ~3;
-    extern __shared__ uint4 split_stage[];  // SPLIT_ROW_STAGE bytes per warp when the output is split in rows
+    extern __shared__ uint4 split_stage[];  // SPLIT_ROW_STAGE bytes per warp when the output is split in rows; the results for the host
     const int frame_in_chunk = blockIdx.y;
     const int frame          = a.f0 + frame_in_chunk;
     const int start          = a.offsets[frame];
@@ -219,6 +236,17 @@ __global__ void __launch_bounds__(T, (CIN == 8 && COUT <= 8 && T == 256) ? 6 : 0
         }
     }
     const size_t out_base = a.out_global ? nb_base : static_cast<size_t>(local_base);
+    if (COUT <= 16 && a.out_host != nullptr) {
+        float v[R][COUTP];
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+#pragma unroll
+            for (int j = 0; j < COUTP / 2; ++j) unpack2(acc[q][j], v[q][2 * j], v[q][2 * j + 1]);
+            activate<COUT>(v[q], a.activation);
+        }
+        store_rows_to_host<R, T>(*a.out_host + (out_base + first) * COUT, rows - first, COUT, v, reinterpret_cast<float*>(split_stage));
+        return;
+    }
 #pragma unroll
     for (int q = 0; q < R; ++q) {
         const int i = first + q * T + static_cast<int>(threadIdx.x);
@@ -258,7 +286,8 @@ __global__ void __launch_bounds__(T, (CIN == 8 && COUT <= 8 && T == 256) ? 6 : 0
 // Layers whose widths are multiples of 4 up to 32 but have no kernel of their own: the padded output width is a template parameter,
 // the input width is not. Input chunks come in batches of four, the next batch (and the next slot's neighbour index) on its way
 // while one is multiplied: with one row per thread an SM holds few warps, and what bounds the layer is the chain of its gathers.
-// Weights in the parameter space as above. Measured on 29 k rows with four neighbours, against the
+// With two rows per thread the weights are in the parameter space as above. With one (few rows) they are in shared memory: the constant
+// cache holds 2 KB of them, and with a few warps per SM nothing hides its misses (24 -> 20 on 29 k rows: ANY_SHARED). Measured on 29 k rows with four neighbours, against the
 // kernel that reads its weights through the cache: 24 -> 20 85 -> 21 us, 20 -> 12 47 -> 15 us, 4 -> 24 30 -> 13 us.
 template <int COUTP, int R, int T, int WMAX>
 __global__ void __launch_bounds__(T) k_graph_conv_any(const ConvArgs a, int32_t cin4, int32_t cout, const __grid_constant__ ConvWeights<WMAX> wp) {
@@ -290,6 +319,12 @@ __global__ void __launch_bounds__(T) k_graph_conv_any(const ConvArgs a, int32_t 
         }
     };
     const int biases = a.n_slots * cin4 * 4 * COUTP;
+    extern __shared__ float4 smem4[];  // the weights (one row per thread), the results for the host
+    constexpr bool SHARED = R == 1;
+    const float* w_s      = reinterpret_cast<const float*>(smem4);
+    auto weights = [&](int at) -> unsigned long long {
+        return SHARED ? *reinterpret_cast<const unsigned long long*>(w_s + at) : pack2(wp.w[at], wp.w[at + 1]);
+    };
 #pragma unroll
     for (int q = 0; q < R; ++q) {
         row[q] = min(first + q * T + static_cast<int>(threadIdx.x), rows - 1);
@@ -299,6 +334,11 @@ __global__ void __launch_bounds__(T) k_graph_conv_any(const ConvArgs a, int32_t 
     }
     if (a.n_slots > 1) fetch_index(1);
     fetch(0);
+    if (SHARED) {
+        const float4* from = reinterpret_cast<const float4*>(a.weights);
+        for (int i = threadIdx.x; i < biases / 4; i += T) smem4[i] = __ldg(from + i);
+        __syncthreads();
+    }
     int at = 0;  // weights of the channel
     for (int s = 0; s < a.n_slots; ++s) {
         for (int c = 0; c < cin4; c += BATCH) {
@@ -327,7 +367,7 @@ __global__ void __launch_bounds__(T) k_graph_conv_any(const ConvArgs a, int32_t 
                     }
 #pragma unroll
                     for (int j = 0; j < COUTP / 2; ++j) {
-                        const unsigned long long w = pack2(wp.w[at + 2 * j], wp.w[at + 2 * j + 1]);
+                        const unsigned long long w = weights(at + 2 * j);
 #pragma unroll
                         for (int q = 0; q < R; ++q) ffma2(acc[q][j], xx[q], w);
                     }
@@ -337,47 +377,55 @@ __global__ void __launch_bounds__(T) k_graph_conv_any(const ConvArgs a, int32_t 
         }
     }
     const size_t out_base = a.out_global ? nb_base : static_cast<size_t>(local_base);
+    float v[R][COUTP];
 #pragma unroll
     for (int q = 0; q < R; ++q) {
-        const int i = first + q * T + static_cast<int>(threadIdx.x);
-        if (i >= rows) continue;
-        float v[COUTP];
 #pragma unroll
-        for (int j = 0; j < COUTP / 2; ++j) unpack2(acc[q][j], v[2 * j], v[2 * j + 1]);
+        for (int j = 0; j < COUTP / 2; ++j) unpack2(acc[q][j], v[q][2 * j], v[q][2 * j + 1]);
         if (a.activation == VM_SOFTMAX) {
             float total = 0.0f;
 #pragma unroll
             for (int j = 0; j < COUTP; ++j) {
                 if (j < cout) {
-                    v[j]  = expf(v[j]);
-                    total = __fadd_rn(total, v[j]);
+                    v[q][j] = expf(v[q][j]);
+                    total   = __fadd_rn(total, v[q][j]);
                 }
             }
 #pragma unroll
-            for (int j = 0; j < COUTP; ++j) v[j] = __fdiv_rn(v[j], total);
+            for (int j = 0; j < COUTP; ++j) v[q][j] = __fdiv_rn(v[q][j], total);
         }
         else {
-            activate<COUTP>(v, a.activation);
+            activate<COUTP>(v[q], a.activation);
         }
+    }
+    if (a.out_host != nullptr) {
+        if (SHARED) __syncthreads();  // the weights have been read
+        store_rows_to_host<R, T>(*a.out_host + (out_base + first) * cout, rows - first, cout, v, reinterpret_cast<float*>(smem4));
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        const int i = first + q * T + static_cast<int>(threadIdx.x);
+        if (i >= rows) continue;
         if (a.out_planar) {
             float4* out4 = reinterpret_cast<float4*>(a.out);
 #pragma unroll
             for (int j4 = 0; j4 < COUTP / 4; ++j4) {
-                out4[static_cast<size_t>(j4) * a.out_stride + out_base + i] = make_float4(v[j4 * 4], v[j4 * 4 + 1], v[j4 * 4 + 2], v[j4 * 4 + 3]);
+                out4[static_cast<size_t>(j4) * a.out_stride + out_base + i] = make_float4(v[q][j4 * 4], v[q][j4 * 4 + 1], v[q][j4 * 4 + 2], v[q][j4 * 4 + 3]);
             }
         }
         else {
             float* dst = a.out + (out_base + i) * cout;
 #pragma unroll
             for (int j = 0; j < COUTP; ++j) {
-                if (j < cout) dst[j] = v[j];
+                if (j < cout) dst[j] = v[q][j];
             }
         }
     }
 }
 
 // Any layer shape: one row per thread, outputs in tiles of 8, weights read through the read-only cache.
-__global__ void __launch_bounds__(CONV_THREADS) k_graph_conv_generic(const ConvArgs a, int32_t cin, int32_t cout, int32_t coutp) {
+static __global__ void __launch_bounds__(CONV_THREADS) k_graph_conv_generic(const ConvArgs a, int32_t cin, int32_t cout, int32_t coutp) {
     const int frame_in_chunk = blockIdx.y;
     const int frame          = a.f0 + frame_in_chunk;
     const int start          = a.offsets[frame];

@@ -340,7 +340,8 @@ static void run_network(vm_engine* e,
                         int max_rows,
                         float* out_final,
                         bool final_global,
-                        int feature_stride) {
+                        int feature_stride,
+                        float* const* out_host = nullptr) {
     // Which kernel runs each layer (VMCUDA_TC: 0 = CUDA cores only; 1, the default, and 2 = tensor cores too).
     // A 16-channel layer whose producer can write the split layout runs as a staged layer (conv_staged.cuh), a dense one with 32
     // channels in on the window kernel (conv_window.cuh; VMCUDA_STAGED=0 turns both off). Otherwise the tcgen05 kernels take a layer when its contraction is dense enough to
@@ -381,6 +382,7 @@ static void run_network(vm_engine* e,
         a.out_stride   = feature_stride;
         a.out_planar   = (!last && e->layers[l].cout % 4 == 0) ? 1 : 0;
         a.out_split    = last ? SPLIT_NONE : kind[l + 1] == CONV_TC_WINDOW ? SPLIT_ROWS : kind[l + 1] >= CONV_TC_SPLIT ? SPLIT_PLANES : SPLIT_NONE;
+        a.out_host     = last ? out_host : nullptr;
         a.range_flag   = e->flags;
         launch_conv(e, e->layers[l], a, n_frames, max_rows, lane.stream, kind[l], plan);
         cur ^= 1;
@@ -743,11 +745,15 @@ static void issue_projection(vm_engine* e, Lane& lane, const Chunk& c, bool samp
     if (fork) VM_CUDA(cudaStreamWaitEvent(s, lane.ev_join, 0));
 }
 
-// All layers, and the classifications to the host when they are wanted there.
+// All layers, and the classifications to the host when they are wanted there: by the last layer itself where its kernel can (one kernel
+// and one trip through memory less: EXPORT_MEASURED).
 static void issue_layers(vm_engine* e, Lane& lane, const Chunk& c, bool sample) {
     if (sample) issue_sample(e, lane, c, lane.stream);
-    run_network(e, lane, c.with_plan, e->d_offsets.p, e->d_nb.p, c.n_neighbours, c.f0, c.f1 - c.f0, c.max_rows, e->d_cls.p, true, c.stride);
-    if (!c.exported) return;
+    const DenseLayer& last = e->layers.back();
+    const bool direct      = c.exported && ffma_stores_to_host(last) && (last.tc_np == 0 || !e->use_tc || e->tc_mode == 1) && last.cin * last.cout < e->tc_min_product;
+    float* const* to_host  = reinterpret_cast<float* const*>(lane.d_staging.p + offsetof(ChunkHeader, cls));
+    run_network(e, lane, c.with_plan, e->d_offsets.p, e->d_nb.p, c.n_neighbours, c.f0, c.f1 - c.f0, c.max_rows, e->d_cls.p, true, c.stride, direct ? to_host : nullptr);
+    if (!c.exported || direct) return;
     begin_stage(e, lane.stream, "export_classes");
     k_export<1><<<EXPORT_BLOCKS, EXPORT_THREADS, 0, lane.stream>>>(device_header(lane), e->d_offsets.p, c.f0, c.f1, e->n_classes, nullptr, nullptr, e->d_cls.p);
     end_stage(e, lane.stream);
