@@ -285,10 +285,7 @@ __global__ void __launch_bounds__(T, (CIN == 8 && COUT <= 8 && T == 256) ? 6 : 0
 
 // Layers whose widths are multiples of 4 up to 32 but have no kernel of their own: the padded output width is a template parameter,
 // the input width is not. Input chunks come in batches of four, the next batch (and the next slot's neighbour index) on its way
-// while one is multiplied: with one row per thread an SM holds few warps, and what bounds the layer is the chain of its gathers.
-// With two rows per thread the weights are in the parameter space as above. With one (few rows) they are in shared memory: the constant
-// cache holds 2 KB of them, and with a few warps per SM nothing hides its misses (24 -> 20 on 29 k rows: ANY_SHARED). Measured on 29 k rows with four neighbours, against the
-// kernel that reads its weights through the cache: 24 -> 20 85 -> 21 us, 20 -> 12 47 -> 15 us, 4 -> 24 30 -> 13 us.
+// while one is multiplied. Weights in the parameter space as above.
 template <int COUTP, int R, int T, int WMAX>
 __global__ void __launch_bounds__(T) k_graph_conv_any(const ConvArgs a, int32_t cin4, int32_t cout, const __grid_constant__ ConvWeights<WMAX> wp) {
     constexpr int BATCH      = 4;  // chunks of 4 channels
@@ -319,12 +316,7 @@ __global__ void __launch_bounds__(T) k_graph_conv_any(const ConvArgs a, int32_t 
         }
     };
     const int biases = a.n_slots * cin4 * 4 * COUTP;
-    extern __shared__ float4 smem4[];  // the weights (one row per thread), the results for the host
-    constexpr bool SHARED = R == 1;
-    const float* w_s      = reinterpret_cast<const float*>(smem4);
-    auto weights = [&](int at) -> unsigned long long {
-        return SHARED ? *reinterpret_cast<const unsigned long long*>(w_s + at) : pack2(wp.w[at], wp.w[at + 1]);
-    };
+    extern __shared__ float4 smem4[];  // the results for the host
 #pragma unroll
     for (int q = 0; q < R; ++q) {
         row[q] = min(first + q * T + static_cast<int>(threadIdx.x), rows - 1);
@@ -334,11 +326,6 @@ __global__ void __launch_bounds__(T) k_graph_conv_any(const ConvArgs a, int32_t 
     }
     if (a.n_slots > 1) fetch_index(1);
     fetch(0);
-    if (SHARED) {
-        const float4* from = reinterpret_cast<const float4*>(a.weights);
-        for (int i = threadIdx.x; i < biases / 4; i += T) smem4[i] = __ldg(from + i);
-        __syncthreads();
-    }
     int at = 0;  // weights of the channel
     for (int s = 0; s < a.n_slots; ++s) {
         for (int c = 0; c < cin4; c += BATCH) {
@@ -367,7 +354,7 @@ __global__ void __launch_bounds__(T) k_graph_conv_any(const ConvArgs a, int32_t 
                     }
 #pragma unroll
                     for (int j = 0; j < COUTP / 2; ++j) {
-                        const unsigned long long w = weights(at + 2 * j);
+                        const unsigned long long w = pack2(wp.w[at + 2 * j], wp.w[at + 2 * j + 1]);
 #pragma unroll
                         for (int q = 0; q < R; ++q) ffma2(acc[q][j], xx[q], w);
                     }
@@ -399,7 +386,6 @@ __global__ void __launch_bounds__(T) k_graph_conv_any(const ConvArgs a, int32_t 
         }
     }
     if (a.out_host != nullptr) {
-        if (SHARED) __syncthreads();  // the weights have been read
         store_rows_to_host<R, T>(*a.out_host + (out_base + first) * cout, rows - first, cout, v, reinterpret_cast<float*>(smem4));
         return;
     }
@@ -420,6 +406,131 @@ __global__ void __launch_bounds__(T) k_graph_conv_any(const ConvArgs a, int32_t 
             for (int j = 0; j < COUTP; ++j) {
                 if (j < cout) dst[j] = v[q][j];
             }
+        }
+    }
+}
+
+// Few rows: a block owns 128 rows and OW of the outputs (blockIdx.z), a thread one row. With all outputs of a row to a thread an SM would
+// hold a block or two, four to eight warps, too few to hide either the gather or the arithmetic's own latency; part of the outputs
+// makes it three or four times as many, each with a chain as much shorter (the rows read again come from the L1 cache). The weights of
+// those outputs sit in shared memory. Input chunks come in batches of four, the next batch (and the next slot's neighbour index) on its
+// way while one is multiplied.
+template <int OW, int T>
+__global__ void __launch_bounds__(T) k_graph_conv_few(const ConvArgs a, int32_t cin4, int32_t cout, int32_t coutp) {
+    constexpr int BATCH      = 4;  // chunks of 4 channels
+    const int frame_in_chunk = blockIdx.y;
+    const int frame          = a.f0 + frame_in_chunk;
+    const int start          = a.offsets[frame];
+    const int rows           = a.offsets[frame + 1] - start + 1;
+    const int first          = blockIdx.x * T;
+    if (first >= rows) return;
+    const int local_base = start - a.offsets[a.f0] + frame_in_chunk;
+    const size_t nb_base = static_cast<size_t>(start + frame);
+    const float4* in4    = reinterpret_cast<const float4*>(a.in);
+    const int o0         = blockIdx.z * OW;
+    extern __shared__ float4 smem4[];  // weights [channel][OW], then the results for the host
+
+    const int i   = first + static_cast<int>(threadIdx.x);
+    const int row = min(i, rows - 1);
+    int src = local_base + row, next_src = src;
+    float4 next[BATCH];
+    auto fetch_index = [&](int s) { next_src = local_base + __ldg(a.nb + (nb_base + row) * a.n_neighbours + (s - 1)); };
+    auto fetch       = [&](int c) {
+#pragma unroll
+        for (int k = 0; k < BATCH; ++k) {
+            if (c + k < cin4) next[k] = __ldg(in4 + static_cast<size_t>(c + k) * a.in_stride + src);
+        }
+    };
+    if (a.n_slots > 1) fetch_index(1);
+    fetch(0);
+    const int channels = a.n_slots * cin4 * 4;
+    for (int k = threadIdx.x; k < channels * (OW / 4); k += T) {
+        const int o = o0 + (k % (OW / 4)) * 4;
+        smem4[k]    = o < coutp ? __ldg(reinterpret_cast<const float4*>(a.weights + static_cast<size_t>(k / (OW / 4)) * coutp + o)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    unsigned long long acc[OW / 2];
+#pragma unroll
+    for (int j = 0; j < OW / 2; ++j) {
+        const bool there = o0 + 2 * j < coutp;
+        acc[j]           = there ? pack2(__ldg(a.biases + o0 + 2 * j), __ldg(a.biases + o0 + 2 * j + 1)) : 0ull;
+    }
+    __syncthreads();
+    const ulonglong2* w = reinterpret_cast<const ulonglong2*>(smem4);  // of the channel
+    auto multiply       = [&](const float4& x) {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            const float xv              = kk == 0 ? x.x : kk == 1 ? x.y : kk == 2 ? x.z : x.w;
+            const unsigned long long xx = pack2(xv, xv);
+#pragma unroll
+            for (int j = 0; j < OW / 4; ++j) {
+                const ulonglong2 w2 = w[kk * (OW / 4) + j];
+                ffma2(acc[2 * j], xx, w2.x);
+                ffma2(acc[2 * j + 1], xx, w2.y);
+            }
+        }
+        w += OW;
+    };
+    for (int s = 0; s < a.n_slots; ++s) {
+        for (int c = 0; c < cin4; c += BATCH) {
+            float4 x[BATCH];
+#pragma unroll
+            for (int k = 0; k < BATCH; ++k) x[k] = next[k];
+            if (c + BATCH < cin4) { fetch(c + BATCH); }
+            else if (s + 1 < a.n_slots) {
+                src = next_src;
+                fetch(0);
+                if (s + 2 < a.n_slots) fetch_index(s + 2);
+            }
+            if (c + BATCH <= cin4) {
+#pragma unroll
+                for (int k = 0; k < BATCH; ++k) multiply(x[k]);
+            }
+            else {
+#pragma unroll
+                for (int k = 0; k < BATCH - 1; ++k) {
+                    if (c + k < cin4) multiply(x[k]);
+                }
+            }
+        }
+    }
+    const size_t out_base = a.out_global ? nb_base : static_cast<size_t>(local_base);
+    float v[1][OW];
+#pragma unroll
+    for (int j = 0; j < OW / 2; ++j) unpack2(acc[j], v[0][2 * j], v[0][2 * j + 1]);
+    if (a.activation == VM_SOFTMAX) {  // all outputs are this block's
+        float total = 0.0f;
+#pragma unroll
+        for (int j = 0; j < OW; ++j) {
+            if (j < cout) {
+                v[0][j] = expf(v[0][j]);
+                total   = __fadd_rn(total, v[0][j]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < OW; ++j) v[0][j] = __fdiv_rn(v[0][j], total);
+    }
+    else {
+        activate<OW>(v[0], a.activation);
+    }
+    if (a.out_host != nullptr) {
+        store_rows_to_host<1, T>(*a.out_host + (out_base + first) * cout, rows - first, cout, v, reinterpret_cast<float*>(smem4 + channels * (OW / 4)));
+        return;
+    }
+    if (i >= rows) return;
+    if (a.out_planar) {
+        float4* out4 = reinterpret_cast<float4*>(a.out);
+#pragma unroll
+        for (int j4 = 0; j4 < OW / 4; ++j4) {
+            if (o0 + j4 * 4 < coutp) {
+                out4[static_cast<size_t>(o0 / 4 + j4) * a.out_stride + out_base + i] = make_float4(v[0][j4 * 4], v[0][j4 * 4 + 1], v[0][j4 * 4 + 2], v[0][j4 * 4 + 3]);
+            }
+        }
+    }
+    else {
+        float* dst = a.out + (out_base + i) * cout;
+#pragma unroll
+        for (int j = 0; j < OW; ++j) {
+            if (o0 + j < cout) dst[o0 + j] = v[0][j];
         }
     }
 }

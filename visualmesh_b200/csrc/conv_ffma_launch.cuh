@@ -24,6 +24,7 @@ bool launch_conv_narrow(const DenseLayer& L, const ConvArgs& a, dim3 grid, int m
 bool launch_conv_mid(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s);
 bool launch_conv_wide(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s);
 bool launch_conv_any(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s);
+bool launch_conv_few(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s);
 
 constexpr int CW_MAX  = 2320;  // floats: a 16 -> 16 layer with 8 neighbours and its biases
 constexpr int CW_MOST = 8120;  // what the parameter space holds beside the other arguments: 28 -> 32 with 8 neighbours
@@ -95,7 +96,7 @@ template <int CIN, int COUT, int RR>
 static bool launch_conv_shape(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s) {
     if (L.cin != CIN || L.cout != COUT) return false;
     if (const_weights() && few_rows(max_rows, grid.y)) {
-        if (L.host_packed.size() > 640 && launch_conv_any(L, a, grid, max_rows, s)) return true;
+        if (L.host_packed.size() > 640 && launch_conv_few(L, a, grid, max_rows, s)) return true;
         if (launch_conv_cw<CIN, COUT, 1, CW_MAX, 128>(L, a, grid, max_rows, s)) return true;
     }
     if (const_weights() && launch_conv_cw<CIN, COUT, 2, CW_MAX, 256>(L, a, grid, max_rows, s)) return true;

