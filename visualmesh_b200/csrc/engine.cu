@@ -119,6 +119,7 @@ struct Lane {
     cudaStream_t side   = nullptr;     // runs beside `stream` within a chunk: sampling next to the neighbour remap, result copies
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaEvent_t ev_offsets = nullptr;  // this chunk's offsets are on the device
+    cudaEvent_t ev_projected = nullptr;  // everything of its projection is
     cudaEvent_t ev_images  = nullptr;  // its images are
     cudaEvent_t ev_done    = nullptr;  // everything of this chunk, result copies included, has finished
     bool busy = false;
@@ -685,9 +686,15 @@ static const ChunkHeader* device_header(const Lane& lane) {
 // Exported arrays are copied by a few blocks that leave the SMs to the layers: 32 blocks of 512 threads keep the bus busy.
 constexpr int EXPORT_BLOCKS = 32;
 
-static void issue_export_points(vm_engine* e, Lane& lane, const Chunk& c, cudaStream_t s) {
+static void issue_export_points(vm_engine* e, Lane& lane, const Chunk& c, cudaStream_t s, bool neighbours) {
     begin_stage(e, s, "export_points");
-    k_export<0><<<EXPORT_BLOCKS, EXPORT_THREADS, 0, s>>>(device_header(lane), e->d_offsets.p, c.f0, c.f1, c.n_neighbours, e->d_px.p, e->d_gi.p, e->d_nb.p);
+    k_export<0><<<EXPORT_BLOCKS, EXPORT_THREADS, 0, s>>>(device_header(lane), e->d_offsets.p, c.f0, c.f1, c.n_neighbours, e->d_px.p, e->d_gi.p,
+                                                         neighbours ? e->d_nb.p : nullptr);
+    end_stage(e, s);
+}
+static void issue_export_neighbours(vm_engine* e, Lane& lane, const Chunk& c, cudaStream_t s) {
+    begin_stage(e, s, "export_neighbours");
+    k_export<2><<<EXPORT_BLOCKS, EXPORT_THREADS, 0, s>>>(device_header(lane), e->d_offsets.p, c.f0, c.f1, c.n_neighbours, nullptr, nullptr, e->d_nb.p);
     end_stage(e, s);
 }
 
@@ -702,9 +709,24 @@ static void issue_sample(vm_engine* e, Lane& lane, const Chunk& c, cudaStream_t 
     end_stage(e, s);
 }
 
+static void issue_remap(vm_engine* e, Lane& lane, const Chunk& c) {
+    cudaStream_t s = lane.stream;
+    const dim3 g((c.max_rows + ROW_THREADS - 1) / ROW_THREADS, c.f1 - c.f0);
+    const st::PlanOut plan = c.with_plan ? tile_plan(lane) : st::PlanOut{nullptr, nullptr, nullptr};
+    begin_stage(e, s, "remap_neighbours");
+#define VM_REMAP(NN)                                                                                                                      \
+    if (c.n_neighbours == NN) {                                                                                                           \
+        if (c.with_plan) k_remap<NN, true><<<g, ROW_THREADS, 0, s>>>(device_frames(lane), e->d_offsets.p, c.f0, e->d_gi.p, lane.d_node_rank.p, e->d_nb.p, plan); \
+        else k_remap<NN, false><<<g, ROW_THREADS, 0, s>>>(device_frames(lane), e->d_offsets.p, c.f0, e->d_gi.p, lane.d_node_rank.p, e->d_nb.p, plan);  \
+    }
+    VM_REMAP(4) VM_REMAP(6) VM_REMAP(8)
+#undef VM_REMAP
+    end_stage(e, s);
+}
+
 // Staging copy, lookup, projection, compaction, neighbour remap; images that are on the device already are sampled beside the
 // remap (neither needs the other: 178 -> 140 us on 4.4 M rows).
-static void issue_projection(vm_engine* e, Lane& lane, const Chunk& c, bool sample) {
+static void issue_projection(vm_engine* e, Lane& lane, const Chunk& c, bool sample, bool remap = true) {
     cudaStream_t s            = lane.stream;
     const int nf              = c.f1 - c.f0;
     const FrameParams* frames = device_frames(lane);
@@ -724,24 +746,20 @@ static void issue_projection(vm_engine* e, Lane& lane, const Chunk& c, bool samp
       frames, device_header(lane), lane.d_cand_px.p, lane.d_cand_node.p, lane.d_block_counts.p, groups, c.blocks_per_frame, c.n_groups, e->d_offsets.p,
       c.f0, e->d_px.p, e->d_gi.p, lane.d_node_rank.p);
     end_stage(e, s);
-    const bool fork = sample && !e->timing;
+    if (!remap) return;
+    // What the scatter leaves can go to the host while the remap runs: a chunk that only projects has nothing else to overlap the bus
+    // with (RING8, 1193 pixels wide, six cameras: 443 -> 427 us; with layers to overlap, the second kernel costs what it saves).
+    const bool early = !c.classify && c.exported && !e->timing;
+    const bool fork  = (sample && !e->timing) || early;
     if (fork) {
         VM_CUDA(cudaEventRecord(lane.ev_fork, s));
         VM_CUDA(cudaStreamWaitEvent(lane.side, lane.ev_fork, 0));
     }
     if (sample) issue_sample(e, lane, c, fork ? lane.side : s);
+    if (early) issue_export_points(e, lane, c, lane.side, false);
     if (fork) VM_CUDA(cudaEventRecord(lane.ev_join, lane.side));
-    const dim3 g((c.max_rows + ROW_THREADS - 1) / ROW_THREADS, nf);
-    const st::PlanOut plan = c.with_plan ? tile_plan(lane) : st::PlanOut{nullptr, nullptr, nullptr};
-    begin_stage(e, s, "remap_neighbours");
-#define VM_REMAP(NN)                                                                                                                      \
-    if (c.n_neighbours == NN) {                                                                                                           \
-        if (c.with_plan) k_remap<NN, true><<<g, ROW_THREADS, 0, s>>>(frames, e->d_offsets.p, c.f0, e->d_gi.p, lane.d_node_rank.p, e->d_nb.p, plan); \
-        else k_remap<NN, false><<<g, ROW_THREADS, 0, s>>>(frames, e->d_offsets.p, c.f0, e->d_gi.p, lane.d_node_rank.p, e->d_nb.p, plan);  \
-    }
-    VM_REMAP(4) VM_REMAP(6) VM_REMAP(8)
-#undef VM_REMAP
-    end_stage(e, s);
+    issue_remap(e, lane, c);
+    if (early) issue_export_neighbours(e, lane, c, s);
     if (fork) VM_CUDA(cudaStreamWaitEvent(s, lane.ev_join, 0));
 }
 
@@ -779,7 +797,7 @@ static GraphKey graph_key(const vm_engine* e, const Lane& lane, const Chunk& c, 
     k.n_neighbours     = c.n_neighbours;
     k.blocks_per_frame = c.blocks_per_frame;
     k.bsp_blocks       = c.bsp_blocks;
-    k.options          = c.classify | c.exported << 1 | c.device_lookup << 2 | c.packed4 << 3 | c.with_plan << 4 | c.images_apart << 5 | int(e->use_tc) << 6;
+    k.options          = c.classify | c.exported << 1 | c.device_lookup << 2 | c.packed4 << 3 | c.with_plan << 4 | c.images_apart << 5 | int(e->use_tc) << 6 | c.copied << 7;
     k.wait_limit       = e->tc_wait_limit;
     k.feature_stride   = c.stride;
     k.staging_bytes    = c.staging_bytes;
@@ -874,19 +892,24 @@ static Chunk enqueue_chunk(vm_engine* e, Lane& lane, Lane* prev, bool after_prev
                 VM_CUDA(cudaEventRecord(lane.ev_fork, lane.stream));
                 VM_CUDA(cudaStreamWaitEvent(lane.side, lane.ev_fork, 0));
             }
-            if (c.exported) issue_export_points(e, lane, c, fork ? lane.side : lane.stream);
+            if (c.exported && (classify || e->timing)) issue_export_points(e, lane, c, fork ? lane.side : lane.stream, true);
             if (fork) VM_CUDA(cudaEventRecord(lane.ev_join, lane.side));
             if (classify) issue_layers(e, lane, c, false);
             if (fork) VM_CUDA(cudaStreamWaitEvent(lane.stream, lane.ev_join, 0));
         });
     }
     else {
-        run_part(e, lane, c, PART_PROJECTION, [&] { issue_projection(e, lane, c, classify && !c.images_apart); });
+        // results that are copied once their number is known, and no layers beside which to copy them: the copies begin before the remap
+        // (six cameras of 1280 x 1024, 14 MB: 338 -> 332 us)
+        const bool split = !classify && c.copied;
+        run_part(e, lane, c, PART_PROJECTION, [&] { issue_projection(e, lane, c, classify && !c.images_apart, !split); });
         VM_CUDA(cudaEventRecord(lane.ev_offsets, lane.stream));
+        if (split) issue_remap(e, lane, c);
+        VM_CUDA(cudaEventRecord(lane.ev_projected, lane.stream));
         if (c.exported) {
             cudaStream_t beside = e->timing ? lane.stream : lane.side;
             VM_CUDA(cudaStreamWaitEvent(beside, lane.ev_offsets, 0));
-            issue_export_points(e, lane, c, beside);
+            issue_export_points(e, lane, c, beside, true);
             VM_CUDA(cudaEventRecord(lane.ev_join, beside));
         }
         if (upload != nullptr) upload->finish();
@@ -916,6 +939,7 @@ static void copy_results(vm_engine* e, Lane& lane, const Chunk& c) {
         VM_CUDA(cudaMemcpyAsync(to.px.p + p0, e->d_px.p + p0, sizeof(float2) * (p1 - p0), cudaMemcpyDeviceToHost, beside));
         VM_CUDA(cudaMemcpyAsync(to.gi.p + p0, e->d_gi.p + p0, sizeof(int32_t) * (p1 - p0), cudaMemcpyDeviceToHost, beside));
     }
+    VM_CUDA(cudaStreamWaitEvent(beside, lane.ev_projected, 0));
     VM_CUDA(cudaMemcpyAsync(to.nb.p + r0 * N, e->d_nb.p + r0 * N, sizeof(int32_t) * (r1 - r0) * N, cudaMemcpyDeviceToHost, beside));
     if (c.classify) VM_CUDA(cudaMemcpyAsync(to.cls.p + r0 * C, e->d_cls.p + r0 * C, sizeof(float) * (r1 - r0) * C, cudaMemcpyDeviceToHost, lane.stream));
     if (beside != lane.stream) {
@@ -1213,7 +1237,7 @@ vm_status vm_engine_create(int device, const vm_layer* layers, const int32_t* la
             Lane& lane = e->lanes[l];
             VM_CUDA(cudaStreamCreateWithFlags(&lane.stream, cudaStreamNonBlocking));
             VM_CUDA(cudaStreamCreateWithFlags(&lane.side, cudaStreamNonBlocking));
-            for (cudaEvent_t* ev : {&lane.ev_fork, &lane.ev_join, &lane.ev_images}) VM_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
+            for (cudaEvent_t* ev : {&lane.ev_fork, &lane.ev_join, &lane.ev_images, &lane.ev_projected}) VM_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
             // the events the host waits on: spinning (lowest latency) or, with VMCUDA_BLOCKING_SYNC=1, sleeping - for boxes where
             // several engines' host threads share few cores
             for (cudaEvent_t* ev : {&lane.ev_offsets, &lane.ev_done}) {
@@ -1373,7 +1397,7 @@ void vm_engine_destroy(vm_engine* e) {
         lane.d_halo_count.release();
         if (lane.stream) cudaStreamDestroy(lane.stream);
         if (lane.side) cudaStreamDestroy(lane.side);
-        for (cudaEvent_t ev : {lane.ev_fork, lane.ev_join, lane.ev_offsets, lane.ev_images, lane.ev_done})
+        for (cudaEvent_t ev : {lane.ev_fork, lane.ev_join, lane.ev_offsets, lane.ev_projected, lane.ev_images, lane.ev_done})
             if (ev) cudaEventDestroy(ev);
     }
     if (e->copy_stream) cudaStreamDestroy(e->copy_stream);

@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(ROW_THREADS) k_sample(const FrameParams* __res
 // ---- results to the host -----------------------------------------------------------------------------------------
 // Writes a chunk's results into pinned host memory. The device knows how many there are, so the copy needs no count on the host
 // and no wait for one in the middle of a call; the bus takes 64 KB in 3 us more than a copy engine would and 5 MB in 10 us more
-// (112 us against 102). WHICH: 0 = pixel coordinates, node indices and neighbourhood; 1 = classifications.
+// (112 us against 102). WHICH: 0 = pixel coordinates, node indices and (rows given) neighbourhood, 1 = classifications, 2 = neighbourhood.
 __device__ __forceinline__ void export_words(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, size_t begin, size_t end) {
     // 16-byte pieces between the first and the last whole one (both arrays start on 256-byte boundaries), words at the ends
     const size_t first = (begin + 3) / 4, last = end / 4;
@@ -394,8 +394,9 @@ __global__ void __launch_bounds__(EXPORT_THREADS) k_export(const ChunkHeader* __
     if (WHICH == 0) {
         export_words(reinterpret_cast<uint32_t*>(header->px), reinterpret_cast<const uint32_t*>(px), 2 * p0, 2 * p1);
         export_words(reinterpret_cast<uint32_t*>(header->gi), reinterpret_cast<const uint32_t*>(gi), p0, p1);
+        if (rows == nullptr) return;
     }
-    uint32_t* dst = WHICH == 0 ? reinterpret_cast<uint32_t*>(header->nb) : reinterpret_cast<uint32_t*>(header->cls);
+    uint32_t* dst = WHICH == 1 ? reinterpret_cast<uint32_t*>(header->cls) : reinterpret_cast<uint32_t*>(header->nb);
     export_words(dst, static_cast<const uint32_t*>(rows), (p0 + f0) * width, (p1 + f1) * width);
 }
 
