@@ -285,7 +285,8 @@ __global__ void __launch_bounds__(T, (CIN == 8 && COUT <= 8 && T == 256) ? 6 : 0
 
 // Layers whose widths are multiples of 4 up to 32 but have no kernel of their own: the padded output width is a template parameter,
 // the input width is not. Input chunks come in batches of four, the next batch (and the next slot's neighbour index) on its way
-// while one is multiplied. Weights in the parameter space as above.
+// while one is multiplied. Weights in the parameter space as above. Measured on 29 k rows with four neighbours, against the kernel that
+// reads its weights through the cache: 24 -> 20 85 -> 21 us, 20 -> 12 47 -> 15 us, 4 -> 24 30 -> 13 us.
 template <int COUTP, int R, int T, int WMAX>
 __global__ void __launch_bounds__(T) k_graph_conv_any(const ConvArgs a, int32_t cin4, int32_t cout, const __grid_constant__ ConvWeights<WMAX> wp) {
     constexpr int BATCH      = 4;  // chunks of 4 channels

@@ -22,11 +22,13 @@ static bool launch_conv_few_t(const DenseLayer& L, const ConvArgs& a, dim3 grid_
 }
 bool launch_conv_few(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s) {
     if (L.cin % 4 != 0 || L.cin > 32 || L.coutp > 32 || a.out_split) return false;
-    // eight outputs per block while that makes no more than four blocks per SM (then the arithmetic counts, and what the threads of a
-    // row would do twice); all of them where a row's outputs meet
+    // While eight outputs per block make no more than four blocks per SM: beyond that the arithmetic counts, and what the threads of a row
+    // would do twice (24,20,12,5 with four or six neighbours on 13 k rows 86 -> 80 and 96 -> 86 us a call; with eight on 25 k rows,
+    // which this line leaves to the other kernels, 112 -> 114).
     const int64_t blocks = static_cast<int64_t>((max_rows + 127) / 128) * grid.y * ((L.coutp + 7) / 8);
-    const bool together  = a.activation == VM_SOFTMAX || a.out_host != nullptr || blocks > 4 * 148;
-    const int outputs    = together ? L.coutp : std::min(L.coutp, 8);
+    if (blocks > 4 * 148) return false;
+    // all outputs in a block where a row's outputs meet
+    const int outputs = a.activation == VM_SOFTMAX || a.out_host != nullptr ? L.coutp : std::min(L.coutp, 8);
     if (outputs <= 4) return launch_conv_few_t<4>(L, a, grid, max_rows, s);
     if (outputs <= 8) return launch_conv_few_t<8>(L, a, grid, max_rows, s);
     if (outputs <= 16) return launch_conv_few_t<16>(L, a, grid, max_rows, s);
