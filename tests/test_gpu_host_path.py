@@ -66,6 +66,30 @@ def test_host_ranges_of_changing_poses_leave_nothing_behind():
     engine.close()
 
 
+def test_a_recorded_graph_serves_one_layout_of_the_staging_block_only():
+    """Two shapes whose staging blocks have the same size and all their launches the same grids, but the group counts in another
+    place: 24576 bytes of images against 12288 of images and 12288 of range slots."""
+    case = G.Case("ring4_rectilinear_grey")
+    mesh = Mesh.from_arrays(case.rays, case.nbrs, case.bsp)
+    engine = Engine(case.network)
+    Hoc, code = case.frames[0]["Hoc"], W.fourcc("GREY")
+    everything = np.array([[0, mesh.n_nodes]], np.int32)
+
+    def frame(width, height, ranges):
+        lens = W.Lens((width, height), W.EQUISOLID, 0.35 * width, (0.0, 0.0), (0.0, 0.0), np.pi)
+        return FrameInput(mesh, Hoc, lens, W.random_bytes(width, width * height), code, ranges)
+
+    batches = [[frame(128, 96, None), frame(128, 96, None)], [frame(64, 96, None), frame(64, 96, everything)]]
+    want = [[engine.run_batch([fr]).frame(0) for fr in batch] for batch in batches]
+    assert all(len(w.global_indices) > 100 for batch in want for w in batch)
+    for _ in range(3):
+        for batch, expected in zip(batches, want):
+            out = engine.run_batch(batch)
+            for f in range(2):
+                _same(out.frame(f), expected[f])
+    engine.close()
+
+
 @pytest.mark.parametrize("n_frames", [1, 2, 37])
 def test_batches_left_on_the_device_and_copied_to_the_host_agree(n_frames):
     """Results written to the host by the device (one small chunk), copied by the copy engines (several chunks) and left behind."""

@@ -177,12 +177,14 @@ struct StageTimer {
     cudaEvent_t start, stop;
 };
 
-// What the recorded graph of a chunk's kernels depends on besides the contents of its buffers. Compared byte for byte.
+// What the recorded graph of a chunk's kernels depends on besides the contents of its buffers: everything that ends up in a launch's
+// grid or arguments. Compared byte for byte. The staging block's layout is in it by every offset that a kernel gets (its size alone does
+// not fix where the group counts lie: range slots before them and small images behind them may make up for each other).
 struct GraphKey {
     int32_t part, lane, n_frames, f0, n_neighbours, blocks_per_frame, bsp_blocks, options;
     uint32_t wait_limit;
     int32_t feature_stride;
-    uint64_t staging_bytes;
+    uint64_t staging_bytes, counts_at;
 };
 struct GraphEntry {
     GraphKey key;
@@ -801,6 +803,7 @@ static GraphKey graph_key(const vm_engine* e, const Lane& lane, const Chunk& c, 
     k.wait_limit       = e->tc_wait_limit;
     k.feature_stride   = c.stride;
     k.staging_bytes    = c.staging_bytes;
+    k.counts_at        = c.counts_at;
     return k;
 }
 
