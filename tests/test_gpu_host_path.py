@@ -90,6 +90,30 @@ def test_a_recorded_graph_serves_one_layout_of_the_staging_block_only():
     engine.close()
 
 
+def test_many_frames_with_few_candidates_on_a_mesh_of_many_nodes():
+    """The node tables of the batch's frames together pass 2^31 entries, their candidates are 205 k: a chunk is cut before its
+    32-bit offsets into the node table overflow."""
+    n_nodes, n_frames, part = 8_500_000, 257, 800
+    assert n_nodes * (n_frames - 1) > 2**31
+    rng = np.random.default_rng(7)
+    rays = rng.uniform(-1.0, 1.0, (n_nodes, 3)).astype(np.float32)
+    rays /= np.linalg.norm(rays, axis=1, keepdims=True)
+    near = np.arange(n_nodes, dtype=np.int64)[:, None] + np.array([-2, -1, 1, 2])
+    mesh = Mesh.from_arrays(rays, np.clip(near, 0, n_nodes - 1).astype(np.int32))
+    lens = W.Lens((640, 480), W.EQUIDISTANT, 200.0, (0.0, 0.0), (0.0, 0.0), np.pi)
+    engine = Engine()
+    starts = np.linspace(0, n_nodes - part, n_frames).astype(np.int32)
+    frames = [FrameInput(mesh, W.make_Hoc(-0.01 * f, 0.1, 1.0), lens, None, 0, np.array([[s, s + part]], np.int32)) for f, s in enumerate(starts)]
+    batch = engine.run_batch(frames)
+    got = [batch.frame(f) for f in range(n_frames)]
+    assert sum(len(g.global_indices) for g in got) > 10 * n_frames
+    for f in list(range(0, n_frames, 16)) + [n_frames - 2, n_frames - 1]:
+        want = engine.run_batch([frames[f]]).frame(0)
+        assert np.array_equal(G.bits(got[f].pixel_coordinates), G.bits(want.pixel_coordinates))
+        assert np.array_equal(got[f].global_indices, want.global_indices) and np.array_equal(got[f].neighbourhood, want.neighbourhood)
+    engine.close()
+
+
 @pytest.mark.parametrize("n_frames", [1, 2, 37])
 def test_batches_left_on_the_device_and_copied_to_the_host_agree(n_frames):
     """Results written to the host by the device (one small chunk), copied by the copy engines (several chunks) and left behind."""

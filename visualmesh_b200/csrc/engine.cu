@@ -466,6 +466,7 @@ static size_t aligned(size_t n) {
 
 // Sizes that shape the launches are rounded up (by an eighth at most), so that calls whose poses differ a little share a graph.
 static int64_t rounded(int64_t n) {
+    if (n >= int64_t(1) << 30) return n;  // the next step would pass what the 32-bit indices hold
     int64_t step = 1024;
     while (step * 16 <= n) step *= 2;
     return (n + step - 1) / step * step;
@@ -483,6 +484,11 @@ constexpr int64_t MAX_EXPORT = 16 << 20;
 
 // Host images of one chunk of a batch.
 constexpr size_t CHUNK_IMAGE_BYTES = 21 << 20;
+
+// Nodes, and BSP elements, of the meshes of one chunk's frames. With host ranges the candidates say nothing about either, and the
+// node tables of 256 frames on a mesh of 8.4 M nodes would pass the 32-bit offsets that find them. The limit lies lower: the node table
+// takes 4 bytes a node in every lane (512 MB here; 64 frames on a mesh of 1.7 M nodes fit). One frame is always accepted.
+constexpr int64_t MAX_CHUNK_NODES = int64_t(1) << 27;
 
 struct Chunk {
     int f0 = 0, f1 = 0, n_neighbours = 0;
@@ -1075,13 +1081,18 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
         Chunk last;
         while (f0 < n_frames) {
             int f1 = f0;
-            int64_t c    = 0;
+            int64_t c = 0, nodes = 0, elements = 0;
             size_t bytes = 0;
             while (f1 < n_frames) {
-                const int64_t more      = frame_candidates(frames[f1]);
-                const size_t more_bytes = classify && !frames[f1].image_on_device ? image_bytes(frames[f1]) : 0;
+                const int64_t more          = frame_candidates(frames[f1]);
+                const int64_t more_nodes    = frames[f1].mesh->n_nodes;
+                const int64_t more_elements = frames[f1].ranges == nullptr ? frames[f1].mesh->n_bsp : 0;
+                const size_t more_bytes     = classify && !frames[f1].image_on_device ? image_bytes(frames[f1]) : 0;
+                if (f1 > f0 && (nodes + more_nodes > MAX_CHUNK_NODES || elements + more_elements > MAX_CHUNK_NODES)) break;
                 if (f1 > f0 && (c + more > max_chunk_candidates || f1 - f0 >= max_chunk_frames || (bytes + more_bytes > CHUNK_IMAGE_BYTES && !e->chunk_override))) break;
                 c += more;
+                nodes += more_nodes;
+                elements += more_elements;
                 bytes += more_bytes;
                 ++f1;
             }
