@@ -15,8 +15,10 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -40,6 +42,27 @@ static vm_status fail(vm_status s, const std::string& msg) {
 // the per-frame constants could not be computed: a projection the lens math does not know (the reference throws from
 // unproject, cpp/visualmesh/utility/projection.hpp:224)
 struct UnsupportedLens {};
+
+// The status of the exception in flight: nothing leaves a C entry point as an exception. Called inside a handler.
+static vm_status status_of_exception() {
+    cudaGetLastError();
+    try {
+        throw;
+    }
+    catch (const CudaFailure& f) {
+        const vm_status s = f.code == cudaErrorMemoryAllocation ? VM_ERR_OUT_OF_MEMORY : VM_ERR_CUDA;
+        return fail(s, std::string(cudaGetErrorName(f.code)) + ": " + cudaGetErrorString(f.code) + " in " + f.what);
+    }
+    catch (const UnsupportedLens&) {
+        return fail(VM_ERR_UNSUPPORTED_LENS, "Cannot project: Unknown lens type");
+    }
+    catch (const std::bad_alloc&) {
+        return fail(VM_ERR_OUT_OF_MEMORY, "out of host memory");
+    }
+    catch (const std::exception& x) {
+        return fail(VM_ERR_CUDA, x.what());
+    }
+}
 
 // Grow-only device and pinned-host arrays (the reference's OpenCL engine keeps the same kind of caches,
 // cpp/visualmesh/engine/opencl/engine.hpp:740-835).
@@ -162,6 +185,9 @@ struct Results {
 constexpr int MAX_KEPT_RESULTS = 4;
 static_assert(MAX_KEPT_RESULTS == VM_MAX_KEPT_RESULTS, "as the header says");
 struct ResultPool {
+    ResultPool() {
+        free.reserve(MAX_KEPT_RESULTS + 1);  // all sets there can be: giving one back allocates nothing
+    }
     std::mutex mutex;
     std::vector<std::unique_ptr<Results>> free;
     int kept    = 0;
@@ -855,7 +881,7 @@ static void run_part(vm_engine* e, Lane& lane, const Chunk& c, int part, Issue i
         try {
             issue();
         }
-        catch (const CudaFailure&) {
+        catch (...) {  // the recording must end whatever happened; launched one by one below, it happens again or does not
             recorded = false;
         }
         recorded         = cudaStreamEndCapture(lane.stream, &graph) == cudaSuccess && recorded;
@@ -1160,16 +1186,9 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
         }
         return VM_OK;
     }
-    catch (const CudaFailure& f) {
-        cudaGetLastError();
+    catch (...) {
         drain();
-        cudaGetLastError();
-        const vm_status s = f.code == cudaErrorMemoryAllocation ? VM_ERR_OUT_OF_MEMORY : VM_ERR_CUDA;
-        return fail(s, std::string(cudaGetErrorName(f.code)) + ": " + cudaGetErrorString(f.code) + " in " + f.what);
-    }
-    catch (const UnsupportedLens&) {
-        drain();
-        return fail(VM_ERR_UNSUPPORTED_LENS, "Cannot project: Unknown lens type");
+        return status_of_exception();
     }
 }
 
@@ -1222,8 +1241,9 @@ vm_status vm_engine_create(int device, const vm_layer* layers, const int32_t* la
         cudaGetLastError();
         return fail(VM_ERR_CUDA, "no CUDA device: this engine has no CPU fallback");
     }
-    std::unique_ptr<vm_engine> e(new vm_engine());
+    std::unique_ptr<vm_engine> e;
     try {
+        e.reset(new vm_engine());
         if (device < 0) VM_CUDA(cudaGetDevice(&device));
         if (device >= count) return fail(VM_ERR_INVALID_ARGUMENT, "no such device");
         e->device = device;
@@ -1363,10 +1383,8 @@ vm_status vm_engine_create(int device, const vm_layer* layers, const int32_t* la
             e->may_stage        = e->may_stage || (has_window_kernel(L) && (e->tc_mode != 1 || L.cin * L.cout >= e->tc_min_product));
         }
     }
-    catch (const CudaFailure& f) {
-        cudaGetLastError();
-        return fail(f.code == cudaErrorMemoryAllocation ? VM_ERR_OUT_OF_MEMORY : VM_ERR_CUDA,
-                    std::string(cudaGetErrorName(f.code)) + " in " + f.what);
+    catch (...) {
+        return status_of_exception();
     }
     *out = e.release();
     return VM_OK;
@@ -1438,8 +1456,9 @@ vm_status vm_mesh_upload(vm_engine* e, const float* rays, const int32_t* neighbo
     }
     if (n_neighbours != 4 && n_neighbours != 6 && n_neighbours != 8) return fail(VM_ERR_INVALID_ARGUMENT, "n_neighbours must be 4, 6 or 8");
     *out = nullptr;
-    std::unique_ptr<vm_mesh> m(new vm_mesh());
+    std::unique_ptr<vm_mesh> m;
     try {
+        m.reset(new vm_mesh());
         VM_CUDA(cudaSetDevice(e->device));
         m->owner        = e;
         m->n_nodes      = n_nodes;
@@ -1452,13 +1471,12 @@ vm_status vm_mesh_upload(vm_engine* e, const float* rays, const int32_t* neighbo
         const size_t nb_bytes = sizeof(int32_t) * static_cast<size_t>(n_nodes) * n_neighbours;
         VM_CUDA(cudaMalloc(reinterpret_cast<void**>(&m->d_neighbours), nb_bytes));
         VM_CUDA(cudaMemcpy(m->d_neighbours, neighbours, nb_bytes, cudaMemcpyHostToDevice));
+        e->meshes.push_back(m.get());
     }
-    catch (const CudaFailure& f) {
-        cudaGetLastError();
+    catch (...) {
         free_mesh(m.release());
-        return fail(f.code == cudaErrorMemoryAllocation ? VM_ERR_OUT_OF_MEMORY : VM_ERR_CUDA, std::string(cudaGetErrorName(f.code)) + " in " + f.what);
+        return status_of_exception();
     }
-    e->meshes.push_back(m.get());
     *out = m.release();
     return VM_OK;
 }
@@ -1467,18 +1485,18 @@ vm_status vm_mesh_set_bsp(vm_engine* e, vm_mesh* m, int32_t n, const int32_t* ra
     if (e == nullptr || m == nullptr || n <= 0 || ranges == nullptr || children == nullptr || cones == nullptr) {
         return fail(VM_ERR_INVALID_ARGUMENT, "null argument or empty BSP");
     }
-    std::vector<float4> a(n);
-    std::vector<float> s(n);
-    std::vector<int4> t(n);
-    for (int i = 0; i < n; ++i) {
-        a[i] = make_float4(cones[5 * i], cones[5 * i + 1], cones[5 * i + 2], cones[5 * i + 3]);
-        s[i] = cones[5 * i + 4];
-        const int c0 = children[2 * i], c1 = children[2 * i + 1];
-        if (c0 >= n || c1 >= n || (c0 < 0) != (c1 < 0)) return fail(VM_ERR_INVALID_ARGUMENT, "BSP child out of range");
-        if (ranges[2 * i] < 0 || ranges[2 * i + 1] > m->n_nodes) return fail(VM_ERR_INVALID_ARGUMENT, "BSP range outside the mesh");
-        t[i] = make_int4(c0, c1, c1 >= 0 ? ranges[2 * c1] : 0, 0);
-    }
     try {
+        std::vector<float4> a(n);
+        std::vector<float> s(n);
+        std::vector<int4> t(n);
+        for (int i = 0; i < n; ++i) {
+            a[i] = make_float4(cones[5 * i], cones[5 * i + 1], cones[5 * i + 2], cones[5 * i + 3]);
+            s[i] = cones[5 * i + 4];
+            const int c0 = children[2 * i], c1 = children[2 * i + 1];
+            if (c0 >= n || c1 >= n || (c0 < 0) != (c1 < 0)) return fail(VM_ERR_INVALID_ARGUMENT, "BSP child out of range");
+            if (ranges[2 * i] < 0 || ranges[2 * i + 1] > m->n_nodes) return fail(VM_ERR_INVALID_ARGUMENT, "BSP range outside the mesh");
+            t[i] = make_int4(c0, c1, c1 >= 0 ? ranges[2 * c1] : 0, 0);
+        }
         VM_CUDA(cudaSetDevice(e->device));
         cudaFree(m->d_cones_a);
         cudaFree(m->d_cones_s);
@@ -1495,9 +1513,8 @@ vm_status vm_mesh_set_bsp(vm_engine* e, vm_mesh* m, int32_t n, const int32_t* ra
         VM_CUDA(cudaMemcpy(m->d_topology, t.data(), sizeof(int4) * n, cudaMemcpyHostToDevice));
         m->n_bsp = n;
     }
-    catch (const CudaFailure& f) {
-        cudaGetLastError();
-        return fail(f.code == cudaErrorMemoryAllocation ? VM_ERR_OUT_OF_MEMORY : VM_ERR_CUDA, std::string(cudaGetErrorName(f.code)) + " in " + f.what);
+    catch (...) {
+        return status_of_exception();
     }
     return VM_OK;
 }
@@ -1560,12 +1577,17 @@ vm_status vm_results_keep(vm_engine* e, vm_results** kept) {
     if (e == nullptr || kept == nullptr) return fail(VM_ERR_INVALID_ARGUMENT, "null argument");
     *kept = nullptr;
     if (!e->host) return fail(VM_ERR_INVALID_ARGUMENT, "the engine has no results");
-    {
+    try {
+        std::unique_ptr<KeptResults> k(new KeptResults{e->pool, nullptr});
         std::lock_guard<std::mutex> lock(e->pool->mutex);
         if (e->pool->kept >= MAX_KEPT_RESULTS) return fail(VM_ERR_OUT_OF_MEMORY, "VM_MAX_KEPT_RESULTS results of this engine are kept already");
         ++e->pool->kept;
+        k->results = std::move(e->host);
+        *kept      = reinterpret_cast<vm_results*>(k.release());
     }
-    *kept = reinterpret_cast<vm_results*>(new KeptResults{e->pool, std::move(e->host)});
+    catch (...) {
+        return status_of_exception();
+    }
     return VM_OK;
 }
 
@@ -1609,9 +1631,8 @@ vm_status vm_sample(vm_engine* e, const float* px, int32_t n, const void* image,
         VM_CUDA(cudaMemcpyAsync(out, lane.d_feat[0].p, sizeof(float) * 4 * n, cudaMemcpyDeviceToHost, lane.stream));
         VM_CUDA(cudaStreamSynchronize(lane.stream));
     }
-    catch (const CudaFailure& f) {
-        cudaGetLastError();
-        return fail(f.code == cudaErrorMemoryAllocation ? VM_ERR_OUT_OF_MEMORY : VM_ERR_CUDA, std::string(cudaGetErrorName(f.code)) + " in " + f.what);
+    catch (...) {
+        return status_of_exception();
     }
     return VM_OK;
 }
@@ -1661,9 +1682,8 @@ vm_status vm_network(vm_engine* e, const float* input, const int32_t* neighbourh
             break;
         }
     }
-    catch (const CudaFailure& f) {
-        cudaGetLastError();
-        return fail(f.code == cudaErrorMemoryAllocation ? VM_ERR_OUT_OF_MEMORY : VM_ERR_CUDA, std::string(cudaGetErrorName(f.code)) + " in " + f.what);
+    catch (...) {
+        return status_of_exception();
     }
     return VM_OK;
 }
@@ -1778,9 +1798,8 @@ vm_status vm_project_static(vm_engine* e,
         if (cells[4 + ABORT_BSP_DEPTH] != 0) return fail(VM_ERR_DEVICE_ABORT, "a kernel gave up on a bounded loop (BSP deeper than 128 levels)");
         if (n_points != nullptr) *n_points = cells[1];
     }
-    catch (const CudaFailure& f) {
-        cudaGetLastError();
-        return fail(VM_ERR_CUDA, std::string(cudaGetErrorName(f.code)) + ": " + cudaGetErrorString(f.code) + " in " + f.what);
+    catch (...) {
+        return status_of_exception();
     }
     return VM_OK;
 }
@@ -1802,9 +1821,8 @@ vm_status vm_timer_start(vm_engine* e) {
         for (int l = 0; l < MAX_LANES; ++l) VM_CUDA(cudaStreamSynchronize(e->lanes[l].stream));
         VM_CUDA(cudaEventRecord(e->ev_timer_start, e->lanes[0].stream));
     }
-    catch (const CudaFailure& f) {
-        cudaGetLastError();
-        return fail(VM_ERR_CUDA, std::string(cudaGetErrorName(f.code)) + " in " + f.what);
+    catch (...) {
+        return status_of_exception();
     }
     return VM_OK;
 }
@@ -1822,9 +1840,8 @@ vm_status vm_timer_stop(vm_engine* e, float* milliseconds) {
         VM_CUDA(cudaEventSynchronize(e->ev_timer_stop));
         VM_CUDA(cudaEventElapsedTime(milliseconds, e->ev_timer_start, e->ev_timer_stop));
     }
-    catch (const CudaFailure& f) {
-        cudaGetLastError();
-        return fail(VM_ERR_CUDA, std::string(cudaGetErrorName(f.code)) + " in " + f.what);
+    catch (...) {
+        return status_of_exception();
     }
     return VM_OK;
 }

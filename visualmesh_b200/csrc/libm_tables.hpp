@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -62,27 +63,30 @@ namespace libm {
         const size_t n_words = packed.size();
         unsigned n_threads   = std::thread::hardware_concurrency();
         n_threads            = n_threads == 0 ? 4 : (n_threads > 32 ? 32 : n_threads);
-        std::vector<std::thread> workers;
-        const size_t per = (n_words + n_threads - 1) / n_threads;
-        for (unsigned t = 0; t < n_threads; ++t) {
-            const size_t w0 = t * per;
-            const size_t w1 = w0 + per < n_words ? w0 + per : n_words;
-            if (w0 >= w1) break;
-            workers.emplace_back([fn, first, w0, w1, &packed] {
-                for (size_t w = w0; w < w1; ++w) {
-                    uint32_t word = 0;
-                    for (uint32_t j = 0; j < 16; ++j) {
-                        const uint32_t bits = first + static_cast<uint32_t>(w) * 16u + j;
-                        float x;
-                        std::memcpy(&x, &bits, sizeof(x));
-                        const float y = evaluate(fn, x);
-                        uint32_t yb;
-                        std::memcpy(&yb, &y, sizeof(yb));
-                        word |= (yb & 3u) << (2u * j);
-                    }
-                    packed[w] = word;
+        auto fill = [fn, first, &packed](size_t w0, size_t w1) {
+            for (size_t w = w0; w < w1; ++w) {
+                uint32_t word = 0;
+                for (uint32_t j = 0; j < 16; ++j) {
+                    const uint32_t bits = first + static_cast<uint32_t>(w) * 16u + j;
+                    float x;
+                    std::memcpy(&x, &bits, sizeof(x));
+                    const float y = evaluate(fn, x);
+                    uint32_t yb;
+                    std::memcpy(&yb, &y, sizeof(yb));
+                    word |= (yb & 3u) << (2u * j);
                 }
-            });
+                packed[w] = word;
+            }
+        };
+        std::vector<std::thread> workers;
+        workers.reserve(n_threads);
+        const size_t per = (n_words + n_threads - 1) / n_threads;
+        size_t w0        = 0;
+        try {
+            for (; w0 < n_words; w0 += per) workers.emplace_back(fill, w0, w0 + per < n_words ? w0 + per : n_words);
+        }
+        catch (const std::exception&) {  // a limit on threads: this one does what is left
+            fill(w0, n_words);
         }
         for (auto& w : workers) w.join();
         return packed;

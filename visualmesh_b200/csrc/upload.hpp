@@ -15,6 +15,7 @@
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <mutex>
 #include <thread>
@@ -124,7 +125,11 @@ public:
 private:
     UploadHelpers() {
         const int n = std::min<int>(UPLOAD_HELPERS, static_cast<int>(std::thread::hardware_concurrency()) / 4);
-        for (int i = 0; i < n; ++i) threads_.emplace_back([this] { work(); });
+        threads_.reserve(UPLOAD_HELPERS);
+        try {
+            for (int i = 0; i < n; ++i) threads_.emplace_back([this] { work(); });
+        }
+        catch (const std::exception&) {}  // a limit on threads: those that did start help, and an upload without any copies alone
     }
     void work() {
         uint64_t seen = 0;
