@@ -9,11 +9,17 @@ from visualmesh_b200 import build as vm_build
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 
-@pytest.fixture(scope="module")
-def check(tmp_path_factory):
-    out = str(tmp_path_factory.mktemp("upload") / "upload_check")
+@pytest.fixture(scope="module", params=["this host", "without SSE2"])
+def check(tmp_path_factory, request):
+    folder = tmp_path_factory.mktemp("upload")
+    out, flags = str(folder / "upload_check"), []
+    if request.param == "without SSE2":
+        # a host that is no x86: the macro is not defined and the header does not exist
+        (folder / "emmintrin.h").write_text("#error this host has no SSE2\n")
+        flags = ["-U__SSE2__", "-I", str(folder)]
     include = os.path.join(os.path.dirname(os.path.dirname(vm_build._nvcc())), "include")
-    subprocess.run(["g++", "-O2", "-std=c++17", "-I", include, os.path.join(HERE, "upload_check.cpp"), "-o", out, "-lpthread", "-ldl"], check=True)
+    subprocess.run(["g++", "-O2", "-std=c++17", *flags, "-I", include, os.path.join(HERE, "upload_check.cpp"), "-o", out, "-lpthread", "-ldl"],
+                   check=True)
     return out
 
 

@@ -8,7 +8,9 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#if defined(__SSE2__)
 #include <emmintrin.h>
+#endif
 
 #include <algorithm>
 #include <atomic>
@@ -33,6 +35,7 @@ constexpr size_t UPLOAD_RUN = 512 << 10;
 constexpr int UPLOAD_HELPERS = 2;
 
 inline void copy_past_the_cache(uint8_t* dst, const uint8_t* src, size_t n) {
+#if defined(__SSE2__)
     const size_t head = std::min(n, (16 - (reinterpret_cast<uintptr_t>(dst) & 15)) & 15);
     std::memcpy(dst, src, head);
     size_t i = head;
@@ -48,6 +51,9 @@ inline void copy_past_the_cache(uint8_t* dst, const uint8_t* src, size_t n) {
     }
     std::memcpy(dst + i, src + i, n - i);
     _mm_sfence();
+#else
+    std::memcpy(dst, src, n);  // other hosts
+#endif
 }
 
 struct UploadSlice {
