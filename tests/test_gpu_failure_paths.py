@@ -175,3 +175,24 @@ def test_nvtx_ranges_do_not_change_results():
         out = engine.run_batch([FrameInput(mesh, fr["Hoc"], case.lens, fr["image"], case.format, None)]).frame(0)
         assert P.compare(out, fr, case.lens.dimensions).ok
     engine.close()
+
+
+def test_streams_are_made_when_they_are_first_used():
+    """An engine starts with one stream pair; the stopwatch, a failing call and a batch that needs all lanes meet it in that state."""
+    case = G.Case("ring6_equisolid_rgba")
+    fr = case.frames[0]
+    engine = _engine_with_env(case.network, VMCUDA_CHUNK_FRAMES=1)
+    mesh = Mesh.from_arrays(case.rays, case.nbrs, case.bsp)
+    engine.timer_start()
+    assert engine.timer_stop() >= 0.0
+    children = case.bsp[1].copy()
+    children[[i for i in range(1, len(children)) if children[i][0] >= 0][0]] = (0, 0)
+    looped = Mesh.from_arrays(case.rays, case.nbrs, (case.bsp[0], children, case.bsp[2]))
+    with pytest.raises(VisualMeshError):
+        engine.run_batch([FrameInput(looped, fr["Hoc"], case.lens, fr["image"], case.format, None)])
+    engine.timer_start()
+    batch = engine.run_batch([FrameInput(mesh, fr["Hoc"], case.lens, fr["image"], case.format, None)] * 9)
+    assert engine.timer_stop() > 0.0
+    for f in range(9):
+        assert P.compare(batch.frame(f), fr, case.lens.dimensions).ok
+    engine.close()

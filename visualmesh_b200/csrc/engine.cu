@@ -162,6 +162,19 @@ struct Lane {
     DeviceArray<uint16_t> d_nbl;
     DeviceArray<int32_t> d_halo_rows;
     DeviceArray<int32_t> d_halo_count;
+
+    // Makes the streams and events, when the lane is first used: a call of one chunk takes one lane of the four.
+    void open(bool blocking_sync) {
+        if (stream != nullptr) return;
+        if (side == nullptr) VM_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+        // ev_offsets and ev_done are the ones the host waits on: spinning (lowest latency) or, with VMCUDA_BLOCKING_SYNC=1, sleeping - for
+        // boxes where several engines' host threads share few cores
+        for (cudaEvent_t* ev : {&ev_fork, &ev_join, &ev_images, &ev_projected, &ev_offsets, &ev_done}) {
+            const unsigned waits = (ev == &ev_offsets || ev == &ev_done) && blocking_sync ? cudaEventBlockingSync : 0;
+            if (*ev == nullptr) VM_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming | waits));
+        }
+        VM_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    }
 };
 
 // One set of result arrays in pinned host memory. An engine writes its results into the set it holds; a caller may keep the set
@@ -568,6 +581,7 @@ static ImagePlan plan_images(const vm_frame* frames, int f0, int f1) {
 // turn-around than one 84 MB copy. Pageable frames go through the upload helpers.
 static std::unique_ptr<Upload> start_images(vm_engine* e, Lane& lane, const vm_frame* frames, int f0, int f1, const ImagePlan& plan) {
     need(e, lane.d_images, plan.total + 256);
+    if (e->copy_stream == nullptr) VM_CUDA(cudaStreamCreateWithFlags(&e->copy_stream, cudaStreamNonBlocking));
     std::unique_ptr<Upload> upload;
     if (plan.pageable > 0) {
         if (!e->helpers) e->helpers = UploadHelpers::get();
@@ -1035,11 +1049,11 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
 
     auto drain = [&] {
         for (auto& lane : e->lanes) {
-            cudaStreamSynchronize(lane.stream);
-            cudaStreamSynchronize(lane.side);
+            if (lane.stream != nullptr) cudaStreamSynchronize(lane.stream);
+            if (lane.side != nullptr) cudaStreamSynchronize(lane.side);
             lane.busy = false;
         }
-        cudaStreamSynchronize(e->copy_stream);
+        if (e->copy_stream != nullptr) cudaStreamSynchronize(e->copy_stream);
     };
     try {
         VM_CUDA(cudaSetDevice(e->device));
@@ -1123,6 +1137,7 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
                 ++f1;
             }
             Lane& lane = e->lanes[chunk % n_lanes];
+            lane.open(e->blocking_sync);
             if (lane.busy) {
                 // its previous chunk must have left the lane's staging and scratch
                 VM_CUDA(cudaEventSynchronize(lane.ev_done));
@@ -1267,18 +1282,7 @@ vm_status vm_engine_create(int device, const vm_layer* layers, const int32_t* la
         if (const char* v = std::getenv("VMCUDA_NVTX")) e->nvtx = std::atoi(v) != 0;
         if (const char* v = std::getenv("VMCUDA_GRAPHS")) e->use_graphs = std::atoi(v) != 0;
         if (const char* v = std::getenv("VMCUDA_LANES")) e->n_lanes = std::min(MAX_LANES, std::max(1, std::atoi(v)));
-        for (int l = 0; l < MAX_LANES; ++l) {
-            Lane& lane = e->lanes[l];
-            VM_CUDA(cudaStreamCreateWithFlags(&lane.stream, cudaStreamNonBlocking));
-            VM_CUDA(cudaStreamCreateWithFlags(&lane.side, cudaStreamNonBlocking));
-            for (cudaEvent_t* ev : {&lane.ev_fork, &lane.ev_join, &lane.ev_images, &lane.ev_projected}) VM_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
-            // the events the host waits on: spinning (lowest latency) or, with VMCUDA_BLOCKING_SYNC=1, sleeping - for boxes where
-            // several engines' host threads share few cores
-            for (cudaEvent_t* ev : {&lane.ev_offsets, &lane.ev_done}) {
-                VM_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming | (e->blocking_sync ? cudaEventBlockingSync : 0)));
-            }
-        }
-        VM_CUDA(cudaStreamCreateWithFlags(&e->copy_stream, cudaStreamNonBlocking));
+        e->lanes[0].open(e->blocking_sync);  // the others, and the stream of the images, when they are first used
         VM_CUDA(cudaEventCreate(&e->ev_timer_start));
         VM_CUDA(cudaEventCreate(&e->ev_timer_stop));
         VM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&e->flags), sizeof(int32_t) * ABORT_FLAGS, cudaHostAllocDefault));
@@ -1818,7 +1822,8 @@ vm_status vm_timer_start(vm_engine* e) {
     if (e == nullptr) return fail(VM_ERR_INVALID_ARGUMENT, "null engine");
     try {
         VM_CUDA(cudaSetDevice(e->device));
-        for (int l = 0; l < MAX_LANES; ++l) VM_CUDA(cudaStreamSynchronize(e->lanes[l].stream));
+        for (auto& lane : e->lanes)
+            if (lane.stream != nullptr) VM_CUDA(cudaStreamSynchronize(lane.stream));
         VM_CUDA(cudaEventRecord(e->ev_timer_start, e->lanes[0].stream));
     }
     catch (...) {
@@ -1833,6 +1838,7 @@ vm_status vm_timer_stop(vm_engine* e, float* milliseconds) {
         VM_CUDA(cudaSetDevice(e->device));
         // lane 0 waits for the other lanes, then stamps the end
         for (int l = 1; l < MAX_LANES; ++l) {
+            if (e->lanes[l].stream == nullptr) continue;
             VM_CUDA(cudaEventRecord(e->lanes[l].ev_fork, e->lanes[l].stream));
             VM_CUDA(cudaStreamWaitEvent(e->lanes[0].stream, e->lanes[l].ev_fork, 0));
         }
