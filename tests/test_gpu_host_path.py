@@ -90,6 +90,31 @@ def test_a_recorded_graph_serves_one_layout_of_the_staging_block_only():
     engine.close()
 
 
+def test_staging_blocks_of_every_size_reach_the_device_whole():
+    """Frame constants, ranges and counts come by a copy when the images are on the device already, else they are read by a kernel:
+    from one range to 16810 of one node each (204 KB, more than the kernel's threads read in one turn)."""
+    import torch
+    case = G.Case("ring6_equisolid_rgba")
+    mesh = Mesh.from_arrays(case.rays, case.nbrs, case.bsp)
+    lens = W.Lens((640, 512), W.EQUISOLID, 0.35 * 640, (0.0, 0.0), (0.0, 0.0), np.pi)
+    engine = Engine(case.network)
+    host = W.random_bytes(3, 5 * 640 * 512 * 4).reshape(5, -1)
+    device = torch.from_numpy(host).cuda()
+    torch.cuda.synchronize()
+    nodes = np.arange(mesh.n_nodes, dtype=np.int32)
+    for ranges in (None, np.array([[0, mesh.n_nodes]], np.int32), np.stack([nodes, nodes + 1], axis=1)[::7], np.stack([nodes, nodes + 1], axis=1)):
+        frames = [[FrameInput(mesh, case.frames[f % 3]["Hoc"], lens, device[f].data_ptr() if there else host[f], W.fourcc("RGBA"), ranges, there)
+                   for f in range(5)] for there in (True, False)]
+        batch = engine.run_batch(frames[0])
+        want = [batch.frame(f) for f in range(5)]
+        assert min(len(w.global_indices) for w in want) > 100
+        for _ in range(3):
+            batch = engine.run_batch(frames[1])
+            for f in range(5):
+                _same(batch.frame(f), want[f])
+    engine.close()
+
+
 def test_many_frames_with_few_candidates_on_a_mesh_of_many_nodes():
     """The node tables of the batch's frames together pass 2^31 entries, their candidates are 205 k: a chunk is cut before its
     32-bit offsets into the node table overflow."""
@@ -145,6 +170,29 @@ def test_batches_left_on_the_device_and_copied_to_the_host_agree(n_frames):
                 assert np.array_equal(out.global_indices, gi[p0:p1])
                 assert np.array_equal(out.neighbourhood, nb[p0 + f:p1 + f + 1])
                 assert np.array_equal(G.bits(out.classifications), G.bits(cls[p0 + f:p1 + f + 1]))
+    engine.close()
+
+
+# frames per launch: beyond 64 (two turns of a warp over the table of tiles), and one more than a chunk holds
+@pytest.mark.parametrize("n_frames", [130, 257])
+@pytest.mark.parametrize("widths", [[16, 16, 8, 3], [32, 32, 32, 4]])
+def test_batches_of_many_frames_equal_single_frames(n_frames, widths):
+    import torch
+    case = G.Case("ring6_equisolid_rgba")
+    mesh = Mesh.from_arrays(case.rays, case.nbrs, case.bsp)
+    engine = Engine(W.make_network(23, 6, widths))
+    size = case.lens.dimensions[0] * case.lens.dimensions[1] * 4
+    images = torch.from_numpy(W.random_bytes(29, n_frames * size).reshape(n_frames, size)).cuda()
+    torch.cuda.synchronize()
+    # from straight down to above the horizon: frames of many rows, few and none
+    views = [W.make_Hoc(-1.5 + 3.1 * (7 * f % n_frames) / n_frames, 0.2, 1.0) for f in range(n_frames)]
+    frames = [FrameInput(mesh, H, case.lens, images[f].data_ptr(), W.fourcc("RGBA"), None, True) for f, H in enumerate(views)]
+    batch = engine.run_batch(frames)
+    got = [batch.frame(f) for f in range(n_frames)]
+    points = [len(g.global_indices) for g in got]
+    assert min(points) < 10 and max(points) > 1000 and len(set(points)) > n_frames // 2
+    for f in range(n_frames):
+        _same(got[f], engine.run_batch([frames[f]]).frame(0))
     engine.close()
 
 

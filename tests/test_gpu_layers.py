@@ -66,3 +66,38 @@ def test_layers_of_32_channels_with_neighbours_close_by():
     got = engine.network(x, nb)
     engine.close()
     assert np.abs(got.astype(np.float64) - O.network(x, nb, net).astype(np.float64)).max() <= P.TOL_CLS / 4
+
+
+def test_selu_over_its_range():
+    """A layer that passes its input through: SELU of floats of every size, against double.
+
+    The kernels write lambda alpha (e^s - 1) as one multiply-add of 2^(s log2 e). Its errors: the hardware's 2^x (2^-22.5 relative), the
+    product s log2 e and its constant (together |s| 2^-23 of an exponential of e^s), the multiply-add (half an ulp of at most 1.76) and
+    its rounded constant: 1.7581 (e^s 2^-22.5 + |s| e^s 2^-23) + 2^-24 + 2^-24 < 4.2e-7 for every s. The form with an exponential
+    function, lambda (alpha exp(s) - alpha), rounds three times behind it and is no closer."""
+    import torch
+    down = -np.exp2(np.linspace(-30.0, 7.0, 3_000_000)).astype(np.float32)
+    extremes = np.array([-0.0, 0.0, -1e-45, -1e-38, -87.0, -104.0, -1e4, -3e38, 1e-45, 1e-38, 3e38, 1.0], np.float32)
+    up = np.exp2(np.linspace(-100.0, 100.0, 999_988)).astype(np.float32)
+    ones = np.ones(4, np.float32)  # the last row, which every neighbour is: the zero weights of the gather meet finite values
+    s = np.concatenate([down, up, extremes, ones]).reshape(-1, 4)
+    n = len(s)
+    weights = np.zeros((20, 4), np.float32)
+    weights[:4] = np.eye(4, dtype=np.float32)
+    net = [[W.Layer(weights, np.zeros(4, np.float32), W.SELU)]]
+    nb = np.full((n, 4), n - 1, np.int32)
+    lam, alpha = 1.0507009873554804934193349852946, 1.6732632423543772848170429916717
+    x = s.astype(np.float64)
+    want = np.where(x >= 0, lam * x, lam * alpha * np.expm1(np.minimum(x, 0)))
+    engine = Engine(net)
+    got = engine.network(s, nb).astype(np.float64)
+    engine.close()
+    error, negative = np.abs(got - want), x < 0
+    alpha32 = float(np.float32(alpha))
+    plain = (float(np.float32(lam)) * (alpha32 * torch.exp(torch.from_numpy(s).cuda()) - alpha32)).cpu().numpy().astype(np.float64)
+    plain_error = np.abs(plain - want)[negative].max()
+    print(f"selu: largest error {error[negative].max():.3g}, with an exponential function {plain_error:.3g}")
+    assert error[negative].max() <= min(4.2e-7, plain_error)
+    positive = x > 1e-37
+    assert (error[positive] / want[positive]).max() <= 2.0**-23  # lambda rounded, the product rounded
+    assert error[(x >= 0) & ~positive].max() <= 1e-44

@@ -772,14 +772,31 @@ static void issue_remap(vm_engine* e, Lane& lane, const Chunk& c) {
     end_stage(e, s);
 }
 
-// Staging copy, lookup, projection, compaction, neighbour remap; images that are on the device already are sampled beside the
+// The staging block's way to the device: by a kernel where images are on their way too (k_fetch), else by a copy. A block is a few
+// kilobytes, with ranges at most a few hundred: 32 thread blocks keep enough reads in flight.
+constexpr int FETCH_BLOCKS = 32;
+
+static void issue_staging(vm_engine* e, Lane& lane, const Chunk& c) {
+    cudaStream_t s = lane.stream;
+    if (!c.images_apart) {
+        VM_CUDA(cudaMemcpyAsync(lane.d_staging.p, lane.h_staging.p, c.staging_bytes, cudaMemcpyHostToDevice, s));
+        return;
+    }
+    const int n = static_cast<int>(c.staging_bytes / sizeof(uint4));  // whole pieces: every part of the block is aligned to 256 bytes
+    begin_stage(e, s, "fetch_staging");
+    k_fetch<<<std::min(FETCH_BLOCKS, (n + FETCH_THREADS - 1) / FETCH_THREADS), FETCH_THREADS, 0, s>>>(reinterpret_cast<const uint4*>(lane.h_staging.p),
+                                                                                                    reinterpret_cast<uint4*>(lane.d_staging.p), n);
+    end_stage(e, s);
+}
+
+// Staging block, lookup, projection, compaction, neighbour remap; images that are on the device already are sampled beside the
 // remap (neither needs the other: 178 -> 140 us on 4.4 M rows).
 static void issue_projection(vm_engine* e, Lane& lane, const Chunk& c, bool sample, bool remap = true) {
     cudaStream_t s            = lane.stream;
     const int nf              = c.f1 - c.f0;
     const FrameParams* frames = device_frames(lane);
     int32_t* groups           = reinterpret_cast<int32_t*>(lane.d_staging.p + c.counts_at);
-    VM_CUDA(cudaMemcpyAsync(lane.d_staging.p, lane.h_staging.p, c.staging_bytes, cudaMemcpyHostToDevice, s));
+    issue_staging(e, lane, c);
     if (c.device_lookup) {
         begin_stage(e, s, "bsp_state");
         k_bsp_state<<<dim3(c.bsp_blocks, nf), SELECT_THREADS, 0, s>>>(frames, lane.d_state.p);
@@ -1108,7 +1125,9 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
 
         // Chunks: runs of frames bounded by a candidate budget, a frame count and the bytes of their host images. Small ones let the
         // copies of one chunk overlap the kernels of another: 20 MB are 0.4 ms of the bus (32 frames of 5 MB to results on the
-        // host: 4.28 ms in chunks of 16 frames, 3.98 in chunks of 4, 4.11 in chunks of 2; both directions' bytes alone take 3.45). When no images are to be copied in, a batch is one chunk as far as the scratch allows, and
+        // host: 3.87 ms in chunks of 16 frames, 3.56 in chunks of 8, 3.50 in chunks of 4, 3.60 in chunks of 2; both directions' bytes
+        // alone take 3.45. Two engines with 32 frames each: 6.60, 6.59, 6.78 ms in chunks of 16, 8 and 4; the bytes alone 6.67). When no
+        // images are to be copied in, a batch is one chunk as far as the scratch allows, and
         // chunks follow one another: fewer and fuller launches (64 frames of 1280 x 1024 pixels in one chunk: 1.61 ms, in two that
         // overlap 1.99, in eight 2.06 - persistent layer kernels of two chunks get in one another's way).
         bool host_images = false;

@@ -24,6 +24,7 @@ constexpr int ROW_THREADS    = 256;
 constexpr int SCATTER_UNITS  = 4;    // runs of SELECT_THREADS candidates per block of k_scatter
 constexpr int GROUP_BLOCKS   = 64;   // blocks of k_select whose counts are also summed as a group (a multiple of SCATTER_UNITS)
 constexpr int EXPORT_THREADS = 512;
+constexpr int FETCH_THREADS  = 256;
 
 // Where a chunk's results go when they are wanted on the host: pinned memory that the device writes directly. It heads the
 // chunk's staging block, so that a recorded graph of the chunk's kernels serves results buffers that change from call to call.
@@ -35,6 +36,16 @@ struct alignas(16) ChunkHeader {
     int32_t* offsets;  // every chunk: the batch's offsets array in pinned memory
 };
 constexpr int SAMPLE_ROWS    = 2;    // points per thread of k_sample
+
+// ---- staging block of a chunk, read by the device --------------------------------------------------------------------
+// For chunks whose images travel on the copy stream. A copy of these few kilobytes waits in the copy engine behind every image that is
+// on its way, this chunk's and the next one's, and with it the projection and its results' way back: in a batch of chunks of four
+// 5 MB frames the second projection ended 1.1 ms after the first. Read by a kernel instead (64 such frames, results on the host):
+// one engine 7.46 -> 6.83 ms, two engines with half of them each 7.52 -> 6.78, where the bare copies take 6.67; 32 frames on one engine
+// 3.90 -> 3.50. `n` pieces of 16 bytes, read past the L1 cache because the host rewrites them between launches.
+__global__ void __launch_bounds__(FETCH_THREADS) k_fetch(const uint4* __restrict__ from, uint4* __restrict__ to, int32_t n) {
+    for (int i = blockIdx.x * FETCH_THREADS + threadIdx.x; i < n; i += gridDim.x * FETCH_THREADS) to[i] = __ldcv(from + i);
+}
 
 enum : uint8_t { BSP_DESCEND = 0, BSP_INSIDE = 1, BSP_OUTSIDE = 2 };
 
