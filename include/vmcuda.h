@@ -167,7 +167,7 @@ VM_API vm_status vm_classify(vm_engine* engine,
                       vm_batch_result* out);
 
 /* The reference's calls with their lookup (cpp/visualmesh/engine/opencl/engine.hpp:581): Mesh::lookup runs inside the call, on the
- * device where the mesh's BSP is (vm_mesh_set_bsp), else on the host while the image is on its way; either finds the same nodes.
+ * device where the mesh's BSP is (vm_mesh_set_bsp), else on the host before it; either finds the same nodes.
  * lookup: the host tables that `mesh` was uploaded from (vm_hostmesh, below); image NULL: projection only. Otherwise vm_classify and
  * vm_project. */
 struct vm_hostmesh;

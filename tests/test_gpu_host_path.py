@@ -196,6 +196,40 @@ def test_batches_of_many_frames_equal_single_frames(n_frames, widths):
     engine.close()
 
 
+def test_call_looks_up_on_the_host_when_the_device_has_no_bsp():
+    """vm_call on a mesh that was uploaded without its BSP: the host tables find the same nodes as the device does."""
+    import ctypes as C
+    from visualmesh_b200 import abi
+    from visualmesh_b200.engine import _c_lens
+    lib = abi.load()
+    mesh = Mesh("XYGRID6", "CYLINDER", 0.2, 1.8, 1.0, 4.0, 12.0)
+    lens = W.Lens((320, 240), W.RECTILINEAR, 190.0, (0.0, 0.0), (0.0, 0.0), 1.8)
+    engine = Engine(W.make_network(5, 6, [8, 8, 3]))
+    image = W.random_bytes(11, 320 * 240 * 4)
+    handle = C.c_void_p()
+    abi.check(lib.vm_mesh_upload(engine._ptr, mesh.rays.ctypes.data, mesh.neighbours.ctypes.data, mesh.n_nodes, mesh.n_neighbours, C.byref(handle)))
+    most = 0
+    for pitch in (-0.2, -0.6, -1.2, 1.5):
+        Hoc = W.make_Hoc(pitch, 0.1, 1.0)
+        want = engine(mesh, Hoc, lens, image, W.fourcc("RGBA"))
+        most = max(most, len(mesh.lookup(Hoc, lens)))
+        for _ in range(2):
+            res = abi.vm_batch_result()
+            abi.check(lib.vm_call(engine._ptr, handle, mesh._ptr, Hoc.ctypes.data, C.byref(_c_lens(lens)), image.ctypes.data, W.fourcc("RGBA"), C.byref(res)))
+            n = res.offsets[1]
+            assert n == len(want.global_indices)
+            if n > 0:
+                assert np.array_equal(np.ctypeslib.as_array(res.global_indices, (n,)), want.global_indices)
+                assert np.array_equal(np.ctypeslib.as_array(res.neighbourhood, (n + 1, 6)), want.neighbourhood)
+                assert np.array_equal(G.bits(np.ctypeslib.as_array(res.classifications, (n + 1, 3))), G.bits(want.classifications))
+    assert most > 10
+    bad = _c_lens(lens)
+    bad.projection = 7
+    status = lib.vm_call(engine._ptr, handle, mesh._ptr, Hoc.ctypes.data, C.byref(bad), image.ctypes.data, W.fourcc("RGBA"), C.byref(res))
+    assert status == abi.VM_ERR_UNSUPPORTED_LENS
+    engine.close()
+
+
 def test_results_of_a_call_are_the_callers_own():
     """Results kept over later calls (more of them than the engine hands over without a copy), over the engine's end, and given
     back in another order."""

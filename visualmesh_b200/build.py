@@ -24,7 +24,7 @@ ABI_HEADER = os.path.join("..", "..", "include", "vmcuda.h")
 FFMA_HEADERS = ["conv_ffma_launch.cuh", "conv_ffma.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER]
 # translation unit -> headers it includes (directly or not)
 UNITS = {
-    "engine.cu": ["kernels.cuh", "tile_plan.cuh", "device_math.cuh", "host_math.hpp", "libm_tables.hpp", "upload.hpp", "hostmesh.hpp", "conv_dispatch.hpp", "conv_args.hpp",
+    "engine.cu": ["kernels.cuh", "tile_plan.cuh", "device_math.cuh", "host_math.hpp", "libm_tables.hpp", "upload.hpp", "conv_dispatch.hpp", "conv_args.hpp",
                   ABI_HEADER],
     "conv_ffma.cu": FFMA_HEADERS,
     "conv_ffma_mid.cu": FFMA_HEADERS,
@@ -32,7 +32,7 @@ UNITS = {
     "conv_tc.cu": ["conv_tc.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
     "conv_staged.cu": ["conv_staged.cuh", "tile_plan.cuh", "conv_tc.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
     "conv_window.cu": ["conv_window.cuh", "tile_plan.cuh", "conv_tc.cuh", "conv_common.cuh", "conv_dispatch.hpp", "conv_args.hpp", ABI_HEADER],
-    "hostmesh.cpp": ["host_math.hpp", "hostmesh.hpp", ABI_HEADER],
+    "hostmesh.cpp": ["host_math.hpp", ABI_HEADER],
 }
 NATIVE_SOURCES = ["native.cpp", ABI_HEADER]
 

@@ -24,7 +24,6 @@
 
 #include "../../include/vmcuda.h"
 #include "host_math.hpp"
-#include "hostmesh.hpp"
 #include "kernels.cuh"
 #include "conv_dispatch.hpp"
 #include "upload.hpp"
@@ -265,7 +264,6 @@ struct vm_engine {
     vm::DeviceArray<float> d_cls;
     std::unique_ptr<vm::Results> host;  // ... and where they arrive on the host
     std::shared_ptr<vm::ResultPool> pool = std::make_shared<vm::ResultPool>();
-    std::vector<std::pair<int, int>> looked_up;  // ranges of the frame whose lookup runs inside the call
     int32_t* flags = nullptr;  // abort flags, pinned host memory that the kernels raise them in
     std::vector<vm_mesh*> meshes;
     // recorded graphs
@@ -496,8 +494,6 @@ static int64_t frame_candidates(const vm_frame& fr) {
     for (int r = 0; r < fr.n_ranges; ++r) n += std::max(0, fr.ranges[2 * r + 1] - fr.ranges[2 * r]);
     return n;
 }
-
-static_assert(sizeof(std::pair<int, int>) == 2 * sizeof(int32_t), "range pairs as the frames hold them");
 
 static size_t aligned(size_t n) {
     return (n + 255) & ~size_t(255);
@@ -1015,8 +1011,7 @@ static void copy_results(vm_engine* e, Lane& lane, const Chunk& c) {
     VM_CUDA(cudaEventRecord(lane.ev_done, lane.stream));
 }
 
-// lookup: host mesh tables of the one frame of the batch, whose ranges are looked up inside the call, beside its image's upload.
-static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frames, uint32_t flags, vm_batch_result* out, const vm_hostmesh* lookup = nullptr) {
+static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frames, uint32_t flags, vm_batch_result* out) {
     if (e == nullptr || out == nullptr || n_frames < 0 || (n_frames > 0 && frames == nullptr)) {
         return fail(VM_ERR_INVALID_ARGUMENT, "null engine, frames or result");
     }
@@ -1046,7 +1041,7 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
         }
         if (fr.lens.dimensions[0] <= 0 || fr.lens.dimensions[1] <= 0) return fail(VM_ERR_INVALID_ARGUMENT, "lens dimensions must be positive");
         if (fr.ranges == nullptr && fr.n_ranges != 0) return fail(VM_ERR_INVALID_ARGUMENT, "n_ranges without ranges");
-        if (fr.ranges == nullptr && fr.mesh->n_bsp == 0 && lookup == nullptr) return fail(VM_ERR_NO_BSP, "device lookup needs vm_mesh_set_bsp");
+        if (fr.ranges == nullptr && fr.mesh->n_bsp == 0) return fail(VM_ERR_NO_BSP, "device lookup needs vm_mesh_set_bsp");
         if (fr.n_ranges < 0) return fail(VM_ERR_INVALID_ARGUMENT, "negative n_ranges");
         for (int r = 0; r < fr.n_ranges; ++r) {
             if (fr.ranges[2 * r] < 0 || fr.ranges[2 * r + 1] > fr.mesh->n_nodes || fr.ranges[2 * r] > fr.ranges[2 * r + 1]) {
@@ -1058,7 +1053,7 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
             char code[5] = {char(fr.format & 0xFF), char(fr.format >> 8 & 0xFF), char(fr.format >> 16 & 0xFF), char(fr.format >> 24 & 0xFF), 0};
             return fail(VM_ERR_UNSUPPORTED_FORMAT, std::string("Unsupported image format ") + code);
         }
-        if (lookup == nullptr) cand_all += frame_candidates(fr);
+        cand_all += frame_candidates(fr);
     }
     if (classify && e->layers.front().cin != 4) return fail(VM_ERR_NETWORK_SHAPE, "first layer must take 4 channels");
     if (classify && e->layers.front().n_slots != N + 1) return fail(VM_ERR_NETWORK_SHAPE, "network was built for a different n_neighbours");
@@ -1083,22 +1078,6 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
 
         ImagePlan images;
         std::unique_ptr<Upload> upload;
-        vm_frame looked_up;
-        if (lookup != nullptr) {
-            if (classify) {
-                images = plan_images(frames, 0, 1);
-                if (images.total > 0 && !images.small) upload = start_images(e, e->lanes[0], frames, 0, 1, images);
-            }
-            e->looked_up.clear();
-            if (!vm_hostmesh_ranges_(lookup, frames[0].Hoc, &frames[0].lens, e->looked_up)) throw UnsupportedLens{};
-            if (upload) upload->pump();
-            static const int32_t none[2] = {0, 0};
-            looked_up          = frames[0];
-            looked_up.ranges   = e->looked_up.empty() ? none : &e->looked_up.front().first;
-            looked_up.n_ranges = static_cast<int32_t>(e->looked_up.size());
-            frames             = &looked_up;
-            cand_all           = frame_candidates(looked_up);
-        }
 
         const size_t rows_all = static_cast<size_t>(cand_all) + n_frames;
         need(e, e->d_offsets, n_frames + 1);
@@ -1162,7 +1141,7 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
                 VM_CUDA(cudaEventSynchronize(lane.ev_done));
                 lane.busy = false;
             }
-            if (classify && lookup == nullptr) {
+            if (classify) {
                 images = plan_images(frames, f0, f1);
                 upload.reset();
                 if (images.total > 0 && !images.small) upload = start_images(e, lane, frames, f0, f1, images);
@@ -1190,7 +1169,7 @@ static vm_status run_batch(vm_engine* e, const vm_frame* frames, int32_t n_frame
             // a feature value beyond the range of the fp16 split: this engine goes back to the FFMA kernels for good and
             // the batch is computed again
             e->use_tc = false;
-            return run_batch(e, frames, n_frames, flags, out);  // the frames have their ranges by now
+            return run_batch(e, frames, n_frames, flags, out);
         }
 
         if (e->timing) {
@@ -1592,8 +1571,21 @@ vm_status vm_call(vm_engine* e, const vm_mesh* mesh, const vm_hostmesh* lookup, 
     // With the mesh's BSP on the device the lookup runs there, with the host's arithmetic and the host's result: one more small kernel
     // against 10 to 140 us on the calling thread, which is then free to copy the image (thumbnail on a mesh of 7 k nodes: 62 -> 48 us a
     // call, 21 MB frame on one of 1.7 M: 2.49 -> 2.27 ms, ten calls of both grid models and all sizes: -3 % to +29 %).
-    if (mesh->n_bsp > 0) lookup = nullptr;
-    return run_batch(e, &fr, 1, 0, out, lookup);
+    if (mesh->n_bsp > 0) return run_batch(e, &fr, 1, 0, out);
+    std::vector<int32_t> ranges;
+    try {
+        int32_t held = 1024;
+        do {
+            ranges.resize(2 * static_cast<size_t>(held = std::max(held, fr.n_ranges)));
+            const vm_status s = vm_hostmesh_lookup(lookup, Hoc, lens, ranges.data(), held, &fr.n_ranges);
+            if (s != VM_OK) return s;
+        } while (fr.n_ranges > held);
+    }
+    catch (...) {
+        return status_of_exception();
+    }
+    fr.ranges = ranges.data();
+    return run_batch(e, &fr, 1, 0, out);
 }
 
 vm_status vm_results_keep(vm_engine* e, vm_results** kept) {

@@ -24,7 +24,6 @@
 
 #include "../../include/vmcuda.h"
 #include "host_math.hpp"
-#include "hostmesh.hpp"
 
 namespace vm {
 namespace host {
@@ -478,10 +477,6 @@ struct vm_hostmesh {
     std::unique_ptr<vm::host::HostMesh> mesh;
 };
 
-bool vm_hostmesh_ranges_(const vm_hostmesh* mesh, const float Hoc[16], const vm_lens* lens, std::vector<std::pair<int, int>>& ranges) {
-    return mesh->mesh->lookup(Hoc, *lens, ranges);
-}
-
 extern "C" {
 
 // defined in engine.cu; the host mesh reports through the same channel
@@ -593,17 +588,23 @@ vm_status vm_hostmesh_lookup(const vm_hostmesh* mesh, const float Hoc[16], const
         vm_set_last_error_("null argument");
         return VM_ERR_INVALID_ARGUMENT;
     }
-    std::vector<std::pair<int, int>> out;
-    if (!mesh->mesh->lookup(Hoc, *lens, out)) {
-        vm_set_last_error_("Unknown lens type");
-        return VM_ERR_UNSUPPORTED_LENS;
+    try {
+        std::vector<std::pair<int, int>> out;
+        if (!mesh->mesh->lookup(Hoc, *lens, out)) {
+            vm_set_last_error_("Unknown lens type");
+            return VM_ERR_UNSUPPORTED_LENS;
+        }
+        *n_ranges = int32_t(out.size());
+        for (size_t i = 0; i < out.size() && int32_t(i) < capacity; ++i) {
+            ranges[2 * i]     = out[i].first;
+            ranges[2 * i + 1] = out[i].second;
+        }
+        return VM_OK;
     }
-    *n_ranges = int32_t(out.size());
-    for (size_t i = 0; i < out.size() && int32_t(i) < capacity; ++i) {
-        ranges[2 * i]     = out[i].first;
-        ranges[2 * i + 1] = out[i].second;
+    catch (const std::exception& e) {
+        vm_set_last_error_(e.what());
+        return VM_ERR_OUT_OF_MEMORY;
     }
-    return VM_OK;
 }
 
 }  // extern "C"
