@@ -25,11 +25,20 @@ def _check(net, n, n_neighbours):
     assert np.abs(got.astype(np.float64) - O.network(x, nb, net).astype(np.float64)).max() <= P.TOL_CLS / 4
 
 
-# one row per thread up to 147 blocks of 512 rows, two from there on (75776 is the last size of the one, 75777 the first of the other)
-@pytest.mark.parametrize("n", [1, 127, 129, 75_776, 75_777])
+# on 148 SMs: part of the outputs per block up to 1036 blocks of 128 rows and eight outputs (24 outputs: up to 44160 rows), one row per
+# thread up to 147 blocks of 512 rows (75264 rows), two from there on
+@pytest.mark.parametrize("n", [1, 127, 129, 44_160, 44_161, 75_264, 75_265, 75_776, 75_777])
 @pytest.mark.parametrize("n_neighbours,widths", [(4, [24, 20, 12, 5]), (6, [7, 13, 3]), (8, [28, 32, 31, 2])])
 def test_widths_without_a_kernel_of_their_own(n, n_neighbours, widths):
     _check(W.make_network(41, n_neighbours, widths), n, n_neighbours)
+
+
+# the same for layers with a kernel of their own: 444 blocks (16 outputs: 28416 rows; 8 outputs: 56832), 148 for 12 outputs (9472 rows)
+@pytest.mark.parametrize("n", [1, 128, 129, 9_472, 9_473, 28_416, 28_417, 56_832, 56_833, 75_264, 75_265])
+@pytest.mark.parametrize("n_neighbours,widths", [(4, [16, 8, 16, 5]), (6, [8, 16, 12, 12, 8, 3]), (8, [12, 16, 4, 32, 16, 2])])
+def test_layers_with_a_kernel_of_their_own(n, n_neighbours, widths, monkeypatch):
+    monkeypatch.setenv("VMCUDA_TC", "0")
+    _check(W.make_network(53, n_neighbours, widths), n, n_neighbours)
 
 
 @pytest.mark.parametrize("activation", [W.SELU, W.RELU, W.TANH, W.SOFTMAX])

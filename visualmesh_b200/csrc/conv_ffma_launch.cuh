@@ -24,16 +24,37 @@ bool launch_conv_narrow(const DenseLayer& L, const ConvArgs& a, dim3 grid, int m
 bool launch_conv_mid(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s);
 bool launch_conv_wide(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s);
 bool launch_conv_any(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s);
-bool launch_conv_few(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s);
+bool launch_conv_few(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, int blocks_per_sm, cudaStream_t s);
 
 constexpr int CW_MAX  = 2320;  // floats: a 16 -> 16 layer with 8 neighbours and its biases
 constexpr int CW_MOST = 8120;  // what the parameter space holds beside the other arguments: 28 -> 32 with 8 neighbours
 
-// Two rows per thread and 256 threads per block would leave SMs without a block (148 of them): such launches run one row per thread
-// in blocks of 128 threads.
-inline bool few_rows(int max_rows, int n_frames) {
-    return static_cast<int64_t>((max_rows + 511) / 512) * n_frames < 148;
+inline int sm_count() {
+    static LaunchPlans plans;
+    return plans.get([](int device) {
+        LaunchPlan p;
+        VM_CUDA(cudaDeviceGetAttribute(&p.n_sms, cudaDevAttrMultiProcessorCount, device));
+        return p;
+    }).n_sms;
 }
+// Two rows per thread and 256 threads per block would leave SMs without a block: such launches run one row per thread in blocks of 128
+// threads.
+inline bool few_rows(int max_rows, int n_frames) {
+    return static_cast<int64_t>((max_rows + 511) / 512) * n_frames < sm_count();
+}
+// The kernel with part of the outputs per block (launch_conv_few) pays while those blocks are few. A specialised layer with its weights
+// in the parameter space, one frame, us of that layer less with it: 16 -> 16 with six neighbours 3.5 at 0.9 blocks per SM, 2.0 at 2.2,
+// nothing from 2.8 on, 2.2 more at 7.2; 16 -> 8 1 to 2 up to 1.1, nothing at 2.5. Against the kernels of the other widths, and of the
+// layers too large for the parameter space, it pays further (24,20,12,5, six neighbours, us a call: 4.0 blocks per SM 67.9 -> 64.3, 4.6
+// 70.9 -> 65.8, 6.9 76.6 -> 76.2, 8.0 75.5 -> 79.3; 32 -> 16 13 at 0.5, 10 at 5.0, 5 at 7.2).
+// Twelve outputs leave half of their second part empty: 16 -> 12 gains 0.5 to 2.7 us up to one block per SM, 12 -> 12 and 8 -> 12 nothing,
+// and from there on all three lose, 2 to 3 us at 3.7.
+constexpr int FEW_BLOCKS_SPECIALISED = 3;
+constexpr int FEW_BLOCKS_TWELVE      = 1;
+constexpr int FEW_BLOCKS             = 7;
+// ... and while there are weights to share: below this many floats the parameter space is faster even for few blocks (8 -> 8, 328 to 584
+// floats: 1.1 to 1.5 us a layer; from 648 on, 16 -> 8 and 8 -> 16 with four neighbours, it is 1 to 2 us slower).
+constexpr size_t FEW_WEIGHTS = 640;
 // weights small enough for the kernel parameter space are read through the constant cache (measured 15-40 %
 // faster than the shared-memory copy: the weight reads leave the L1/shared data path to the gather)
 inline bool const_weights() {
@@ -90,13 +111,14 @@ static bool launch_conv_cw(const DenseLayer& L, const ConvArgs& a, dim3 grid_row
     return true;
 }
 
-// One shape: parameter-space weights where they fit (two rows per thread and 256 threads measured best for every shape tried), for few
-// rows one row per thread and, where the weights are more than the constant cache holds, the kernel that keeps them in shared memory.
+// One shape: parameter-space weights where they fit (two rows per thread and 256 threads measured best for every shape tried). For few
+// rows one row per thread, or the kernel that keeps part of the outputs' weights in shared memory.
 template <int CIN, int COUT, int RR>
 static bool launch_conv_shape(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s) {
     if (L.cin != CIN || L.cout != COUT) return false;
     if (const_weights() && few_rows(max_rows, grid.y)) {
-        if (L.host_packed.size() > 640 && launch_conv_few(L, a, grid, max_rows, s)) return true;
+        const int blocks = L.host_packed.size() > static_cast<size_t>(CW_MAX) ? FEW_BLOCKS : COUT == 12 ? FEW_BLOCKS_TWELVE : FEW_BLOCKS_SPECIALISED;
+        if (L.host_packed.size() > FEW_WEIGHTS && launch_conv_few(L, a, grid, max_rows, blocks, s)) return true;
         if (launch_conv_cw<CIN, COUT, 1, CW_MAX, 128>(L, a, grid, max_rows, s)) return true;
     }
     if (const_weights() && launch_conv_cw<CIN, COUT, 2, CW_MAX, 256>(L, a, grid, max_rows, s)) return true;

@@ -20,13 +20,10 @@ static bool launch_conv_few_t(const DenseLayer& L, const ConvArgs& a, dim3 grid_
     k_graph_conv_few<OW, threads><<<grid, threads, smem, s>>>(a, L.cin / 4, L.cout, L.coutp);
     return true;
 }
-bool launch_conv_few(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s) {
+bool launch_conv_few(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, int blocks_per_sm, cudaStream_t s) {
     if (L.cin % 4 != 0 || L.cin > 32 || L.coutp > 32 || a.out_split) return false;
-    // While eight outputs per block make no more than four blocks per SM: beyond that the arithmetic counts, and what the threads of a row
-    // would do twice (24,20,12,5 with four or six neighbours on 13 k rows 86 -> 80 and 96 -> 86 us a call; with eight on 25 k rows,
-    // which this line leaves to the other kernels, 112 -> 114).
     const int64_t blocks = static_cast<int64_t>((max_rows + 127) / 128) * grid.y * ((L.coutp + 7) / 8);
-    if (blocks > 4 * 148) return false;
+    if (blocks > static_cast<int64_t>(blocks_per_sm) * sm_count()) return false;
     // all outputs in a block where a row's outputs meet
     const int outputs = a.activation == VM_SOFTMAX || a.out_host != nullptr ? L.coutp : std::min(L.coutp, 8);
     if (outputs <= 4) return launch_conv_few_t<4>(L, a, grid, max_rows, s);
@@ -45,7 +42,7 @@ static void launch_conv_any_t(const DenseLayer& L, const ConvArgs& a, dim3 grid_
     k_graph_conv_any<COUTP, 2, threads, WMAX><<<grid, threads, stage_bytes(a, L.cout, threads, 2), s>>>(a, L.cin / 4, L.cout, wp);
 }
 bool launch_conv_any(const DenseLayer& L, const ConvArgs& a, dim3 grid, int max_rows, cudaStream_t s) {
-    if (few_rows(max_rows, grid.y) && launch_conv_few(L, a, grid, max_rows, s)) return true;
+    if (few_rows(max_rows, grid.y) && launch_conv_few(L, a, grid, max_rows, FEW_BLOCKS, s)) return true;
     if (L.cin % 4 != 0 || L.coutp > 32 || L.host_packed.size() > static_cast<size_t>(CW_MOST) || a.out_split) return false;
     const bool small = L.host_packed.size() <= static_cast<size_t>(CW_MAX);
 #define VM_ANY(CP)                                                             \
