@@ -21,7 +21,7 @@ prints one JSON line:
 With N > 1 (launched by torchrun, one rank per GPU) every rank runs the same per-GPU batch on its own frames; frames
 are independent, so there is no collective on the data path - only a barrier and a max over ranks around the timing.
 `--impl reference` times the reference's own CPU engine (oracle/_ref, the unmodified reference compiled in place) with
-one engine instance per host core, the pattern of example/benchmark.cpp:86-101,142.
+one engine instance per host core, the pattern of example/benchmark.cpp:86-101,142; where that is not there it says so.
 """
 import argparse
 import hashlib
@@ -173,6 +173,11 @@ def _cpu_reference_run(wl, frames, n_threads):
 
 def run_reference(args, rank, world):
     if rank != 0:
+        return
+    import refharness as R
+    if not R.available():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's CPU engine (header-only C++) is not compiled here: its sources are missing"}),
+              flush=True)
         return
     wl = W.config(args.config, seed=args.seed, n_frames=max(args.frames, 1))
     cores = os.cpu_count() or 1
