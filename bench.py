@@ -49,7 +49,7 @@ USER_SET_BLOCKING_SYNC = "VMCUDA_BLOCKING_SYNC" in os.environ
 # rows of the captured launch); traffic grows in proportion to the rows, so it is scaled to the bench's launches.
 NCU_TRAFFIC_BYTES_PER_ROW = {
     (16, 16): 110.6,  # profiles/graph_conv_staged_16x16_cfg1_16frames.md: 122.6 MB over 1,108,261 rows
-    (32, 32): 250.4,  # profiles/graph_conv_tc_tmem_32x32_cfg3_1frame.md: 233.3 MB over 931,718 rows
+    (32, 32): 229.5,  # profiles/graph_conv_window_32x32_cfg3_1frame.md: 213.8 MB over 931,718 rows
 }
 
 
@@ -57,8 +57,8 @@ def _kernel_of_layer(cin, cout):
     """Which kernel the engine's default policy runs a gather layer on (visualmesh_b200/csrc/engine.cu, run_network)."""
     if cin == 16 and cout in (8, 16, 32):
         return "st::k_graph_conv_mma (shared-memory windows, ldmatrix gather, mma.sync)"
-    if cin in (16, 32) and cout in (16, 32) and cin * cout >= 512:
-        return "tc::k_graph_conv_tc_tmem (tcgen05, A operand in tensor memory)"
+    if cin == 32 and cout >= 16:  # behind a layer of 32 outputs, as in every configuration
+        return "win::k_graph_conv_window (shared-memory windows, tcgen05, A operand in tensor memory)"
     return "k_graph_conv_cw (FFMA)"
 
 
