@@ -184,7 +184,9 @@ VM_API vm_status vm_call(vm_engine* engine,
  * engine and are overwritten by its next call. vm_results_keep hands the host arrays of the engine's last call over to the caller
  * instead of having them copied: they stay valid until vm_results_release, whatever becomes of the engine, and then serve it again.
  * At most VM_MAX_KEPT_RESULTS are kept per engine; one more fails with VM_ERR_OUT_OF_MEMORY and leaves the results where they
- * are. vm_results_release may be called from any thread. */
+ * are. A set of result arrays is pinned memory for all candidates of the largest batch it served, 12 + 4 * (neighbours + classes)
+ * bytes each (its points are not counted when it is made); sets that were given back serve later calls and are freed with the
+ * engine, so that an engine holds up to VM_MAX_KEPT_RESULTS + 1 of them. vm_results_release may be called from any thread. */
 #define VM_MAX_KEPT_RESULTS 4
 typedef struct vm_results vm_results;
 VM_API vm_status vm_results_keep(vm_engine* engine, vm_results** kept);

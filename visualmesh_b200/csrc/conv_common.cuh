@@ -15,9 +15,9 @@ __device__ __forceinline__ float selu(float s) {
     const float lambda       = 1.0507009873554804934193349852946f;
     const float lambda_alpha = 1.7580993408473768599402175208123f;
     // exp is evaluated for every value and the result selected: straight-line code, so the chains of a row's outputs overlap. Written
-    // as one multiply-add of 2^(s log2 e); the product before it loses |s| 2^-24 of an exponential that has become small by then. Five
-    // instructions instead of about fifteen with expf, and over all floats the largest error against double is below that of
-    // lambda * (alpha * expf(s) - alpha), which rounds three times behind the exponential (3.2e-7 against 3.6e-7).
+    // as one multiply-add of 2^(s log2 e); the product before it loses |s| 2^-24 of an exponential that has become small by then. Over
+    // 3 M negative values from 2^-30 to 2^7 the largest error against double is 1.96e-7, that of lambda * (alpha * exp(s) - alpha), which
+    // rounds three times behind the exponential, 2.21e-7. 16 -> 16 layers over 4.4 M rows 223 -> 211 us each with it, 4 -> 16 116 -> 102.
     float e;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__fmul_rn(s, 1.4426950408889634f)));
     const float negative = fmaf(lambda_alpha, e, -lambda_alpha);

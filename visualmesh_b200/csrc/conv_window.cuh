@@ -17,12 +17,13 @@
 // Roles: two gather groups of four warps (128 rows, one MMA tile) that store units of up to three slots of A into a ring in tensor
 // memory, one warp that issues the MMAs (the weights' hi and lo parts side by side as N, so half as many to issue), a group of four
 // warps for the epilogue, one loader warp. They meet at mbarriers only. 14 warps leave 128 registers a thread, and two steps of the
-// gather in flight; three groups with 96 registers and one step measured 6 % slower, with two steps (spills) 28 %, a second group for
-// the epilogue 10 % slower, units of one slot 10 % slower (the barriers).
-// What bounds a 128-row tile with eight neighbours: the load/store path of its SM, about 2300 cycles for the gather's loads (1152 and
-// their conflicts), the stores to tensor memory, the window and the output, while the MMAs take 1190; the tile takes about 4000,
-// the rest being the chain load -> store -> settle -> MMA of a unit with only two groups to overlap it. Measured on the 32 -> 32 layer
-// over 7.4 M rows: 834 us, against 1394 us for the kernel that gathers with global loads (conv_tc.cuh).
+// gather in flight. Measured on the way here, 32 -> 32 over 7.4 M rows, against 820 us when this form was settled: three groups with 96
+// registers and one step 883 us, with two steps (spills) 1064; a second group for the epilogue 970 and units of one slot 1075 (the
+// barriers), either about a tenth more than the form it was tried on; hi and lo parts as two MMAs 978.
+// What bounds a 128-row tile with eight neighbours (counters of one frame, 0.93 M rows): it takes 3420 cycles of its SM. The load/store
+// path works 2120 of them - the gathered rows 1152 and 300 of conflicts, the stores to tensor memory, the window and the output - and
+// the tensor pipe 1150; the rest is the chain load -> store -> settle -> MMA of a unit with only two groups to overlap it. The layer
+// takes 761 us over 7.4 M rows, against 1394 us with the kernel that gathers with global loads (conv_tc.cuh).
 //
 // Every wait is bounded: a wait that runs out raises the abort flag, the CTA stops issuing work, waits (bounded) for its own copies
 // and MMAs, frees its tensor memory and returns. No multicast; all copies read this GPU's own memory.

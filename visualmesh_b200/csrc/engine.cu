@@ -285,7 +285,9 @@ struct vm_engine {
     int64_t launches = 0;
     bool use_tc      = true;
     int tc_mode      = 1;
-    int tc_min_product = 512;   // mode 1: layers with C_in x C_out at least this run on the tensor cores
+    // mode 1: layers with C_in x C_out at least this run on the tensor cores. Narrower ones are slower there: 32 -> 4 over 7.4 M rows takes
+    // 790 us on the CUDA cores and 2241 us on the window kernel.
+    int tc_min_product = 512;
     bool tc_no_split = false;   // debugging: never use the split feature layout
     bool staged          = true;    // tensor-core layers read their gather from shared-memory windows (conv_staged.cuh)
     bool may_stage       = false;   // some layer could run as a staged tensor-core layer under the engine's policy
@@ -867,7 +869,7 @@ static GraphKey graph_key(const vm_engine* e, const Lane& lane, const Chunk& c, 
 }
 
 // Enqueues what `issue` enqueues on the lane's stream. A chunk of this shape that comes back is recorded as a CUDA graph and from
-// then on costs one launch: on the B200 box a launch takes 2.7 to 3.8 us of host time, so that 8 small kernels and a wait take
+// then on costs one launch: on a B200's host of 16 cores a launch takes 2.7 to 3.8 us of host time, so that 8 small kernels and a wait take
 // 32 us one by one and 11 us as a graph, 16 kernels 49 and 15 us. The first time nothing is recorded: recording and instantiating
 // costs more than it saves on a shape that may never return.
 template <typename Issue>

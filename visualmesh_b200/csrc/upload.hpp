@@ -1,7 +1,7 @@
 // Uploads of camera frames from ordinary (pageable) host memory.
 //
 // The driver copies pageable memory through a staging buffer of its own on the calling thread: 294 us for a 5 MB frame and
-// 1.14 ms for a 21 MB one on the B200 box (16 cores), against 102 us and 400 us of bus time. Here the frame is cut into slices
+// 1.14 ms for a 21 MB one on a B200's host of 16 cores, against 102 us and 400 us of bus time. Here the frame is cut into slices
 // that the calling thread and a few helper threads copy into the lane's pinned buffer with non-temporal stores (which leave no
 // dirty lines for the bus to snoop), and every run of finished slices is sent on its way while the next ones are copied: 143 us
 // and 504 us. The helpers sleep between uploads; they belong to all engines of the process, and the last engine ends them.

@@ -300,7 +300,14 @@ class Engine:
     def __call__(self, mesh, Hoc, lens, image=None, format=None, ranges="host"):
         """The two reference calls. ranges="host" looks up the nodes of a mesh with host tables as the reference engines do
         (cpp/visualmesh/engine/opencl/engine.hpp:581; the work itself is done wherever it is faster, with the same result),
-        ranges="device" walks the BSP on the GPU, or pass the ranges."""
+        ranges="device" walks the BSP on the GPU, or pass the ranges.
+
+        The arrays of the result are the engine's own pinned memory, handed over without a copy for as long as one of them (or a view)
+        is alive: up to four results of an engine at a time (VM_MAX_KEPT_RESULTS). While a caller holds four, further results are
+        copied into ordinary arrays (6.3 ms for 930 k points with eight neighbours and four classes). A set of pinned arrays is made
+        before the points are counted, so it is as large as the candidates, the nodes of the mesh or of the given ranges, may need:
+        12 + 4 * (neighbours + classes) bytes each, 117 MB for 1.73 M nodes with eight neighbours and four classes. An engine keeps up
+        to five sets until it is closed and its results are gone."""
         m = mesh.height(np.asarray(Hoc, dtype=np.float32).reshape(4, 4)[2][3]) if isinstance(mesh, VisualMesh) else mesh
         host = None
         if isinstance(ranges, str):
