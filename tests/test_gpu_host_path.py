@@ -53,6 +53,28 @@ def test_images_from_every_kind_of_memory_give_the_same_results(width, height):
     pinned_free(pinned)
 
 
+def test_frames_pinned_one_by_one_that_lie_next_to_one_another():
+    """Frames that follow one another in memory travel as one copy, but no copy reaches from one allocation into the next."""
+    case = G.Case("ring6_equisolid_rgba")
+    mesh = Mesh.from_arrays(case.rays, case.nbrs, case.bsp)
+    lens = W.Lens((512, 512), W.EQUISOLID, 0.35 * 512, (0.0, 0.0), (0.0, 0.0), np.pi)
+    engine = Engine(case.network)
+    buffers = sorted((pinned_empty(512 * 512 * 4) for _ in range(24)), key=lambda b: b.ctypes.data)
+    if not any(b.ctypes.data - a.ctypes.data == a.size for a, b in zip(buffers, buffers[1:])):
+        pytest.skip("no two of these allocations lie next to one another")
+    for i, b in enumerate(buffers):
+        b[:] = W.random_bytes(50 + i, b.size)
+    frames = [FrameInput(mesh, case.frames[i % 3]["Hoc"], lens, b, W.fourcc("RGBA"), None) for i, b in enumerate(buffers)]
+    want = [engine.run_batch([fr]).frame(0) for fr in frames]
+    for _ in range(3):
+        batch = engine.run_batch(frames)
+        for f, w in enumerate(want):
+            _same(batch.frame(f), w)
+    engine.close()
+    for b in buffers:
+        pinned_free(b)
+
+
 def test_host_ranges_of_changing_poses_leave_nothing_behind():
     """With host ranges the node table is not cleared between calls: entries of an earlier pose must not be taken for points."""
     case = G.Case("ring6_equisolid_rgba")

@@ -592,8 +592,23 @@ static std::unique_ptr<Upload> start_images(vm_engine* e, Lane& lane, const vm_f
     }
     const uint8_t* run_src = nullptr;
     size_t run_dst = 0, run_bytes = 0;
-    auto flush = [&] {
-        if (run_bytes > 0) VM_CUDA(cudaMemcpyAsync(lane.d_images.p + run_dst, run_src, run_bytes, cudaMemcpyHostToDevice, e->copy_stream));
+    int run_first = f0;
+    auto copy = [&](const uint8_t* src, size_t dst, size_t bytes) {
+        return cudaMemcpyAsync(lane.d_images.p + dst, src, bytes, cudaMemcpyHostToDevice, e->copy_stream);
+    };
+    auto flush = [&](int end) {
+        if (run_bytes == 0) return;
+        cudaError_t err = copy(run_src, run_dst, run_bytes);
+        if (err == cudaErrorInvalidValue && run_bytes > image_bytes(frames[run_first])) {
+            // frames that follow one another but were pinned one by one: a copy may not reach from one allocation into the next
+            cudaGetLastError();
+            err = cudaSuccess;
+            for (int f = run_first; f < end && err == cudaSuccess; ++f) {
+                if (frames[f].image_on_device || plan.at[f - f0] < plan.pageable) continue;
+                err = copy(static_cast<const uint8_t*>(frames[f].image), plan.at[f - f0], image_bytes(frames[f]));
+            }
+        }
+        VM_CUDA(err);
         run_bytes = 0;
     };
     for (int f = f0; f < f1; ++f) {
@@ -602,13 +617,14 @@ static std::unique_ptr<Upload> start_images(vm_engine* e, Lane& lane, const vm_f
         const uint8_t* src = static_cast<const uint8_t*>(frames[f].image);
         if (run_bytes > 0 && src == run_src + run_bytes && plan.at[f - f0] == run_dst + run_bytes) { run_bytes += bytes; }
         else {
-            flush();
+            flush(f);
+            run_first = f;
             run_src   = src;
             run_dst   = plan.at[f - f0];
             run_bytes = bytes;
         }
     }
-    flush();
+    flush(f1);
     return upload;
 }
 
