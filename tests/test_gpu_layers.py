@@ -77,6 +77,36 @@ def test_layers_of_32_channels_with_neighbours_close_by():
     assert np.abs(got.astype(np.float64) - O.network(x, nb, net).astype(np.float64)).max() <= P.TOL_CLS / 4
 
 
+def _near(n, n_neighbours, reach):
+    """Neighbours within `reach` rows, so that most lie in the row's own window."""
+    near = (W.splitmix64(6, n * n_neighbours) % np.uint64(2 * reach + 1)).astype(np.int64).reshape(n, n_neighbours) - reach
+    return np.clip(np.arange(n)[:, None] + near, 0, n - 1).astype(np.int32)
+
+
+# tiles of 8 rows, groups of 32, super-tiles of 256; 113 921 rows are two super-tiles for some of 444 CTAs. Every layout in front of
+# and behind a 16-channel layer: from the CUDA cores, from the window kernel and from one another, to either of them and to fp32
+@pytest.mark.parametrize("n", [1, 7, 9, 31, 33, 255, 257, 9_472, 113_921])
+@pytest.mark.parametrize("n_neighbours,widths", [(4, [16, 16, 8, 3]), (6, [8, 16, 32, 32, 16, 16, 8, 2]), (8, [16, 32, 16, 12, 16, 8, 5])])
+@pytest.mark.parametrize("activation", [W.SELU, W.TANH])
+def test_layers_of_16_channels_with_neighbours_close_by(n, n_neighbours, widths, activation):
+    net = W.make_network(59, n_neighbours, widths)
+    for group in net[:-1]:
+        group[0].activation = activation
+    x, _ = _rows(n, n_neighbours, 7)
+    nb = _near(n, n_neighbours, 40)
+    engine = Engine(net)
+    got = engine.network(x, nb)
+    engine.close()
+    assert np.abs(got.astype(np.float64) - O.network(x, nb, net).astype(np.float64)).max() <= P.TOL_CLS / 4
+
+
+# random neighbours lie outside the window, most of them beyond its halo
+@pytest.mark.parametrize("n", [1, 33, 257, 9_473])
+@pytest.mark.parametrize("n_neighbours,widths", [(4, [16, 16, 8, 3]), (6, [16, 32, 16, 16, 8, 2]), (8, [16, 16, 8, 5])])
+def test_layers_of_16_channels_with_neighbours_anywhere(n, n_neighbours, widths):
+    _check(W.make_network(61, n_neighbours, widths), n, n_neighbours)
+
+
 def test_selu_over_its_range():
     """A layer that passes its input through: SELU of floats of every size, against double.
 

@@ -27,13 +27,14 @@ struct ConvArgs {
     int32_t in_stride;      // rows per planar chunk of `in`
     int32_t out_stride;     // rows per planar chunk of `out`
     int32_t out_planar;     // write `out` chunk-planar (needs COUT % 4 == 0 and !out_global)
-    int32_t out_split;      // write `out` as fp16 hi/lo parts for a tensor-core consumer: SPLIT_PLANES (COUT % 8 == 0) or SPLIT_ROWS
+    int32_t out_split;      // write `out` as fp16 hi/lo parts for a tensor-core consumer: SPLIT_PLANES (COUT % 8 == 0), SPLIT_ROWS or SPLIT_QUADS
     float* const* out_host; // where the batch-wide classifications go instead of `out`: the device address of a pointer to pinned memory
     int32_t* range_flag;    // the engine's abort flags: ABORT_RANGE is raised when a value is too large for the fp16 split
 };
 
-// ConvArgs::out_split. Planes of 16-byte chunks, or whole rows for the window kernel (its 32 input channels: COUT == 32).
-enum SplitLayout { SPLIT_NONE = 0, SPLIT_PLANES = 1, SPLIT_ROWS = 2 };
+// ConvArgs::out_split. Planes of 16-byte chunks; whole rows for the window kernel (its 32 input channels: COUT == 32), 32 hi parts, then
+// 32 lo parts; whole rows for the staged kernel (its 16 input channels: COUT == 16), pieces of four hi and four lo parts.
+enum SplitLayout { SPLIT_NONE = 0, SPLIT_PLANES = 1, SPLIT_ROWS = 2, SPLIT_QUADS = 3 };
 
 constexpr int CONV_THREADS = 128;
 

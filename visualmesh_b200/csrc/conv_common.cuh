@@ -127,4 +127,40 @@ __device__ __forceinline__ void store_split_rows(float* out, size_t row, bool va
     }
 }
 
+// Rows of 16 channels for the staged kernel (SPLIT_QUADS): four 16-byte pieces a row, each four hi parts and their four lo parts.
+__device__ __forceinline__ uint4 split_quad(const float* v, bool& bad) {
+    uint4 q;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) bad |= fabsf(v[k]) > 60000.0f;
+    split_pair(v[0], v[1], q.x, q.z);
+    split_pair(v[2], v[3], q.y, q.w);
+    return q;
+}
+// the row of a thread
+__device__ __forceinline__ void store_split_quads(float* out, size_t row, const float* v, int32_t* range_flag) {
+    bool bad = false;
+    uint4* dst = reinterpret_cast<uint4*>(out) + row * 4;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) dst[p] = split_quad(v + 4 * p, bad);
+    if (bad) raise_flag(range_flag, ABORT_TC_RANGE);
+}
+// the rows of a warp by way of shared memory (as in store_split_rows; stage: 2 KB of the warp)
+constexpr int SPLIT_QUAD_STAGE = 32 * 64;
+__device__ __forceinline__ void store_split_quads(float* out, size_t row, bool valid, const float* v, uint4* stage, int32_t* range_flag) {
+    const int lane = threadIdx.x & 31;
+    bool bad       = false;
+    __syncwarp();
+#pragma unroll
+    for (int p = 0; p < 4; ++p) stage[lane * 4 + (p ^ (lane >> 1 & 3))] = split_quad(v + 4 * p, bad);
+    if (bad && valid) raise_flag(range_flag, ABORT_TC_RANGE);
+    __syncwarp();
+    const int pieces = __popc(__ballot_sync(0xffffffffu, valid)) * 4;
+    uint4* dst       = reinterpret_cast<uint4*>(out) + (row - lane) * 4;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = k * 32 + lane, r = i / 4, p = i % 4;
+        if (i < pieces) dst[i] = stage[r * 4 + (p ^ (r >> 1 & 3))];
+    }
+}
+
 }  // namespace vm

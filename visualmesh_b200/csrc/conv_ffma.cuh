@@ -110,6 +110,13 @@ __global__ void __launch_bounds__(T, MINB) k_graph_conv(const ConvArgs a) {
                 continue;
             }
         }
+        if constexpr (COUT == 16) {
+            if (a.out_split == SPLIT_QUADS) {
+                uint4* stage = reinterpret_cast<uint4*>(smem4 + (K * COUTP + COUTP) / 4) + (threadIdx.x >> 5) * (SPLIT_QUAD_STAGE / 16);
+                store_split_quads(a.out, out_base + i, i < rows, acc[q], stage, a.range_flag);
+                continue;
+            }
+        }
         if (i >= rows) continue;
         float* dst = a.out + (out_base + i) * COUT;
         if (COUT % 8 == 0 && a.out_split) { store_split<(COUT % 8 == 0 ? COUT : 8)>(a.out, a.out_stride, out_base + i, acc[q], a.range_flag); }
@@ -182,7 +189,7 @@ template <int CIN, int COUT, int R, int WMAX, int T = CONV_THREADS, int NS = 0>
 __global__ void __launch_bounds__(T, (CIN == 8 && COUT <= 8 && T == 256) ? 6 : 0) k_graph_conv_cw(const ConvArgs a, const __grid_constant__ ConvWeights<WMAX> wp) {
     static_assert(CIN % 4 == 0, "vector loads of the input rows");
     constexpr int COUTP = (COUT + 3) & ~3;
-    extern __shared__ uint4 split_stage[];  // SPLIT_ROW_STAGE bytes per warp when the output is split in rows; the results for the host
+    extern __shared__ uint4 split_stage[];  // SPLIT_ROW_STAGE (SPLIT_QUAD_STAGE) bytes per warp when the output is split in rows; the results for the host
     const int frame_in_chunk = blockIdx.y;
     const int frame          = a.f0 + frame_in_chunk;
     const int start          = a.offsets[frame];
@@ -257,6 +264,12 @@ __global__ void __launch_bounds__(T, (CIN == 8 && COUT <= 8 && T == 256) ? 6 : 0
         if constexpr (COUT == 32) {
             if (a.out_split == SPLIT_ROWS) {
                 store_split_rows(a.out, out_base + i, i < rows, v, split_stage + (threadIdx.x >> 5) * (SPLIT_ROW_STAGE / 16), a.range_flag);
+                continue;
+            }
+        }
+        if constexpr (COUT == 16) {
+            if (a.out_split == SPLIT_QUADS) {
+                store_split_quads(a.out, out_base + i, i < rows, v, split_stage + (threadIdx.x >> 5) * (SPLIT_QUAD_STAGE / 16), a.range_flag);
                 continue;
             }
         }

@@ -68,7 +68,8 @@ inline bool const_weights() {
 // shared memory in which the warps of a block arrange split rows, or the block its results for the host, before they store them
 inline size_t stage_bytes(const ConvArgs& a, int cout, int threads, int rows_per_thread) {
     if (a.out_host != nullptr) return static_cast<size_t>(threads) * rows_per_thread * cout * sizeof(float);
-    return a.out_split == SPLIT_ROWS ? static_cast<size_t>(threads / 32) * SPLIT_ROW_STAGE : 0;
+    const int warp = a.out_split == SPLIT_ROWS ? SPLIT_ROW_STAGE : a.out_split == SPLIT_QUADS ? SPLIT_QUAD_STAGE : 0;
+    return static_cast<size_t>(threads / 32) * warp;
 }
 
 template <int CIN, int COUT, int R, int T = CONV_THREADS, int MINB = 1>

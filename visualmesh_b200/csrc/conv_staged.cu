@@ -10,12 +10,12 @@ namespace vm {
 static_assert(STAGED_NBL_STRIDE == st::NBL_STRIDE && STAGED_ST == st::ST && STAGED_HALO == st::HALO,
               "the engine sizes the plan with the kernels' own constants");
 
-template <int CIN, int COUT, int NSLOTS>
+template <int COUT, int NSLOTS>
 static void launch_conv_staged_t(const DenseLayer& L, const ConvArgs& a, const st::Plan& plan, int n_frames, int max_rows, int32_t* abort_flags,
                                  uint32_t wait_limit, cudaStream_t s) {
-    constexpr int THREADS = (CIN == 16 ? 8 : 16) * 32 + 32;  // compute warps + the loader warp
-    constexpr auto kernel = st::k_graph_conv_mma<CIN, COUT, NSLOTS, THREADS>;
-    constexpr size_t smem = st::smem_bytes<CIN, COUT, NSLOTS, THREADS>();
+    constexpr int THREADS = 4 * 32 + 32;  // compute warps + the loader warp
+    constexpr auto kernel = st::k_graph_conv_mma<COUT, NSLOTS, 4, THREADS, COUT == 32 ? 2 : 3>;
+    constexpr size_t smem = st::smem_bytes<COUT, NSLOTS>();
     static LaunchPlans plans;
     const LaunchPlan& lp = plans.get([](int dev) {
         LaunchPlan p;
@@ -51,7 +51,7 @@ bool launch_conv_staged(const DenseLayer& L, const ConvArgs& a, const StagedPlan
     const st::Plan p{plan.nbl, plan.halo_rows, plan.halo_count};
 #define VM_STG(CI, CO, NS)                                                                             \
     if (L.cin == CI && L.cout == CO && L.n_slots == NS) {                                                \
-        launch_conv_staged_t<CI, CO, NS>(L, a, p, n_frames, max_rows, abort_flags, wait_limit, s);        \
+        launch_conv_staged_t<CO, NS>(L, a, p, n_frames, max_rows, abort_flags, wait_limit, s);        \
         return true;                                                                                     \
     }
     VM_STG(16, 8, 5) VM_STG(16, 8, 7) VM_STG(16, 8, 9) VM_STG(16, 16, 5) VM_STG(16, 16, 7) VM_STG(16, 16, 9)

@@ -10,16 +10,32 @@
 // So the rows of a frame are cut into super-tiles of consecutive rows and a tile plan (tile_plan.cuh) is made once per
 // chunk of frames: the list of outside rows each super-tile needs (its halo) and every row's neighbours as 16-bit
 // positions inside "super-tile + halo". A layer then runs as a persistent kernel whose loader warp brings a
-// super-tile's own rows into shared memory with one bulk asynchronous copy per 16-byte plane and its halo rows with
-// 16-byte asynchronous copies - every byte of the feature buffer is requested once per super-tile that needs it, in
-// large contiguous pieces, a super-tile ahead of its use - and whose compute warps read neighbour rows from shared
-// memory only: ldmatrix takes one row address per lane, so the gather of sixteen neighbour rows IS the load of an MMA
-// operand fragment. The product runs on the warp-level tensor-core path (mma.sync m16n8k16, fp16 hi/lo parts of both
-// operands, fp32 accumulators in registers) rather than tcgen05: a 16-channel slot is a 16x16x16 product per sixteen
-// rows, far too little work per instruction to amortise moving a gathered tile into tensor memory and a single-thread
-// issue pipeline, while here every warp is an independent worker with nothing to hand over (measured on the 16 -> 16
-// layer over 4.4 M rows: tcgen05 with global-load gather 337 us, tcgen05 with this staging 740 us at one CTA per SM,
-// this kernel 222 us; the FFMA kernel 308 us). The epilogue runs on the accumulator registers.
+// super-tile's own rows and their positions into shared memory with one bulk asynchronous copy each and its halo rows with
+// 16-byte asynchronous copies - every byte of the feature buffer is requested once per super-tile that needs it, a
+// super-tile ahead of its use - and whose compute warps read neighbour rows from shared memory only. The product runs on
+// the warp-level tensor-core path (mma.sync m16n8k16, fp16 hi/lo parts of both operands, fp32 accumulators in registers)
+// rather than tcgen05: a 16-channel slot is a 16x16x16 product per sixteen rows, far too little work per instruction to
+// amortise moving a gathered tile into tensor memory and a single-thread issue pipeline, while here every warp is an
+// independent worker with nothing to hand over (the 16 -> 16 layer over 4.4 M rows: tcgen05 with global-load gather
+// 337 us, tcgen05 with this staging 740 us at one CTA per SM; the FFMA kernel 308 us).
+//
+// What bounds it is the shared-memory data path, then the rate of mma.sync (measured: one m16n8k16 per 8.5 cycles and SM
+// sub-partition, 89 cycles for the 42 of sixteen rows of the 16 -> 16 layer with six neighbours). Three choices keep that path short:
+//   - The weights are the operand with sixteen rows and the gathered rows the one with eight columns. A feature row is four
+//     16-byte pieces, each the hi and the lo parts of four channels, and a thread's piece of a row IS its two registers
+//     of that operand, hi and lo: one 16-byte load, no register is moved. (As the operand with sixteen rows its four
+//     registers come from two loads: 170 moves more per sixteen rows.)
+//   - A quarter-warp reads two whole rows of 64 bytes, so only two rows of the same parity meet in a bank (a third of the
+//     pairs on the meshes here: consecutive rows have neighbours that follow one another). Rows in planes of 16-byte
+//     pieces, eight of them per quarter-warp as ldmatrix takes them, took 2.25 passes where this takes 1.4.
+//   - Twelve warps per SM with 128 registers instead of 24 with 72: loads of the next slot are in flight during the products of
+//     one, and nothing spills. The eight-channel layers also keep their weights in registers (the sixteen-channel ones
+//     have twice as many, which spills).
+// 16 -> 16 over 4.48 M rows with six neighbours 212 -> 169 us (the weights' fragments are 28 of its 115 wavefronts of shared-memory
+// loads per sixteen rows, the rows 56 and 24 of conflicts), 16 -> 8 176 -> 123 us (138 with the weights read for each slot). On the way:
+// planes and ldmatrix with fewer instructions 212; the layout alone 219 and 152; weights as the first operand with 24 warps 200 and 152;
+// with twelve 182 and 138; split rows transposed before they are stored (stores of a quarter-warp in one 128-byte line, not
+// four) 169. Sixteen compute warps in two CTAs 192; groups of 64 rows 177 (spills).
 // A neighbour whose halo slot did not fit (more outside rows than halo slots) is marked and fetched from global memory
 // by its warp, so any neighbourhood is computed correctly, only slower.
 //
@@ -82,16 +98,22 @@ namespace st {
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
     }
     // ---- warp-level tensor-core pieces ----------------------------------------------------------------------------------
-    // Four 8x8 fp16 matrices, one 16-byte row address per lane: the A fragment of mma.m16n8k16 for sixteen ARBITRARY
-    // rows of shared memory - the gather of a slot is this one instruction.
-    __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
-        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+    __device__ __forceinline__ uint4 load_shared(uint32_t addr) {
+        uint4 v;
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+        return v;
     }
     // D += A . B, A 16x16 fp16 (row), B 16x8 fp16 (col), D 16x8 fp32
-    __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    __device__ __forceinline__ void mma_16816(float (&d)[4], const uint4& a, uint32_t b0, uint32_t b1) {
         asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                     : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+                     : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+    }
+    // an 8x8 matrix of fp16 values, two neighbours of row g per thread
+    __device__ __forceinline__ uint32_t transpose(uint32_t v) {
+        uint32_t r;
+        asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+        return r;
     }
     struct Args {
         int32_t n_frames;
@@ -102,59 +124,54 @@ namespace st {
 
     constexpr uint32_t WAIT_LIMIT  = tc::WAIT_LIMIT;
     constexpr int MAX_FRAMES       = tc::MAX_FRAMES;
-    constexpr int TILE             = 16;  // rows of one warp-level MMA tile
+    constexpr int TILE             = 8;   // rows of one warp-level MMA tile (its N)
+    constexpr int CIN              = 16;  // input channels
+    constexpr int ROW              = 4 * CIN;  // bytes of a feature row: four pieces of four channels, hi parts then lo parts each
+    constexpr int WINDOW           = (ST + HALO) * ROW;
+    constexpr int NBL_BYTES        = ST * NBL_STRIDE * 2;
 
-    constexpr int PAIR = 2;  // 16-row tiles a warp works on at a time: two independent chains of MMAs to interleave
-
-    template <int CIN, int COUT, int NSLOTS, int THREADS>
+    // 16x16 fragments of a slot's weights: hi and lo parts of 16 output channels each, or of eight channels in one
+    template <int COUT>
+    __host__ __device__ constexpr int weight_fragments() {
+        return COUT == 8 ? 1 : COUT / 8;
+    }
+    template <int COUT, int NSLOTS>
     __host__ __device__ constexpr size_t smem_bytes() {
-        return static_cast<size_t>(2) * (2 * (CIN / 8)) * (ST + HALO) * 16                     // two windows
-               + static_cast<size_t>(THREADS / 32 - 1) * (2 * (CIN / 8)) * TILE * 16           // per-warp rows fetched from global memory
-               + static_cast<size_t>(NSLOTS) * (CIN / 16) * (COUT / 8) * 2 * 32 * 8;           // B fragments, hi and lo
-    }
-    template <int CIN, int COUT>
-    __host__ __device__ constexpr int ctas_per_sm_wanted() {
-        return CIN == 16 ? (COUT <= 16 ? 3 : 2) : 1;
+        return static_cast<size_t>(2) * (WINDOW + NBL_BYTES)                  // two windows and their neighbour positions
+               + static_cast<size_t>(NSLOTS) * weight_fragments<COUT>() * 32 * 16;
     }
 
-    // One CTA walks super-tiles; while it computes on one window the next is on its way. Every warp owns pairs of 16-row
-    // tiles of the super-tile: for each slot one ldmatrix per fp16 part and tile gathers the sixteen neighbour rows from
-    // the window, three MMAs per 8 output columns add hi.hi, hi.lo and lo.hi into fp32 accumulators in registers
-    // (dropping only lo.lo keeps ~2^-21 relative accuracy), and the epilogue (bias, activation, store as fp32 chunks or
-    // split again for the next such layer) runs on the accumulator registers. The weights sit in shared memory as
-    // ready-made B fragments (8 bytes per lane, read once per slot for both tiles). The last warp of the CTA is the
-    // loader; a compute warp waits only for a window to land and tells the loader when it is done with one, so no
-    // compute warp ever waits for another.
-    template <int CIN, int COUT, int NSLOTS, int THREADS>
-    __global__ void __launch_bounds__(THREADS, ctas_per_sm_wanted<CIN, COUT>()) k_graph_conv_mma(const ConvArgs a, const Args t, const Plan plan) {
-        static_assert(CIN % 16 == 0 && COUT % 8 == 0 && ST % (PAIR * TILE) == 0, "whole K steps, whole column blocks, whole tile pairs");
-        constexpr int PLANES    = CIN / 8;   // 16-byte chunks of the hi (or lo) half of a row
-        constexpr int ALLP      = 2 * PLANES;
-        constexpr int KSTEPS    = CIN / 16;
-        constexpr int NBLK      = COUT / 8;
-        constexpr int WARPS     = THREADS / 32 - 1;       // compute warps; the last warp of the CTA is the loader
-        constexpr int WROWS     = ST + HALO;
-        constexpr int PSTRIDE   = WROWS * 16;             // bytes between planes of a window
-        constexpr int WIN_BYTES = ALLP * PSTRIDE;
-        constexpr int SCR_BYTES = ALLP * TILE * 16;       // per warp: rows of one tile that were not staged
-        constexpr int NFRAG     = NSLOTS * KSTEPS * NBLK; // B fragments per part
+    // One CTA walks super-tiles; while it computes on one window the next is on its way. Every warp owns groups of TILES 8-row
+    // tiles of the super-tile: for each slot four threads read a neighbour row, 16 bytes each, and hold with it their part of the
+    // operand; three MMAs per 16 output channels add hi.hi, lo.hi and hi.lo into fp32 accumulators in registers (dropping only lo.lo
+    // keeps ~2^-21 relative accuracy; with 8 output channels two MMAs do all four), and the epilogue (activation, store as fp32
+    // chunks or split again for the next such layer) runs on the accumulator registers. The weights sit in shared memory as
+    // ready-made fragments (16 bytes per lane, read once per slot for all tiles of the group), or in registers. The last warp
+    // of the CTA is the loader; a compute warp waits only for a window to land and tells the loader when it is done with one,
+    // so no compute warp ever waits for another.
+    template <int COUT, int NSLOTS, int TILES, int THREADS, int CTAS>
+    __global__ void __launch_bounds__(THREADS, CTAS) k_graph_conv_mma(const ConvArgs a, const Args t, const Plan plan) {
+        static_assert((COUT == 8 || COUT == 16 || COUT == 32) && ST % (TILES * TILE) == 0, "whole fragments, whole groups of tiles");
+        constexpr int MBLK  = COUT == 32 ? 2 : 1;  // blocks of 16 rows of the weights' operand
+        constexpr int FRAGS = weight_fragments<COUT>();
+        constexpr int WARPS = THREADS / 32 - 1;    // compute warps; the last warp of the CTA is the loader
 
         extern __shared__ __align__(1024) unsigned char smem_raw[];
         __shared__ uint64_t bars[4];                      // full[2]: a window has landed; empty[2]: every compute warp is done with it
         __shared__ int32_t tile_prefix[MAX_FRAMES + 1];   // in super-tiles
         __shared__ int32_t frame_start[MAX_FRAMES + 1];   // offsets[f0 + f]
+        __shared__ int32_t window_miss[2];                // some neighbour of the super-tile was left out of its window
         __shared__ int32_t failed_s;
         volatile int32_t* failed = &failed_s;
 
         const int tid  = threadIdx.x;
         const int warp = tid >> 5;
         const int lane = tid & 31;
-        const int g    = lane >> 2;  // row of the accumulator fragment (and g + 8)
-        const int tq   = lane & 3;   // column pair of the accumulator fragment
+        const int g    = lane >> 2;  // row of a tile that the thread reads; output channels of the accumulator fragment
+        const int tq   = lane & 3;   // its piece of that row; rows 2 tq and 2 tq + 1 of the accumulator fragment
         const uint32_t win_addr = tc::smem_u32(smem_raw);
-        const uint32_t scr_addr = win_addr + 2 * WIN_BYTES + warp * SCR_BYTES;
-        unsigned char* scr_ptr  = smem_raw + 2 * WIN_BYTES + warp * SCR_BYTES;
-        const uint32_t frag_addr = win_addr + 2 * WIN_BYTES + WARPS * SCR_BYTES + lane * 8;  // this lane's 8 bytes of fragment 0, hi part
+        const uint32_t nbl_addr  = win_addr + 2 * WINDOW;
+        const uint32_t frag_addr = nbl_addr + 2 * NBL_BYTES + lane * 16;  // this lane's 16 bytes of fragment 0
         const uint32_t bar_full  = tc::smem_u32(&bars[0]);
         const uint32_t bar_empty = tc::smem_u32(&bars[2]);
 
@@ -170,32 +187,36 @@ namespace st {
         __syncthreads();
         tc::tiles_before<ST>(tile_prefix, frame_start, t.n_frames);
 
-        // ---- B fragments: weights [k][n] split into fp16 hi and lo, in the register layout of mma.m16n8k16 ----
-        // fragment of (slot s, K step ks, column block nb), lane (g, tq): b0 = {W[k0 + 2 tq][n], W[k0 + 2 tq + 1][n]} and b1 =
-        // the same 8 rows further, with k0 = s * CIN + ks * 16 and n = nb * 8 + g
+        // ---- the weights' fragments: split into fp16 hi and lo parts, in the register layout of mma.m16n8k16's A ----
+        // The contraction's K axis may come in any order that both operands share: thread (g, tq) holds input channels 4 tq .. 4 tq + 3 of
+        // a row (its 16-byte piece) as k = 2 tq, 2 tq + 1, 2 tq + 8, 2 tq + 9. Which output channel a row of the operand stands for is free
+        // too; a thread gets rows g and g + 8 of each block, and those are neighbouring channels. Eight channels are one block: their
+        // hi parts are its rows 0 to 7, their lo parts rows 8 to 15.
+        auto channel = [&](int block, int half) { return COUT == 8 ? g : COUT == 16 ? 4 * (g >> 1) + 2 * half + (g & 1) : 4 * g + 2 * block + half; };
         {
             constexpr int COUTP = (COUT + 3) & ~3;
-            uint2* w_frag       = reinterpret_cast<uint2*>(smem_raw + 2 * WIN_BYTES + WARPS * SCR_BYTES);  // [part][fragment][lane]
-            for (int frag = warp; frag < NFRAG; frag += WARPS + 1) {
-                const int nb = frag % NBLK, ks = (frag / NBLK) % KSTEPS, sl = frag / (NBLK * KSTEPS);
-                const int n  = nb * 8 + g;
-                const int k0 = sl * CIN + ks * 16 + 2 * tq;
-                uint32_t h[2], l[2];
+            uint4* w_frag       = reinterpret_cast<uint4*>(smem_raw + 2 * WINDOW + 2 * NBL_BYTES);  // [slot][block][part][lane]
+            for (int i = warp; i < NSLOTS * MBLK; i += WARPS + 1) {
+                const int block = i % MBLK, slot = i / MBLK;
+                const float* w  = a.weights + static_cast<size_t>(slot * CIN + 4 * tq) * COUTP;
+                uint32_t h[4], l[4];  // register 2 k + half: channels 4 tq + 2 k, + 1 of the block's row g + 8 half
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const float w0 = __ldg(a.weights + static_cast<size_t>(k0 + 8 * half) * COUTP + n);
-                    const float w1 = __ldg(a.weights + static_cast<size_t>(k0 + 8 * half + 1) * COUTP + n);
-                    split_pair(w0, w1, h[half], l[half]);
+                for (int r = 0; r < 4; ++r) {
+                    const float* from = w + (r & 2) * COUTP + channel(block, r & 1);
+                    split_pair(__ldg(from), __ldg(from + COUTP), h[r], l[r]);
                 }
-                w_frag[frag * 32 + lane]           = make_uint2(h[0], h[1]);
-                w_frag[(NFRAG + frag) * 32 + lane] = make_uint2(l[0], l[1]);
+                if (COUT == 8) { w_frag[slot * 32 + lane] = make_uint4(h[0], l[0], h[2], l[2]); }
+                else {
+                    w_frag[(2 * i) * 32 + lane]     = make_uint4(h[0], h[1], h[2], h[3]);
+                    w_frag[(2 * i + 1) * 32 + lane] = make_uint4(l[0], l[1], l[2], l[3]);
+                }
             }
         }
-        float bias[NBLK][2];
+        float bias[MBLK][2];
 #pragma unroll
-        for (int nb = 0; nb < NBLK; ++nb) {
-            bias[nb][0] = __ldg(a.biases + nb * 8 + 2 * tq);
-            bias[nb][1] = __ldg(a.biases + nb * 8 + 2 * tq + 1);
+        for (int m = 0; m < MBLK; ++m) {
+            bias[m][0] = __ldg(a.biases + channel(m, 0));
+            bias[m][1] = COUT == 8 ? 0.0f : __ldg(a.biases + channel(m, 1));
         }
         __syncthreads();
         const int total_st = tile_prefix[t.n_frames];
@@ -220,8 +241,6 @@ namespace st {
             return r;
         };
         const unsigned char* in_bytes = reinterpret_cast<const unsigned char*>(a.in);
-        const uint4* in4              = reinterpret_cast<const uint4*>(a.in);
-        const uint4* nbl4             = reinterpret_cast<const uint4*>(plan.nbl);
 
         if (warp == WARPS) {
             // ================= loader warp: one window ahead of the compute warps per buffer =================
@@ -229,10 +248,11 @@ namespace st {
             // the loader waits for a buffer anyway: the copies of a window then start the moment its buffer is free
             // instead of two dependent trips to global memory later.
             constexpr int PER_LANE = (HALO + 31) / 32;
-            int n_halo = 0;
+            int n_halo = 0, listed = 0;
             int32_t halo_row[PER_LANE];
             auto fetch_halo_list = [&](int st) {
-                n_halo                = min(__ldg(plan.halo_count + st), HALO);
+                listed                = __ldg(plan.halo_count + st);
+                n_halo                = min(listed, HALO);
                 const int32_t* h_rows = plan.halo_rows + static_cast<size_t>(st) * HALO;
 #pragma unroll
                 for (int k = 0; k < PER_LANE; ++k) halo_row[k] = __ldg(h_rows + min(lane + 32 * k, HALO - 1));  // entries past n_halo are never used
@@ -249,24 +269,23 @@ namespace st {
                 }
                 const StRef r      = locate(s);
                 const int own      = min(ST, r.rows - r.t0);
-                const uint32_t dst = win_addr + b * WIN_BYTES;
+                const uint32_t dst = win_addr + b * WINDOW;
                 const uint32_t bar = bar_full + 8 * b;
                 if (lane == 0) {
-                    mbar_expect_tx(bar, static_cast<uint32_t>(ALLP * own * 16));
-#pragma unroll
-                    for (int p = 0; p < ALLP; ++p) {
-                        bulk_copy(dst + p * PSTRIDE, in_bytes + (static_cast<size_t>(p) * a.in_stride + r.local_base + r.t0) * 16,
-                                  static_cast<uint32_t>(own * 16), bar);
-                    }
+                    window_miss[b] = listed > HALO;
+                    mbar_expect_tx(bar, static_cast<uint32_t>(own * (ROW + 2 * NBL_STRIDE)));
+                    bulk_copy(nbl_addr + b * NBL_BYTES, reinterpret_cast<const uint4*>(plan.nbl) + r.local_base + r.t0, static_cast<uint32_t>(own * 2 * NBL_STRIDE),
+                              bar);
+                    bulk_copy(dst, in_bytes + static_cast<size_t>(r.local_base + r.t0) * ROW, static_cast<uint32_t>(own * ROW), bar);
                 }
+                // four lanes to a halo row: whole rows per request
+                const unsigned char* from = in_bytes + (lane & 3) * 16;
+                const uint32_t to         = dst + ST * ROW + lane * 16;
 #pragma unroll
-                for (int k = 0; k < PER_LANE; ++k) {
-                    const int h = lane + 32 * k;
-                    if (h < n_halo) {
-                        const size_t src_row = static_cast<size_t>(halo_row[k]);
-#pragma unroll
-                        for (int p = 0; p < ALLP; ++p) copy16(dst + p * PSTRIDE + (ST + h) * 16, in_bytes + (static_cast<size_t>(p) * a.in_stride + src_row) * 16);
-                    }
+                for (int k = 0; k < HALO / 8; ++k) {
+                    if (8 * k >= n_halo) break;
+                    const int32_t row = __shfl_sync(0xffffffffu, halo_row[k / 4], 8 * (k % 4) + (lane >> 2));
+                    if (8 * k + (lane >> 2) < n_halo) copy16(to + k * 8 * ROW, from + static_cast<size_t>(row) * ROW);
                 }
                 if (s + static_cast<int>(gridDim.x) < total_st) fetch_halo_list(s + gridDim.x);
                 copies_arrive(bar);
@@ -283,182 +302,212 @@ namespace st {
         }
         else {
         // ================= compute warps =================
+        constexpr bool HELD = COUT == 8;  // weights in registers
+        uint4 held[HELD ? NSLOTS : 1];
+        if (HELD) {
+#pragma unroll
+            for (int i = 0; i < NSLOTS; ++i) held[i] = load_shared(frag_addr + i * 512);
+        }
         uint32_t n = 0;
         bool ok    = true;
         for (int s = blockIdx.x; s < total_st; s += gridDim.x, ++n) {
             const uint32_t b  = n & 1u;
             const StRef r     = locate(s);
             const int own     = min(ST, r.rows - r.t0);
-            const int n_pairs = (own + PAIR * TILE - 1) / (PAIR * TILE);
-            // neighbour positions of this warp's first pair of tiles, fetched while the window is on its way
-            // (lanes 0-15 and 16-31 address the same sixteen rows; tile i of the pair is rows 16 i .. 16 i + 15)
-            int arow[PAIR];
-            uint4 pos[PAIR];
-            auto fetch_positions = [&](int pair, int (&rows_out)[PAIR], uint4 (&pos_out)[PAIR]) {
-#pragma unroll
-                for (int i = 0; i < PAIR; ++i) {
-                    rows_out[i] = min((pair * PAIR + i) * TILE + (lane & 15), own - 1);
-                    pos_out[i]  = __ldg(nbl4 + r.local_base + r.t0 + rows_out[i]);
-                }
-            };
-            if (warp < n_pairs) fetch_positions(warp, arow, pos);
+            const int n_groups = (own + TILES * TILE - 1) / (TILES * TILE);
             ok = __all_sync(0xffffffffu, tc::mbar_wait_or_fail(bar_full + 8 * b, (n >> 1) & 1u, failed, t.wait_limit));
             if (!ok) {
                 *failed = 1;
                 break;
             }
-            const uint32_t win = win_addr + b * WIN_BYTES;
-            for (int pair = warp; pair < n_pairs; pair += WARPS) {
-                int cur_row[PAIR];
-                uint4 cur_pos[PAIR];
+            const uint32_t win = win_addr + b * WINDOW + tq * 16;
+            const uint32_t nbl = nbl_addr + b * NBL_BYTES;
+            const bool miss    = *static_cast<volatile int32_t*>(&window_miss[b]) != 0;
+            for (int group = warp; group < n_groups; group += WARPS) {
+                float acc[TILES][MBLK][4];
 #pragma unroll
-                for (int i = 0; i < PAIR; ++i) {
-                    cur_row[i] = arow[i];
-                    cur_pos[i] = pos[i];
-                }
-                if (pair + WARPS < n_pairs) fetch_positions(pair + WARPS, arow, pos);  // for the next round, in flight during this one
-                float acc[PAIR][NBLK][4];
+                for (int i = 0; i < TILES; ++i) {
 #pragma unroll
-                for (int i = 0; i < PAIR; ++i) {
+                    for (int m = 0; m < MBLK; ++m) {
 #pragma unroll
-                    for (int nb = 0; nb < NBLK; ++nb) {
-                        acc[i][nb][0] = bias[nb][0];
-                        acc[i][nb][1] = bias[nb][1];
-                        acc[i][nb][2] = bias[nb][0];
-                        acc[i][nb][3] = bias[nb][1];
+                        for (int k = 0; k < 4; ++k) acc[i][m][k] = bias[m][k >> 1];
                     }
                 }
+                // the products of a slot for all tiles, x[i]: this thread's piece of tile i, {hi, hi, lo, lo} of four channels; no
+                // accumulator twice in a row
+                auto products = [&](const uint4 (&x)[TILES], int slot, auto rolled) {
+                    constexpr bool ROLLED = decltype(rolled)::value;  // the slot is not known at compile time
 #pragma unroll
-                for (int sl = 0; sl < NSLOTS; ++sl) {
-                    uint32_t base[PAIR], pstride[PAIR];
-                    bool miss[PAIR];
-                    bool any_miss = false;
+                    for (int m = 0; m < MBLK; ++m) {
+                        const uint4 wh = HELD && !ROLLED ? held[slot] : load_shared(frag_addr + (slot * FRAGS + (COUT == 8 ? 0 : 2 * m)) * 512);
 #pragma unroll
-                    for (int i = 0; i < PAIR; ++i) {
-                        uint32_t p;
-                        if (sl == 0) { p = static_cast<uint32_t>(cur_row[i]); }
-                        else {
-                            const uint4& q      = cur_pos[i];
-                            const uint32_t word = ((sl - 1) >> 1) == 0 ? q.x : ((sl - 1) >> 1) == 1 ? q.y : ((sl - 1) >> 1) == 2 ? q.z : q.w;
-                            p                   = ((sl - 1) & 1) ? (word >> 16) : (word & 0xFFFFu);
+                        for (int i = 0; i < TILES; ++i) mma_16816(acc[i][m], wh, x[i].x, x[i].y);
+                        if constexpr (COUT != 8) {
+                            const uint4 wl = load_shared(frag_addr + (slot * FRAGS + 2 * m + 1) * 512);
+#pragma unroll
+                            for (int i = 0; i < TILES; ++i) mma_16816(acc[i][m], wl, x[i].x, x[i].y);
                         }
-                        // address of this lane's row in plane 0 of the window, and the distance between planes
-                        base[i]    = win + p * 16;
-                        pstride[i] = PSTRIDE;
-                        miss[i]    = sl > 0 && p == NBL_GLOBAL;
-                        any_miss |= miss[i];
+#pragma unroll
+                        for (int i = 0; i < TILES; ++i) mma_16816(acc[i][m], wh, x[i].z, x[i].w);
                     }
-                    // the slot's products for tiles [I0, I1) of the pair: one B fragment load serves all of them
-                    auto products = [&](auto i0, auto i1) {
-                        constexpr int I0 = decltype(i0)::value, I1 = decltype(i1)::value;
+                };
+                // rows past the super-tile's last are copies of it
+                auto window_row = [&](int i) { return static_cast<uint32_t>(min((group * TILES + i) * TILE + g, own - 1)); };
+                if (!miss) {
+                    uint32_t row[TILES];
+                    uint4 pos[TILES];
 #pragma unroll
-                        for (int ks = 0; ks < KSTEPS; ++ks) {
-                            uint32_t a_hi[PAIR][4], a_lo[PAIR][4];
+                    for (int i = 0; i < TILES; ++i) {
+                        row[i] = window_row(i);
+                        pos[i] = load_shared(nbl + row[i] * (2 * NBL_STRIDE));
+                    }
 #pragma unroll
-                            for (int i = I0; i < I1; ++i) {
-                                // lanes 16-31 address the second 16-byte chunk of the K step
-                                const uint32_t at = base[i] + (2 * ks + (lane >> 4)) * pstride[i];
-                                ldmatrix_x4(a_hi[i], at);
-                                ldmatrix_x4(a_lo[i], at + PLANES * pstride[i]);
+                    for (int slot = 0; slot < NSLOTS; ++slot) {
+                        uint4 x[TILES];
+#pragma unroll
+                        for (int i = 0; i < TILES; ++i) {
+                            uint32_t p = row[i];
+                            if (slot > 0) {
+                                const int k         = slot - 1;
+                                const uint32_t word = (k >> 1) == 0 ? pos[i].x : (k >> 1) == 1 ? pos[i].y : (k >> 1) == 2 ? pos[i].z : pos[i].w;
+                                p                   = (k & 1) ? (word >> 16) : (word & 0xFFFFu);
                             }
+                            x[i] = load_shared(win + p * ROW);
+                        }
+                        products(x, slot, std::false_type{});
+                    }
+                }
+                else {
+                    // some neighbour of the super-tile was not staged (more outside rows than halo slots): it comes from global memory
+#pragma unroll 1
+                    for (int slot = 0; slot < NSLOTS; ++slot) {
+                        uint4 x[TILES];
 #pragma unroll
-                            for (int nb = 0; nb < NBLK; ++nb) {
-                                const int frag = (sl * KSTEPS + ks) * NBLK + nb;
-                                uint32_t h0, h1, l0, l1;
-                                asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(h0), "=r"(h1) : "r"(frag_addr + frag * 256));
-                                asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(l0), "=r"(l1) : "r"(frag_addr + (NFRAG + frag) * 256));
-#pragma unroll
-                                for (int i = I0; i < I1; ++i) {
-                                    mma_16816(acc[i][nb], a_hi[i], h0, h1);
-                                    mma_16816(acc[i][nb], a_hi[i], l0, l1);
-                                    mma_16816(acc[i][nb], a_lo[i], h0, h1);
-                                }
+                        for (int i = 0; i < TILES; ++i) {
+                            const uint32_t row = window_row(i);
+                            uint32_t p         = row;
+                            if (slot > 0) asm volatile("ld.shared.u16 %0, [%1];" : "=r"(p) : "r"(nbl + row * (2 * NBL_STRIDE) + 2 * (slot - 1)));
+                            if (slot > 0 && p == NBL_GLOBAL) {
+                                const int idx = __ldg(a.nb + (r.nb_base + r.t0 + row) * a.n_neighbours + (slot - 1));
+                                x[i]          = __ldg(reinterpret_cast<const uint4*>(in_bytes + static_cast<size_t>(r.local_base + idx) * ROW + tq * 16));
+                            }
+                            else {
+                                x[i] = load_shared(win + p * ROW);
                             }
                         }
-                    };
-                    if (!__any_sync(0xffffffffu, any_miss)) { products(std::integral_constant<int, 0>{}, std::integral_constant<int, PAIR>{}); }
+                        __syncwarp();
+                        products(x, slot, std::true_type{});
+                    }
+                }
+                if constexpr (COUT == 8) {  // what the hi and the lo parts of the weights gave
+#pragma unroll
+                    for (int i = 0; i < TILES; ++i) {
+                        acc[i][0][0] += acc[i][0][2];
+                        acc[i][0][1] += acc[i][0][3];
+                    }
+                }
+                // ---- epilogue on the accumulator fragments: rows 2 tq and 2 tq + 1 of each tile, COUT / 8 neighbouring channels ----
+                auto apply = [&](auto f) {
+#pragma unroll
+                    for (int i = 0; i < TILES; ++i) {
+#pragma unroll
+                        for (int m = 0; m < MBLK; ++m) {
+#pragma unroll
+                            for (int k = 0; k < (COUT == 8 ? 2 : 4); ++k) acc[i][m][k] = f(acc[i][m][k]);
+                        }
+                    }
+                };
+                if (a.activation == VM_SELU) apply([](float x) { return selu(x); });
+                else if (a.activation == VM_RELU) apply([](float x) { return x < 0.0f ? 0.0f : x; });
+                else if (a.activation == VM_TANH) apply([](float x) { return tanhf(x); });
+                // fp32 is stored by threads g and g ^ 1 together, which hold channels of the same four (8 channels: two) of the same two
+                // rows: each takes one of the rows and the other's part of it. With 32 channels a thread's own part is wide enough. Split
+                // rows of 16 channels are transposed, so that four threads write the 64 bytes of row g.
+                const bool odd       = (g & 1) != 0;
+                const bool quads     = COUT == 16 && a.out_split != SPLIT_NONE;
+                const int row0       = r.t0 + group * TILES * TILE + (quads ? g : 2 * tq + (COUT != 32 && odd ? 1 : 0));  // within the frame
+                const int left       = r.rows - row0;  // row row0 + k exists: k < left
+                const size_t out_row = static_cast<size_t>(r.local_base) + row0;
+                unsigned char* out_b = reinterpret_cast<unsigned char*>(a.out);
+                auto swap            = [&](uint32_t first, uint32_t second) { return __shfl_xor_sync(0xffffffffu, odd ? first : second, 4); };
+                auto swap_f          = [&](float first, float second) { return __uint_as_float(swap(__float_as_uint(first), __float_as_uint(second))); };
+                if constexpr (COUT == 8) {
+                    // chunk-planar fp32 (no consumer takes 8 channels split)
+                    unsigned char* to = out_b + (static_cast<size_t>(g >> 2) * a.out_stride + out_row) * 16 + (g >> 1 & 1) * 8;
+#pragma unroll
+                    for (int i = 0; i < TILES; ++i) {
+                        const float other = swap_f(acc[i][0][0], acc[i][0][1]);
+                        if (TILE * i < left) *reinterpret_cast<float2*>(to + TILE * i * 16) = odd ? make_float2(other, acc[i][0][1]) : make_float2(acc[i][0][0], other);
+                    }
+                }
+                else if (a.out_split) {
+                    __half2 largest = __float2half2_rn(0.0f);
+                    if constexpr (COUT == 16) {
+                        unsigned char* to  = out_b + out_row * ROW + tq * 16;
+                        const size_t plane = static_cast<size_t>(a.out_stride) * 16;
+                        if (a.out_split == SPLIT_PLANES) to = out_b + (tq >> 1) * plane + out_row * 16 + (tq & 1) * 8;
+#pragma unroll
+                        for (int i = 0; i < TILES; ++i) {
+                            uint32_t h[2], l[2];
+#pragma unroll
+                            for (int k = 0; k < 2; ++k) {
+                                split_pair(acc[i][0][2 * k], acc[i][0][2 * k + 1], h[k], l[k]);
+                                largest = __hmax2(largest, __habs2(*reinterpret_cast<const __half2*>(&h[k])));
+                            }
+                            const uint4 piece = make_uint4(transpose(h[0]), transpose(h[1]), transpose(l[0]), transpose(l[1]));
+                            if (TILE * i >= left) continue;
+                            if (a.out_split == SPLIT_QUADS) { *reinterpret_cast<uint4*>(to + TILE * i * ROW) = piece; }
+                            else {
+                                *reinterpret_cast<uint2*>(to + TILE * i * 16)             = make_uint2(piece.x, piece.y);
+                                *reinterpret_cast<uint2*>(to + 2 * plane + TILE * i * 16) = make_uint2(piece.z, piece.w);
+                            }
+                        }
+                    }
                     else {
-                        // Some neighbour of this slot was not staged (more outside rows than halo slots): one tile at a time,
-                        // its missing rows are fetched from global memory into the warp's scratch rows and addressed there.
-                        auto one_tile = [&](auto which) {
-                            constexpr int I = decltype(which)::value;
-                            __syncwarp();
-                            if (miss[I] && lane < 16) {
-                                const int idx        = __ldg(a.nb + (r.nb_base + r.t0 + cur_row[I]) * a.n_neighbours + (sl - 1));
-                                const size_t src_row = static_cast<size_t>(r.local_base + idx);
+                        // 32 channels, the thread's 4 g .. 4 g + 3: eight bytes of the hi parts and of the lo parts of either row
+                        const bool rowed   = a.out_split == SPLIT_ROWS;
+                        const size_t plane = static_cast<size_t>(a.out_stride) * 16;
+                        const int pitch    = rowed ? 128 : 16;
+                        unsigned char* to  = rowed ? out_b + out_row * 128 + g * 8 : out_b + (g >> 1) * plane + out_row * 16 + (g & 1) * 8;
+                        const size_t lo_at = rowed ? 64 : 4 * plane;
 #pragma unroll
-                                for (int pl = 0; pl < ALLP; ++pl) {
-                                    *reinterpret_cast<uint4*>(scr_ptr + (pl * TILE + lane) * 16) = __ldg(in4 + static_cast<size_t>(pl) * a.in_stride + src_row);
+                        for (int i = 0; i < TILES; ++i) {
+#pragma unroll
+                            for (int k = 0; k < 2; ++k) {
+                                uint32_t h[2], l[2];
+#pragma unroll
+                                for (int m = 0; m < MBLK; ++m) {
+                                    split_pair(acc[i][m][k], acc[i][m][2 + k], h[m], l[m]);
+                                    largest = __hmax2(largest, __habs2(*reinterpret_cast<const __half2*>(&h[m])));
                                 }
-                            }
-                            __syncwarp();
-                            if (miss[I]) {
-                                base[I]    = scr_addr + (lane & 15) * 16;
-                                pstride[I] = TILE * 16;
-                            }
-                            products(std::integral_constant<int, I>{}, std::integral_constant<int, I + 1>{});
-                        };
-                        one_tile(std::integral_constant<int, 0>{});
-                        one_tile(std::integral_constant<int, 1>{});
-                        static_assert(PAIR == 2, "the fallback above is written out for two tiles");
-                    }
-                }
-                // ---- epilogue on the accumulator fragments: rows g and g + 8 of each tile, columns nb * 8 + 2 tq, + 1 ----
-                bool bad = false;
-#pragma unroll
-                for (int i = 0; i < PAIR; ++i) {
-#pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        const int row = r.t0 + (pair * PAIR + i) * TILE + g + 8 * half;  // within the frame
-                        float v[NBLK][2];
-#pragma unroll
-                        for (int nb = 0; nb < NBLK; ++nb) {
-                            v[nb][0] = acc[i][nb][2 * half];
-                            v[nb][1] = acc[i][nb][2 * half + 1];
-                            if (a.activation == VM_SELU) {
-                                v[nb][0] = selu(v[nb][0]);
-                                v[nb][1] = selu(v[nb][1]);
-                            }
-                            else if (a.activation == VM_RELU) {
-                                v[nb][0] = v[nb][0] < 0.0f ? 0.0f : v[nb][0];
-                                v[nb][1] = v[nb][1] < 0.0f ? 0.0f : v[nb][1];
-                            }
-                            else if (a.activation == VM_TANH) {
-                                v[nb][0] = tanhf(v[nb][0]);
-                                v[nb][1] = tanhf(v[nb][1]);
+                                if (TILE * i + k >= left) continue;
+                                *reinterpret_cast<uint2*>(to + (TILE * i + k) * pitch)         = make_uint2(h[0], h[MBLK - 1]);
+                                *reinterpret_cast<uint2*>(to + lo_at + (TILE * i + k) * pitch) = make_uint2(l[0], l[MBLK - 1]);
                             }
                         }
-                        if (row >= r.rows) continue;
-                        const size_t out_row = static_cast<size_t>(r.local_base) + row;
-                        unsigned char* out_b = reinterpret_cast<unsigned char*>(a.out);
-                        if (a.out_split) {
-                            // column block nb is 16-byte chunk nb of the row's hi part (and of its lo part): this thread's two
-                            // values are 4 bytes of it, the four threads of a row write the chunk, eight rows 128 contiguous bytes
+                    }
+                    if (__hgt(__hmax(__low2half(largest), __high2half(largest)), __float2half_rn(60000.0f))) raise_flag(a.range_flag, ABORT_TC_RANGE);
+                }
+                else {
+                    // chunk-planar fp32
+                    unsigned char* to = out_b + (static_cast<size_t>(COUT == 16 ? g >> 1 : g) * a.out_stride + out_row) * 16;
 #pragma unroll
-                            for (int nb = 0; nb < NBLK; ++nb) {
-                                uint32_t h, l;
-                                split_pair(v[nb][0], v[nb][1], h, l);
-                                bad |= fabsf(v[nb][0]) > 60000.0f || fabsf(v[nb][1]) > 60000.0f;
-                                if (COUT == 32 && a.out_split == SPLIT_ROWS) {
-                                    *reinterpret_cast<uint32_t*>(out_b + out_row * 128 + nb * 16 + tq * 4)      = h;
-                                    *reinterpret_cast<uint32_t*>(out_b + out_row * 128 + 64 + nb * 16 + tq * 4) = l;
-                                    continue;
-                                }
-                                *reinterpret_cast<uint32_t*>(out_b + (static_cast<size_t>(nb) * a.out_stride + out_row) * 16 + tq * 4)        = h;
-                                *reinterpret_cast<uint32_t*>(out_b + (static_cast<size_t>(NBLK + nb) * a.out_stride + out_row) * 16 + tq * 4) = l;
-                            }
+                    for (int i = 0; i < TILES; ++i) {
+                        if constexpr (COUT == 16) {
+                            const float o0 = swap_f(acc[i][0][0], acc[i][0][1]), o1 = swap_f(acc[i][0][2], acc[i][0][3]);
+                            const float4 v = odd ? make_float4(o0, acc[i][0][1], o1, acc[i][0][3]) : make_float4(acc[i][0][0], o0, acc[i][0][2], o1);
+                            if (TILE * i < left) *reinterpret_cast<float4*>(to + TILE * i * 16) = v;
                         }
                         else {
-                            // chunk-planar fp32: this thread's two values are half of 16-byte chunk 2 nb + tq / 2
 #pragma unroll
-                            for (int nb = 0; nb < NBLK; ++nb) {
-                                *reinterpret_cast<float2*>(out_b + (static_cast<size_t>(2 * nb + (tq >> 1)) * a.out_stride + out_row) * 16 + (tq & 1) * 8) =
-                                  make_float2(v[nb][0], v[nb][1]);
+                            for (int k = 0; k < 2; ++k) {
+                                if (TILE * i + k >= left) continue;
+                                *reinterpret_cast<float4*>(to + (TILE * i + k) * 16) =
+                                  make_float4(acc[i][0][k], acc[i][0][2 + k], acc[i][MBLK - 1][k], acc[i][MBLK - 1][2 + k]);
                             }
                         }
                     }
                 }
-                if (bad) raise_flag(a.range_flag, ABORT_TC_RANGE);
             }
             // this warp is done with the window: the loader may refill it once every compute warp has said so
             __syncwarp();

@@ -441,7 +441,8 @@ namespace tc {
                     else {
                         activate<NP>(v, a.activation);  // one branch on the activation, then NP independent chains
                     }
-                    if (a.out_split && t.cout == NP) { store_split<NP>(a.out, a.out_stride, out_row, v, a.range_flag); }
+                    if (NP == 16 && a.out_split == SPLIT_QUADS && t.cout == NP) { store_split_quads(a.out, out_row, v, a.range_flag); }
+                    else if (a.out_split && t.cout == NP) { store_split<NP>(a.out, a.out_stride, out_row, v, a.range_flag); }
                     else if (a.out_planar) {
                         float4* out4 = reinterpret_cast<float4*>(a.out);
 #pragma unroll
@@ -779,7 +780,8 @@ namespace tc {
                     else {
                         activate<NP>(v, a.activation);  // one branch on the activation, then NP independent chains
                     }
-                    if (a.out_split && t.cout == NP) { store_split<NP>(a.out, a.out_stride, out_row, v, a.range_flag); }
+                    if (NP == 16 && a.out_split == SPLIT_QUADS && t.cout == NP) { store_split_quads(a.out, out_row, v, a.range_flag); }
+                    else if (a.out_split && t.cout == NP) { store_split<NP>(a.out, a.out_stride, out_row, v, a.range_flag); }
                     else if (a.out_planar) {
                         float4* out4 = reinterpret_cast<float4*>(a.out);
 #pragma unroll

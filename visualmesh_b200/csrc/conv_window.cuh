@@ -610,6 +610,16 @@ namespace win {
                                 dst += 32 * t.cout;
                             }
                         }
+                        else if (a.out_split == SPLIT_QUADS) {
+                            // 16 channels; pieces of four hi and four lo parts
+                            if (OWN == 4) {
+                                uint4* dst = reinterpret_cast<uint4*>(a.out) + (static_cast<size_t>(r.local_base) + first_row) * 4 + piece;
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    if (8 * j < rows) dst[32 * j] = make_uint4(hi[j][0], hi[j][1], lo[j][0], lo[j][1]);
+                                }
+                            }
+                        }
                         else {
                             // planes of 16-byte chunks of 8 channels, the hi planes first
                             const int n        = piece * OWN < t.cout ? rows : 0;

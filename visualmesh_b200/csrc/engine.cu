@@ -423,7 +423,7 @@ static void run_network(vm_engine* e,
         a.in_stride    = feature_stride;
         a.out_stride   = feature_stride;
         a.out_planar   = (!last && e->layers[l].cout % 4 == 0) ? 1 : 0;
-        a.out_split    = last ? SPLIT_NONE : kind[l + 1] == CONV_TC_WINDOW ? SPLIT_ROWS : kind[l + 1] >= CONV_TC_SPLIT ? SPLIT_PLANES : SPLIT_NONE;
+        a.out_split    = last ? SPLIT_NONE : kind[l + 1] == CONV_TC_WINDOW ? SPLIT_ROWS : kind[l + 1] == CONV_TC_STAGED ? SPLIT_QUADS : kind[l + 1] >= CONV_TC_SPLIT ? SPLIT_PLANES : SPLIT_NONE;
         a.out_host     = last ? out_host : nullptr;
         a.range_flag   = e->flags;
         launch_conv(e, e->layers[l], a, n_frames, max_rows, lane.stream, kind[l], plan);
