@@ -107,6 +107,21 @@ def test_layers_of_16_channels_with_neighbours_anywhere(n, n_neighbours, widths)
     _check(W.make_network(61, n_neighbours, widths), n, n_neighbours)
 
 
+# super-tiles with 200, 340 and 460 outside rows: more than the staged kernel keeps, than the window kernel's loaders read ahead, than
+# the plan has slots for; 64-row tiles and their edges
+@pytest.mark.parametrize("reach", [100, 170, 230])
+@pytest.mark.parametrize("n", [63, 65, 20_001])
+@pytest.mark.parametrize("n_neighbours,widths", [(4, [32, 32, 16, 16, 3]), (6, [16, 16, 32, 32, 8, 3]), (8, [32, 32, 32, 4])])
+def test_layers_with_large_halos(n, reach, n_neighbours, widths):
+    net = W.make_network(67, n_neighbours, widths)
+    x, _ = _rows(n, n_neighbours, 11)
+    nb = _near(n, n_neighbours, reach)
+    engine = Engine(net)
+    got = engine.network(x, nb)
+    engine.close()
+    assert np.abs(got.astype(np.float64) - O.network(x, nb, net).astype(np.float64)).max() <= P.TOL_CLS / 4
+
+
 def test_selu_over_its_range():
     """A layer that passes its input through: SELU of floats of every size, against double.
 

@@ -32,8 +32,8 @@ struct ConvArgs {
     int32_t* range_flag;    // the engine's abort flags: ABORT_RANGE is raised when a value is too large for the fp16 split
 };
 
-// ConvArgs::out_split. Planes of 16-byte chunks; whole rows for the window kernel (its 32 input channels: COUT == 32), 32 hi parts, then
-// 32 lo parts; whole rows for the staged kernel (its 16 input channels: COUT == 16), pieces of four hi and four lo parts.
+// ConvArgs::out_split. Planes of 16-byte chunks; whole rows for the window kernel (its 32 input channels: COUT == 32), pieces of
+// two hi, two lo, two hi and two lo parts, odd rows with their second half first; whole rows for the staged kernel (its 16 input channels: COUT == 16), pieces of four hi and four lo parts.
 enum SplitLayout { SPLIT_NONE = 0, SPLIT_PLANES = 1, SPLIT_ROWS = 2, SPLIT_QUADS = 3 };
 
 constexpr int CONV_THREADS = 128;

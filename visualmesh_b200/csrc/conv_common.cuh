@@ -94,27 +94,28 @@ __device__ __forceinline__ void store_split(float* out, int stride, size_t row, 
     if (bad) raise_flag(range_flag, ABORT_TC_RANGE);
 }
 
-// The same values row after row (32 hi parts, then 32 lo parts) for the window kernel. Stores the rows of a warp, one per thread and one
-// after another; all threads call (valid: the row exists; those that do come first). stage: shared memory of the warp, 4 KB. A thread
-// that stored its own row would write 16-byte pieces 128 bytes apart, half a sector and one line per thread and store; from shared
+// The same values row after row for the window kernel (SPLIT_ROWS): eight 16-byte pieces a row, each the hi and lo parts of two channels,
+// then of the next two; odd rows begin with their second half, so that two rows of different parity never meet in a bank of shared
+// memory. Stores the rows of a warp, one per thread and one after another; all threads call (valid: the row exists; those that do come
+// first). stage: shared memory of the warp, 4 KB. A thread that stored its own row would write 16-byte pieces 128 bytes apart, half a sector and one line per thread and store; from shared
 // memory a store writes 512 consecutive bytes. Pieces are swizzled by their row, so that neither side meets bank conflicts.
 constexpr int SPLIT_ROW_STAGE = 32 * 128;  // bytes of shared memory per warp
 __device__ __forceinline__ void store_split_rows(float* out, size_t row, bool valid, const float* v, uint4* stage, int32_t* range_flag) {
-    constexpr int P = 4, Q = 8;  // 16-byte pieces of the hi (or lo) part, of a row
+    constexpr int Q = 8;  // 16-byte pieces of a row
     const int lane  = threadIdx.x & 31;
+    const int odd   = static_cast<int>(row & 1) * 4;
     bool bad        = false;
     __syncwarp();
 #pragma unroll
-    for (int p = 0; p < P; ++p) {
-        uint32_t h[4], l[4];
+    for (int p = 0; p < Q; ++p) {
+        uint32_t h[2], l[2];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float x0 = v[8 * p + 2 * q], x1 = v[8 * p + 2 * q + 1];
+        for (int q = 0; q < 2; ++q) {
+            const float x0 = v[4 * p + 2 * q], x1 = v[4 * p + 2 * q + 1];
             bad |= fabsf(x0) > 60000.0f || fabsf(x1) > 60000.0f;
             split_pair(x0, x1, h[q], l[q]);
         }
-        stage[lane * Q + (p ^ (lane & (Q - 1)))]       = make_uint4(h[0], h[1], h[2], h[3]);
-        stage[lane * Q + ((P + p) ^ (lane & (Q - 1)))] = make_uint4(l[0], l[1], l[2], l[3]);
+        stage[lane * Q + ((p ^ odd) ^ (lane & (Q - 1)))] = make_uint4(h[0], l[0], h[1], l[1]);
     }
     if (bad && valid) raise_flag(range_flag, ABORT_TC_RANGE);
     __syncwarp();

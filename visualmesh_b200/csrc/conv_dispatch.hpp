@@ -81,7 +81,7 @@ struct StagedPlan {
 };
 constexpr int STAGED_NBL_STRIDE = 8;    // 16-bit neighbour positions per row
 constexpr int STAGED_ST         = 256;  // rows of a super-tile
-constexpr int STAGED_HALO       = 192;  // halo slots of a super-tile
+constexpr int STAGED_HALO       = 384;  // halo slots of a super-tile
 bool has_staged_kernel(const DenseLayer& L);
 bool launch_conv_staged(const DenseLayer& L, const ConvArgs& a, const StagedPlan& plan, int n_frames, int max_rows, int32_t* abort_flags,
                         uint32_t wait_limit, cudaStream_t s);

@@ -127,7 +127,8 @@ namespace st {
     constexpr int TILE             = 8;   // rows of one warp-level MMA tile (its N)
     constexpr int CIN              = 16;  // input channels
     constexpr int ROW              = 4 * CIN;  // bytes of a feature row: four pieces of four channels, hi parts then lo parts each
-    constexpr int WINDOW           = (ST + HALO) * ROW;
+    constexpr int KEPT             = 192;  // halo slots of a window: the rest of a super-tile's comes from global memory (rings of six neighbours have 188 at most)
+    constexpr int WINDOW           = (ST + KEPT) * ROW;
     constexpr int NBL_BYTES        = ST * NBL_STRIDE * 2;
 
     // 16x16 fragments of a slot's weights: hi and lo parts of 16 output channels each, or of eight channels in one
@@ -247,15 +248,15 @@ namespace st {
             // The halo list of a super-tile (its length, then this lane's entries) is read one super-tile ahead, while
             // the loader waits for a buffer anyway: the copies of a window then start the moment its buffer is free
             // instead of two dependent trips to global memory later.
-            constexpr int PER_LANE = (HALO + 31) / 32;
+            constexpr int PER_LANE = (KEPT + 31) / 32;
             int n_halo = 0, listed = 0;
             int32_t halo_row[PER_LANE];
             auto fetch_halo_list = [&](int st) {
                 listed                = __ldg(plan.halo_count + st);
-                n_halo                = min(listed, HALO);
+                n_halo                = min(listed, KEPT);
                 const int32_t* h_rows = plan.halo_rows + static_cast<size_t>(st) * HALO;
 #pragma unroll
-                for (int k = 0; k < PER_LANE; ++k) halo_row[k] = __ldg(h_rows + min(lane + 32 * k, HALO - 1));  // entries past n_halo are never used
+                for (int k = 0; k < PER_LANE; ++k) halo_row[k] = __ldg(h_rows + min(lane + 32 * k, KEPT - 1));  // entries past n_halo are never used
             };
             uint32_t n = 0;
             bool ok    = true;
@@ -272,7 +273,7 @@ namespace st {
                 const uint32_t dst = win_addr + b * WINDOW;
                 const uint32_t bar = bar_full + 8 * b;
                 if (lane == 0) {
-                    window_miss[b] = listed > HALO;
+                    window_miss[b] = listed > KEPT;
                     mbar_expect_tx(bar, static_cast<uint32_t>(own * (ROW + 2 * NBL_STRIDE)));
                     bulk_copy(nbl_addr + b * NBL_BYTES, reinterpret_cast<const uint4*>(plan.nbl) + r.local_base + r.t0, static_cast<uint32_t>(own * 2 * NBL_STRIDE),
                               bar);
@@ -282,7 +283,7 @@ namespace st {
                 const unsigned char* from = in_bytes + (lane & 3) * 16;
                 const uint32_t to         = dst + ST * ROW + lane * 16;
 #pragma unroll
-                for (int k = 0; k < HALO / 8; ++k) {
+                for (int k = 0; k < KEPT / 8; ++k) {
                     if (8 * k >= n_halo) break;
                     const int32_t row = __shfl_sync(0xffffffffu, halo_row[k / 4], 8 * (k % 4) + (lane >> 2));
                     if (8 * k + (lane >> 2) < n_halo) copy16(to + k * 8 * ROW, from + static_cast<size_t>(row) * ROW);
@@ -387,7 +388,7 @@ namespace st {
                             const uint32_t row = window_row(i);
                             uint32_t p         = row;
                             if (slot > 0) asm volatile("ld.shared.u16 %0, [%1];" : "=r"(p) : "r"(nbl + row * (2 * NBL_STRIDE) + 2 * (slot - 1)));
-                            if (slot > 0 && p == NBL_GLOBAL) {
+                            if (slot > 0 && p >= static_cast<uint32_t>(ST + KEPT)) {
                                 const int idx = __ldg(a.nb + (r.nb_base + r.t0 + row) * a.n_neighbours + (slot - 1));
                                 x[i]          = __ldg(reinterpret_cast<const uint4*>(in_bytes + static_cast<size_t>(r.local_base + idx) * ROW + tq * 16));
                             }
@@ -464,12 +465,8 @@ namespace st {
                         }
                     }
                     else {
-                        // 32 channels, the thread's 4 g .. 4 g + 3: eight bytes of the hi parts and of the lo parts of either row
-                        const bool rowed   = a.out_split == SPLIT_ROWS;
+                        // 32 channels, the thread's 4 g .. 4 g + 3 of either row: a piece of it, or eight bytes of the hi and of the lo planes
                         const size_t plane = static_cast<size_t>(a.out_stride) * 16;
-                        const int pitch    = rowed ? 128 : 16;
-                        unsigned char* to  = rowed ? out_b + out_row * 128 + g * 8 : out_b + (g >> 1) * plane + out_row * 16 + (g & 1) * 8;
-                        const size_t lo_at = rowed ? 64 : 4 * plane;
 #pragma unroll
                         for (int i = 0; i < TILES; ++i) {
 #pragma unroll
@@ -481,8 +478,15 @@ namespace st {
                                     largest = __hmax2(largest, __habs2(*reinterpret_cast<const __half2*>(&h[m])));
                                 }
                                 if (TILE * i + k >= left) continue;
-                                *reinterpret_cast<uint2*>(to + (TILE * i + k) * pitch)         = make_uint2(h[0], h[MBLK - 1]);
-                                *reinterpret_cast<uint2*>(to + lo_at + (TILE * i + k) * pitch) = make_uint2(l[0], l[MBLK - 1]);
+                                const size_t row = out_row + TILE * i + k;
+                                if (a.out_split == SPLIT_ROWS) {
+                                    // the halves of odd rows lie the other way round
+                                    reinterpret_cast<uint4*>(out_b)[row * 8 + (g ^ (static_cast<int>(row & 1) * 4))] = make_uint4(h[0], l[0], h[MBLK - 1], l[MBLK - 1]);
+                                    continue;
+                                }
+                                unsigned char* dst                     = out_b + (g >> 1) * plane + row * 16 + (g & 1) * 8;
+                                *reinterpret_cast<uint2*>(dst)             = make_uint2(h[0], h[MBLK - 1]);
+                                *reinterpret_cast<uint2*>(dst + 4 * plane) = make_uint2(l[0], l[MBLK - 1]);
                             }
                         }
                     }

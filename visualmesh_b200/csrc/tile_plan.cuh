@@ -1,7 +1,7 @@
 // The tile plan of a chunk of frames for the staged graph-convolution layers (conv_staged.cuh).
 //
 // The rows of a frame are cut into super-tiles of ST consecutive rows. For every super-tile the plan lists the rows
-// outside it that its rows have as neighbours (its halo, at most HALO rows - mesh nodes are stored in the order of the
+// outside it that its rows have as neighbours (its halo; at most HALO of them get a slot - mesh nodes are stored in the order of the
 // reference's BSP, cpp/visualmesh/mesh.hpp:450-466, which is spatially compact, so a 256-row super-tile has ~95 of
 // them), and for every row its neighbours as 16-bit positions inside "super-tile rows, then halo slots". A neighbour
 // whose halo slot did not fit is marked NBL_GLOBAL and fetched from global memory by the layer kernels.
@@ -15,7 +15,7 @@ namespace vm {
 namespace st {
 
     constexpr int ST               = 256;     // rows of a super-tile = threads of the block that plans it
-    constexpr int HALO             = 192;     // halo slots of a super-tile
+    constexpr int HALO             = 384;     // halo slots of a super-tile: rings of eight neighbours have 113 on average, 331 at most
     constexpr int HASH_SIZE        = 1024;    // open-addressing table of a super-tile's outside rows
     constexpr uint32_t NBL_GLOBAL  = 0xFFFFu; // neighbour position: not staged, fetch from global memory
     constexpr int NBL_STRIDE       = 8;       // 16-bit positions per row (N <= 8), one 16-byte load
