@@ -122,6 +122,25 @@ def test_layers_with_large_halos(n, reach, n_neighbours, widths):
     assert np.abs(got.astype(np.float64) - O.network(x, nb, net).astype(np.float64)).max() <= P.TOL_CLS / 4
 
 
+# 296 blocks of 128 rows (32 channels: half super-tiles), 592 super-tiles or 296 blocks of 512 rows: up to there layers start early
+@pytest.mark.parametrize("n", [1, 300, 37_888, 37_889, 151_552, 151_553])
+@pytest.mark.parametrize("n_neighbours,widths", [(6, [16, 16, 16, 8, 8, 8, 5]), (8, [32, 32, 32, 16, 8, 4, 3])])
+def test_layers_that_start_early(n, n_neighbours, widths):
+    """Layers whose buffers take turns, over inputs that take turns: a row read too early would be another input's or another layer's."""
+    net = W.make_network(71, n_neighbours, widths)
+    x, _ = _rows(n, n_neighbours, 13)
+    inputs = [x, np.ascontiguousarray(-x[::-1])]
+    nb = _near(n, n_neighbours, 40)
+    engine = Engine(net)
+    got = [engine.network(inputs[i % 2], nb).copy() for i in range(6)]
+    engine.close()
+    for i, result in enumerate(got):
+        if i >= 2:
+            assert np.array_equal(result, got[i - 2])
+            continue
+        assert np.abs(result.astype(np.float64) - O.network(inputs[i], nb, net).astype(np.float64)).max() <= P.TOL_CLS / 4
+
+
 def test_selu_over_its_range():
     """A layer that passes its input through: SELU of floats of every size, against double.
 

@@ -30,6 +30,7 @@ struct ConvArgs {
     int32_t out_split;      // write `out` as fp16 hi/lo parts for a tensor-core consumer: SPLIT_PLANES (COUT % 8 == 0), SPLIT_ROWS or SPLIT_QUADS
     float* const* out_host; // where the batch-wide classifications go instead of `out`: the device address of a pointer to pinned memory
     int32_t* range_flag;    // the engine's abort flags: ABORT_RANGE is raised when a value is too large for the fp16 split
+    int32_t early;          // for the launch: may start while the layer before finishes (launch_kernel)
 };
 
 // ConvArgs::out_split. Planes of 16-byte chunks; whole rows for the window kernel (its 32 input channels: COUT == 32), pieces of
@@ -42,6 +43,18 @@ constexpr int CONV_THREADS = 128;
 // call neither clears nor copies anything.
 enum AbortReason { ABORT_BSP_DEPTH = 1, ABORT_TC_TIMEOUT = 2, ABORT_TC_RANGE = 3, ABORT_FLAGS = 4 };
 #ifdef __CUDACC__
+// A layer that launch_kernel starts early begins before the one in front of it has ended. Before it reads what that one writes, or
+// writes what that one reads, it calls this: everything of the layer in front is then done and visible, and the next layer may start in
+// turn. Not sooner: a layer must not run beside the one two in front of it, which reads the buffer that the layer between them writes and
+// could leave its old lines in an L1 cache that was cleaned when the layer behind started. The pointer goes through the wait, so
+// that no load from it is scheduled in front of it. Launched the ordinary way a kernel passes at once. At least one block of every launch
+// must call; blocks without work may leave before.
+template <typename T>
+__device__ __forceinline__ T* after_previous(T* p) {
+    asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    return p;
+}
 __device__ __forceinline__ void raise_flag(int32_t* flags, int reason) {
     *static_cast<volatile int32_t*>(flags + reason) = 1;
 }

@@ -58,6 +58,33 @@ struct LaunchPlans {
     }
 };
 
+// Whether a layer's launch starts early: only while its blocks (as many as there may be rows for) find room beside those of the
+// layer in front. A pass with a network's layers started early, us, one frame of 2.7 | 11 | 25 | 57 | 121 | 242 k nodes: thirteen layers of 16 and 8
+// channels 86.9 | 90.3 | 92.8 | 101 | 128 | 154 -> 76.0 | 80.6 | 82.9 | 93.6 | 118 | 169; four layers 50.5 | 51.5 | 53.2 | 54.4 | 64.0 | 76.6 -> 45.7 | 48.5 |
+// 48.4 | 53.2 | 63.6 | 85.9; ten of 32 channels, a CTA per SM, 105 | 107 | 112 | 126 | 157 | 239 -> 84.7 | 85.9 | 104 | 134 | 193 | 255. So two blocks
+// per SM, and four of the staged layers' small CTAs. Layers that few rows send to the kernel with part of the outputs per block lose (50
+// -> 57 us at 11 k nodes, five times the blocks) and start the ordinary way, and so do the kernels of the projection (no gain),
+// and a last layer that writes to the host (a call of two layers 36.9 -> 37.7 us).
+inline bool starts_early(int64_t blocks, int blocks_per_sm, int n_sms) {
+    return blocks <= static_cast<int64_t>(blocks_per_sm) * n_sms;
+}
+// A launch; early: it may start while the kernel in front of it in the stream finishes, and waits for that one's results itself
+// (after_previous), with its own preparations - barriers, weights into shared memory - behind it.
+template <typename... Params, typename... Args>
+void launch_kernel(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t s, bool early, const Args&... args) {
+    cudaLaunchAttribute attribute{};
+    attribute.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim          = grid;
+    config.blockDim         = dim3(threads);
+    config.dynamicSmemBytes = smem;
+    config.stream           = s;
+    config.attrs            = &attribute;
+    config.numAttrs         = early ? 1 : 0;
+    VM_CUDA(cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...));
+}
+
 // ---- conv_ffma.cu: layers on the CUDA cores ----------------------------------------------------------------------
 // a specialised kernel exists for this shape (anything else runs the generic kernel, which ignores ConvArgs::out_split)
 bool has_fast_ffma_kernel(int cin, int cout);

@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(T, (CIN == 8 && COUT <= 8 && T == 256) ? 6 : 0
 #pragma unroll
         for (int j = 0; j < COUTP / 2; ++j) acc[q][j] = pack2(wp.w[K * COUTP + 2 * j], wp.w[K * COUTP + 2 * j + 1]);
     }
-    const float4* in4 = reinterpret_cast<const float4*>(a.in);
+    const float4* in4 = after_previous(reinterpret_cast<const float4*>(a.in));
 #pragma unroll(NS ? NS : 1)
     for (int s = 0; s < n_slots; ++s) {
         int src_row[R];

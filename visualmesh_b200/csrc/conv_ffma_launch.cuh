@@ -97,17 +97,18 @@ static bool launch_conv_cw(const DenseLayer& L, const ConvArgs& a, dim3 grid_row
     // (with the weights in the parameter space instead of shared memory), 8 -> 8 133 -> 112 us, 32 -> 4 448 -> 413 us;
     // the 16- and 32-channel layers in between, bound by the FP32 pipe, measured 3-6 % slower unrolled and stay rolled.
     const size_t smem            = stage_bytes(a, COUT, T, R);
+    const bool early             = a.early && starts_early(static_cast<int64_t>(grid.x) * grid.y, 2, sm_count());
     // 12 -> 8 and 8 -> 12 go with the narrow ones.
     constexpr bool LATENCY_BOUND = CIN * COUT <= 96 || CIN == 4 || COUT <= 4;
-    if (LATENCY_BOUND && a.n_slots == 5) { k_graph_conv_cw<CIN, COUT, R, WMAX, T, LATENCY_BOUND ? 5 : 0><<<grid, T, smem, s>>>(a, wp); }
+    if (LATENCY_BOUND && a.n_slots == 5) { launch_kernel(k_graph_conv_cw<CIN, COUT, R, WMAX, T, LATENCY_BOUND ? 5 : 0>, grid, T, smem, s, early, a, wp); }
     else if (LATENCY_BOUND && a.n_slots == 7) {
-        k_graph_conv_cw<CIN, COUT, R, WMAX, T, LATENCY_BOUND ? 7 : 0><<<grid, T, smem, s>>>(a, wp);
+        launch_kernel(k_graph_conv_cw<CIN, COUT, R, WMAX, T, LATENCY_BOUND ? 7 : 0>, grid, T, smem, s, early, a, wp);
     }
     else if (LATENCY_BOUND && a.n_slots == 9) {
-        k_graph_conv_cw<CIN, COUT, R, WMAX, T, LATENCY_BOUND ? 9 : 0><<<grid, T, smem, s>>>(a, wp);
+        launch_kernel(k_graph_conv_cw<CIN, COUT, R, WMAX, T, LATENCY_BOUND ? 9 : 0>, grid, T, smem, s, early, a, wp);
     }
     else {
-        k_graph_conv_cw<CIN, COUT, R, WMAX, T><<<grid, T, smem, s>>>(a, wp);
+        launch_kernel(k_graph_conv_cw<CIN, COUT, R, WMAX, T>, grid, T, smem, s, early, a, wp);
     }
     return true;
 }

@@ -35,7 +35,7 @@ static void launch_conv_staged_t(const DenseLayer& L, const ConvArgs& a, const s
     t.wait_limit = wait_limit;
     const int tiles_upper = n_frames * ((max_rows + st::ST - 1) / st::ST);
     const int grid        = std::max(1, std::min(tiles_upper, lp.n_sms * lp.ctas_per_sm));
-    kernel<<<grid, THREADS, smem, s>>>(a, t, plan);
+    launch_kernel(kernel, dim3(grid), THREADS, smem, s, a.early && starts_early(tiles_upper, 4, lp.n_sms), a, t, plan);
 }
 
 bool has_staged_kernel(const DenseLayer& L) {

@@ -241,6 +241,7 @@ namespace st {
             r.nb_base    = static_cast<size_t>(start + a.f0 + f);
             return r;
         };
+        // all that read the features: the loader, and the compute warps behind its first window
         const unsigned char* in_bytes = reinterpret_cast<const unsigned char*>(a.in);
 
         if (warp == WARPS) {
@@ -261,6 +262,7 @@ namespace st {
             uint32_t n = 0;
             bool ok    = true;
             if (static_cast<int>(blockIdx.x) < total_st) fetch_halo_list(blockIdx.x);
+            in_bytes = after_previous(in_bytes);
             for (int s = blockIdx.x; s < total_st; s += gridDim.x, ++n) {
                 const uint32_t b = n & 1u;
                 // every compute warp must be done with the super-tile that used this buffer before

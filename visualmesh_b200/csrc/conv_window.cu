@@ -29,7 +29,7 @@ static void launch_conv_window_t(const DenseLayer& L, const ConvArgs& a, const s
     t.wait_limit  = wait_limit;
     const int tiles_upper = n_frames * 2 * ((max_rows + st::ST - 1) / st::ST);  // few super-tiles: half a super-tile per CTA
     const int grid        = std::max(1, std::min(tiles_upper, lp.n_sms));
-    kernel<<<grid, win::THREADS, smem, s>>>(a, t, plan);
+    launch_kernel(kernel, dim3(grid), win::THREADS, smem, s, a.early && starts_early(tiles_upper, 2, lp.n_sms), a, t, plan);
 }
 
 bool has_window_kernel(const DenseLayer& L) {

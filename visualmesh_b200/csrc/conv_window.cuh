@@ -299,6 +299,7 @@ namespace win {
             int start[2] = {0, 0}, end[2] = {0, 0};
             HaloList next = {};
             if (static_cast<int>(blockIdx.x) < total_items) fetch_halo_list(next, blockIdx.x);
+            in_bytes = after_previous(in_bytes);  // what the other warps read and write comes behind a window
             for (int item = blockIdx.x; item < total_items; item += gridDim.x, ++n) {
                 const HaloList list = next;
                 if (item + static_cast<int>(gridDim.x) < total_items) fetch_halo_list(next, item + gridDim.x);

@@ -426,6 +426,10 @@ static void run_network(vm_engine* e,
         a.out_split    = last ? SPLIT_NONE : kind[l + 1] == CONV_TC_WINDOW ? SPLIT_ROWS : kind[l + 1] == CONV_TC_STAGED ? SPLIT_QUADS : kind[l + 1] >= CONV_TC_SPLIT ? SPLIT_PLANES : SPLIT_NONE;
         a.out_host     = last ? out_host : nullptr;
         a.range_flag   = e->flags;
+        // not the first layer, which follows two streams that have joined, and none behind a window kernel but another: a CTA of that one
+        // fills its SM, and the 32 -> 4 layer started behind ten of them cost 45 us of 157 (121 k nodes)
+        const bool behind_window = l > 0 && kind[l - 1] == CONV_TC_WINDOW && kind[l] != CONV_TC_WINDOW;
+        a.early                  = l > 0 && !behind_window && a.out_host == nullptr && !e->timing ? 1 : 0;
         launch_conv(e, e->layers[l], a, n_frames, max_rows, lane.stream, kind[l], plan);
         cur ^= 1;
     }
