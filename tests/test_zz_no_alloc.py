@@ -132,3 +132,29 @@ def test_static_projection_rejects_what_does_not_fit():
     assert lib.vm_launch_count(engine._ptr) == n
     other.close()
     engine.close()
+
+
+# an array of the caller's own may begin on any multiple of four bytes; the wide stores of 4, 6 and 8 neighbours begin on 16 or 8
+@pytest.mark.parametrize("words", [0, 1, 2, 3])
+@pytest.mark.parametrize("name", ["ring4_rectilinear_grey", "ring6_equisolid_rgba", "ring8_equidistant_bgra"])
+def test_static_projection_into_arrays_of_any_alignment(name, words):
+    import torch
+    case = G.Case(name)
+    engine = Engine()
+    mesh = Mesh.from_arrays(case.rays, case.nbrs, case.bsp)
+    n_nodes, N = case.nbrs.shape
+    handle, lens, fr = engine._device_mesh(mesh), _c_lens(case.lens), case.frames[0]
+    px = torch.empty((n_nodes, 2), dtype=torch.float32, device="cuda")
+    gi = torch.empty((n_nodes,), dtype=torch.int32, device="cuda")
+    nb = torch.full(((n_nodes + 1) * N + 8,), -7, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()  # the engine has streams of its own
+    H = np.ascontiguousarray(fr["Hoc"], dtype=np.float32)
+    n = C.c_int32(-1)
+    abi.check(abi.load().vm_project_static(engine._ptr, handle, H.ctypes.data, C.byref(lens), px.data_ptr(), gi.data_ptr(),
+                                           nb.data_ptr() + 4 * words, None, C.byref(n)))
+    torch.cuda.synchronize()
+    rows = (n.value + 1) * N
+    got = nb.cpu().numpy()
+    assert np.array_equal(got[words:words + rows].reshape(-1, N), fr["neighbourhood"])
+    assert np.all(got[:words] == -7) and np.all(got[words + rows:] == -7)
+    engine.close()
