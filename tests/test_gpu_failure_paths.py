@@ -85,6 +85,22 @@ def test_poll_limit_zero_makes_the_tensor_core_kernels_give_up_cleanly(n_neighbo
     engine.close()
 
 
+# A poll of a wait lasts a few microseconds. With the waits of a layer counting from the end of the layer in front, these chains were
+# computed twenty times of twenty with limits of 1 and 8 (4: 19 times); counting from their early starts, never with 2 and 8.
+@pytest.mark.parametrize("widths,n,polls", [([16] * 7 + [3], 37_888, 2), ([32] * 7 + [4], 20_000, 8)])
+def test_poll_limit_does_not_count_the_layer_in_front(widths, n, polls):
+    """Layers of few rows start early. Their bounded waits are for what the block itself brings and computes, so a limit that is
+    enough for a layer's own work is enough however long the layer in front takes (neighbours all over the rows make it slow)."""
+    net = W.make_network(73, 8, widths)
+    x, nb = _random_rows(n, 8, 41)
+    engine = Engine(net)
+    want = engine.network(x, nb).copy()
+    engine.set_wait_limit(polls)
+    for _ in range(5):
+        assert np.array_equal(engine.network(x, nb), want)
+    engine.close()
+
+
 def test_fp16_range_overflow_in_an_early_chunk_of_a_batch_is_not_missed():
     """Six one-frame chunks rotate over the engine's three streams. Only the first frame drives a feature beyond the
     range of the fp16 split (its image is bright, the others are black), so the flag is raised by an early chunk while

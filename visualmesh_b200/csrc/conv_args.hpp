@@ -44,14 +44,21 @@ constexpr int CONV_THREADS = 128;
 enum AbortReason { ABORT_BSP_DEPTH = 1, ABORT_TC_TIMEOUT = 2, ABORT_TC_RANGE = 3, ABORT_FLAGS = 4 };
 #ifdef __CUDACC__
 // A layer that launch_kernel starts early begins before the one in front of it has ended. Before it reads what that one writes, or
-// writes what that one reads, it calls this: everything of the layer in front is then done and visible, and the next layer may start in
-// turn. Not sooner: a layer must not run beside the one two in front of it, which reads the buffer that the layer between them writes and
-// could leave its old lines in an L1 cache that was cleaned when the layer behind started. The pointer goes through the wait, so
-// that no load from it is scheduled in front of it. Launched the ordinary way a kernel passes at once. At least one block of every launch
-// must call; blocks without work may leave before.
+// writes what that one reads, it waits for it here: everything of the layer in front is then done and visible. The pointer goes through
+// the wait, so that no load from it is scheduled in front of it. Launched the ordinary way a kernel passes at once. All warps make this
+// wait, also those that only read what others of their block bring: their bounded waits (vm_set_wait_limit) then count polls of this
+// layer's work alone, and the issue slots stay with the layer in front.
+template <typename T>
+__device__ __forceinline__ T* wait_previous(T* p) {
+    asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");
+    return p;
+}
+// The same, and the next layer may start in turn. Not sooner: a layer must not run beside the one two in front of it, which reads the
+// buffer that the layer between them writes and could leave its old lines in an L1 cache that was cleaned when the layer behind started.
+// At least one block of every launch must call; blocks without work may leave before.
 template <typename T>
 __device__ __forceinline__ T* after_previous(T* p) {
-    asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");
+    p = wait_previous(p);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     return p;
 }

@@ -311,6 +311,7 @@ namespace st {
 #pragma unroll
             for (int i = 0; i < NSLOTS; ++i) held[i] = load_shared(frag_addr + i * 512);
         }
+        in_bytes = wait_previous(in_bytes);
         uint32_t n = 0;
         bool ok    = true;
         for (int s = blockIdx.x; s < total_st; s += gridDim.x, ++n) {

@@ -299,7 +299,7 @@ namespace win {
             int start[2] = {0, 0}, end[2] = {0, 0};
             HaloList next = {};
             if (static_cast<int>(blockIdx.x) < total_items) fetch_halo_list(next, blockIdx.x);
-            in_bytes = after_previous(in_bytes);  // what the other warps read and write comes behind a window
+            in_bytes = after_previous(in_bytes);
             for (int item = blockIdx.x; item < total_items; item += gridDim.x, ++n) {
                 const HaloList list = next;
                 if (item + static_cast<int>(gridDim.x) < total_items) fetch_halo_list(next, item + gridDim.x);
@@ -378,6 +378,7 @@ namespace win {
             uint32_t phase = 0;
             int turn = 0;
             bool ok  = true;
+            in_bytes = wait_previous(in_bytes);
             for (int item = blockIdx.x; ok && item < total_items; item += gridDim.x) {
                 const Item r = locate(item);
                 for (int tile = r.first; tile < r.end; ++tile) {
@@ -432,6 +433,7 @@ namespace win {
             uint32_t buf = 0, phase = 0, done_phase = 1;  // the first waits for a part to be multiplied pass at once
             int turn = 0;  // the group whose tile is next
             bool ok  = true;
+            in_bytes = wait_previous(in_bytes);
             for (int item = blockIdx.x; ok && item < total_items; item += gridDim.x) {
                 int last, first_tile, end_tile;
                 uint32_t parity;  // 64 where even places of the window hold odd rows
@@ -547,7 +549,8 @@ namespace win {
 #pragma unroll
             for (int j = 0; j < OWN; ++j) bias[j] = __ldg(t.bias + piece * OWN + j);
             uint32_t acc = 0, phase = 0;
-            bool ok = true;
+            bool ok  = true;
+            in_bytes = wait_previous(in_bytes);
             for (int item = blockIdx.x; ok && item < total_items; item += gridDim.x) {
                 const Item r = locate(item);
                 for (int tile = r.first; ok && tile < r.end; ++tile) {
