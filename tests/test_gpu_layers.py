@@ -141,6 +141,23 @@ def test_layers_that_start_early(n, n_neighbours, widths):
         assert np.abs(result.astype(np.float64) - O.network(inputs[i], nb, net).astype(np.float64)).max() <= P.TOL_CLS / 4
 
 
+# neighbours beyond every halo: rows that the layer in front writes are read past the windows, from memory
+@pytest.mark.parametrize("n", [300, 37_888])
+@pytest.mark.parametrize("n_neighbours,widths", [(6, [16, 16, 32, 32, 16, 16, 5]), (8, [16, 16, 16, 16, 8, 3]), (8, [32, 32, 32, 32, 4])])
+def test_layers_that_start_early_with_neighbours_anywhere(n, n_neighbours, widths):
+    net = W.make_network(79, n_neighbours, widths)
+    x, nb = _rows(n, n_neighbours, 17)
+    inputs = [x, np.ascontiguousarray(-x[::-1])]
+    engine = Engine(net)
+    got = [engine.network(inputs[i % 2], nb).copy() for i in range(6)]
+    engine.close()
+    for i, result in enumerate(got):
+        if i >= 2:
+            assert np.array_equal(result, got[i - 2])
+            continue
+        assert np.abs(result.astype(np.float64) - O.network(inputs[i], nb, net).astype(np.float64)).max() <= P.TOL_CLS / 4
+
+
 def test_selu_over_its_range():
     """A layer that passes its input through: SELU of floats of every size, against double.
 

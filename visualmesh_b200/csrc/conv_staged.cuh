@@ -393,7 +393,7 @@ namespace st {
                             if (slot > 0) asm volatile("ld.shared.u16 %0, [%1];" : "=r"(p) : "r"(nbl + row * (2 * NBL_STRIDE) + 2 * (slot - 1)));
                             if (slot > 0 && p >= static_cast<uint32_t>(ST + KEPT)) {
                                 const int idx = __ldg(a.nb + (r.nb_base + r.t0 + row) * a.n_neighbours + (slot - 1));
-                                x[i]          = __ldg(reinterpret_cast<const uint4*>(in_bytes + static_cast<size_t>(r.local_base + idx) * ROW + tq * 16));
+                                x[i]          = *reinterpret_cast<const uint4*>(in_bytes + static_cast<size_t>(r.local_base + idx) * ROW + tq * 16);
                             }
                             else {
                                 x[i] = load_shared(win + p * ROW);

@@ -516,7 +516,7 @@ namespace win {
                                     const int idx            = f.local_base + __ldg(a.nb + (nb_base + row) * a.n_neighbours + (slot - 1));
                                     const unsigned char* src = in_bytes + static_cast<size_t>(idx) * ROW + piece * 16;
 #pragma unroll
-                                    for (int h = 0; h < 2; ++h) x[0].v[h] = __ldg(reinterpret_cast<const uint4*>(src + 64 * ((h ^ idx) & 1)));
+                                    for (int h = 0; h < 2; ++h) x[0].v[h] = *reinterpret_cast<const uint4*>(src + 64 * ((h ^ idx) & 1));
                                 }
                                 else {
                                     load(x[0], p);
