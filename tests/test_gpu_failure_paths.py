@@ -6,6 +6,7 @@ run out with well-formed but useless inputs (a BSP with a cycle, a poll limit of
 use the same engine again.
 """
 import os
+import time
 
 import numpy as np
 import pytest
@@ -98,6 +99,27 @@ def test_poll_limit_does_not_count_the_layer_in_front(widths, n, polls):
     engine.set_wait_limit(polls)
     for _ in range(5):
         assert np.array_equal(engine.network(x, nb), want)
+    engine.close()
+
+
+def test_wait_that_runs_out_for_one_loader_of_a_window_ends_the_call_at_once():
+    """The two loader warps of a 32-channel layer fill every window together. With limits near what their waits need one of them may
+    run out where the other passes: neither may then begin the window, whose copies the other would wait for until the default limit
+    (seconds). Several windows per block, so that their buffers are used again."""
+    net = W.make_network(75, 8, [32, 32, 32, 4])
+    x, nb = _random_rows(151_552, 8, 43)
+    engine = Engine(net)
+    want = engine.network(x, nb).copy()
+    for i in range(120):
+        engine.set_wait_limit(1 + i % 12)
+        begin = time.perf_counter()
+        try:
+            assert np.array_equal(engine.network(x, nb), want)
+        except VisualMeshError as e:
+            assert e.status == abi.VM_ERR_DEVICE_ABORT, str(e)
+        assert time.perf_counter() - begin < 0.5
+    engine.set_wait_limit(4_000_000)
+    assert np.array_equal(engine.network(x, nb), want)
     engine.close()
 
 

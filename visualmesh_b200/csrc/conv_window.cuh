@@ -115,6 +115,22 @@ namespace win {
         asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(addr));
         return v;
     }
+    // Whether both loader warps may go on. A window is filled by both or by neither: one that a single loader had begun would never become
+    // full, and the other's wait for its copies at the end would last until the default limit runs out.
+    __device__ __forceinline__ bool loaders_agree(bool ok) {
+        uint32_t r;
+        asm volatile(
+          "{\n\t"
+          ".reg .pred p, q;\n\t"
+          "setp.ne.u32 p, %1, 0;\n\t"
+          "barrier.cta.red.and.pred q, 1, %2, p;\n\t"
+          "selp.u32 %0, 1, 0, q;\n\t"
+          "}\n"
+          : "=r"(r)
+          : "r"(static_cast<uint32_t>(ok)), "n"(32 * LOADERS)
+          : "memory");
+        return r != 0;
+    }
     // one lane of a converged warp; what it alone does keeps its operands uniform
     __device__ __forceinline__ bool elect_one() {
         uint32_t r;
@@ -303,19 +319,18 @@ namespace win {
             for (int item = blockIdx.x; item < total_items; item += gridDim.x, ++n) {
                 const HaloList list = next;
                 if (item + static_cast<int>(gridDim.x) < total_items) fetch_halo_list(next, item + gridDim.x);
-                if (n >= BUFFERS && !wait(bar_free + 8 * buf, phase ^ 1u)) break;
+                bool there = n < BUFFERS || wait(bar_free + 8 * buf, phase ^ 1u);
                 const int n_halo = min(list.count, HALO);
                 // behind the last window, or from the pool's beginning; whatever window lies there still must have been read
                 const int size = ST + n_halo;
                 const int at   = end[0] + size <= POOL ? end[0] : 0;
-                bool there     = true;
 #pragma unroll
                 for (int back = 2; back >= 1; --back) {
                     const bool meets = n >= static_cast<uint32_t>(back) && at < end[back - 1] && start[back - 1] < at + size;
                     const uint32_t m = n - back;
                     if (there && meets) there = wait(bar_free + 8 * (m % BUFFERS), (m / BUFFERS) & 1u);
                 }
-                if (!there) break;
+                if (!loaders_agree(there)) break;
                 start[1] = start[0];
                 end[1]   = end[0];
                 start[0] = at;
