@@ -102,12 +102,13 @@ def test_poll_limit_does_not_count_the_layer_in_front(widths, n, polls):
     engine.close()
 
 
-def test_wait_that_runs_out_for_one_loader_of_a_window_ends_the_call_at_once():
-    """The two loader warps of a 32-channel layer fill every window together. With limits near what their waits need one of them may
-    run out where the other passes: neither may then begin the window, whose copies the other would wait for until the default limit
-    (seconds). Several windows per block, so that their buffers are used again."""
-    net = W.make_network(75, 8, [32, 32, 32, 4])
-    x, nb = _random_rows(151_552, 8, 43)
+@pytest.mark.parametrize("widths,n", [([32, 32, 32, 4], 151_552), ([16, 16, 16, 3], 400_000)])
+def test_wait_that_runs_out_for_one_loader_of_a_window_ends_the_call_at_once(widths, n):
+    """The two loader warps of a 32-channel layer fill every window together, and the lanes of the one of a 16-channel layer. With limits
+    near what their waits need some may run out where the others pass: none may then begin the window, whose copies they would wait
+    for until the default limit (seconds). Several windows per block, so that their buffers are used again."""
+    net = W.make_network(75, 8, widths)
+    x, nb = _random_rows(n, 8, 43)
     engine = Engine(net)
     want = engine.network(x, nb).copy()
     for i in range(120):

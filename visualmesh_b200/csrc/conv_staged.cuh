@@ -266,10 +266,9 @@ namespace st {
             for (int s = blockIdx.x; s < total_st; s += gridDim.x, ++n) {
                 const uint32_t b = n & 1u;
                 // every compute warp must be done with the super-tile that used this buffer before
-                if (n >= 2 && !tc::mbar_wait_or_fail(bar_empty + 8 * b, ((n >> 1) - 1) & 1u, failed, t.wait_limit)) {
-                    ok = false;
-                    break;
-                }
+                // the warp decides together: what follows needs all of its lanes, and a window that some had begun would never become full
+                ok = __all_sync(0xffffffffu, n < 2 || tc::mbar_wait_or_fail(bar_empty + 8 * b, ((n >> 1) - 1) & 1u, failed, t.wait_limit));
+                if (!ok) break;
                 const StRef r      = locate(s);
                 const int own      = min(ST, r.rows - r.t0);
                 const uint32_t dst = win_addr + b * WINDOW;
