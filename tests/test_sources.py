@@ -44,3 +44,18 @@ def test_kernels_that_start_early_read_no_features_by_the_read_only_path():
                 argument = re.sub(r"^reinterpret_cast<[^>]*>\(", "", _argument(body, load.end()))
                 assert CONSTANT.match(argument), f"{kernel}: __ldg({argument})"
     assert seen == {"k_graph_conv_cw", "k_graph_conv_mma", "k_graph_conv_window"}
+
+
+def test_a_layer_runs_on_the_kernel_whose_layout_its_input_has():
+    """A kind of layer gets its features in a layout of its own, so no other kind's kernel, nor the CUDA cores', may take its place."""
+    with open(os.path.join(CSRC, "engine.cu")) as f:
+        text = f.read()
+    begin = text.index("{", text.index("static void launch_conv("))
+    body = _argument(text.replace("{", "(").replace("}", ")"), begin + 1)
+    calls = list(re.finditer(r"launch_conv_(\w+)\(", body))
+    assert {c.group(1) for c in calls} == {"window", "staged", "tc_split", "tc_gather", "ffma"}
+    for call in calls:
+        kind = {"window": "TC_WINDOW", "staged": "TC_STAGED"}.get(call.group(1), call.group(1).upper())
+        line = body[body.rindex("case ", 0, call.start()):call.start()] if "case " in body[:call.start()] else body[:call.start()]
+        assert re.findall(r"CONV_(\w+)", line) == [kind], call.group(0)
+    assert "throw" in body[calls[-1].end():]

@@ -19,6 +19,7 @@
 #include <memory>
 #include <mutex>
 #include <new>
+#include <stdexcept>
 #include <string>
 #include <vector>
 
@@ -360,13 +361,19 @@ static void launch_conv(vm_engine* e, const DenseLayer& L, ConvArgs a, int n_fra
     a.n_slots     = L.n_slots;
     a.activation  = L.activation;
     begin_stage(e, s, L.stage.c_str());
-    if (kind == CONV_TC_WINDOW && launch_conv_window(L, a, plan, n_frames, max_rows, e->flags, e->tc_wait_limit, s)) {}
-    else if (kind == CONV_TC_STAGED && launch_conv_staged(L, a, plan, n_frames, max_rows, e->flags, e->tc_wait_limit, s)) {}
-    else if ((kind == CONV_TC_SPLIT || kind == CONV_TC_STAGED) && launch_conv_tc_split(L, a, n_frames, max_rows, e->flags, e->tc_wait_limit, s)) {}
-    else if (kind == CONV_TC_GATHER && launch_conv_tc_gather(L, a, n_frames, max_rows, e->flags, e->tc_wait_limit, s)) {}
-    else {
-        launch_conv_ffma(L, a, n_frames, max_rows, s);
+    // A layer's kind fixes the layout of its input: there is no other kernel to fall back to.
+    bool launched = false;
+    switch (kind) {
+        case CONV_TC_WINDOW: launched = launch_conv_window(L, a, plan, n_frames, max_rows, e->flags, e->tc_wait_limit, s); break;
+        case CONV_TC_STAGED: launched = launch_conv_staged(L, a, plan, n_frames, max_rows, e->flags, e->tc_wait_limit, s); break;
+        case CONV_TC_SPLIT: launched = launch_conv_tc_split(L, a, n_frames, max_rows, e->flags, e->tc_wait_limit, s); break;
+        case CONV_TC_GATHER: launched = launch_conv_tc_gather(L, a, n_frames, max_rows, e->flags, e->tc_wait_limit, s); break;
+        case CONV_FFMA:
+            launch_conv_ffma(L, a, n_frames, max_rows, s);
+            launched = true;
+            break;
     }
+    if (!launched) throw std::logic_error("no kernel for layer " + L.stage + " in the layout of its input");
     end_stage(e, s);
 }
 
