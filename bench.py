@@ -56,7 +56,7 @@ NCU_TRAFFIC_BYTES_PER_ROW = {
 def _kernel_of_layer(cin, cout):
     """Which kernel the engine's default policy runs a gather layer on (visualmesh_b200/csrc/engine.cu, run_network)."""
     if cin == 16 and cout in (8, 16, 32):
-        return "st::k_graph_conv_mma (shared-memory windows, ldmatrix gather, mma.sync)"
+        return "st::k_graph_conv_mma (shared-memory windows, mma.sync)"
     if cin == 32 and cout >= 16:  # behind a layer of 32 outputs, as in every configuration
         return "win::k_graph_conv_window (shared-memory windows, tcgen05, A operand in tensor memory)"
     return "k_graph_conv_cw (FFMA)"

@@ -155,6 +155,34 @@ def test_fp16_range_overflow_in_an_early_chunk_of_a_batch_is_not_missed():
     engine.close()
 
 
+# (widths, the layer that overflows): staged to staged, to a last layer of 32 channels, to the window kernel; window to window, to staged and
+# to a last layer of 32 channels
+@pytest.mark.parametrize("widths,layer", [([16, 16, 16, 3], 1), ([16, 16, 32], 1), ([16, 32, 32, 3], 1), ([32, 32, 32, 3], 1),
+                                          ([32, 32, 16, 16, 3], 2), ([32, 16, 32], 1)])
+@pytest.mark.parametrize("n_neighbours,n", [(6, 257), (8, 20_001)])
+@pytest.mark.parametrize("last_row_only", [False, True])
+def test_fp16_range_overflow_in_a_tensor_core_layer_is_not_missed(widths, layer, n_neighbours, n, last_row_only):
+    """A tensor-core layer whose input is in the range of the fp16 split and whose output is not, in all rows or in the last one alone, behind
+    whole tiles: the call must come back bit for bit as an engine without tensor-core kernels computes it."""
+    net = W.make_network(77, n_neighbours, widths)
+    for group in net:
+        group[0].biases[:] = 0.0  # rows of zeros stay zeros
+    net[layer][0].weights[:] *= 3.0e6
+    net[layer + 1][0].weights[:] *= 1.0e-6
+    x, nb = _random_rows(n, n_neighbours, 47)
+    if last_row_only:
+        x[:-1] = 0.0
+        nb[:-1] = np.minimum(nb[:-1], n - 2)
+    plain = _engine_with_env(net, VMCUDA_TC=0)
+    want = plain.network(x, nb).copy()
+    plain.close()
+    assert np.all(np.isfinite(want))
+    engine = Engine(net)
+    for _ in range(2):
+        assert np.array_equal(G.bits(engine.network(x, nb)), G.bits(want))
+    engine.close()
+
+
 def test_layer_without_a_tensor_core_kernel_between_two_that_have_one():
     """8 -> 32 has a tensor-core weight layout but no kernel instantiation: it must run on the FFMA kernels and the
     32 -> 32 layer behind it must still be fed the layout its kernel expects (tensor cores forced on wherever a kernel
