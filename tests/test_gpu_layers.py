@@ -122,6 +122,22 @@ def test_layers_with_large_halos(n, reach, n_neighbours, widths):
     assert np.abs(got.astype(np.float64) - O.network(x, nb, net).astype(np.float64)).max() <= P.TOL_CLS / 4
 
 
+# three blocks per SM walk the super-tiles: three or more windows each from 227 329 rows on. Halos of 30 to 520 rows in any order: windows
+# that share the pool with the one before, that wait for it, and super-tiles beyond the plan's slots
+@pytest.mark.parametrize("n", [227_329, 350_001])
+@pytest.mark.parametrize("n_neighbours,widths", [(4, [16, 16, 8, 3]), (6, [16, 32, 16, 16, 3]), (8, [16, 16, 8, 3])])
+def test_layers_of_16_channels_with_halos_of_every_size(n, n_neighbours, widths):
+    net = W.make_network(83, n_neighbours, widths)
+    x, _ = _rows(n, n_neighbours, 19)
+    reach = np.array([15, 90, 120, 170, 190, 260])[(W.splitmix64(8, n // 256 + 1) % np.uint64(6)).astype(np.int64)][np.arange(n) // 256]
+    step = (W.splitmix64(9, n * n_neighbours) % (2 * reach.astype(np.uint64) + 1).repeat(n_neighbours)).astype(np.int64).reshape(n, n_neighbours)
+    nb = np.clip(np.arange(n)[:, None] + step - reach[:, None], 0, n - 1).astype(np.int32)
+    engine = Engine(net)
+    got = engine.network(x, nb)
+    engine.close()
+    assert np.abs(got.astype(np.float64) - O.network(x, nb, net).astype(np.float64)).max() <= P.TOL_CLS / 4
+
+
 # 296 blocks of 128 rows (32 channels: half super-tiles), 592 super-tiles or 296 blocks of 512 rows: up to there layers start early
 @pytest.mark.parametrize("n", [1, 300, 37_888, 37_889, 151_552, 151_553])
 @pytest.mark.parametrize("n_neighbours,widths", [(6, [16, 16, 16, 8, 8, 8, 5]), (8, [32, 32, 32, 16, 8, 4, 3])])

@@ -127,8 +127,10 @@ namespace st {
     constexpr int TILE             = 8;   // rows of one warp-level MMA tile (its N)
     constexpr int CIN              = 16;  // input channels
     constexpr int ROW              = 4 * CIN;  // bytes of a feature row: four pieces of four channels, hi parts then lo parts each
-    constexpr int KEPT             = 192;  // halo slots of a window: the rest of a super-tile's comes from global memory (rings of six neighbours have 188 at most)
-    constexpr int WINDOW           = (ST + KEPT) * ROW;
+    constexpr int POOL             = 896;  // rows of the two windows together: a window takes as many as its super-tile and its halo have
+    // Windows of 192 halo slots each made every super-tile with more outside rows a slow one: none of the rings', three in four of an XYGRID8's
+    // (269 on average with 2.3 M rows, 16 % have more than the plan's 384 slots), half of an XYGRID6's, 43 % of an XYGRID4's.
+    static_assert(ST + HALO <= POOL, "a window fits");
     constexpr int NBL_BYTES        = ST * NBL_STRIDE * 2;
 
     // 16x16 fragments of a slot's weights: hi and lo parts of 16 output channels each, or of eight channels in one
@@ -138,7 +140,7 @@ namespace st {
     }
     template <int COUT, int NSLOTS>
     __host__ __device__ constexpr size_t smem_bytes() {
-        return static_cast<size_t>(2) * (WINDOW + NBL_BYTES)                  // two windows and their neighbour positions
+        return static_cast<size_t>(POOL) * ROW + 2 * NBL_BYTES                // two windows, their neighbour positions
                + static_cast<size_t>(NSLOTS) * weight_fragments<COUT>() * 32 * 16;
     }
 
@@ -162,6 +164,7 @@ namespace st {
         __shared__ int32_t tile_prefix[MAX_FRAMES + 1];   // in super-tiles
         __shared__ int32_t frame_start[MAX_FRAMES + 1];   // offsets[f0 + f]
         __shared__ int32_t window_miss[2];                // some neighbour of the super-tile was left out of its window
+        __shared__ int32_t window_start[2];               // its first row in the pool
         __shared__ int32_t failed_s;
         volatile int32_t* failed = &failed_s;
 
@@ -171,7 +174,7 @@ namespace st {
         const int g    = lane >> 2;  // row of a tile that the thread reads; output channels of the accumulator fragment
         const int tq   = lane & 3;   // its piece of that row; rows 2 tq and 2 tq + 1 of the accumulator fragment
         const uint32_t win_addr = tc::smem_u32(smem_raw);
-        const uint32_t nbl_addr  = win_addr + 2 * WINDOW;
+        const uint32_t nbl_addr  = win_addr + POOL * ROW;
         const uint32_t frag_addr = nbl_addr + 2 * NBL_BYTES + lane * 16;  // this lane's 16 bytes of fragment 0
         const uint32_t bar_full  = tc::smem_u32(&bars[0]);
         const uint32_t bar_empty = tc::smem_u32(&bars[2]);
@@ -196,7 +199,7 @@ namespace st {
         auto channel = [&](int block, int half) { return COUT == 8 ? g : COUT == 16 ? 4 * (g >> 1) + 2 * half + (g & 1) : 4 * g + 2 * block + half; };
         {
             constexpr int COUTP = (COUT + 3) & ~3;
-            uint4* w_frag       = reinterpret_cast<uint4*>(smem_raw + 2 * WINDOW + 2 * NBL_BYTES);  // [slot][block][part][lane]
+            uint4* w_frag       = reinterpret_cast<uint4*>(smem_raw + POOL * ROW + 2 * NBL_BYTES);  // [slot][block][part][lane]
             for (int i = warp; i < NSLOTS * MBLK; i += WARPS + 1) {
                 const int block = i % MBLK, slot = i / MBLK;
                 const float* w  = a.weights + static_cast<size_t>(slot * CIN + 4 * tq) * COUTP;
@@ -248,18 +251,20 @@ namespace st {
             // ================= loader warp: one window ahead of the compute warps per buffer =================
             // The halo list of a super-tile (its length, then this lane's entries) is read one super-tile ahead, while
             // the loader waits for a buffer anyway: the copies of a window then start the moment its buffer is free
-            // instead of two dependent trips to global memory later.
-            constexpr int PER_LANE = (KEPT + 31) / 32;
+            // instead of two dependent trips to global memory later. As much of it as most have: the rest is read when it is copied.
+            constexpr int EARLY    = 192;
+            constexpr int PER_LANE = EARLY / 32;
             int n_halo = 0, listed = 0;
             int32_t halo_row[PER_LANE];
             auto fetch_halo_list = [&](int st) {
                 listed                = __ldg(plan.halo_count + st);
-                n_halo                = min(listed, KEPT);
+                n_halo                = min(listed, HALO);
                 const int32_t* h_rows = plan.halo_rows + static_cast<size_t>(st) * HALO;
 #pragma unroll
-                for (int k = 0; k < PER_LANE; ++k) halo_row[k] = __ldg(h_rows + min(lane + 32 * k, KEPT - 1));  // entries past n_halo are never used
+                for (int k = 0; k < PER_LANE; ++k) halo_row[k] = __ldg(h_rows + lane + 32 * k);  // entries past n_halo are never used
             };
             uint32_t n = 0;
+            int before = 0;  // rows of the window before
             bool ok    = true;
             if (static_cast<int>(blockIdx.x) < total_st) fetch_halo_list(blockIdx.x);
             in_bytes = after_previous(in_bytes);
@@ -269,12 +274,21 @@ namespace st {
                 // the warp decides together: what follows needs all of its lanes, and a window that some had begun would never become full
                 ok = __all_sync(0xffffffffu, n < 2 || tc::mbar_wait_or_fail(bar_empty + 8 * b, ((n >> 1) - 1) & 1u, failed, t.wait_limit));
                 if (!ok) break;
+                // windows lie at the pool's beginning and at its end in turn; two that do not fit beside each other follow one another
+                const int size = ST + n_halo;
+                if (size + before > POOL) {
+                    ok = __all_sync(0xffffffffu, tc::mbar_wait_or_fail(bar_empty + 8 * (b ^ 1u), ((n - 1) >> 1) & 1u, failed, t.wait_limit));
+                    if (!ok) break;
+                }
+                before             = size;
+                const int at       = b == 0 ? 0 : POOL - size;
                 const StRef r      = locate(s);
                 const int own      = min(ST, r.rows - r.t0);
-                const uint32_t dst = win_addr + b * WINDOW;
+                const uint32_t dst = win_addr + at * ROW;
                 const uint32_t bar = bar_full + 8 * b;
                 if (lane == 0) {
-                    window_miss[b] = listed > KEPT;
+                    window_miss[b]  = listed > HALO;
+                    window_start[b] = at;
                     mbar_expect_tx(bar, static_cast<uint32_t>(own * (ROW + 2 * NBL_STRIDE)));
                     bulk_copy(nbl_addr + b * NBL_BYTES, reinterpret_cast<const uint4*>(plan.nbl) + r.local_base + r.t0, static_cast<uint32_t>(own * 2 * NBL_STRIDE),
                               bar);
@@ -284,11 +298,17 @@ namespace st {
                 const unsigned char* from = in_bytes + (lane & 3) * 16;
                 const uint32_t to         = dst + ST * ROW + lane * 16;
 #pragma unroll
-                for (int k = 0; k < KEPT / 8; ++k) {
+                for (int k = 0; k < EARLY / 8; ++k) {
                     if (8 * k >= n_halo) break;
                     const int32_t row = __shfl_sync(0xffffffffu, halo_row[k / 4], 8 * (k % 4) + (lane >> 2));
                     if (8 * k + (lane >> 2) < n_halo) copy16(to + k * 8 * ROW, from + static_cast<size_t>(row) * ROW);
                 }
+                const int32_t* rest = plan.halo_rows + static_cast<size_t>(s) * HALO;
+#pragma unroll 4
+                for (int h = EARLY + (lane >> 2); h < n_halo; h += 8) {
+                    copy16(dst + (ST + h) * ROW + (lane & 3) * 16, from + static_cast<size_t>(__ldg(rest + h)) * ROW);
+                }
+                __syncwarp();
                 if (s + static_cast<int>(gridDim.x) < total_st) fetch_halo_list(s + gridDim.x);
                 copies_arrive(bar);
             }
@@ -323,7 +343,7 @@ namespace st {
                 *failed = 1;
                 break;
             }
-            const uint32_t win = win_addr + b * WINDOW + tq * 16;
+            const uint32_t win = win_addr + *static_cast<volatile int32_t*>(&window_start[b]) * ROW + tq * 16;
             const uint32_t nbl = nbl_addr + b * NBL_BYTES;
             const bool miss    = *static_cast<volatile int32_t*>(&window_miss[b]) != 0;
             for (int group = warp; group < n_groups; group += WARPS) {
@@ -390,7 +410,7 @@ namespace st {
                             const uint32_t row = window_row(i);
                             uint32_t p         = row;
                             if (slot > 0) asm volatile("ld.shared.u16 %0, [%1];" : "=r"(p) : "r"(nbl + row * (2 * NBL_STRIDE) + 2 * (slot - 1)));
-                            if (slot > 0 && p >= static_cast<uint32_t>(ST + KEPT)) {
+                            if (slot > 0 && p == NBL_GLOBAL) {
                                 const int idx = __ldg(a.nb + (r.nb_base + r.t0 + row) * a.n_neighbours + (slot - 1));
                                 x[i]          = *reinterpret_cast<const uint4*>(in_bytes + static_cast<size_t>(r.local_base + idx) * ROW + tq * 16);
                             }
