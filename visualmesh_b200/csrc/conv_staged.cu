@@ -14,8 +14,9 @@ template <int COUT, int NSLOTS>
 static void launch_conv_staged_t(const DenseLayer& L, const ConvArgs& a, const st::Plan& plan, int n_frames, int max_rows, int32_t* abort_flags,
                                  uint32_t wait_limit, cudaStream_t s) {
     constexpr int THREADS = 4 * 32 + 32;  // compute warps + the loader warp
-    constexpr auto kernel = st::k_graph_conv_mma<COUT, NSLOTS, 4, THREADS, COUT == 32 ? 2 : 3>;
-    constexpr size_t smem = st::smem_bytes<COUT, NSLOTS>();
+    constexpr int CTAS    = COUT == 32 ? 2 : 3;  // per SM
+    constexpr auto kernel = st::k_graph_conv_mma<COUT, NSLOTS, 4, THREADS, CTAS>;
+    constexpr size_t smem = st::smem_bytes<COUT, NSLOTS, CTAS>();
     static LaunchPlans plans;
     const LaunchPlan& lp = plans.get([](int dev) {
         LaunchPlan p;

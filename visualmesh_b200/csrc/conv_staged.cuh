@@ -28,15 +28,15 @@
 //   - A quarter-warp reads two whole rows of 64 bytes, so only two rows of the same parity meet in a bank (a third of the
 //     pairs on the meshes here: consecutive rows have neighbours that follow one another). Rows in planes of 16-byte
 //     pieces, eight of them per quarter-warp as ldmatrix takes them, took 2.25 passes where this takes 1.4.
-//   - Twelve warps per SM with 128 registers instead of 24 with 72: loads of the next slot are in flight during the products of
-//     one, and nothing spills. The eight-channel layers also keep their weights in registers (the sixteen-channel ones
-//     have twice as many, which spills).
+//   - Twelve warps per SM with 106 to 128 registers instead of 24 with 72: loads of the next slot are in flight during the products of
+//     one, and nothing spills but a register of 16 -> 8 with eight neighbours. The eight-channel layers also keep their weights in
+//     registers (the sixteen-channel ones have twice as many, which spills).
 // 16 -> 16 over 4.48 M rows with six neighbours 212 -> 169 us (the weights' fragments are 28 of its 115 wavefronts of shared-memory
 // loads per sixteen rows, the rows 56 and 24 of conflicts), 16 -> 8 176 -> 123 us (138 with the weights read for each slot). On the way:
 // planes and ldmatrix with fewer instructions 212; the layout alone 219 and 152; weights as the first operand with 24 warps 200 and 152;
 // with twelve 182 and 138; split rows transposed before they are stored (stores of a quarter-warp in one 128-byte line, not
 // four) 169. Sixteen compute warps in two CTAs 192; groups of 64 rows 177 (spills).
-// A neighbour whose halo slot did not fit (more outside rows than halo slots) is marked and fetched from global memory
+// A neighbour without a halo slot (more outside rows than the plan has slots) is marked and fetched from global memory
 // by its warp, so any neighbourhood is computed correctly, only slower.
 //
 // The only waits are for a window's copies (compute warps) and for a window to be handed back (loader), and they are
@@ -127,10 +127,6 @@ namespace st {
     constexpr int TILE             = 8;   // rows of one warp-level MMA tile (its N)
     constexpr int CIN              = 16;  // input channels
     constexpr int ROW              = 4 * CIN;  // bytes of a feature row: four pieces of four channels, hi parts then lo parts each
-    constexpr int POOL             = 896;  // rows of the two windows together: a window takes as many as its super-tile and its halo have
-    // Windows of 192 halo slots each made every super-tile with more outside rows a slow one: none of the rings', three in four of an XYGRID8's
-    // (269 on average with 2.3 M rows, 16 % have more than the plan's 384 slots), half of an XYGRID6's, 43 % of an XYGRID4's.
-    static_assert(ST + HALO <= POOL, "a window fits");
     constexpr int NBL_BYTES        = ST * NBL_STRIDE * 2;
 
     // 16x16 fragments of a slot's weights: hi and lo parts of 16 output channels each, or of eight channels in one
@@ -139,9 +135,27 @@ namespace st {
         return COUT == 8 ? 1 : COUT / 8;
     }
     template <int COUT, int NSLOTS>
+    __host__ __device__ constexpr int weight_bytes() {
+        return NSLOTS * weight_fragments<COUT>() * 32 * 16;
+    }
+    // Rows of the two windows together: as many as let CTAS blocks share an SM, which has 228 KB and keeps 1 KB of them for every block. A
+    // window takes as many as its super-tile and its halo have. Windows of 192 halo slots each made every super-tile with more outside rows a slow
+    // one: none of the rings', three in four of an XYGRID8's (269 on average with 2.3 M rows, 16 % have more than the plan's 384 slots), half of an
+    // XYGRID6's, 43 % of an XYGRID4's. And 896 rows with sixteen channels and eight neighbours left room for two blocks, not three: 16 -> 16
+    // over 4.5 M rows of RING8 217 -> 202 us, over 2.3 M of XYGRID8 322 -> 240 (348 with windows of 192 slots).
+    constexpr int SMEM_ALIGN  = 128;
+    constexpr int SMEM_STATIC = (4 * 8 + 2 * 4 * (MAX_FRAMES + 1) + 5 * 4 + SMEM_ALIGN - 1) / SMEM_ALIGN * SMEM_ALIGN;  // the kernel's other variables
+    template <int COUT, int NSLOTS, int CTAS>
+    __host__ __device__ constexpr int pool_rows() {
+        constexpr int room = 228 * 1024 / CTAS - 1024 - SMEM_STATIC - 2 * NBL_BYTES - weight_bytes<COUT, NSLOTS>();
+        constexpr int rows = room / (2 * ROW) * 2;
+        static_assert(rows >= ST + HALO, "a window fits");
+        return rows < 2 * (ST + HALO) ? rows : 2 * (ST + HALO);
+    }
+    // windows, their neighbour positions, weights
+    template <int COUT, int NSLOTS, int CTAS>
     __host__ __device__ constexpr size_t smem_bytes() {
-        return static_cast<size_t>(POOL) * ROW + 2 * NBL_BYTES                // two windows, their neighbour positions
-               + static_cast<size_t>(NSLOTS) * weight_fragments<COUT>() * 32 * 16;
+        return static_cast<size_t>(pool_rows<COUT, NSLOTS, CTAS>()) * ROW + 2 * NBL_BYTES + weight_bytes<COUT, NSLOTS>();
     }
 
     // One CTA walks super-tiles; while it computes on one window the next is on its way. Every warp owns groups of TILES 8-row
@@ -158,8 +172,9 @@ namespace st {
         constexpr int MBLK  = COUT == 32 ? 2 : 1;  // blocks of 16 rows of the weights' operand
         constexpr int FRAGS = weight_fragments<COUT>();
         constexpr int WARPS = THREADS / 32 - 1;    // compute warps; the last warp of the CTA is the loader
+        constexpr int POOL  = pool_rows<COUT, NSLOTS, CTAS>();
 
-        extern __shared__ __align__(1024) unsigned char smem_raw[];
+        extern __shared__ __align__(SMEM_ALIGN) unsigned char smem_raw[];
         __shared__ uint64_t bars[4];                      // full[2]: a window has landed; empty[2]: every compute warp is done with it
         __shared__ int32_t tile_prefix[MAX_FRAMES + 1];   // in super-tiles
         __shared__ int32_t frame_start[MAX_FRAMES + 1];   // offsets[f0 + f]
@@ -303,10 +318,10 @@ namespace st {
                     const int32_t row = __shfl_sync(0xffffffffu, halo_row[k / 4], 8 * (k % 4) + (lane >> 2));
                     if (8 * k + (lane >> 2) < n_halo) copy16(to + k * 8 * ROW, from + static_cast<size_t>(row) * ROW);
                 }
-                const int32_t* rest = plan.halo_rows + static_cast<size_t>(s) * HALO;
+                const int32_t* h_rows = plan.halo_rows + static_cast<size_t>(s) * HALO;
 #pragma unroll 4
                 for (int h = EARLY + (lane >> 2); h < n_halo; h += 8) {
-                    copy16(dst + (ST + h) * ROW + (lane & 3) * 16, from + static_cast<size_t>(__ldg(rest + h)) * ROW);
+                    copy16(dst + (ST + h) * ROW + (lane & 3) * 16, from + static_cast<size_t>(__ldg(h_rows + h)) * ROW);
                 }
                 __syncwarp();
                 if (s + static_cast<int>(gridDim.x) < total_st) fetch_halo_list(s + gridDim.x);
