@@ -58,11 +58,13 @@ struct LaunchPlans {
     }
 };
 
-// Whether a layer's launch starts early: only while its blocks (as many as there may be rows for) find room beside those of the
-// layer in front. A pass with a network's layers started early, us, one frame of 2.7 | 11 | 25 | 57 | 121 | 242 k nodes: thirteen layers of 16 and 8
-// channels 86.9 | 90.3 | 92.8 | 101 | 128 | 154 -> 76.0 | 80.6 | 82.9 | 93.6 | 118 | 169; four layers 50.5 | 51.5 | 53.2 | 54.4 | 64.0 | 76.6 -> 45.7 | 48.5 |
-// 48.4 | 53.2 | 63.6 | 85.9; ten of 32 channels, a CTA per SM, 105 | 107 | 112 | 126 | 157 | 239 -> 84.7 | 85.9 | 104 | 134 | 193 | 255. So two blocks
-// per SM, and four of the staged layers' small CTAs. Layers that few rows send to the kernel with part of the outputs per block lose (50
+// Whether a layer's launch starts early: while its blocks (as many as there may be rows for) are few. The lines were found by trial on three
+// networks; they do not follow from what a kernel's blocks take of an SM (a window layer's CTA takes all of it, and three or two of the
+// staged ones: those of the next layer then start as the ones in front end). A pass with the layers started early, us, one frame of 2.7 | 11 | 25 |
+// 57 | 121 | 242 k nodes: thirteen layers of 16 and 8 channels 86.9 | 90.3 | 92.8 | 101 | 128 | 154 -> 76.0 | 80.6 | 82.9 | 93.6 | 118 | 169; four layers
+// 50.5 | 51.5 | 53.2 | 54.4 | 64.0 | 76.6 -> 45.7 | 48.5 | 48.4 | 53.2 | 63.6 | 85.9; ten of 32 channels 105 | 107 | 112 | 126 | 157 | 239 -> 84.7 | 85.9 | 104 |
+// 134 | 193 | 255. So two blocks (of a window layer, two halves of a super-tile: 37.9 k rows) per SM, and four super-tiles of the staged layers
+// (151.6 k rows): what measured slower lies beyond. Layers that few rows send to the kernel with part of the outputs per block lose (50
 // -> 57 us at 11 k nodes, five times the blocks) and start the ordinary way, and so do the kernels of the projection (no gain),
 // and a last layer that writes to the host (a call of two layers 36.9 -> 37.7 us).
 inline bool starts_early(int64_t blocks, int blocks_per_sm, int n_sms) {

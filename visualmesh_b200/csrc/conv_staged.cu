@@ -30,10 +30,9 @@ static void launch_conv_staged_t(const DenseLayer& L, const ConvArgs& a, const s
         return p;
     });
     st::Args t{};
-    t.n_frames   = n_frames;
-    t.cout       = L.cout;
+    t.n_frames    = n_frames;
     t.abort_flags = abort_flags;
-    t.wait_limit = wait_limit;
+    t.wait_limit  = wait_limit;
     const int tiles_upper = n_frames * ((max_rows + st::ST - 1) / st::ST);
     const int grid        = std::max(1, std::min(tiles_upper, lp.n_sms * lp.ctas_per_sm));
     launch_kernel(kernel, dim3(grid), THREADS, smem, s, a.early && starts_early(tiles_upper, 4, lp.n_sms), a, t, plan);
@@ -41,8 +40,7 @@ static void launch_conv_staged_t(const DenseLayer& L, const ConvArgs& a, const s
 
 bool has_staged_kernel(const DenseLayer& L) {
     // tc_half: the layer's weights are within the range of the fp16 split
-    // 16-channel inputs: on 32-channel layers the tcgen05 kernel of conv_tc.cuh measured faster (94 against 102 ms for the
-    // eight 32 -> 32 layers of 64 frames with 0.93 M rows each), the warp-level MMA rate being what bounds this one there
+    // 16-channel inputs: layers with 32 have kernels on tcgen05 (conv_window.cuh, conv_tc.cuh)
     return L.tc_np != 0 && L.tc_half && L.cin == 16 && (L.cout == 8 || L.cout == 16 || L.cout == 32)
            && (L.n_slots == 5 || L.n_slots == 7 || L.n_slots == 9) && L.activation != VM_SOFTMAX;
 }
@@ -75,9 +73,3 @@ void launch_tile_plan_kernel(int n_neighbours, const int32_t* offsets, const int
 }
 
 }  // namespace vm
-
-#ifdef VM_PROFILE_STAGED
-extern "C" __attribute__((visibility("default"))) int vm_debug_staged_profile(long long* out, int n) {
-    return (int)cudaMemcpyFromSymbol(out, vm::st::g_prof, sizeof(long long) * n);
-}
-#endif

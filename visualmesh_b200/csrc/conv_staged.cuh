@@ -80,29 +80,13 @@ namespace st {
         plan_super_tile<N>(idx, valid, t0, f, a.offsets, a.f0, a.out);
     }
 
-    // ---- asynchronous copies ------------------------------------------------------------------------------------------
-    __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-    }
-    // contiguous global -> shared, completion counted in bytes on the mbarrier; no multicast
-    __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
-                     "r"(bytes), "r"(bar)
-                     : "memory");
-    }
-    __device__ __forceinline__ void copy16(uint32_t dst, const void* src) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-    }
-    // one arrival on the mbarrier once all earlier 16-byte copies of this thread have landed (counted at init)
-    __device__ __forceinline__ void copies_arrive(uint32_t bar) {
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-    }
+    using tc::bulk_copy;
+    using tc::copies_arrive;
+    using tc::copy16;
+    using tc::expect_bytes;
+    using tc::load_shared;
+
     // ---- warp-level tensor-core pieces ----------------------------------------------------------------------------------
-    __device__ __forceinline__ uint4 load_shared(uint32_t addr) {
-        uint4 v;
-        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-        return v;
-    }
     // D += A . B, A 16x16 fp16 (row), B 16x8 fp16 (col), D 16x8 fp32
     __device__ __forceinline__ void mma_16816(float (&d)[4], const uint4& a, uint32_t b0, uint32_t b1) {
         asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -117,7 +101,6 @@ namespace st {
     }
     struct Args {
         int32_t n_frames;
-        int32_t cout;
         int32_t* abort_flags;
         uint32_t wait_limit;  // polls of one wait for a window before the kernel gives up (0: the first wait fails at once)
     };
@@ -142,7 +125,7 @@ namespace st {
     // window takes as many as its super-tile and its halo have. Windows of 192 halo slots each made every super-tile with more outside rows a slow
     // one: none of the rings', three in four of an XYGRID8's (269 on average with 2.3 M rows, 16 % have more than the plan's 384 slots), half of an
     // XYGRID6's, 43 % of an XYGRID4's. And 896 rows with sixteen channels and eight neighbours left room for two blocks, not three: 16 -> 16
-    // over 4.5 M rows of RING8 217 -> 202 us, over 2.3 M of XYGRID8 322 -> 240 (348 with windows of 192 slots).
+    // over 4.5 M rows of RING8 217 -> 203 us, over 2.3 M of XYGRID8 314 -> 236 (343 with windows of 192 slots).
     constexpr int SMEM_ALIGN  = 128;
     constexpr int SMEM_STATIC = (4 * 8 + 2 * 4 * (MAX_FRAMES + 1) + 5 * 4 + SMEM_ALIGN - 1) / SMEM_ALIGN * SMEM_ALIGN;  // the kernel's other variables
     template <int COUT, int NSLOTS, int CTAS>
@@ -304,7 +287,7 @@ namespace st {
                 if (lane == 0) {
                     window_miss[b]  = listed > HALO;
                     window_start[b] = at;
-                    mbar_expect_tx(bar, static_cast<uint32_t>(own * (ROW + 2 * NBL_STRIDE)));
+                    expect_bytes(bar, static_cast<uint32_t>(own * (ROW + 2 * NBL_STRIDE)));
                     bulk_copy(nbl_addr + b * NBL_BYTES, reinterpret_cast<const uint4*>(plan.nbl) + r.local_base + r.t0, static_cast<uint32_t>(own * 2 * NBL_STRIDE),
                               bar);
                     bulk_copy(dst, in_bytes + static_cast<size_t>(r.local_base + r.t0) * ROW, static_cast<uint32_t>(own * ROW), bar);

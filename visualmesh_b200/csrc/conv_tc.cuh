@@ -57,6 +57,28 @@ namespace tc {
         return false;
     }
 
+    // Asynchronous copies into shared memory, counted on an mbarrier.
+    __device__ __forceinline__ void expect_bytes(uint32_t bar, uint32_t bytes) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    }
+    // contiguous global -> shared, completion counted in bytes; no multicast
+    __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+                     : "memory");
+    }
+    __device__ __forceinline__ void copy16(uint32_t dst, const void* src) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    }
+    // one arrival once all earlier 16-byte copies of this thread have landed (counted at init)
+    __device__ __forceinline__ void copies_arrive(uint32_t bar) {
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+    }
+    __device__ __forceinline__ uint4 load_shared(uint32_t addr) {
+        uint4 v;
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+        return v;
+    }
+
     // prefix[f] = tiles of the frames before frame f of the launch, prefix[n_frames] = all of them; by the first warp of the block,
     // 32 frames at a time. The caller synchronises.
     template <int ROWS>

@@ -25,7 +25,8 @@
 // 1290 cycles. Measured on the way, 32 -> 32, one frame of 0.92 M rows | eight frames: 110 | 762 us at first (units of three slots in a
 // ring, A as two loads interleaved, one issuer); registers in order but more and smaller units 127 | 870 - the issuer and the chain of
 // barriers were what took the time, with row loads, stores to tensor memory or the epilogue left out one by one it stayed the same;
-// a tile's A as one unit 107 | 742; in two parts with an issuer per group 102 | 706; windows from a pool 85 | 610: before, a
+// a tile's A as one unit 107 | 742; in two parts with an issuer per group 102 | 706; windows from a pool 85 | 631 (the
+// mean of eight layers, as the others; the last, which writes fp32, 610): before, a
 // super-tile with more than 192 halo rows (3 % of them) was gathered by a slow path, and the CTAs that had two or three of those
 // finished 25 % later than the others; and one loader warp was busy all along. Four and six steps of loads in flight instead of two: 2 %.
 // Sixteen gather or epilogue warps (96 registers): 5 to 17 % slower. Registers shared out with setmaxnreg: 9 % slower.
@@ -90,26 +91,11 @@ namespace win {
         return static_cast<size_t>(POOL) * ROW + static_cast<size_t>(BUFFERS) * NBL_BYTES + static_cast<size_t>(n_slots) * 4 * 2 * NP * 16;
     }
 
-    __device__ __forceinline__ void expect_bytes(uint32_t bar, uint32_t bytes) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-    }
-    // contiguous global -> shared, completion counted in bytes on the mbarrier; no multicast
-    __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-                     : "memory");
-    }
-    __device__ __forceinline__ void copy16(uint32_t dst, const void* src) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-    }
-    // one arrival on the mbarrier once all earlier 16-byte copies of this thread have landed (counted at init)
-    __device__ __forceinline__ void copies_arrive(uint32_t bar) {
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-    }
-    __device__ __forceinline__ uint4 load_shared(uint32_t addr) {
-        uint4 v;
-        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-        return v;
-    }
+    using tc::bulk_copy;
+    using tc::copies_arrive;
+    using tc::copy16;
+    using tc::expect_bytes;
+    using tc::load_shared;
     __device__ __forceinline__ uint32_t load_position(uint32_t addr) {
         uint32_t v;
         asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(addr));
