@@ -48,8 +48,8 @@ USER_SET_BLOCKING_SYNC = "VMCUDA_BLOCKING_SYNC" in os.environ
 # DRAM traffic per row of the dominant kernels from their ncu captures (dram__bytes_read + dram__bytes_write over the
 # rows of the captured launch); traffic grows in proportion to the rows, so it is scaled to the bench's launches.
 NCU_TRAFFIC_BYTES_PER_ROW = {
-    (16, 16): 110.6,  # profiles/graph_conv_staged_16x16_cfg1_16frames.md: 122.6 MB over 1,108,261 rows
-    (32, 32): 229.5,  # profiles/graph_conv_window_32x32_cfg3_1frame.md: 213.8 MB over 931,718 rows
+    (16, 16): 110.4,  # profiles/graph_conv_staged_quads_16x16_16frames.md: 121.8 MB over 1,103,036 rows
+    (32, 32): 225.2,  # profiles/graph_conv_window_rows_32x32_1frame.md: 206.9 MB over 918,909 rows
 }
 
 
