@@ -293,18 +293,18 @@ namespace st {
                     bulk_copy(dst, in_bytes + static_cast<size_t>(r.local_base + r.t0) * ROW, static_cast<uint32_t>(own * ROW), bar);
                 }
                 // four lanes to a halo row: whole rows per request
-                const unsigned char* from = in_bytes + (lane & 3) * 16;
+                const unsigned char* feat = in_bytes + (lane & 3) * 16;
                 const uint32_t to         = dst + ST * ROW + lane * 16;
 #pragma unroll
                 for (int k = 0; k < EARLY / 8; ++k) {
                     if (8 * k >= n_halo) break;
                     const int32_t row = __shfl_sync(0xffffffffu, halo_row[k / 4], 8 * (k % 4) + (lane >> 2));
-                    if (8 * k + (lane >> 2) < n_halo) copy16(to + k * 8 * ROW, from + static_cast<size_t>(row) * ROW);
+                    if (8 * k + (lane >> 2) < n_halo) copy16(to + k * 8 * ROW, feat + static_cast<size_t>(row) * ROW);
                 }
                 const int32_t* h_rows = plan.halo_rows + static_cast<size_t>(s) * HALO;
 #pragma unroll 4
                 for (int h = EARLY + (lane >> 2); h < n_halo; h += 8) {
-                    copy16(dst + (ST + h) * ROW + (lane & 3) * 16, from + static_cast<size_t>(__ldg(h_rows + h)) * ROW);
+                    copy16(dst + (ST + h) * ROW + (lane & 3) * 16, feat + static_cast<size_t>(__ldg(h_rows + h)) * ROW);
                 }
                 __syncwarp();
                 if (s + static_cast<int>(gridDim.x) < total_st) fetch_halo_list(s + gridDim.x);

@@ -339,7 +339,7 @@ namespace win {
                 __syncwarp();
                 // LPR lanes to a row: whole rows per request; pieces of a row that goes to a place of other parity trade halves
                 const int first           = loader * (32 / LPR) + lane / LPR;
-                const unsigned char* from = in_bytes + (lane % LPR) * 16;
+                const unsigned char* feat = in_bytes + (lane % LPR) * 16;
                 const uint32_t to         = dst + ST * ROW + (lane % LPR) * 16;
                 const uint32_t place      = static_cast<uint32_t>(first + r.local_base + r.t0);  // parity of this lane's places: they are an even number apart
                 for (int h = first; h < n_halo; h += BATCH * STEP) {
@@ -348,7 +348,7 @@ namespace win {
                     for (int k = 0; k < BATCH; ++k) row[k] = halo[min(h + k * STEP, HALO - 1)];
 #pragma unroll
                     for (int k = 0; k < BATCH; ++k) {
-                        if (h + k * STEP < n_halo) copy16((to + (h + k * STEP) * ROW) ^ ((place ^ row[k]) & 1u) << 6, from + static_cast<size_t>(row[k]) * ROW);
+                        if (h + k * STEP < n_halo) copy16((to + (h + k * STEP) * ROW) ^ ((place ^ row[k]) & 1u) << 6, feat + static_cast<size_t>(row[k]) * ROW);
                     }
                 }
                 __syncwarp();
